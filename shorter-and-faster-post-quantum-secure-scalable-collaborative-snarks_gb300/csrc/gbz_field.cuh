@@ -100,7 +100,8 @@ struct dot_cols {
   uint32_t x0, x1, x2, x3;  // S, least significant word first
 };
 // Requires a, c < 2^62 and b, d <= 2^61: S < 2^124.
-__device__ __forceinline__ dot_cols dot2_cols(uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
+// add: a constant added to S.
+__device__ __forceinline__ dot_cols dot2_cols(uint64_t a, uint64_t b, uint64_t c, uint64_t d, uint32_t add = 0) {
   dot_cols s;
   asm("{\n\t"
       ".reg .u32 al, ah, bl, bh, cl, ch, dl, dh, ml, mh;\n\t"
@@ -114,8 +115,8 @@ __device__ __forceinline__ dot_cols dot2_cols(uint64_t a, uint64_t b, uint64_t c
       "mad.wide.u32 m, cl, dh, m;\n\t"
       "mad.wide.u32 m, ch, dl, m;\n\t"
       "mov.b64 {ml, mh}, m;\n\t"
-      "mul.lo.u32 %0, al, bl;\n\t"
-      "mul.hi.u32 %1, al, bl;\n\t"
+      "mad.lo.cc.u32 %0, al, bl, %8;\n\t"
+      "madc.hi.u32 %1, al, bl, 0;\n\t"
       "mad.lo.cc.u32 %0, cl, dl, %0;\n\t"
       "madc.hi.cc.u32 %1, cl, dl, %1;\n\t"
       "madc.lo.cc.u32 %2, ah, bh, 0;\n\t"
@@ -127,7 +128,7 @@ __device__ __forceinline__ dot_cols dot2_cols(uint64_t a, uint64_t b, uint64_t c
       "addc.u32 %3, %3, 0;\n\t"
       "}"
       : "=&r"(s.x0), "=&r"(s.x1), "=&r"(s.x2), "=&r"(s.x3)
-      : "l"(a), "l"(b), "l"(c), "l"(d));
+      : "l"(a), "l"(b), "l"(c), "l"(d), "r"(add));
   return s;
 }
 // A single product a b, a < 2^62, b < 2^62.

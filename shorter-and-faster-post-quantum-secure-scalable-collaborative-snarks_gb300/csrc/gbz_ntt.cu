@@ -8,21 +8,21 @@
 // of the factorisation, so the GPU uses its own:
 //
 //  * lengths up to 2^13: one shared-memory pass;
-//  * longer lengths L = N1 * N2 (N1, N2 <= 2^13): the four-step algorithm.
-//      pass A: for each column n1 < N1, a length-N2 DFT over x[n1 + N1*n2]
-//              (zero beyond n_valid: the Reed-Solomon padding is never
-//              read), times omega_L^{n1*k2}, stored at n1 + N1*k2;
-//      pass B: for each row k2 < N2, a length-N1 DFT over the row,
-//              stored at k2 + N2*k1 (natural order, no bit reversal pass).
+//  * longer lengths: two or three passes (schedule()).  With L = S C, a pass
+//    over columns computes, for each column l < C, the length-S DFT of
+//    x[l + C j] (zero beyond n_valid: the Reed-Solomon padding is never
+//    read), times omega_L^{l k}, stored at l + C k; what remains are S rows
+//    of length C, transformed by the next passes.  The last pass stores in
+//    natural order (no bit reversal pass).
 //
 // Inside a pass every CTA holds B sub-transforms of length S in shared
 // memory and runs self-sorting (Stockham) stages on them, radix 8 after one
 // radix-2 or radix-4 stage when log2 S is not a multiple of 3.  The first
-// stage runs on the values as they are loaded from global memory; the
-// others read and write shared memory with __syncthreads between them.  The
-// outer twiddle and the inverse scale are applied on the way out.  Groups of
-// B >= 2 neighbouring columns make the strided pass read whole 32-byte
-// sectors.
+// stage runs on the values as they are loaded from global memory and the
+// last one stores from registers; between stages the values cross shared
+// memory, with a barrier among the threads of one sub-transform only.
+// Groups of B >= 2 neighbouring columns make the strided pass read whole
+// 32-byte sectors.
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -39,22 +39,27 @@ constexpr int kTwLoBits = 12;        // outer twiddle table split
 constexpr int kMaxThreads = 1024;
 constexpr int kCtaElems = 1 << kSubLog;  // most elements staged per CTA
 constexpr int kPerThread = 8;            // elements per thread (CTA = max(32, E/8) threads)
-constexpr int kLoadGroup = 4;            // global loads a thread issues back to back
 
-// Four-step shape per length: the pass split (k1 = log2 of the contiguous
-// pass B length) and the sub-transforms staged per CTA in each pass.  Set
-// by ntt_set_shape (the autotuner) or derived by ntt_default_shape.
+// Two-pass shape of a length set by ntt_set_shape (the autotuner): k1 = log2
+// of the contiguous second pass and the sub-transforms staged per CTA in each
+// pass.  Lengths without one take the passes of schedule().
 NttShape g_shape[kMaxLogN + 1];
 
 struct PassArgs {
   const fe *in;
   fe *out;
   uint64_t n_valid;
-  uint64_t in_gstride, in_jstride, out_gstride, out_kstride;
-  const fe *wh;      // omega_{2^13}^t, t < 2^12 (first half), direction-specific
+  // Sub-transform g = h 2^logG + l reads its entry j at l in_gstride + h
+  // in_hstride + j in_jstride and writes its output k at l out_gstride + h
+  // out_hstride + k out_kstride; l is the column of the outer twiddle.
+  uint64_t in_gstride, in_hstride, in_jstride, out_gstride, out_hstride, out_kstride;
+  int logG;
+  const fe *stages;  // stage twiddles of the direction
+  // The outer twiddle of output k is omega_L^{l k 2^tw_shift}.
   const fe *tw_lo;   // omega_L^t, t < 2^12 (nullptr: no outer twiddle)
   const fe *tw_hi;   // omega_L^{2^12 t}
-  const fe *tw_full; // pass A: omega_L^{n1 k2} at the output address n1 + N1 k2 (optional)
+  const fe *tw_full; // the twiddle at l out_gstride + k out_kstride (optional)
+  int tw_shift;
   fe scale;
   int logS, logB, has_scale, inverse;
   // Sparse rows (second pass of a sparse transform, the first pass folded
@@ -72,6 +77,8 @@ struct PassArgs {
   // Accumulating output: out[addr] += v for addr < acc_n, other outputs dropped.
   uint64_t acc_n;
   int acc;
+  // Every entry is present: n_valid and j_valid need no test (set at launch).
+  int dense;
   // Entries j >= j_valid of every sub-transform are zero (per-transform
   // padding of batched transforms; S when unused).
   uint32_t j_valid;
@@ -87,341 +94,266 @@ struct PassArgs {
   const uint32_t *run_if;
 };
 
-// Shared-memory swizzle: element a lives at a ^ ((a >> 3) & 7), which keeps
-// both contiguous runs and stride-8 runs of 16-byte elements free of bank
-// conflicts.
-__device__ __forceinline__ uint32_t swz(uint32_t a) { return a ^ ((a >> 3) & 7u); }
-
-// ---- lazy arithmetic inside one radix-8 butterfly -----------------------
-// Values are kept below k*p (k <= 8 < 2^64 / p) and reduced once at the end.
-// p - x for 0 <= x <= p is a bitwise complement within 61 bits.
-__device__ __forceinline__ uint64_t lz_add(uint64_t a, uint64_t b) { return a + b; }
-// a - b + m*p for b < m*p (m a power of two times p keeps it cheap: kp - b).
-__device__ __forceinline__ uint64_t lz_sub(uint64_t a, uint64_t b, uint64_t mp) { return a + (mp - b); }
+// ---- lazy arithmetic inside one butterfly --------------------------------
+// Words are residues held mod 2^64: additions and subtractions are plain
+// 64-bit instructions, and the window of every word is argued once, here, so
+// that a result is read as the integer it stands for when it is folded.
 // Fold any 64-bit value to [0, p + 7] (p itself stands for zero).
 __device__ __forceinline__ uint64_t fold(uint64_t x) { return (x & P) + (x >> 61); }
 __device__ __forceinline__ uint64_t canon(uint64_t x) {  // [0, p + 7] -> [0, p)
   return x >= P ? x - P : x;
 }
-// A staged value (folded to [0, p + 7] by the last radix-8 stage, or
-// canonical) made canonical for the output.
+// A staged value (folded to [0, p + 7] by the last stage, or canonical) made
+// canonical for the output.
 __device__ __forceinline__ fe canon_fe(fe x) { return fe_make(canon(x.re), canon(x.im)); }
-
-struct lz {
-  uint64_t re, im;
-};
-__device__ __forceinline__ lz lz_of(fe x) { return lz{x.re, x.im}; }
-__device__ __forceinline__ lz lzadd(lz a, lz b) { return lz{lz_add(a.re, b.re), lz_add(a.im, b.im)}; }
-__device__ __forceinline__ lz lzsub(lz a, lz b, uint64_t mp) { return lz{lz_sub(a.re, b.re, mp), lz_sub(a.im, b.im, mp)}; }
-
-// Multiplications by the small roots on lazy values below 2p.
-// getRootOfUnity(2) = -i and getRootOfUnity(3) = 2^30 (1 - i).
-template <bool INV>
-__device__ __forceinline__ lz lz_w4(lz x) {  // forward * (-i), inverse * i; input < 2p, output < 2p
-  const uint64_t p2 = 2 * P;
-  return INV ? lz{p2 - x.im, x.re} : lz{x.im, p2 - x.re};
+__device__ __forceinline__ fe lz_add(fe a, fe b) { return fe_make(a.re + b.re, a.im + b.im); }
+__device__ __forceinline__ fe lz_sub(fe a, fe b) { return fe_make(a.re - b.re, a.im - b.im); }
+__device__ __forceinline__ fe lz_fold(fe a) { return fe_make(fold(a.re), fold(a.im)); }
+// a + w4 b (PLUS) or a - w4 b: getRootOfUnity(2) = -i, inverse i.
+template <bool INV, bool PLUS>
+__device__ __forceinline__ fe lz_w4_add(fe a, fe b) {
+  return INV == PLUS ? fe_make(a.re - b.im, a.im + b.re) : fe_make(a.re + b.im, a.im - b.re);
 }
-// s * 2^30 (mod p) for s < 2^63: s = h 2^31 + l gives h 2^61 + l 2^30 = h + l 2^30;
-// the result is below p + 2^32.
-__device__ __forceinline__ uint64_t mul2e30(uint64_t s) { return ((s << 30) & P) + (s >> 31); }
-// On inputs <= 2p per component the sums below stay within 4p; outputs < p + 2^32.
-template <bool INV>
-__device__ __forceinline__ lz lz_w8(lz x) {  // forward * 2^30 (1 - i), inverse * 2^30 (1 + i)
-  const uint64_t s = mul2e30(x.re + x.im);
-  const uint64_t d = INV ? mul2e30(x.re + (2 * P - x.im)) : mul2e30(x.im + (2 * P - x.re));
-  return INV ? lz{d, s} : lz{s, d};
-}
-template <bool INV>
-__device__ __forceinline__ lz lz_w8_3(lz x) {  // forward * 2^30 (-1 - i), inverse * 2^30 (-1 + i)
-  const uint64_t ns = mul2e30(4 * P - (x.re + x.im));
-  const uint64_t d = INV ? mul2e30(x.re + (2 * P - x.im)) : mul2e30(x.im + (2 * P - x.re));
-  return INV ? lz{ns, d} : lz{d, ns};
-}
+// z 2^30 (mod p) for a signed z, |z| < 2^63: z = h 2^31 + l gives
+// h 2^61 + l 2^30 = h + l 2^30, in [-2^32, p + 2^32].
+__device__ __forceinline__ uint64_t mul2e30(uint64_t z) { return ((z << 30) & P) + (uint64_t)((int64_t)z >> 31); }
 
-// In-register DFTs with natural-order output: V[k] = sum_q v[q] w_R^{qk}.
-// dft2 and dft4 take and return canonical values (they only run as the first
-// stage); dft8 keeps its additions lazy (bounds at its definition).
+// x w + (1 + i) for a staged x (words <= p + 7) and a table twiddle w, each
+// word in [1, p + 1].  The constant keeps the fold away from zero, which
+// makes the window p wide instead of p + 1: with S + 1 <= (p + 7)(2p - 64) + 1
+// (tw_margin) the wrapped sum stays below 3 2^61 - 50, so its quotient 2
+// leaves at most p - 50 and quotients 0, 1 at most p and p + 1.
+__device__ __forceinline__ fe tw_mul(fe x, fe w) {
+  const uint64_t nb = w.im ^ P;
+  return fe_make(dot_fold(dot2_cols(x.re, w.re, x.im, nb, 1)), dot_fold(dot2_cols(x.re, w.im, x.im, w.re, 1)));
+}
+// In-register DFTs with natural-order output: V[k] = sum_q v[q] w_R^{qk},
+// words folded to [0, p + 7].
+// dft2 and dft4 only run as a first stage, on words in [0, p + 7]: a sum of
+// four of them and a difference biased by 2p or 4p stay within 64 bits.
 template <bool INV>
 __device__ __forceinline__ void dft2(fe *v) {
-  fe a = v[0], b = v[1];
-  v[0] = fadd(a, b);
-  v[1] = fsub(a, b);
+  const fe a = v[0], b = v[1], c = fe_make(a.re + 2 * P, a.im + 2 * P);
+  v[0] = lz_fold(lz_add(a, b));
+  v[1] = lz_fold(lz_sub(c, b));
 }
 template <bool INV>
 __device__ __forceinline__ void dft4(fe *v) {
-  fe c0 = fadd(v[0], v[2]), c1 = fadd(v[1], v[3]);
-  fe d0 = fsub(v[0], v[2]), d1 = fsub(v[1], v[3]);
-  d1 = INV ? fe_make(subp(0, d1.im), d1.re) : fe_make(d1.im, subp(0, d1.re));
-  v[0] = fadd(c0, c1);
-  v[2] = fsub(c0, c1);
-  v[1] = fadd(d0, d1);
-  v[3] = fsub(d0, d1);
+  const fe z = fe_make(v[0].re + 4 * P, v[0].im + 4 * P);
+  const fe c0 = lz_add(v[0], v[2]), c1 = lz_add(v[1], v[3]);
+  const fe c0b = lz_add(z, v[2]), d0 = lz_sub(z, v[2]), d1 = lz_sub(v[1], v[3]);
+  v[0] = lz_fold(lz_add(c0, c1));
+  v[2] = lz_fold(lz_sub(c0b, c1));
+  v[1] = lz_fold(lz_w4_add<INV, true>(d0, d1));
+  v[3] = lz_fold(lz_w4_add<INV, false>(d0, d1));
 }
-// Inputs: v[0] <= p + 7 (a folded output of the previous stage), v[1..7]
-// <= p (canonical, or p standing for zero).  Every intermediate below stays
-// within 8p + 7 = 2^64 - 1, and the outputs are folded once to [0, p + 7]:
-// the next stage multiplies v[1..7] by twiddles (canonical products) and
-// takes v[0] as it is; the pass epilogue makes the last stage's values
-// canonical.
-template <bool INV>
+// Radix 8.  v[0] in [0, p + 7]; v[1..7] hold x + (1 + i) in [1, p + 1]
+// (OFF, the outputs of tw_mul) or x in [0, p + 7] with x <= p - 1 except for
+// v[0] (first stage, canonical).  Every output is v[0] plus signed inputs:
+// v[0] carries the bias 4p (and the constant, which then cancels everywhere
+// but in V[0], where both are taken out again), so
+//   V[0] = sum of eight                                  in [0, 8p + 7],
+//   V[2], V[4], V[6] + 4p: four inputs with either sign  in [0, 8p + 7],
+//   odd V + 4p: b0 and w4 b2 in +-p, c1 and d1 of the rotated pair in
+//     +-(p + 2^33) once the sum of two of them is shifted by p,
+//     so within +-(3p + 2^34)                            in [0, 8p],
+// and 8p + 7 = 2^64 - 1: no word wraps, and one fold each ends the stage.
+// Against the previous form (biased subtractions of two instructions more
+// and canonical products) a radix-8 stage issues 62 instead of 106
+// arithmetic instructions an element.
+template <bool INV, bool OFF>
 __device__ __forceinline__ void dft8(fe *v) {
-  const uint64_t P2 = 2 * P, P4 = 4 * P;
-  lz a[4], b[4];
+  constexpr uint64_t B = 4 * P + (OFF ? 1 : 0);  // bias of v[0]
+  constexpr uint64_t Z = 4 * P + (OFF ? 8 : 0);  // what V[0] holds of biases and constants
+  v[0] = fe_make(v[0].re + B, v[0].im + B);
+  fe a[4], b[4];
 #pragma unroll
-  for (int q = 0; q < 4; q++) {  // <= 2p (<= 2p + 7 for q = 0)
-    a[q] = lzadd(lz_of(v[q]), lz_of(v[q + 4]));
-    b[q] = lzsub(lz_of(v[q]), lz_of(v[q + 4]), P);
+  for (int q = 0; q < 4; q++) {
+    a[q] = lz_add(v[q], v[q + 4]);
+    b[q] = lz_sub(v[q], v[q + 4]);
   }
-  b[1] = lz_w8<INV>(b[1]);    // < p + 2^32
-  b[2] = lz_w4<INV>(b[2]);    // <= 2p
-  b[3] = lz_w8_3<INV>(b[3]);  // < p + 2^32
-  // two radix-4 DFTs on inputs <= 2p (x[0] <= 2p + 7): c, d <= 4p + 7,
-  // outputs <= 8p + 7
-  lz out[8];
-#pragma unroll
-  for (int h = 0; h < 2; h++) {
-    lz *x = h ? b : a;
-    lz c0 = lzadd(x[0], x[2]), c1 = lzadd(x[1], x[3]);
-    lz d0 = lzsub(x[0], x[2], P2), d1 = lzsub(x[1], x[3], P2);
-    // d1 * w4 on a value <= 4p: fold to <= p + 3 first
-    d1 = lz{fold(d1.re), fold(d1.im)};
-    d1 = INV ? lz{P2 - d1.im, d1.re} : lz{d1.im, P2 - d1.re};  // < 2p
-    out[h + 0] = lzadd(c0, c1);       // V[0 + h]
-    out[h + 4] = lzsub(c0, c1, P4);   // V[4 + h]
-    out[h + 2] = lzadd(d0, d1);       // V[2 + h]
-    out[h + 6] = lzsub(d0, d1, P4);   // V[6 + h]
+  {
+    const fe c0 = lz_add(a[0], a[2]), c1 = lz_add(a[1], a[3]);
+    const fe d0 = lz_sub(a[0], a[2]), d1 = lz_sub(a[1], a[3]);
+    v[0] = lz_fold(fe_make(c0.re + c1.re - Z, c0.im + c1.im - Z));
+    v[4] = lz_fold(lz_sub(c0, c1));
+    v[2] = lz_fold(lz_w4_add<INV, true>(d0, d1));
+    v[6] = lz_fold(lz_w4_add<INV, false>(d0, d1));
   }
-#pragma unroll
-  for (int k = 0; k < 8; k++) v[k] = fe_make(fold(out[k].re), fold(out[k].im));
-}
-
-// omega_S^e from the half table T[t] = omega_S^t (t < S/2):
-// omega_S^{t + S/2} = -omega_S^t.
-__device__ __forceinline__ fe twiddle(const fe *T, uint32_t e, int logS) {
-  const uint32_t hshift = logS - 1;
-  const fe w = T[e & ((1u << hshift) - 1)];
-  if (e >> hshift) return fe_make(w.re ? P - w.re : 0, w.im ? P - w.im : 0);
-  return w;
-}
-
-// One radix-R Stockham stage over E staged elements (B sub-transforms of
-// length S = 2^LOGS), Ns = 2^LOGNS = product of the earlier radices:
-//   butterfly (b, j): v[r] = x[j + r S/R] * omega_{Ns R}^{r (j mod Ns)},
-//   DFT_R(v), x'[(j/Ns) Ns R + (j mod Ns) + r Ns] = v[r].
-// S and Ns are compile-time, so shifts, masks and the swizzled offsets of a
-// butterfly's elements fold into immediates: when the stride between them is
-// a multiple of 64 elements, swz(a + r stride) = swz(a) + r stride.
-template <int R, bool INV, int LOGS, int LOGNS>
-__device__ __forceinline__ void stockham_stage(fe *sm, const fe *T, int logE) {
-  constexpr int LOGR = R == 8 ? 3 : (R == 4 ? 2 : 1);
-  constexpr int PER = kPerThread / R;
-  constexpr int logSR = LOGS - LOGR;
-  const uint32_t nb = 1u << (logE - LOGR);
-  fe v[PER * R];
-#pragma unroll
-  for (int i = 0; i < PER; i++) {
-    const uint32_t u = threadIdx.x + i * blockDim.x;
-    if (u < nb) {
-      const uint32_t b = u >> logSR, j = u & ((1u << logSR) - 1);
-      const uint32_t base = (b << LOGS) + j;
-      if constexpr (logSR >= 6) {
-        const fe *src = sm + swz(base);
-#pragma unroll
-        for (int r = 0; r < R; r++) v[i * R + r] = src[(uint32_t)r << logSR];
-      } else {
-#pragma unroll
-        for (int r = 0; r < R; r++) v[i * R + r] = sm[swz(base + ((uint32_t)r << logSR))];
-      }
-      if (LOGNS > 0) {
-        const uint32_t k = j & ((1u << LOGNS) - 1);
-        constexpr int sh = LOGS - LOGNS - LOGR;
-        if (R == 8) {
-          // k << sh < S/8, so the exponents r (k << sh) of r <= 4 stay in the
-          // half table and only r = 5..7 may need the negation.
-          const fe *tw = T + (k << sh);
-          constexpr uint32_t half = 1u << (LOGS - 1);
-#pragma unroll
-          for (int r = 1; r <= 4; r++) v[i * R + r] = fmul(v[i * R + r], tw[(r - 1) * (k << sh)]);  // T[r (k << sh)]
-#pragma unroll
-          for (int r = 5; r < 8; r++) {
-            const uint32_t e = r * (k << sh);
-            const bool hi = e >= half;
-            const fe w = T[hi ? e - half : e];
-            v[i * R + r] = fmul(v[i * R + r], hi ? fe_make(P - w.re, P - w.im) : w);
-          }
-        } else {
-#pragma unroll
-          for (int r = 1; r < R; r++) v[i * R + r] = fmul(v[i * R + r], twiddle(T, (r * k) << sh, LOGS));
-        }
-      }
-      if (R == 8) dft8<INV>(&v[i * R]);
-      else if (R == 4) dft4<INV>(&v[i * R]);
-      else dft2<INV>(&v[i * R]);
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < PER; i++) {
-    const uint32_t u = threadIdx.x + i * blockDim.x;
-    if (u < nb) {
-      const uint32_t b = u >> logSR, j = u & ((1u << logSR) - 1);
-      const uint32_t k = j & ((1u << LOGNS) - 1);
-      const uint32_t dst = (b << LOGS) + ((j >> LOGNS) << (LOGNS + LOGR)) + k;
-      if constexpr (LOGNS >= 6) {
-        fe *d = sm + swz(dst);
-#pragma unroll
-        for (int r = 0; r < R; r++) d[(uint32_t)r << LOGNS] = v[i * R + r];
-      } else {
-#pragma unroll
-        for (int r = 0; r < R; r++) sm[swz(dst + ((uint32_t)r << LOGNS))] = v[i * R + r];
-      }
-    }
-  }
-  __syncthreads();
-}
-
-template <bool INV, int LOGS, int LOGNS>
-__device__ __forceinline__ void stockham_radix8(fe *sm, const fe *T, int logE) {
-  if constexpr (LOGNS < LOGS) {
-    stockham_stage<8, INV, LOGS, LOGNS>(sm, T, logE);
-    stockham_radix8<INV, LOGS, LOGNS + 3>(sm, T, logE);
-  }
-}
-
-// The stages of a length-2^LOGS transform: a radix-2 or radix-4 stage when
-// LOGS is not a multiple of 3, then radix-8 stages.
-template <bool INV, int LOGS>
-__device__ __forceinline__ void stockham(fe *sm, const fe *T, int logE) {
-  if constexpr (LOGS % 3 == 1) {
-    stockham_stage<2, INV, LOGS, 0>(sm, T, logE);
-    stockham_radix8<INV, LOGS, 1>(sm, T, logE);
-  } else if constexpr (LOGS % 3 == 2) {
-    stockham_stage<4, INV, LOGS, 0>(sm, T, logE);
-    stockham_radix8<INV, LOGS, 2>(sm, T, logE);
+  // w8 = 2^30 (1 - i) and w8^3 = 2^30 (-1 - i), inverse conjugates: with
+  // s = re + im, d = im - re
+  //   forward: w8 b1 = (m(s1), m(d1)),   w8^3 b3 = (m(d3), -m(s3))
+  //   inverse: w8 b1 = (m(-d1), m(s1)),  w8^3 b3 = (-m(s3), m(-d3))
+  const uint64_t m1s = mul2e30(b[1].re + b[1].im), m3s = mul2e30(b[3].re + b[3].im);
+  const uint64_t m1d = mul2e30(INV ? b[1].re - b[1].im : b[1].im - b[1].re);
+  const uint64_t m3d = mul2e30(INV ? b[3].re - b[3].im : b[3].im - b[3].re);
+  const fe c0 = lz_w4_add<INV, true>(b[0], b[2]), d0 = lz_w4_add<INV, false>(b[0], b[2]);
+  fe c1, d1;
+  if (INV) {
+    c1 = fe_make(m1d - m3s, m1s + m3d - P);
+    d1 = fe_make(m1d + m3s - P, m1s - m3d);
   } else {
-    stockham_radix8<INV, LOGS, 0>(sm, T, logE);
+    c1 = fe_make(m1s + m3d - P, m1d - m3s);
+    d1 = fe_make(m1s - m3d, m1d + m3s - P);
+  }
+  v[1] = lz_fold(lz_add(c0, c1));
+  v[5] = lz_fold(lz_sub(c0, c1));
+  v[3] = lz_fold(lz_w4_add<INV, true>(d0, d1));
+  v[7] = lz_fold(lz_w4_add<INV, false>(d0, d1));
+}
+
+// ---- one pass ------------------------------------------------------------
+// The stages of a length-2^LOGS sub-transform: a first one of radix 2, 4 or
+// 8 (whatever makes the rest a multiple of three levels), then radix 8.
+__host__ __device__ constexpr int first_log(int logs) { return logs <= 3 ? logs : (logs % 3 == 0 ? 3 : logs % 3); }
+// Stage twiddles: the products of a stage depend on Ns alone (omega_{8 Ns}^{r
+// k}, k < Ns, r = 1..7), so one table in global memory serves every length:
+// Ns = 2, 4, ..., 2^10 one after the other, each [r - 1][k].  Lanes of a warp
+// read neighbouring k, whole lines out of L1 (57 KB for the last stage of
+// S = 2^12, beside 128 KB of staged data).  As a half table of omega_S in
+// shared memory, loaded by every CTA, the strided reads cost up to eight
+// wavefronts for one (60 % of a pass's shared-memory wavefronts were
+// conflicts) and r = 5..7 a conditional negation.
+__host__ __device__ constexpr uint32_t stage_table_offset(int logns) { return 7u * ((1u << logns) - 2); }
+
+// Entry j of sub-transform b in shared memory.  The exclusive or with j / 8
+// keeps contiguous and stride-8 runs of 16-byte elements free of bank
+// conflicts, the one with xb the runs that take the same j of neighbouring
+// sub-transforms.
+template <int LOGS>
+__device__ __forceinline__ uint32_t slot(uint32_t b, uint32_t xb, uint32_t j) {
+  return (b << LOGS) + (j ^ ((j >> 3) & 7u) ^ xb);
+}
+// The slot of entry j + (r << LR) from the slot s0 of entry j, where j has
+// zeros at those bits: the exclusive or is linear.
+template <int LR>
+__device__ __forceinline__ uint32_t slot_step(uint32_t s0, uint32_t r) {
+  const uint32_t x = r << LR;
+  return LR >= 6 ? s0 + x : s0 ^ (x ^ ((x >> 3) & 7u));
+}
+// Spreads neighbouring sub-transforms over the banks so that eight lanes with
+// 2 or 4 of them and 4 or 2 consecutive butterflies of radix 2, 4 or 8 meet
+// no bank twice (the shifts lie outside the spans of the lanes' own offsets).
+__device__ __forceinline__ uint32_t bank_shift(uint32_t b, int logB) {
+  if (logB >= 3) return b & 7u;
+  return logB == 2 ? (b & 1 ? 3u : 0u) ^ (b & 2 ? 5u : 0u) : (b & 1 ? 7u : 0u);
+}
+
+// Waits for the threads that share a sub-transform: a warp, or a named
+// barrier of the S/8 threads where a CTA holds several sub-transforms, so
+// that one group's memory phase overlaps another's arithmetic.
+template <int LOGS>
+__device__ __forceinline__ void group_sync() {
+  constexpr uint32_t G = LOGS >= 3 ? 1u << (LOGS - 3) : 1u;
+  if (G <= 32) {
+    __syncwarp();
+  } else if (blockDim.x <= G || blockDim.x / G > 15) {
+    __syncthreads();
+  } else {
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + threadIdx.x / G), "r"(G) : "memory");
   }
 }
 
-template <bool INV>
-__device__ __forceinline__ void stockham_dispatch(fe *sm, const fe *T, int logS, int logE) {
-  switch (logS) {
-    case 1: stockham<INV, 1>(sm, T, logE); break;
-    case 2: stockham<INV, 2>(sm, T, logE); break;
-    case 3: stockham<INV, 3>(sm, T, logE); break;
-    case 4: stockham<INV, 4>(sm, T, logE); break;
-    case 5: stockham<INV, 5>(sm, T, logE); break;
-    case 6: stockham<INV, 6>(sm, T, logE); break;
-    case 7: stockham<INV, 7>(sm, T, logE); break;
-    case 8: stockham<INV, 8>(sm, T, logE); break;
-    case 9: stockham<INV, 9>(sm, T, logE); break;
-    case 10: stockham<INV, 10>(sm, T, logE); break;
-    case 11: stockham<INV, 11>(sm, T, logE); break;
-    case 12: stockham<INV, 12>(sm, T, logE); break;
-    case 13: stockham<INV, 13>(sm, T, logE); break;
-    default: break;  // length 1: nothing to do
+// Twiddle products of one butterfly of a stage with Ns = 2^LOGNS.
+template <int LOGNS>
+__device__ __forceinline__ void twiddle_inputs(fe *v, const fe *stages, uint32_t j) {
+  const uint4 *t = reinterpret_cast<const uint4 *>(stages + stage_table_offset(LOGNS) + (j & ((1u << LOGNS) - 1)));
+#pragma unroll
+  for (int r = 1; r < 8; r++) {
+    const uint4 w = __ldg(t + ((r - 1) << LOGNS));
+    v[r] = tw_mul(v[r], fe_make(words64(w.x, w.y), words64(w.z, w.w)));
   }
 }
 
-// The first stage (Ns = 1, no twiddles) fused into the staging from global
-// memory: a thread loads the R inputs x[b, j + r S/R] of its butterflies,
-// transforms them in registers and stores x'[b, R j + r], so the stage costs
-// no shared-memory round trip.  Contiguous sub-transforms give consecutive
-// threads consecutive j; strided ones (columns of the first four-step pass)
-// consecutive sub-transforms b, whose columns are adjacent in memory.
-template <bool INV, int LOGS, bool PACK>
-__device__ __forceinline__ void staged_first_stage(fe *sm, const PassArgs &a, uint64_t g0, int logB, int logE) {
-  constexpr int LOGR = LOGS % 3 == 1 ? 1 : (LOGS % 3 == 2 ? 2 : 3);
-  constexpr int R = 1 << LOGR, PER = kPerThread / R, logSR = LOGS - LOGR;
-  const uint32_t nb = 1u << (logE - LOGR);
-  const bool contiguous = a.in_jstride == 1;
-  fe v[PER][R];
-  uint64_t nonreal = 0;
-#pragma unroll
-  for (int i = 0; i < PER; i++) {  // all loads first: PER * R = 8 in flight
-    const uint32_t u = threadIdx.x + i * blockDim.x;
-    const uint32_t b = contiguous ? u >> logSR : u & ((1u << logB) - 1);
-    const uint32_t j = contiguous ? u & ((1u << logSR) - 1) : u >> logB;
-    const uint64_t row = (g0 + b) * a.in_gstride;
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      const uint32_t jj = j + ((uint32_t)r << logSR);
-      const uint64_t addr = row + (uint64_t)jj * a.in_jstride;
-      const bool ok = u < nb && addr < a.n_valid && jj < a.j_valid;
-      if (!PACK) {
-        v[i][r] = ok ? a.in[addr] : fe_zero();
-      } else {
-        const fe e0 = ok ? a.in[2 * addr] : fe_zero(), e1 = ok ? a.in[2 * addr + 1] : fe_zero();
-        nonreal |= e0.im | e1.im;
-        v[i][r] = fe_make(e0.re, e1.re);
-      }
-    }
-  }
-  if (PACK && nonreal) atomicOr(a.nonreal, 1u);
-#pragma unroll
-  for (int i = 0; i < PER; i++) {
-    const uint32_t u = threadIdx.x + i * blockDim.x;
+// The stages between the first and the last, in place in shared memory:
+//   v[r] = x[j + r S/8] omega_{8 Ns}^{r (j mod Ns)}, DFT_8(v),
+//   x'[(j / Ns) 8 Ns + (j mod Ns) + r Ns] = v[r].
+template <bool INV, int LOGS, int LOGNS>
+__device__ __forceinline__ void middle_stages(fe *sm, const fe *stages, int logB, uint32_t nb, uint32_t u) {
+  if constexpr (LOGNS + 3 < LOGS) {
+    const uint32_t b = u >> (LOGS - 3), j = u & ((1u << (LOGS - 3)) - 1), xb = bank_shift(b, logB);
+    fe v[8];
     if (u < nb) {
-      const uint32_t b = contiguous ? u >> logSR : u & ((1u << logB) - 1);
-      const uint32_t j = contiguous ? u & ((1u << logSR) - 1) : u >> logB;
-      if (R == 8) dft8<INV>(v[i]);
-      else if (R == 4) dft4<INV>(v[i]);
-      else dft2<INV>(v[i]);
-      const uint32_t dst = (b << LOGS) + (j << LOGR);
+      const uint32_t s0 = slot<LOGS>(b, xb, j);
 #pragma unroll
-      for (int r = 0; r < R; r++) sm[swz(dst + r)] = v[i][r];
+      for (int r = 0; r < 8; r++) v[r] = sm[slot_step<LOGS - 3>(s0, r)];
+      twiddle_inputs<LOGNS>(v, stages, j);
+      dft8<INV, true>(v);
     }
+    group_sync<LOGS>();
+    if (u < nb) {
+      const uint32_t s0 = slot<LOGS>(b, xb, ((j >> LOGNS) << (LOGNS + 3)) + (j & ((1u << LOGNS) - 1)));
+#pragma unroll
+      for (int r = 0; r < 8; r++) sm[slot_step<LOGNS>(s0, r)] = v[r];
+    }
+    if constexpr (LOGNS + 6 < LOGS) group_sync<LOGS>();  // the caller waits before the last stage
+    middle_stages<INV, LOGS, LOGNS + 3>(sm, stages, logB, nb, u);
   }
 }
 
-template <bool INV, int LOGS, bool PACK>
-__device__ __forceinline__ void staged_transform(fe *sm, const fe *T, const PassArgs &a, uint64_t g0, int logB,
-                                                 int logE) {
-  constexpr int LOGR = LOGS % 3 == 1 ? 1 : (LOGS % 3 == 2 ? 2 : 3);
-  staged_first_stage<INV, LOGS, PACK>(sm, a, g0, logB, logE);
-  __syncthreads();
-  stockham_radix8<INV, LOGS, LOGR>(sm, T, logE);
+// A 16-byte copy from global to shared memory, waited for by copies_wait.
+__device__ __forceinline__ void copy_async(fe *dst, const fe *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// Staged data is read once: it should not displace the twiddles in L1.
+__device__ __forceinline__ fe load_once(const fe *p) {
+  fe x;
+  asm volatile("ld.global.L1::no_allocate.v2.u64 {%0, %1}, [%2];" : "=l"(x.re), "=l"(x.im) : "l"(p));
+  return x;
 }
 
-template <bool INV, bool PACK>
-__device__ __forceinline__ void staged_dispatch(fe *sm, const fe *T, const PassArgs &a, uint64_t g0, int logS,
-                                                int logB, int logE) {
-  switch (logS) {
-    case 1: staged_transform<INV, 1, PACK>(sm, T, a, g0, logB, logE); break;
-    case 2: staged_transform<INV, 2, PACK>(sm, T, a, g0, logB, logE); break;
-    case 3: staged_transform<INV, 3, PACK>(sm, T, a, g0, logB, logE); break;
-    case 4: staged_transform<INV, 4, PACK>(sm, T, a, g0, logB, logE); break;
-    case 5: staged_transform<INV, 5, PACK>(sm, T, a, g0, logB, logE); break;
-    case 6: staged_transform<INV, 6, PACK>(sm, T, a, g0, logB, logE); break;
-    case 7: staged_transform<INV, 7, PACK>(sm, T, a, g0, logB, logE); break;
-    case 8: staged_transform<INV, 8, PACK>(sm, T, a, g0, logB, logE); break;
-    case 9: staged_transform<INV, 9, PACK>(sm, T, a, g0, logB, logE); break;
-    case 10: staged_transform<INV, 10, PACK>(sm, T, a, g0, logB, logE); break;
-    case 11: staged_transform<INV, 11, PACK>(sm, T, a, g0, logB, logE); break;
-    case 12: staged_transform<INV, 12, PACK>(sm, T, a, g0, logB, logE); break;
-    case 13: staged_transform<INV, 13, PACK>(sm, T, a, g0, logB, logE); break;
-    default: break;
+// Writes one output group: values v[q] at positions k + q dk of column l,
+// times the outer twiddle and the scale where the pass has them.
+template <int N>
+__device__ __forceinline__ void emit(const PassArgs &a, fe *out, uint64_t l, uint32_t k, uint32_t dk, const fe *v) {
+  const uint64_t base = l * a.out_gstride + (uint64_t)k * a.out_kstride, step = (uint64_t)dk * a.out_kstride;
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    fe x = v[q];
+    const uint64_t addr = base + q * step;
+    if (a.tw_full) {
+      x = fmul(x, a.tw_full[addr]);
+    } else if (a.tw_lo) {
+      const uint64_t ex = l * (k + q * dk) << a.tw_shift;
+      x = fmul(x, fmul(a.tw_lo[ex & ((1u << kTwLoBits) - 1)], a.tw_hi[ex >> kTwLoBits]));
+    }
+    if (a.has_scale) x = fmul(x, a.scale);
+    else if (!a.tw_lo && !a.tw_full) x = canon_fe(x);
+    if (!a.acc) out[addr] = x;
+    else if (addr < a.acc_n) out[addr] = fadd(out[addr], x);
   }
 }
 
-// PACK: the first pass of a packed real transform (a separate instantiation,
-// so that the general kernel keeps its register allocation).
-template <bool PACK>
-__global__ void __launch_bounds__(kMaxThreads) ntt_pass_kernel(PassArgs a) {
+// One pass: a CTA takes tiles of B = 2^logB sub-transforms of length S, E =
+// S B elements, with E/8 threads.  The first stage runs on the values as
+// they arrive from global memory, the last one ends in registers and stores
+// them: a tile crosses shared memory once less than it has stages.  What
+// bounds it: the integer pipes and the register file's read ports (a
+// radix-8 stage alone takes 115 cycles an element on a full SM, 64 of them
+// the FMA pipe's for the wide products); small CTAs (64 to 256 threads, 1024
+// threads an SM at 64 registers) keep other tiles computing while one waits
+// for memory or a barrier.  A pass of 2^8 over 2^24 elements takes 183 us,
+// 0.8 of the sum of its stages alone.
+// PACK: the first pass of a packed real transform.
+template <int LOGS, bool INV, bool PACK>
+__global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs a) {
   if (a.run_if && *a.run_if == 0) return;  // uniform over the grid
   extern __shared__ fe smem[];
-  a.in += blockIdx.y * a.row_in;
-  a.out += blockIdx.y * a.row_out;
-  const int logS = a.logS, logB = a.logB, logE = logS + logB;
-  const uint32_t S = 1u << logS, total = 1u << logE;
+  constexpr int LOGR = first_log(LOGS), R = 1 << LOGR, PER = kPerThread / R, LOGJ = LOGS - LOGR;
+  constexpr uint32_t S = 1u << LOGS;
+  const int logB = a.logB;
+  const uint32_t total = S << logB;
   fe *sm = smem;
-  fe *T = smem + total;  // S/2 twiddles omega_S^t
+  const bool in_rows = a.in_jstride == 1, out_rows = a.out_kstride == 1 || logB == 0;
+  const uint32_t tid = threadIdx.x;
   const uint64_t g0 = (uint64_t)blockIdx.x << logB;
-
-  if (logS >= 1) {
-    const uint32_t nT = S >> 1;
-    for (uint32_t t = threadIdx.x; t < nT; t += blockDim.x) T[t] = a.wh[t << (kSubLog - logS)];
-  }
+  const uint64_t l0 = g0 & ((1ull << a.logG) - 1), h = g0 >> a.logG;
+  const fe *in = a.in + blockIdx.y * a.row_in + h * a.in_hstride;
+  fe *out = a.out + blockIdx.y * a.row_out + h * a.out_hstride;
+  fe v[PER][R];
+  // first stage: v[r] = x[j + r S/R]
   if (a.sp_l > 0) {
     // Sparse rows: row k2 of the intermediate holds, in column n1, the sum
     // over the entries q = n1 (mod row length) of c * omega_L^{q k2}: the
@@ -435,138 +367,133 @@ __global__ void __launch_bounds__(kMaxThreads) ntt_pass_kernel(PassArgs a) {
       const uint32_t i = t % l, b = t / l;
       if (!a.sp_lead[i]) continue;
       const uint64_t k2 = g0 + b;
-      fe v = fe_zero();
+      fe x = fe_zero();
       int u = (int)i;
       for (uint32_t it = 0; it < l && u >= 0; it++, u = a.sp_next[u]) {
         const uint64_t q = (uint64_t)((uint32_t)a.sp_q[u] >> a.sp_shift);
         const uint64_t ex = (q * k2) & a.sp_mask;
-        v = fadd(v, fmul(a.sp_c[u], fmul(a.sp_lo[ex & ((1u << kTwLoBits) - 1)], a.sp_hi[ex >> kTwLoBits])));
+        x = fadd(x, fmul(a.sp_c[u], fmul(a.sp_lo[ex & ((1u << kTwLoBits) - 1)], a.sp_hi[ex >> kTwLoBits])));
       }
-      const uint32_t n1 = ((uint32_t)a.sp_q[i] >> a.sp_shift) & (S - 1);
-      sm[swz((b << logS) + n1)] = v;
+      sm[(b << LOGS) + (((uint32_t)a.sp_q[i] >> a.sp_shift) & (S - 1))] = x;
     }
     __syncthreads();
-    if (a.inverse) stockham_dispatch<true>(sm, T, logS, logE);
-    else stockham_dispatch<false>(sm, T, logS, logE);
-  } else if (logS >= 1) {
-    if (a.inverse) staged_dispatch<true, PACK>(sm, T, a, g0, logS, logB, logE);
-    else staged_dispatch<false, PACK>(sm, T, a, g0, logS, logB, logE);
-  } else {
-    // Sub-transforms of length 1: staging only.
-    // A thread stages at most kPerThread elements (blockDim >= total / 8);
-    // groups of kLoadGroup loads are issued before their shared-memory
-    // stores so that several global loads are in flight per thread.
-    if (a.in_jstride == 1) {
-      for (int i0 = 0; i0 < kPerThread; i0 += kLoadGroup) {
-        fe v[kLoadGroup];
 #pragma unroll
-        for (int i = 0; i < kLoadGroup; i++) {
-          const uint32_t e = threadIdx.x + (i0 + i) * blockDim.x;
-          const uint32_t b = e >> logS, j = e & (S - 1);
-          const uint64_t addr = (g0 + b) * a.in_gstride + j;
-          v[i] = (e < total && addr < a.n_valid && j < a.j_valid) ? a.in[addr] : fe_zero();
-        }
+    for (int i = 0; i < PER; i++) {
+      const uint32_t u = tid + i * blockDim.x;
 #pragma unroll
-        for (int i = 0; i < kLoadGroup; i++) {
-          const uint32_t e = threadIdx.x + (i0 + i) * blockDim.x;
-          if (e < total) sm[swz(e)] = v[i];
-        }
-      }
-    } else {
-      for (int i0 = 0; i0 < kPerThread; i0 += kLoadGroup) {
-        fe v[kLoadGroup];
-#pragma unroll
-        for (int i = 0; i < kLoadGroup; i++) {
-          const uint32_t e = threadIdx.x + (i0 + i) * blockDim.x;
-          const uint32_t b = e & ((1u << logB) - 1), j = e >> logB;
-          const uint64_t addr = (g0 + b) * a.in_gstride + (uint64_t)j * a.in_jstride;
-          v[i] = (e < total && addr < a.n_valid && j < a.j_valid) ? a.in[addr] : fe_zero();
-        }
-#pragma unroll
-        for (int i = 0; i < kLoadGroup; i++) {
-          const uint32_t e = threadIdx.x + (i0 + i) * blockDim.x;
-          const uint32_t b = e & ((1u << logB) - 1), j = e >> logB;
-          if (e < total) sm[swz((b << logS) + j)] = v[i];
-        }
+      for (int r = 0; r < R; r++) {
+        const uint32_t e = (u >> LOGJ << LOGS) + (u & ((1u << LOGJ) - 1)) + ((uint32_t)r << LOGJ);
+        v[i][r] = e < total ? sm[e] : fe_zero();
       }
     }
     __syncthreads();
-  }
-
-  if (a.out_kstride == 1) {
-    for (uint32_t e = threadIdx.x; e < total; e += blockDim.x) {
-      const uint32_t b = e >> logS, k = e & (S - 1);
-      fe v = canon_fe(sm[swz(e)]);
-      if (a.tw_lo) {
-        const uint64_t ex = (g0 + b) * k;
-        v = fmul(v, fmul(a.tw_lo[ex & ((1u << kTwLoBits) - 1)], a.tw_hi[ex >> kTwLoBits]));
+  } else {
+    uint64_t nonreal = 0;
+#pragma unroll
+    for (int i = 0; i < PER; i++) {  // all loads first: PER * R = 8 in flight
+      const uint32_t u = tid + i * blockDim.x;
+      const uint32_t b = in_rows ? u >> LOGJ : u & ((1u << logB) - 1);
+      const uint32_t j = in_rows ? u & ((1u << LOGJ) - 1) : u >> logB;
+      const uint64_t base = (l0 + b) * a.in_gstride + (uint64_t)j * a.in_jstride;
+      const uint64_t step = a.in_jstride << LOGJ;
+      if (u >= (total >> LOGR)) {
+#pragma unroll
+        for (int r = 0; r < R; r++) v[i][r] = fe_zero();
+      } else if (a.dense) {
+        const fe *p = in + (PACK ? 2 * base : base);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          if (!PACK) {
+            v[i][r] = load_once(p + r * step);
+          } else {
+            const fe e0 = load_once(p + 2 * r * step), e1 = load_once(p + 2 * r * step + 1);
+            nonreal |= e0.im | e1.im;
+            v[i][r] = fe_make(e0.re, e1.re);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          const uint64_t addr = base + r * step;
+          const bool ok = addr < a.n_valid && j + ((uint32_t)r << LOGJ) < a.j_valid;
+          if (!PACK) {
+            v[i][r] = ok ? in[addr] : fe_zero();
+          } else {
+            const fe e0 = ok ? in[2 * addr] : fe_zero(), e1 = ok ? in[2 * addr + 1] : fe_zero();
+            nonreal |= e0.im | e1.im;
+            v[i][r] = fe_make(e0.re, e1.re);
+          }
+        }
       }
-      if (a.has_scale) v = fmul(v, a.scale);
-      const uint64_t addr = (g0 + b) * a.out_gstride + k;
-      if (!a.acc) a.out[addr] = v;
-      else if (addr < a.acc_n) a.out[addr] = fadd(a.out[addr], v);
     }
-  } else if (a.tw_full && !a.has_scale && !a.acc) {
-    // first pass with the full twiddle table: issue each group's table
-    // loads before its multiplies
-    for (int i0 = 0; i0 < kPerThread; i0 += kLoadGroup) {
-      fe tw[kLoadGroup];
+    if (PACK && nonreal) atomicOr(a.nonreal, 1u);
+  }
 #pragma unroll
-      for (int i = 0; i < kLoadGroup; i++) {
-        const uint32_t e = threadIdx.x + (i0 + i) * blockDim.x;
-        const uint32_t b = e & ((1u << logB) - 1), k = e >> logB;
-        const uint64_t addr = (g0 + b) * a.out_gstride + (uint64_t)k * a.out_kstride;
-        tw[i] = e < total ? a.tw_full[addr] : fe_zero();
-      }
+  for (int i = 0; i < PER; i++) {
+    if (R == 8) dft8<INV, false>(v[i]);
+    else if (R == 4) dft4<INV>(v[i]);
+    else if (R == 2) dft2<INV>(v[i]);
+  }
+  const bool in_order = in_rows || a.sp_l > 0;
+  if constexpr (LOGS <= 3) {  // the first stage is the last
 #pragma unroll
-      for (int i = 0; i < kLoadGroup; i++) {
-        const uint32_t e = threadIdx.x + (i0 + i) * blockDim.x;
-        if (e >= total) continue;
-        const uint32_t b = e & ((1u << logB) - 1), k = e >> logB;
-        const uint64_t addr = (g0 + b) * a.out_gstride + (uint64_t)k * a.out_kstride;
-        a.out[addr] = fmul(sm[swz((b << logS) + k)], tw[i]);  // takes the folded value as it is
-      }
+    for (int i = 0; i < PER; i++) {
+      const uint32_t u = tid + i * blockDim.x;
+      const uint32_t b = in_order ? u >> LOGJ : u & ((1u << logB) - 1);
+      if (u < (total >> LOGR)) emit<R>(a, out, l0 + b, 0, 1, v[i]);
     }
   } else {
-    for (uint32_t e = threadIdx.x; e < total; e += blockDim.x) {
-      const uint32_t b = e & ((1u << logB) - 1), k = e >> logB;
-      fe v = canon_fe(sm[swz((b << logS) + k)]);
-      const uint64_t addr = (g0 + b) * a.out_gstride + (uint64_t)k * a.out_kstride;
-      if (a.tw_full) {
-        v = fmul(v, a.tw_full[addr]);
-      } else if (a.tw_lo) {
-        const uint64_t ex = (g0 + b) * k;
-        v = fmul(v, fmul(a.tw_lo[ex & ((1u << kTwLoBits) - 1)], a.tw_hi[ex >> kTwLoBits]));
+#pragma unroll
+    for (int i = 0; i < PER; i++) {  // x'[R j + r]
+      const uint32_t u = tid + i * blockDim.x;
+      const uint32_t b = in_order ? u >> LOGJ : u & ((1u << logB) - 1);
+      const uint32_t j = in_order ? u & ((1u << LOGJ) - 1) : u >> logB;
+      const uint32_t s0 = slot<LOGS>(b, bank_shift(b, logB), j << LOGR);
+      if (u < (total >> LOGR)) {
+#pragma unroll
+        for (int r = 0; r < R; r++) sm[slot_step<0>(s0, r)] = v[i][r];
       }
-      if (a.has_scale) v = fmul(v, a.scale);
-      if (!a.acc) a.out[addr] = v;
-      else if (addr < a.acc_n) a.out[addr] = fadd(a.out[addr], v);
+    }
+    __syncthreads();
+    const uint32_t nb = total >> 3;
+    middle_stages<INV, LOGS, LOGR>(sm, a.stages, logB, nb, tid);
+    if (LOGR + 3 < LOGS) {
+      if (out_rows) group_sync<LOGS>();
+      else __syncthreads();
+    }
+    // last stage (Ns = S/8): outputs k = j + r S/8 leave from registers.
+    // Columns stored side by side are taken by neighbouring threads.
+    const uint32_t u = tid;
+    const uint32_t b = out_rows ? u >> (LOGS - 3) : u & ((1u << logB) - 1);
+    const uint32_t j = out_rows ? u & (S / 8 - 1) : u >> logB;
+    const uint32_t s0 = slot<LOGS>(b, bank_shift(b, logB), j);
+    fe w[8];
+    if (u < nb) {
+#pragma unroll
+      for (int r = 0; r < 8; r++) w[r] = sm[slot_step<LOGS - 3>(s0, r)];
+      const uint64_t base = (l0 + b) * a.out_gstride + (uint64_t)j * a.out_kstride;
+      const uint64_t step = a.out_kstride * (S / 8);
+      const bool staged_tw = a.tw_full && !a.has_scale && !a.acc;
+      twiddle_inputs<LOGS - 3>(w, a.stages, j);
+      if (staged_tw) {
+        // The outer twiddles arrive during the butterfly, in the slots that
+        // this thread alone has read.  Those reads have returned: w[1..7]
+        // went through the products, and the first address waits for w[0]
+        // (below 2^62, so its top bit adds nothing).
+        copy_async(sm + s0, a.tw_full + base + (w[0].re >> 63));
+#pragma unroll
+        for (int r = 1; r < 8; r++) copy_async(sm + slot_step<LOGS - 3>(s0, r), a.tw_full + base + r * step);
+      }
+      dft8<INV, true>(w);
+      if (staged_tw) {
+        copies_wait();
+#pragma unroll
+        for (int r = 0; r < 8; r++) out[base + r * step] = fmul(w[r], sm[slot_step<LOGS - 3>(s0, r)]);
+      } else {
+        emit<8>(a, out, l0 + b, j, S / 8, w);
+      }
     }
   }
-}
-
-// First half of the omega_{2^13} powers, per direction; shared by every length.
-fe *g_wq[2] = {nullptr, nullptr};
-int g_wq_device = -1;
-constexpr size_t kMaxSmem = sizeof(fe) * (kCtaElems + kCtaElems / 2);
-
-void ensure_wq() {
-  int dev;
-  GBZ_CUDA(cudaGetDevice(&dev));
-  if (g_wq[0] && g_wq_device == dev) return;
-  const int n = 1 << (kSubLog - 1);
-  std::vector<fe> h(n);
-  for (int dir = 0; dir < 2; dir++) {
-    fe w = root_of_unity(kSubLog);
-    if (dir) w = finv(w);
-    fe x = fe_one();
-    for (int t = 0; t < n; t++) { h[t] = x; x = fmul(x, w); }
-    GBZ_CUDA(cudaMalloc(&g_wq[dir], sizeof(fe) * n));
-    GBZ_CUDA(cudaMemcpy(g_wq[dir], h.data(), sizeof(fe) * n, cudaMemcpyHostToDevice));
-  }
-  g_wq_device = dev;
-  GBZ_CUDA(cudaFuncSetAttribute(ntt_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-  GBZ_CUDA(cudaFuncSetAttribute(ntt_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
 }
 
 // Column chains of a sparse input: next[t] = the next entry with the same
@@ -590,14 +517,70 @@ __global__ void sparse_chain_kernel(const int32_t *q, int l, int shift, uint32_t
   lead[t] = first;
 }
 
-void launch_pass(const PassArgs &a, uint64_t groups, cudaStream_t s, int rows = 1) {
-  const uint64_t blocks = groups >> a.logB;
+typedef void (*PassKernel)(const PassArgs);
+template <int LOGS>
+PassKernel pass_kernel(bool inverse, bool pack) {
+  if (pack) return ntt_pass_kernel<LOGS, false, true>;
+  return inverse ? ntt_pass_kernel<LOGS, true, false> : ntt_pass_kernel<LOGS, false, false>;
+}
+PassKernel pass_kernel(int logS, bool inverse, bool pack) {
+  switch (logS) {
+    case 0: return pass_kernel<0>(inverse, pack);
+    case 1: return pass_kernel<1>(inverse, pack);
+    case 2: return pass_kernel<2>(inverse, pack);
+    case 3: return pass_kernel<3>(inverse, pack);
+    case 4: return pass_kernel<4>(inverse, pack);
+    case 5: return pass_kernel<5>(inverse, pack);
+    case 6: return pass_kernel<6>(inverse, pack);
+    case 7: return pass_kernel<7>(inverse, pack);
+    case 8: return pass_kernel<8>(inverse, pack);
+    case 9: return pass_kernel<9>(inverse, pack);
+    case 10: return pass_kernel<10>(inverse, pack);
+    case 11: return pass_kernel<11>(inverse, pack);
+    case 12: return pass_kernel<12>(inverse, pack);
+    default: return pass_kernel<13>(inverse, pack);
+  }
+}
+
+// Stage twiddle tables per direction, shared by every length.
+fe *g_stages[2] = {nullptr, nullptr};
+int g_stages_device = -1;
+
+void ensure_stages() {
+  int dev;
+  GBZ_CUDA(cudaGetDevice(&dev));
+  if (g_stages[0] && g_stages_device == dev) return;
+  std::vector<fe> h(stage_table_offset(kSubLog - 2));
+  for (int dir = 0; dir < 2; dir++) {
+    for (int ns = 1; ns <= kSubLog - 3; ns++) {
+      fe w = root_of_unity(ns + 3);
+      if (dir) w = finv(w);
+      fe wr = w;
+      for (int r = 1; r < 8; r++, wr = fmul(wr, w)) {
+        fe x = fe_one();
+        for (uint32_t k = 0; k < (1u << ns); k++, x = fmul(x, wr)) h[stage_table_offset(ns) + ((r - 1) << ns) + k] = x;
+      }
+    }
+    GBZ_CUDA(cudaMalloc(&g_stages[dir], sizeof(fe) * h.size()));
+    GBZ_CUDA(cudaMemcpy(g_stages[dir], h.data(), sizeof(fe) * h.size(), cudaMemcpyHostToDevice));
+  }
+  g_stages_device = dev;
+  for (int logS = 0; logS <= kSubLog; logS++)
+    for (int kind = 0; kind < 3; kind++)
+      GBZ_CUDA(cudaFuncSetAttribute(pass_kernel(logS, kind == 1, kind == 2), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)(sizeof(fe) * kCtaElems)));
+}
+
+void launch_pass(PassArgs a, uint64_t groups, cudaStream_t s, int rows = 1) {
+  const uint64_t tiles = groups >> a.logB;
   const uint32_t E = 1u << (a.logS + a.logB);
-  const size_t smem = sizeof(fe) * (E + (a.logS >= 1 ? (1u << (a.logS - 1)) : 0));
+  const size_t smem = a.logS > 3 || a.sp_l > 0 ? sizeof(fe) * E : 0;
   const unsigned threads = E / kPerThread > 32 ? E / kPerThread : 32;
   if (rows < 1 || rows > 65535) throw ArgError("transform: 1..65535 rows per launch");
-  if (a.pack_real) ntt_pass_kernel<true><<<dim3((unsigned)blocks, (unsigned)rows), threads, smem, s>>>(a);
-  else ntt_pass_kernel<false><<<dim3((unsigned)blocks, (unsigned)rows), threads, smem, s>>>(a);
+  if (a.logG == 0) a.logG = 40;  // every g is a column of its own
+  const uint64_t last = (groups - 1) * a.in_gstride + ((1ull << a.logS) - 1) * a.in_jstride;
+  a.dense = a.j_valid >= (1u << a.logS) && (a.n_valid == ~0ull || last < a.n_valid);
+  pass_kernel(a.logS, a.inverse != 0, a.pack_real != 0)<<<dim3((unsigned)tiles, (unsigned)rows), threads, smem, s>>>(a);
   GBZ_CUDA(cudaGetLastError());
 }
 
@@ -628,20 +611,25 @@ __global__ void outer_table_kernel(fe w, int logL, int k1, fe *T) {
   }
 }
 
-const fe *outer_table_get(int logn, int k1, bool inverse) {
+// Tables of the default schedules (kScheduleTable added to the split) stay
+// for the process, whatever the autotuner does with its own.
+constexpr int kScheduleTable = 64;
+
+const fe *outer_table_get(int logn, int key_k1, bool inverse) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
   std::lock_guard<std::mutex> lk(g_outer_mu);
-  auto it = g_outer.find(std::make_tuple(dev, logn, k1, inverse ? 1 : 0));
+  auto it = g_outer.find(std::make_tuple(dev, logn, key_k1, inverse ? 1 : 0));
   return it == g_outer.end() ? nullptr : it->second;
 }
 
-void outer_table_build(int logn, int k1) {
-  if (logn <= kSubLog || k1 < 1 || k1 >= logn) return;
+void outer_table_build(int logn, int key_k1) {
+  const int k1 = key_k1 & (kScheduleTable - 1);
+  if (k1 < 1 || k1 >= logn) return;
   int dev = 0;
   GBZ_CUDA(cudaGetDevice(&dev));
   for (int dir = 0; dir < 2; dir++) {
-    const auto key = std::make_tuple(dev, logn, k1, dir);
+    const auto key = std::make_tuple(dev, logn, key_k1, dir);
     {
       std::lock_guard<std::mutex> lk(g_outer_mu);
       if (g_outer.count(key)) continue;
@@ -669,7 +657,8 @@ void outer_table_keep_only(int logn, int k1) {
   GBZ_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(g_outer_mu);
   for (auto it = g_outer.begin(); it != g_outer.end();) {
-    if (std::get<0>(it->first) == dev && std::get<1>(it->first) == logn && std::get<2>(it->first) != k1) {
+    if (std::get<0>(it->first) == dev && std::get<1>(it->first) == logn && std::get<2>(it->first) != k1 &&
+        std::get<2>(it->first) < kScheduleTable) {
       GBZ_CUDA(cudaDeviceSynchronize());
       cudaFree(it->second);
       it = g_outer.erase(it);
@@ -681,11 +670,67 @@ void outer_table_keep_only(int logn, int k1) {
 
 void ntt_use_full_twiddles(bool on) { g_use_outer = on; }
 
+namespace {
+// The passes of a transform whose shape nobody set: sub-transforms of 2^log[i]
+// and 2^logB[i] of them a CTA, in order.
+struct Schedule {
+  int passes, log[3], logB[3];
+};
+
+// Cycles an element of a pass of length 2^log, as measured for its parts with
+// every SM busy: a first stage of radix 2, 4 or 8, twiddled radix-8 stages,
+// loads, stores and the outer product.  From 2^10 on the barriers of a
+// sub-transform span several warps and cost more the longer it is (a pass of
+// 2^8 reaches 0.8 of its arithmetic, one of 2^12 0.55).
+double pass_cost(int log) {
+  static const double first[4] = {0, 17, 23, 34};
+  const double c = first[first_log(log)] + 115.0 * ((log - first_log(log)) / 3);
+  return c * (log < 10 ? 1.0 : log == 10 ? 1.05 : log == 11 ? 1.1 : 1.35) + 125;
+}
+
+// Two or three passes by that cost: two up to 2^20 (2^20 as 9 + 11: 41 us,
+// three passes 43), three above, where each further level would fall into
+// passes of 2^11 and more (one transform, two passes of the old shapes ->
+// three: 2^21 85 -> 74 us, 2^22 163 -> 142, 2^23 335 -> 280, 2^24 677 -> 541,
+// 2^25 1594 -> 1121, 2^26 3908 -> 2223).  A pass of 2^6 goes last and the
+// others in ascending order (2^22 as 8 + 8 + 6: 140 us, 6 + 8 + 8: 147).
+// Equal costs: the longer shortest pass.  CTAs stage 2^11 elements (2^10 in
+// three passes up to 2^22: 2^22 140 us, with 2^11 147), less where the rows
+// of a launch are too short to give every SM one.
+Schedule schedule(int logn, int rows = 1) {
+  Schedule best{};
+  double least = 1e30;
+  for (int x = 5; x <= 12; x++)
+    for (int y = x; y <= 12; y++) {
+      if (x + y == logn && pass_cost(x) + pass_cost(y) <= least) {
+        least = pass_cost(x) + pass_cost(y);
+        best = Schedule{2, {x, y, 0}, {0, 0, 0}};
+      }
+      const int z = logn - x - y;
+      if (z >= y && z <= 12 && pass_cost(x) + pass_cost(y) + pass_cost(z) <= least) {
+        least = pass_cost(x) + pass_cost(y) + pass_cost(z);
+        best = Schedule{3, {x, y, z}, {0, 0, 0}};
+      }
+    }
+  int *l = best.log;
+  if (l[0] == 6) std::rotate(l, l + 1, l + best.passes);
+  if (best.passes == 3 && l[0] > l[1]) std::swap(l[0], l[1]);
+  const int stage = std::min(best.passes == 3 && logn <= 22 ? 10 : 11, logn + ilog2((uint64_t)rows) - 8);
+  int rest = logn;
+  for (int i = 0; i < best.passes; i++) {
+    rest -= l[i];
+    const int cols = i + 1 < best.passes ? rest : l[0];  // neighbouring sub-transforms
+    best.logB[i] = std::min(cols, std::max(stage - l[i], logn >= 18 ? 1 : 0));
+  }
+  return best;
+}
+}  // namespace
+
 void ntt_tables_build(NttTables &t, int logn) {
-  ensure_wq();
+  ensure_stages();
   t.logn = logn;
-  t.sub_fwd = g_wq[0];
-  t.sub_inv = g_wq[1];
+  t.sub_fwd = g_stages[0];
+  t.sub_inv = g_stages[1];
   t.inv_len = finv(fe_make(1ull << logn, 0));
   const uint64_t L = 1ull << logn;
   const int nlo = 1 << kTwLoBits;
@@ -705,10 +750,21 @@ void ntt_tables_build(NttTables &t, int logn) {
     GBZ_CUDA(cudaMemcpy(*plo, lo.data(), sizeof(fe) * nlo, cudaMemcpyHostToDevice));
     GBZ_CUDA(cudaMemcpy(*phi, hi.data(), sizeof(fe) * nhi, cudaMemcpyHostToDevice));
   }
-  if (logn > kSubLog) outer_table_build(logn, ntt_get_shape(logn).k1);
+  if (logn > kSubLog) {
+    if (g_shape[logn].k1 > 0) outer_table_build(logn, g_shape[logn].k1);
+    const Schedule sc = schedule(logn);
+    int rest = logn;
+    for (int i = 0; i + 1 < sc.passes; i++) {
+      outer_table_build(rest, (rest - sc.log[i]) + kScheduleTable);
+      rest -= sc.log[i];
+    }
+  }
 }
 
-int ntt_launch_count(int logn) { return logn <= kSubLog ? 1 : 2; }
+int ntt_launch_count(int logn) {
+  if (logn <= kSubLog) return 1;
+  return g_shape[logn].k1 > 0 ? 2 : schedule(logn).passes;
+}
 
 NttShape ntt_default_shape(int logn) {
   NttShape sh;
@@ -738,6 +794,11 @@ NttShape ntt_get_shape(int logn) {
 
 void ntt_set_shape(int logn, const NttShape &sh) {
   if (!ntt_shape_valid(logn, sh)) throw ArgError("ntt shape: invalid split or staging for this length");
+  const NttShape d = ntt_default_shape(logn);
+  if (sh.k1 == d.k1 && sh.logBA == d.logBA && sh.logBB == d.logBB) {  // back to the default schedule
+    g_shape[logn] = NttShape{};
+    return;
+  }
   outer_table_build(logn, sh.k1);
   g_shape[logn] = sh;
 }
@@ -750,7 +811,7 @@ std::vector<NttShape> ntt_shape_candidates(int logn) {
     for (int a = 0; a <= std::min(k1, kSubLog - k2); a++)
       for (int b = 0; b <= std::min(k2, kSubLog - k1); b++) {
         NttShape sh{k1, a, b};
-        if ((a == 0 && k2 < kSubLog) || a > 4 || b > 3) continue;  // keep sector-sized column groups
+        if (a > 4 || b > 3) continue;
         if (ntt_shape_valid(logn, sh)) out.push_back(sh);
       }
   }
@@ -777,12 +838,12 @@ struct PassGate {
   const uint32_t *run_if = nullptr;
 };
 
-void ntt_two_pass(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe *tmp, bool inverse,
+void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe *tmp, bool inverse,
                   cudaStream_t s, int rows = 1, uint64_t row_in = 0, uint64_t row_out = 0,
                   const PassGate &gate = PassGate(), uint64_t out_elem_stride = 1) {
   const int logn = t.logn;
   const uint64_t L = 1ull << logn;
-  if (logn > kMaxNttLogN) throw ArgError("transform longer than 2^26 (two passes of at most 2^13)");
+  if (logn > kMaxNttLogN) throw ArgError("transform longer than 2^26");
   if (gate.pack_real && (logn < 1 || rows != 1)) throw ArgError("packed real transform: one row, length >= 2");
   if (n_valid > L) n_valid = L;
   PassArgs a{};
@@ -791,7 +852,7 @@ void ntt_two_pass(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, f
   a.run_if = gate.run_if;
   a.row_in = row_in;
   a.row_out = row_out;
-  a.wh = inverse ? t.sub_inv : t.sub_fwd;
+  a.stages = inverse ? t.sub_inv : t.sub_fwd;
   a.scale = t.inv_len;
   a.inverse = inverse ? 1 : 0;
   a.j_valid = 1u << kSubLog;
@@ -811,55 +872,71 @@ void ntt_two_pass(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, f
     launch_pass(a, 1, s, rows);
     return;
   }
-  const NttShape sh = g_shape[logn].k1 > 0 ? g_shape[logn] : ntt_default_shape(logn);
-  const int k1 = sh.k1;       // pass B (contiguous rows)
-  const int k2 = logn - k1;   // pass A (strided columns)
-  const uint64_t N1 = 1ull << k1, N2 = 1ull << k2;
-  // pass A: columns n1 < N1, length N2, stride N1
-  a.in = in;
-  a.out = tmp;
-  a.n_valid = n_valid;
-  a.in_gstride = 1;
-  a.in_jstride = N1;
-  a.out_gstride = 1;
-  a.out_kstride = N1;
-  a.logS = k2;
-  // Strided pass: at least two neighbouring columns per CTA (whole 32-byte
-  // sectors) and up to 2^13 staged elements, fewer when the transform is
-  // small so that it still spreads over many CTAs.
-  a.logB = sh.logBA;
-  a.tw_lo = inverse ? t.lo_inv : t.lo_fwd;
-  a.tw_hi = inverse ? t.hi_inv : t.hi_fwd;
-  a.tw_full = g_use_outer ? outer_table_get(logn, k1, inverse) : nullptr;
-  a.has_scale = 0;
-  a.row_out = L;  // the intermediate holds one full row per transform
-  launch_pass(a, N1, s, rows);
-  // pass B: rows k2 < N2, length N1, contiguous
+  Schedule sc;
+  const bool set = g_shape[logn].k1 > 0;
+  if (set) {
+    const NttShape sh = g_shape[logn];
+    sc = Schedule{2, {logn - sh.k1, sh.k1, 0}, {sh.logBA, sh.logBB, 0}};
+  } else {
+    sc = schedule(logn, rows);
+  }
+  // Pass i transforms the columns of what is left of the length, 2^rest: for
+  // each of the 2^done blocks that earlier passes made, columns l < C = 2^rest
+  // / S at stride C, times omega_{2^rest}^{l k}, in place.  The last pass
+  // transforms contiguous rows; its outputs go to natural order.
+  int done = 0, rest = logn;
+  for (int i = 0; i + 1 < sc.passes; i++) {
+    const int lc = rest - sc.log[i];
+    const uint64_t C = 1ull << lc;
+    PassArgs b = a;
+    b.pack_real = i == 0 ? gate.pack_real : 0;  // only the first pass reads the input
+    b.in = i == 0 ? in : tmp;
+    b.row_in = i == 0 ? row_in : L;
+    b.n_valid = i == 0 ? n_valid : ~0ull;
+    b.out = tmp;
+    b.row_out = L;  // the intermediate holds one full row per transform
+    b.in_gstride = b.out_gstride = 1;
+    b.in_hstride = b.out_hstride = 1ull << rest;
+    b.in_jstride = b.out_kstride = C;
+    b.logG = lc;
+    b.logS = sc.log[i];
+    b.logB = sc.logB[i];
+    b.tw_lo = inverse ? t.lo_inv : t.lo_fwd;
+    b.tw_hi = inverse ? t.hi_inv : t.hi_fwd;
+    b.tw_shift = done;
+    b.tw_full = g_use_outer ? outer_table_get(rest, lc + (set ? 0 : kScheduleTable), inverse) : nullptr;
+    launch_pass(b, L >> sc.log[i], s, rows);
+    done += sc.log[i];
+    rest = lc;
+  }
+  // Row (k0, k1) of the last pass starts at k0 2^(logn - log0) + k1 2^rest and
+  // its output k goes to k0 + 2^log0 k1 + 2^done k; neighbouring k0 are taken
+  // together, so that a CTA's outputs lie side by side.
   PassArgs b = a;
-  b.pack_real = 0;  // only the first pass reads the input
+  b.pack_real = 0;
   b.in = tmp;
+  b.row_in = L;
+  b.n_valid = ~0ull;
   b.out = out;
-  b.n_valid = L;
-  b.in_gstride = N1;
+  b.row_out = row_out;
+  b.logG = sc.log[0];
+  b.in_gstride = 1ull << (logn - sc.log[0]);
+  b.in_hstride = 1ull << rest;
   b.in_jstride = 1;
   b.out_gstride = out_elem_stride;
-  b.out_kstride = N2 * out_elem_stride;
-  b.logS = k1;
-  b.logB = sh.logBB;
-  b.tw_lo = nullptr;
-  b.tw_hi = nullptr;
-  b.tw_full = nullptr;
+  b.out_hstride = out_elem_stride << sc.log[0];
+  b.out_kstride = out_elem_stride << done;
+  b.logS = rest;
+  b.logB = sc.logB[sc.passes - 1];
   b.has_scale = inverse;
-  b.row_in = L;
-  b.row_out = row_out;
-  launch_pass(b, N2, s, rows);
+  launch_pass(b, L >> rest, s, rows);
 }
 
 }  // namespace
 
 void ntt_launch(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe *tmp, bool inverse,
                 cudaStream_t s) {
-  ntt_two_pass(t, in, n_valid, out, tmp, inverse, s);
+  ntt_passes(t, in, n_valid, out, tmp, inverse, s);
 }
 
 namespace {
@@ -903,14 +980,14 @@ void ntt_launch_real(const NttTables &t_half, const NttTables &t_full, const fe 
   PassGate g;
   g.pack_real = 1;
   g.nonreal = nonreal;
-  ntt_two_pass(t_half, in, n_valid / 2, Z, tmp, false, s, 1, 0, 0, g);
+  ntt_passes(t_half, in, n_valid / 2, Z, tmp, false, s, 1, 0, 0, g);
   const uint64_t threads = M / 2 + 1;
   real_unpack_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(Z, M, t_full.lo_fwd, t_full.hi_fwd, out);
   GBZ_CUDA(cudaGetLastError());
   // any imaginary word: the general transform replaces the result
   PassGate f;
   f.run_if = nonreal;
-  ntt_two_pass(t_full, in, n_valid, out, tmp, false, s, 1, 0, 0, f);
+  ntt_passes(t_full, in, n_valid, out, tmp, false, s, 1, 0, 0, f);
 }
 
 int ntt_launch_real_count(int logn) { return ntt_launch_count(logn - 1) + 1 + ntt_launch_count(logn); }
@@ -919,7 +996,7 @@ void ntt_launch_rows(const NttTables &t, const fe *in, uint64_t n_valid, uint64_
                      uint64_t out_stride, int rows, fe *tmp, bool inverse, cudaStream_t s, uint64_t out_elem_stride) {
   if (rows < 1) return;
   if (out_elem_stride < 1) throw ArgError("transform: output element stride >= 1");
-  ntt_two_pass(t, in, n_valid, out, tmp, inverse, s, rows, in_stride, out_stride, PassGate(), out_elem_stride);
+  ntt_passes(t, in, n_valid, out, tmp, inverse, s, rows, in_stride, out_stride, PassGate(), out_elem_stride);
 }
 
 void ntt_batched(const NttTables &t, const fe *in, uint64_t in_stride, uint32_t j_valid, fe *out, uint64_t count,
@@ -928,7 +1005,7 @@ void ntt_batched(const NttTables &t, const fe *in, uint64_t in_stride, uint32_t 
   if (logS > kSubLog) throw ArgError("batched transform longer than 2^13");
   if (!count) return;
   PassArgs a{};
-  a.wh = inverse ? t.sub_inv : t.sub_fwd;
+  a.stages = inverse ? t.sub_inv : t.sub_fwd;
   a.scale = t.inv_len;
   a.inverse = inverse ? 1 : 0;
   a.in = in;
@@ -963,7 +1040,7 @@ void ntt_batched_strided(const NttTables &t, const fe *in, uint64_t col_stride, 
   if (logS > kSubLog) throw ArgError("batched transform longer than 2^13");
   if (!count) return;
   PassArgs a{};
-  a.wh = inverse ? t.sub_inv : t.sub_fwd;
+  a.stages = inverse ? t.sub_inv : t.sub_fwd;
   a.scale = t.inv_len;
   a.inverse = inverse ? 1 : 0;
   a.in = in;
@@ -1008,7 +1085,7 @@ void ntt_sparse_accumulate(const NttTables &t, const int32_t *q, const fe *c, in
   sparse_chain_kernel<<<1, kMaxQueries, 0, s>>>(q, l, q_shift, (uint32_t)(N1 - 1), next, lead);
   GBZ_CUDA(cudaGetLastError());
   PassArgs b{};
-  b.wh = t.sub_fwd;
+  b.stages = t.sub_fwd;
   b.scale = t.inv_len;
   b.inverse = 0;
   b.j_valid = 1u << kSubLog;
