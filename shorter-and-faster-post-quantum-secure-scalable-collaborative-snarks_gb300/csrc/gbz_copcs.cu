@@ -58,10 +58,10 @@ multifold5_kernel(const fe *cw, uint64_t n, const fe *a, fe *out, const fe *inv_
 #pragma unroll
     for (int q = 0; q < D; q++) buf[q] = nb[q];
   }
-  fe acc = fe_zero();
+  facc acc = facc_zero();
 #pragma unroll
-  for (int q = 0; q < D; q++) acc = fadd(acc, fmul(a[q], buf[q]));
-  out[i] = fmul(acc, len_inv);
+  for (int q = 0; q < D; q++) facc_mul(acc, buf[q], a[q]);
+  out[i] = fmul(facc_value(acc), len_inv);
 }
 
 __global__ void powers_kernel(fe r, uint64_t n, fe *out) {
@@ -129,9 +129,9 @@ shares_kernel(const fe *v, const fe *fill, uint64_t groups, int N, int k, int kk
   for (int t = 0; t < k; t++) buf[t] = v[i * k + t];
   for (int t = k; t < kk; t++) buf[t] = fill ? fill[i * (kk - k) + (t - k)] : fe_zero();
   for (int j = 0; j < N; j++) {
-    fe acc = fe_zero();
-    for (int t = 0; t < kk; t++) acc = fadd(acc, fmul(smu[j * kk + t], buf[t]));
-    shares[(uint64_t)j * groups + i] = acc;
+    facc acc = facc_zero();
+    for (int t = 0; t < kk; t++) facc_mul(acc, buf[t], smu[j * kk + t]);
+    shares[(uint64_t)j * groups + i] = facc_value(acc);
   }
 }
 
@@ -144,10 +144,10 @@ __global__ void __launch_bounds__(kAggrCols * kAggrRows)
 aggregate_kernel(const fe *msgs, int N, uint64_t len, const fe *lambda, fe *out) {
   __shared__ fe red[kAggrRows][kAggrCols];
   const uint64_t i = (uint64_t)blockIdx.x * kAggrCols + threadIdx.x;
-  fe acc = fe_zero();
+  facc acc = facc_zero();
   if (i < len)
-    for (int p = threadIdx.y; p < N; p += kAggrRows) acc = fadd(acc, fmul(lambda[p], msgs[(uint64_t)p * len + i]));
-  red[threadIdx.y][threadIdx.x] = acc;
+    for (int p = threadIdx.y; p < N; p += kAggrRows) facc_mul(acc, msgs[(uint64_t)p * len + i], lambda[p]);
+  red[threadIdx.y][threadIdx.x] = facc_value(acc);
   __syncthreads();
   if (threadIdx.y == 0 && i < len) {
     fe s = red[0][threadIdx.x];
@@ -214,14 +214,14 @@ cophase1_partial_kernel(const fe *e1, const fe *e2, const fe *e3, const fe *e4, 
   const uint32_t k = blockIdx.y * Dc + (threadIdx.x & (Dc - 1));
   const uint64_t b0 = (uint64_t)blockIdx.x * blocks_per_cta;
   const uint64_t b1 = min(b0 + blocks_per_cta, nblocks);
-  fe acc = fe_zero();
+  facc sum = facc_zero();
   for (uint64_t b = b0 + lane; b < b1; b += lanes) {
     if (flags && !flags[b]) continue;
     const uint64_t at = (b << logD) + k;
-    fe t = fmul(e1[at], e2[at]);
-    if (e3) t = fmul(fsub(t, e4[at]), e3[at]);
-    acc = fadd(acc, t);
+    if (e3) facc_mul(sum, fsub(fmul(e1[at], e2[at]), e4[at]), e3[at]);
+    else facc_mul(sum, e1[at], e2[at]);
   }
+  fe acc = facc_value(sum);
   red[threadIdx.x] = acc;
   __syncthreads();
   if (lane == 0) {
@@ -247,17 +247,32 @@ __global__ void sum_partials_kernel(const fe *partial, uint64_t nparts, uint32_t
   if (lane == 0) H[(uint64_t)blockIdx.y * D + k] = acc;
 }
 
-// coSumcheck phase 2: out[j] = sum_k L[k] v[j d + k].
+// coSumcheck phase 2: out[j] = sum_k L[k] v[j d + k].  2^LOGW neighbouring
+// lanes share an output and read consecutive entries of its block (whole
+// lines; one thread per output walked a block of its own, a line a lane and
+// step): 2^24 entries by 128 78 us, then 63; 1024 outputs of 1024 entries 38
+// us, then 3.
+template <int LOGW>
 __global__ void __launch_bounds__(256) cophase2_kernel(const fe *v, uint64_t nout, const fe *L, int logd, fe *out) {
   __shared__ fe sl[1024];
-  const uint32_t d = 1u << logd;
+  const uint32_t d = 1u << logd, lane = threadIdx.x & ((1u << LOGW) - 1);
   for (uint32_t k = threadIdx.x; k < d; k += blockDim.x) sl[k] = L[k];
   __syncthreads();
-  const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nout) return;
-  fe acc = fe_zero();
-  for (uint32_t k = 0; k < d; k++) acc = fadd(acc, fmul(sl[k], v[(j << logd) + k]));
-  out[j] = acc;
+  const uint64_t j = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> LOGW;
+  facc acc = facc_zero();
+  if (j < nout) {
+#pragma unroll 4
+    for (uint32_t k = lane; k < d; k += 1u << LOGW) facc_mul(acc, v[(j << logd) + k], sl[k]);
+  }
+  fe x = facc_value(acc);
+#pragma unroll
+  for (int s = 1; s < (1 << LOGW); s <<= 1) {
+    // eight canonical words fit 64 bits
+    x.re += __shfl_xor_sync(0xffffffffu, x.re, s);
+    x.im += __shfl_xor_sync(0xffffffffu, x.im, s);
+    if (s == 4 || 2 * s == (1 << LOGW)) x = fe_make(canon64(fold64(x.re)), canon64(fold64(x.im)));
+  }
+  if (j < nout && lane == 0) out[j] = x;
 }
 
 unsigned grid(uint64_t n, unsigned t = 256) { return (unsigned)((n + t - 1) / t); }
@@ -431,7 +446,13 @@ void cophase1_reduce_launch(const fe *e1, const fe *e2, const fe *e3, const fe *
 
 void cophase2_launch(const fe *v, uint64_t n, const fe *L, int logd, fe *out, cudaStream_t s) {
   if (logd > 10) throw ArgError("coSumcheck phase 2: block longer than 1024");
-  cophase2_kernel<<<grid(n >> logd), 256, 0, s>>>(v, n >> logd, L, logd, out);
+  const uint64_t nout = n >> logd;
+  // eight lanes an output; a warp where that leaves SMs without work (1024
+  // outputs of 1024 entries: 38 us with one lane, 3 with 32); blocks below
+  // eight entries have no work for more lanes
+  if (logd < 3) cophase2_kernel<0><<<grid(nout), 256, 0, s>>>(v, nout, L, logd, out);
+  else if (logd < 5 || nout >= (1u << 14)) cophase2_kernel<3><<<grid(nout << 3), 256, 0, s>>>(v, nout, L, logd, out);
+  else cophase2_kernel<5><<<grid(nout << 5), 256, 0, s>>>(v, nout, L, logd, out);
   GBZ_CUDA(cudaGetLastError());
 }
 

@@ -219,9 +219,10 @@ __global__ void k_rowsum(const fe *rows, int nrows, uint64_t len, const fe *w, f
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= len) return;
   const fe *r = rows + (uint64_t)blockIdx.y * nrows * len + k;
-  fe acc = fe_zero();
-  for (int h = 0; h < nrows; h++) acc = fadd(acc, fmul(w[h], r[(uint64_t)h * len]));
-  out[(uint64_t)blockIdx.y * len + k] = acc;
+  facc acc = facc_zero();
+#pragma unroll 4
+  for (int h = 0; h < nrows; h++) facc_mul(acc, r[(uint64_t)h * len], w[h]);
+  out[(uint64_t)blockIdx.y * len + k] = facc_value(acc);
 }
 
 // The row-batched global codeword from every party's codeword rows (party
@@ -233,9 +234,10 @@ __global__ void k_rowsum_global(const fe *cw, int nrows, uint64_t L, int N, cons
   const int r = blockIdx.y;
   const uint64_t blk = L / N, m = i / blk, j = i % blk;
   const fe *src = cw + (uint64_t)r * nrows * L + i;
-  fe acc = fe_zero();
-  for (int h = 0; h < nrows; h++) acc = fadd(acc, fmul(w[h], src[(uint64_t)h * L]));
-  X[r * blk + j + m * L] = acc;
+  facc acc = facc_zero();
+#pragma unroll 4
+  for (int h = 0; h < nrows; h++) facc_mul(acc, src[(uint64_t)h * L], w[h]);
+  X[r * blk + j + m * L] = facc_value(acc);
 }
 
 // One CTA per (i, j != i, party): sum_k b2_j[k] cdb_i[p][k] (the local
@@ -245,9 +247,10 @@ __global__ void k_cross_dots(const fe *cdb, const fe *b2, uint64_t S, int P, int
   const int p = blockIdx.x % N, pair = blockIdx.x / N;
   const int i = pair / (P - 1), jj = pair % (P - 1), j = jj < i ? jj : jj + 1;
   const fe *a = cdb + ((uint64_t)i * N + p) * S, *b = b2 + (uint64_t)j * S;
-  fe acc = fe_zero();
-  for (uint64_t k = threadIdx.x; k < S; k += blockDim.x) acc = fadd(acc, fmul(a[k], b[k]));
-  red[threadIdx.x] = acc;
+  facc acc = facc_zero();
+#pragma unroll 4
+  for (uint64_t k = threadIdx.x; k < S; k += blockDim.x) facc_mul(acc, a[k], b[k]);
+  red[threadIdx.x] = facc_value(acc);
   __syncthreads();
   for (int s = 128; s > 0; s >>= 1) {
     if (threadIdx.x < s) red[threadIdx.x] = fadd(red[threadIdx.x], red[threadIdx.x + s]);
@@ -263,23 +266,22 @@ __global__ void k_batch_vectors(const fe *cdb, const fe *b2, uint64_t S, int P, 
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= S) return;
   const int p = blockIdx.y;
-  const fe w[3] = {fe_one(), w1, w2};
-  fe a = fe_zero(), bt = fe_zero();
+  fe a = cdb[(uint64_t)p * S + k];
+  facc bt = facc_zero();
   for (int l = 0; l < P; l++) {
-    a = fadd(a, fmul(w[l], cdb[((uint64_t)l * N + p) * S + k]));
-    bt = fadd(bt, fmul(v[l * N + p], b2[(uint64_t)l * S + k]));
+    if (l > 0) a = fadd(a, fmul(cdb[((uint64_t)l * N + p) * S + k], l == 1 ? w1 : w2));
+    facc_mul(bt, b2[(uint64_t)l * S + k], v[l * N + p]);
   }
   arr[(uint64_t)p * S + k] = a;
-  betas[(uint64_t)p * S + k] = bt;
+  betas[(uint64_t)p * S + k] = facc_value(bt);
 }
 
 // X = sum_l w[l] Xl[l] over n entries.
 __global__ void k_combine3(const fe *Xl, uint64_t n, int P, fe w1, fe w2, fe *X) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const fe w[3] = {fe_one(), w1, w2};
-  fe acc = fe_zero();
-  for (int l = 0; l < P; l++) acc = fadd(acc, fmul(w[l], Xl[(uint64_t)l * n + i]));
+  fe acc = Xl[i];
+  for (int l = 1; l < P; l++) acc = fadd(acc, fmul(Xl[(uint64_t)l * n + i], l == 1 ? w1 : w2));
   X[i] = acc;
 }
 

@@ -171,10 +171,10 @@ __device__ __forceinline__ uint64_t dot_fold(const dot_cols &s) {
       : "r"(tl), "r"(th >> 29), "r"(th & 0x1fffffffu));
   return words64(ol, oh);
 }
-// S mod p in [0, p): t < 5 p has the quotient floor((t + floor(t / 2^61) + 1) / 2^61).
-__device__ __forceinline__ uint64_t dot_canon(const dot_cols &s) {
-  uint32_t tl, th, qh, ol, oh;
-  dot_wrap(s, tl, th);
+// t mod p in [0, p) for t < 2^64 - 16, in two words: the quotient is
+// floor((t + floor(t / 2^61) + 1) / 2^61).
+__device__ __forceinline__ uint64_t canon_words(uint32_t tl, uint32_t th) {
+  uint32_t qh, ol, oh;
   asm("{\n\t"
       ".reg .u32 t;\n\t"
       "add.cc.u32 t, %1, %2;\n\t"
@@ -185,12 +185,78 @@ __device__ __forceinline__ uint64_t dot_canon(const dot_cols &s) {
   asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, %4, 0;" : "=r"(ol), "=r"(oh) : "r"(tl), "r"(qh >> 29), "r"(th));
   return words64(ol, oh & 0x1fffffffu);
 }
-// The product with each component only folded to [0, p + 4]: a's words below
-// 2^62, b's at most p.
-__device__ __forceinline__ fe fmul_fold(fe a, fe b) {
-  const uint64_t nb = b.im ^ P;  // p - b.im
-  return fe_make(dot_fold(dot2_cols(a.re, b.re, a.im, nb)), dot_fold(dot2_cols(a.re, b.im, a.im, b.re)));
+__device__ __forceinline__ uint64_t canon64(uint64_t t) { return canon_words((uint32_t)t, (uint32_t)(t >> 32)); }
+// S mod p in [0, p).
+__device__ __forceinline__ uint64_t dot_canon(const dot_cols &s) {
+  uint32_t tl, th;
+  dot_wrap(s, tl, th);
+  return canon_words(tl, th);
 }
+__device__ __forceinline__ uint64_t dot_wrap64(const dot_cols &s) {
+  uint32_t tl, th;
+  dot_wrap(s, tl, th);
+  return words64(tl, th);
+}
+// Products with lazy words.  a's words may be up to 2p (a difference below),
+// b's at most p.
+__device__ __forceinline__ dot_cols mul_re(fe a, fe b) { return dot2_cols(a.re, b.re, a.im, b.im ^ P); }  // p - b.im
+__device__ __forceinline__ dot_cols mul_im(fe a, fe b) { return dot2_cols(a.re, b.im, a.im, b.re); }
+// Each component folded to [0, p + 4].
+__device__ __forceinline__ fe fmul_fold(fe a, fe b) { return fe_make(dot_fold(mul_re(a, b)), dot_fold(mul_im(a, b))); }
+// a - b + p, words in [0, 2p], for words in [0, p].
+__device__ __forceinline__ fe fsub_lazy(fe a, fe b) { return fe_make(a.re + (b.re ^ P), a.im + (b.im ^ P)); }
+__device__ __forceinline__ fe fadd_lazy(fe a, fe b) { return fe_make(a.re + b.re, a.im + b.im); }
+// x0 + r (x1 - x0), canonical: x0 joins the wrapped sum.
+__device__ __forceinline__ fe ffold(fe x0, fe x1, fe r) {
+  const fe d = fsub_lazy(x1, x0);
+  return fe_make(canon64(dot_wrap64(mul_re(d, r)) + x0.re), canon64(dot_wrap64(mul_im(d, r)) + x0.im));
+}
+// The same for base-field x0, x1 (imaginary words zero).
+__device__ __forceinline__ fe ffold_base(uint64_t x0, uint64_t x1, fe r) {
+  const uint64_t d = x1 + (x0 ^ P);
+  return fe_make(canon64(dot_wrap64(dot1_cols(d, r.re)) + x0), dot_canon(dot1_cols(d, r.im)));
+}
+
+// A sum of products, each component 96 bits wide: a product is added after
+// the first wrap (below 2^63 + 2^61), so a term costs 34 instructions beside
+// its wide products instead of the 45 of a canonical product and a canonical
+// addition, and the reduction comes once at the end.  Up to 2^32 terms.
+struct facc {
+  uint32_t re[3], im[3];
+};
+__device__ __forceinline__ facc facc_zero() { return facc{{0, 0, 0}, {0, 0, 0}}; }
+__device__ __forceinline__ void acc96(uint32_t *w, const dot_cols &s) {
+  uint32_t tl, th;
+  dot_wrap(s, tl, th);
+  asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, 0;"
+      : "+r"(w[0]), "+r"(w[1]), "+r"(w[2])
+      : "r"(tl), "r"(th));
+}
+__device__ __forceinline__ void facc_mul(facc &s, fe a, fe b) {
+  acc96(s.re, mul_re(a, b));
+  acc96(s.im, mul_im(a, b));
+}
+__device__ __forceinline__ void facc_mul_base(facc &s, fe a, uint64_t c) {
+  acc96(s.re, dot1_cols(a.re, c));
+  acc96(s.im, dot1_cols(a.im, c));
+}
+__device__ __forceinline__ uint64_t canon96(const uint32_t *w) {
+  const uint64_t lo = words64(w[0], w[1]);  // 2^64 = 8 (mod p)
+  return canon64((lo & P) + (lo >> 61) + 8ull * w[2]);
+}
+__device__ __forceinline__ fe facc_value(const facc &s) { return fe_make(canon96(s.re), canon96(s.im)); }
+
+// The same sum in four registers instead of six (kernels with many of them):
+// each component folded after every term, ten instructions instead of three.
+struct facc64 {
+  uint64_t re, im;
+};
+__device__ __forceinline__ uint64_t fold64(uint64_t t) { return (t & P) + (t >> 61); }
+__device__ __forceinline__ void facc_mul(facc64 &s, fe a, fe b) {
+  s.re = fold64(s.re + dot_fold(mul_re(a, b)));
+  s.im = fold64(s.im + dot_fold(mul_im(a, b)));
+}
+__device__ __forceinline__ fe facc_value(const facc64 &s) { return fe_make(canon64(s.re), canon64(s.im)); }
 #endif
 
 // operator* (fieldElement.cpp:49-78).  Both forms combine the four 122-bit

@@ -102,9 +102,10 @@ __global__ void k_lincomb(const fe *rows, uint64_t pstride, uint64_t rstride, in
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= len) return;
   const fe *r = rows + blockIdx.y * pstride + j;
-  fe acc = fe_zero();
-  for (int i = 0; i < nrows; i++) acc = fadd(acc, fmul(coef[i], r[(uint64_t)i * rstride]));
-  out[blockIdx.y * ostride + j] = acc;
+  facc acc = facc_zero();
+#pragma unroll 4
+  for (int i = 0; i < nrows; i++) facc_mul(acc, r[(uint64_t)i * rstride], coef[i]);
+  out[blockIdx.y * ostride + j] = facc_value(acc);
 }
 
 // After the inverse transforms: bcd, cdl *= omega^{-j}; B = b2 omega^j b3'[p]
@@ -127,14 +128,14 @@ __global__ void __launch_bounds__(kRedThreads)
 k_first_partial(const fe *bcd, const fe *cdl, const fe *B, uint64_t Bs, fe *partial) {
   __shared__ fe ra[kRedThreads], rb[kRedThreads];
   const uint64_t base = blockIdx.y * Bs;
-  fe a = fe_zero(), b = fe_zero();
+  facc a = facc_zero(), b = facc_zero();
   for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < Bs; j += (uint64_t)gridDim.x * blockDim.x) {
     const fe x = bcd[base + j], y = cdl[base + j], w = B[base + j];
-    a = fadd(a, fmul(fsub(x, y), w));
-    b = fadd(b, fmul(y, w));
+    facc_mul(a, fsub_lazy(x, y), w);
+    facc_mul(b, y, w);
   }
-  ra[threadIdx.x] = a;
-  rb[threadIdx.x] = b;
+  ra[threadIdx.x] = facc_value(a);
+  rb[threadIdx.x] = facc_value(b);
   __syncthreads();
   for (int s = kRedThreads / 2; s > 0; s >>= 1) {
     if (threadIdx.x < s) {
@@ -193,13 +194,13 @@ __global__ void k_first_fold(fe *bcd, const fe *cdl, fe *B, fe *Cp, const fe *cw
                              uint64_t Bs, uint64_t L, const PcsDev *st) {
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= L) return;
-  const fe r = st->r_first, om = fsub(fe_one(), r);
+  const fe r = st->r_first;
   const uint64_t p = blockIdx.y;
-  Cp[p * L + j] = fadd(fmul(r, Cp[p * L + j]), fmul(om, cw_last[p * cw_pstride + j]));
+  Cp[p * L + j] = ffold(cw_last[p * cw_pstride + j], Cp[p * L + j], r);
   if (j < Bs) {
     const uint64_t at = p * Bs + j;
     B[at] = fmul(r, B[at]);
-    bcd[at] = fadd(fmul(r, bcd[at]), fmul(om, cdl[at]));
+    bcd[at] = ffold(cdl[at], bcd[at], r);
   }
 }
 
@@ -437,9 +438,10 @@ __global__ void k_fold_q(const fe *cw, uint64_t n, int logd, const fe *iQ, fe sc
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   const fe *c = cw + blockIdx.y * n;
-  fe acc = fe_zero();
-  for (int t = 0; t < (1 << logd); t++) acc = fadd(acc, fmul(c[i + t * m], iQ[i + t * m]));
-  out[blockIdx.y * ostride + i] = fmul(acc, scale);
+  facc acc = facc_zero();
+#pragma unroll 4
+  for (int t = 0; t < (1 << logd); t++) facc_mul(acc, c[i + t * m], iQ[i + t * m]);
+  out[blockIdx.y * ostride + i] = fmul(facc_value(acc), scale);
 }
 
 // F_ip's local inner product (MPI_utils.cpp:489-491) of every party:
@@ -455,14 +457,15 @@ k_fip_partial(const fe *rows, uint64_t pstride, int nrows, uint64_t len, const f
   __shared__ fe sr[32];
   if (threadIdx.x < 32) sr[threadIdx.x] = brow[threadIdx.x];
   __syncthreads();
-  fe acc = fe_zero();
+  facc acc = facc_zero();
   const fe *r = rows + blockIdx.y * pstride;
   for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < len; j += (uint64_t)gridDim.x * blockDim.x) {
-    fe c = fe_zero();
-    for (int i = 0; i < nrows; i++) c = fadd(c, fmul(r[(uint64_t)i * len + j], sr[i]));
-    acc = fadd(acc, fmul(c, bcol[j]));
+    facc c = facc_zero();
+#pragma unroll 4
+    for (int i = 0; i < nrows; i++) facc_mul(c, r[(uint64_t)i * len + j], sr[i]);
+    facc_mul(acc, facc_value(c), bcol[j]);
   }
-  red[threadIdx.x] = acc;
+  red[threadIdx.x] = facc_value(acc);
   __syncthreads();
   for (int s = kRedThreads / 2; s > 0; s >>= 1) {
     if (threadIdx.x < s) red[threadIdx.x] = fadd(red[threadIdx.x], red[threadIdx.x + s]);

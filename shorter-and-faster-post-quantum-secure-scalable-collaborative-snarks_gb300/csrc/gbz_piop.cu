@@ -204,12 +204,12 @@ __global__ void k_r1cs_rows(R1csView m, uint64_t nrows, const fe *beta1, const f
   fe acc = fe_zero();
   for (int t = 0; t < 3; t++) {
     if (!m.ptr[t]) continue;
-    fe s = fe_zero();
+    facc s = facc_zero();
     for (uint32_t e = m.ptr[t][g]; e < m.ptr[t][g + 1]; e++) {
       const uint32_t c = m.cols[t][e];
-      s = fadd(s, fmul(beta1[c & S1], beta2[c >> logS]));
+      facc_mul(s, beta1[c & S1], beta2[c >> logS]);
     }
-    acc = fadd(acc, fmul(m.w[t], s));
+    acc = fadd(acc, fmul(m.w[t], facc_value(s)));
   }
   out[g] = fmul(scale, acc);
 }
@@ -229,9 +229,9 @@ __global__ void k_reshare_segments(const fe *v, uint64_t rows, int N, const fe *
   const int p = blockIdx.y;
   const uint64_t q = s / per, i = s % per;
   const fe *src = v + q * rows + i * k;
-  fe acc = fe_zero();
-  for (int t = 0; t < k; t++) acc = fadd(acc, fmul(mu[p * kk + t], src[t]));
-  out[(uint64_t)p * pstride + (s / fill) * seg + s % fill] = acc;
+  facc acc = facc_zero();
+  for (int t = 0; t < k; t++) facc_mul(acc, src[t], mu[p * kk + t]);
+  out[(uint64_t)p * pstride + (s / fill) * seg + s % fill] = facc_value(acc);
 }
 
 // out[p ostride + off + j] = v[j] scal[p] for j < n.

@@ -17,6 +17,8 @@
 // a single bit of the result.
 #include "gbz_rounds.cuh"
 
+#include <type_traits>
+
 namespace gbz {
 
 namespace {
@@ -46,6 +48,7 @@ __device__ __forceinline__ fe fhalf(fe x) { return fe_make(halfp(x.re), halfp(x.
 // are the coefficient sums the reference forms pair by pair.
 template <int FORM>
 __device__ __forceinline__ void acc_to_coeffs(fe *acc) {
+  if (FORM == SC_QUADRATIC) acc[1] = fsub(fsub(acc[1], acc[0]), acc[2]);  // q(1) = q2 + q1 + q0
   if (FORM == SC_CUBIC) {
     const fe e_inf = acc[0], e1 = acc[1], em = acc[2], e0 = acc[3];
     acc[1] = fsub(fhalf(fadd(e1, em)), e0);     // c(1) + c(-1) = 2 (c2 + c0)
@@ -67,29 +70,49 @@ __device__ __forceinline__ void qlmul(const fe q[3], const Line &l, fe c[4]) {
   c[3] = fmul(q[2], l.b);
 }
 
+// The sums of a thread: 96-bit accumulators for the forms of plain products
+// (quadratic, cubic, quadruple), reduced once per thread; canonical sums for
+// the two weighted forms, whose coefficients are combined before they are
+// added.
+template <int FORM> struct Sums {
+  static constexpr bool kLazy = FORM == SC_QUADRATIC || FORM == SC_CUBIC || FORM == SC_QUADRUPLE;
+  typedef typename std::conditional<kLazy, facc, fe>::type type;
+};
+__device__ __forceinline__ void sum_zero(facc &s) { s = facc_zero(); }
+__device__ __forceinline__ void sum_zero(fe &s) { s = fe_zero(); }
+__device__ __forceinline__ fe sum_value(const facc &s) { return facc_value(s); }
+__device__ __forceinline__ fe sum_value(const fe &s) { return s; }
+
+// What each accumulator of a form holds: quadratic the leading coefficient,
+// the values at 1 and 0; cubic the leading coefficient, the values at 1, -1
+// and 0; the others the coefficients.  acc_to_coeffs turns a thread's sums
+// into coefficients.
 template <int FORM>
-__device__ __forceinline__ void accumulate(const Line *l, fe b, fe *acc) {
+__device__ __forceinline__ void accumulate(const Line *l, fe b, typename Sums<FORM>::type *acc) {
   fe q[3], c[4];
-  if (FORM == SC_QUADRATIC) {
-    lmul(l[0], l[1], q);
-    for (int k = 0; k < 3; k++) acc[k] = fadd(acc[k], q[k]);
-  } else if (FORM == SC_CUBIC) {
-    // leading coefficient, values at 1, -1 (b - a) and 0 (acc_to_coeffs)
-    const fe m0 = fsub(l[0].b, l[0].a), m1 = fsub(l[1].b, l[1].a), m2 = fsub(l[2].b, l[2].a);
-    acc[0] = fadd(acc[0], fmul(fmul(l[0].a, l[1].a), l[2].a));
-    acc[1] = fadd(acc[1], fmul(fmul(l[0].h, l[1].h), l[2].h));
-    acc[2] = fadd(acc[2], fmul(fmul(m0, m1), m2));
-    acc[3] = fadd(acc[3], fmul(fmul(l[0].b, l[1].b), l[2].b));
-  } else if (FORM == SC_QUADRUPLE) {
+  if constexpr (FORM == SC_QUADRATIC) {
+    facc_mul(acc[0], l[0].a, l[1].a);
+    facc_mul(acc[1], l[0].h, l[1].h);
+    facc_mul(acc[2], l[0].b, l[1].b);
+  } else if constexpr (FORM == SC_CUBIC) {
+    const fe m0 = fsub_lazy(l[0].b, l[0].a), m1 = fsub(l[1].b, l[1].a), m2 = fsub(l[2].b, l[2].a);
+    facc_mul(acc[0], fmul_fold(l[0].a, l[1].a), l[2].a);
+    facc_mul(acc[1], fmul_fold(l[0].h, l[1].h), l[2].h);
+    facc_mul(acc[2], fmul_fold(m0, m1), m2);
+    facc_mul(acc[3], fmul_fold(l[0].b, l[1].b), l[2].b);
+  } else if constexpr (FORM == SC_QUADRUPLE) {
     // ((l1 l2) l3) l4 as the reference multiplies them (polynomial.cpp:91-101)
     lmul(l[0], l[1], q);
     qlmul(q, l[2], c);
-    acc[0] = fadd(acc[0], fmul(c[0], l[3].a));
-    acc[1] = fadd(acc[1], fadd(fmul(c[1], l[3].a), fmul(c[0], l[3].b)));
-    acc[2] = fadd(acc[2], fadd(fmul(c[2], l[3].a), fmul(c[1], l[3].b)));
-    acc[3] = fadd(acc[3], fadd(fmul(c[3], l[3].a), fmul(c[2], l[3].b)));
-    acc[4] = fadd(acc[4], fmul(c[3], l[3].b));
-  } else if (FORM == SC_BATCH) {
+    facc_mul(acc[0], c[0], l[3].a);
+    facc_mul(acc[1], c[1], l[3].a);
+    facc_mul(acc[1], c[0], l[3].b);
+    facc_mul(acc[2], c[2], l[3].a);
+    facc_mul(acc[2], c[1], l[3].b);
+    facc_mul(acc[3], c[3], l[3].a);
+    facc_mul(acc[3], c[2], l[3].b);
+    facc_mul(acc[4], c[3], l[3].b);
+  } else if constexpr (FORM == SC_BATCH) {
     fe q2[3], qr[3];
     lmul(l[0], l[1], q);
     lmul(l[2], l[3], q2);
@@ -144,9 +167,9 @@ __device__ void block_sum(fe *x) {
 template <int FORM, int MODE>
 __global__ void __launch_bounds__(kThreads) form_step_kernel(RoundArgs a) {
   constexpr int NV = Form<FORM>::NV, NC = Form<FORM>::NC;
-  fe acc[NC];
+  typename Sums<FORM>::type sums[NC];
 #pragma unroll
-  for (int k = 0; k < NC; k++) acc[k] = fe_zero();
+  for (int k = 0; k < NC; k++) sum_zero(sums[k]);
   const fe r = MODE ? *a.r : fe_zero();
   const fe b = a.b ? *a.b : fe_zero();
   const uint64_t stride = (uint64_t)gridDim.x * kThreads;
@@ -162,7 +185,7 @@ __global__ void __launch_bounds__(kThreads) form_step_kernel(RoundArgs a) {
         }
         l[k] = line(lo, hi);
       }
-      accumulate<FORM>(l, b, acc);
+      accumulate<FORM>(l, b, sums);
     } else if (MODE == 1) {
       // every vector's four entries are loaded before any output is stored
       // (the stores could alias later loads, so the compiler would not
@@ -183,13 +206,12 @@ __global__ void __launch_bounds__(kThreads) form_step_kernel(RoundArgs a) {
           x2 = fmul(x2, a.scale[(4 * g + 2) >> a.scale_log]);
           x3 = fmul(x3, a.scale[(4 * g + 3) >> a.scale_log]);
         }
-        const fe f0 = fadd(x0, fmul(r, fsub(x1, x0)));
-        const fe f1 = fadd(x2, fmul(r, fsub(x3, x2)));
+        const fe f0 = ffold(x0, x1, r), f1 = ffold(x2, x3, r);
         a.out[k][2 * g] = f0;
         a.out[k][2 * g + 1] = f1;
         l[k] = line(f0, f1);
       }
-      accumulate<FORM>(l, b, acc);
+      accumulate<FORM>(l, b, sums);
     } else {
 #pragma unroll
       for (int k = 0; k < NV; k++) {
@@ -198,11 +220,14 @@ __global__ void __launch_bounds__(kThreads) form_step_kernel(RoundArgs a) {
           x0 = fmul(x0, a.scale[(2 * g) >> a.scale_log]);
           x1 = fmul(x1, a.scale[(2 * g + 1) >> a.scale_log]);
         }
-        a.out[k][g] = fadd(x0, fmul(r, fsub(x1, x0)));
+        a.out[k][g] = ffold(x0, x1, r);
       }
     }
   }
   if (MODE == 2) return;
+  fe acc[NC];
+#pragma unroll
+  for (int k = 0; k < NC; k++) acc[k] = sum_value(sums[k]);
   acc_to_coeffs<FORM>(acc);
   block_sum<NC>(acc);
   if (threadIdx.x == 0)
@@ -328,9 +353,9 @@ __global__ void __launch_bounds__(kTailThreads) form_tail_kernel(TailArgs t) {
   uint64_t cur = t.cur;
   int pp = 0;
   for (int i = t.i0; i < t.total; i++) {
-    fe acc[NC];
+    typename Sums<FORM>::type sums[NC];
 #pragma unroll
-    for (int k = 0; k < NC; k++) acc[k] = fe_zero();
+    for (int k = 0; k < NC; k++) sum_zero(sums[k]);
     const uint64_t pairs = cur / 4;
     for (uint64_t g = threadIdx.x; g < pairs; g += kTailThreads) {
       fe xs[NV][4];
@@ -341,14 +366,16 @@ __global__ void __launch_bounds__(kTailThreads) form_tail_kernel(TailArgs t) {
       Line l[NV];
 #pragma unroll
       for (int k = 0; k < NV; k++) {
-        const fe f0 = fadd(xs[k][0], fmul(r, fsub(xs[k][1], xs[k][0])));
-        const fe f1 = fadd(xs[k][2], fmul(r, fsub(xs[k][3], xs[k][2])));
+        const fe f0 = ffold(xs[k][0], xs[k][1], r), f1 = ffold(xs[k][2], xs[k][3], r);
         t.buf[pp][k][2 * g] = f0;
         t.buf[pp][k][2 * g + 1] = f1;
         l[k] = line(f0, f1);
       }
-      accumulate<FORM>(l, fe_zero(), acc);
+      accumulate<FORM>(l, fe_zero(), sums);
     }
+    fe acc[NC];
+#pragma unroll
+    for (int k = 0; k < NC; k++) acc[k] = sum_value(sums[k]);
     acc_to_coeffs<FORM>(acc);
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1)
@@ -410,23 +437,25 @@ __global__ void __launch_bounds__(kTailThreads) form_tail_drawn_kernel(DrawnTail
   if (threadIdx.x == 0) y = *t.y;
   int pp = 0;
   for (int i = t.i0; i < t.rounds; i++) {
-    fe acc[NC];
+    typename Sums<FORM>::type sums[NC];
 #pragma unroll
-    for (int k = 0; k < NC; k++) acc[k] = fe_zero();
+    for (int k = 0; k < NC; k++) sum_zero(sums[k]);
     const uint64_t pairs = t.n >> (i + 1);
     for (uint64_t g = threadIdx.x; g < pairs; g += kTailThreads) {
       Line l[NV];
 #pragma unroll
       for (int k = 0; k < NV; k++) {
         const fe *p = in[k] + 4 * g;
-        const fe f0 = fadd(p[0], fmul(r, fsub(p[1], p[0])));
-        const fe f1 = fadd(p[2], fmul(r, fsub(p[3], p[2])));
+        const fe f0 = ffold(p[0], p[1], r), f1 = ffold(p[2], p[3], r);
         t.buf[pp][k][2 * g] = f0;
         t.buf[pp][k][2 * g + 1] = f1;
         l[k] = line(f0, f1);
       }
-      accumulate<FORM>(l, fe_zero(), acc);
+      accumulate<FORM>(l, fe_zero(), sums);
     }
+    fe acc[NC];
+#pragma unroll
+    for (int k = 0; k < NC; k++) acc[k] = sum_value(sums[k]);
     acc_to_coeffs<FORM>(acc);
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1)

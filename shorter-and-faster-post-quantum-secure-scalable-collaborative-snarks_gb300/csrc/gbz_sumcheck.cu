@@ -54,21 +54,22 @@ __device__ void block_sum3(fe &x, fe &y, fe &z) {
   }
 }
 
-__device__ __forceinline__ void acc_pair(fe a0, fe a1, fe b0, fe b1, fe &A, fe &C, fe &D) {
-  A = fadd(A, fmul(fsub(a1, a0), fsub(b1, b0)));
-  C = fadd(C, fmul(a0, b0));
-  D = fadd(D, fmul(a1, b1));
+__device__ __forceinline__ void acc_pair(fe a0, fe a1, fe b0, fe b1, facc &A, facc &C, facc &D) {
+  facc_mul(A, fsub_lazy(a1, a0), fsub(b1, b0));
+  facc_mul(C, a0, b0);
+  facc_mul(D, a1, b1);
 }
 
 // partial[3*blk + {0,1,2}] = (sum A, sum C, sum D) of the block.
 __global__ void __launch_bounds__(kScThreads)
 sc_reduce_kernel(const fe *__restrict__ a, const fe *__restrict__ b, uint64_t pairs, fe *partial) {
-  fe A = fe_zero(), C = fe_zero(), D = fe_zero();
+  facc sA = facc_zero(), sC = facc_zero(), sD = facc_zero();
   const uint64_t stride = (uint64_t)gridDim.x * kScThreads;
   for (uint64_t j = (uint64_t)blockIdx.x * kScThreads + threadIdx.x; j < pairs; j += stride) {
     fe a0 = a[2 * j], a1 = a[2 * j + 1], b0 = b[2 * j], b1 = b[2 * j + 1];
-    acc_pair(a0, a1, b0, b1, A, C, D);
+    acc_pair(a0, a1, b0, b1, sA, sC, sD);
   }
+  fe A = facc_value(sA), C = facc_value(sC), D = facc_value(sD);
   block_sum3(A, C, D);
   if (threadIdx.x == 0) {
     partial[3 * blockIdx.x] = A;
@@ -83,23 +84,23 @@ __global__ void __launch_bounds__(kScThreads)
 sc_fold_kernel(const fe *__restrict__ a, const fe *__restrict__ b, uint64_t m, const fe *chal,
                fe *__restrict__ a2, fe *__restrict__ b2, int reduce, fe *partial) {
   const fe r = *chal;
-  fe A = fe_zero(), C = fe_zero(), D = fe_zero();
+  facc sA = facc_zero(), sC = facc_zero(), sD = facc_zero();
   const uint64_t stride = (uint64_t)gridDim.x * kScThreads;
   const uint64_t quads = m / 4;
   for (uint64_t t = (uint64_t)blockIdx.x * kScThreads + threadIdx.x; t < quads; t += stride) {
     fe x0 = a[4 * t], x1 = a[4 * t + 1], x2 = a[4 * t + 2], x3 = a[4 * t + 3];
     fe y0 = b[4 * t], y1 = b[4 * t + 1], y2 = b[4 * t + 2], y3 = b[4 * t + 3];
-    fe fa0 = fadd(fmul(r, fsub(x1, x0)), x0), fa1 = fadd(fmul(r, fsub(x3, x2)), x2);
-    fe fb0 = fadd(fmul(r, fsub(y1, y0)), y0), fb1 = fadd(fmul(r, fsub(y3, y2)), y2);
+    const fe fa0 = ffold(x0, x1, r), fa1 = ffold(x2, x3, r), fb0 = ffold(y0, y1, r), fb1 = ffold(y2, y3, r);
     a2[2 * t] = fa0; a2[2 * t + 1] = fa1;
     b2[2 * t] = fb0; b2[2 * t + 1] = fb1;
-    if (reduce) acc_pair(fa0, fa1, fb0, fb1, A, C, D);
+    if (reduce) acc_pair(fa0, fa1, fb0, fb1, sA, sC, sD);
   }
   if (m == 2 && blockIdx.x == 0 && threadIdx.x == 0) {  // fold to a single entry
     a2[0] = fadd(fmul(r, fsub(a[1], a[0])), a[0]);
     b2[0] = fadd(fmul(r, fsub(b[1], b[0])), b[0]);
   }
   if (!reduce) return;
+  fe A = facc_value(sA), C = facc_value(sC), D = facc_value(sD);
   block_sum3(A, C, D);
   if (threadIdx.x == 0) {
     partial[3 * blockIdx.x] = A;
@@ -114,7 +115,7 @@ sc_fold_kernel(const fe *__restrict__ a, const fe *__restrict__ b, uint64_t m, c
 // pairs to the first round's message, folds them by r0, adds the folded pair
 // to the second round's message and folds it by r1 into (a4, b4) of length
 // m/4.  One read of (a, b) instead of three passes.
-__global__ void __launch_bounds__(kScThreads)
+__global__ void __launch_bounds__(kScThreads, 2)
 sc_fold2_kernel(const fe *__restrict__ a, const fe *__restrict__ b, uint64_t m, const fe *chal0, const fe *chal1,
                 fe *__restrict__ a4, fe *__restrict__ b4, fe *partial0, fe *partial1, BStr bs) {
   const uint32_t pb = blockIdx.y;
@@ -127,20 +128,22 @@ sc_fold2_kernel(const fe *__restrict__ a, const fe *__restrict__ b, uint64_t m, 
   partial0 = badv(partial0, bs.s[6], pb);
   partial1 = badv(partial1, bs.s[7], pb);
   const fe r0 = *chal0, r1 = *chal1;
-  fe A0 = fe_zero(), C0 = fe_zero(), D0 = fe_zero(), A1 = fe_zero(), C1 = fe_zero(), D1 = fe_zero();
+  facc sA0 = facc_zero(), sC0 = facc_zero(), sD0 = facc_zero();
+  facc sA1 = facc_zero(), sC1 = facc_zero(), sD1 = facc_zero();
   const uint64_t stride = (uint64_t)gridDim.x * kScThreads;
   const uint64_t quads = m / 4;
   for (uint64_t t = (uint64_t)blockIdx.x * kScThreads + threadIdx.x; t < quads; t += stride) {
     const fe x0 = a[4 * t], x1 = a[4 * t + 1], x2 = a[4 * t + 2], x3 = a[4 * t + 3];
     const fe y0 = b[4 * t], y1 = b[4 * t + 1], y2 = b[4 * t + 2], y3 = b[4 * t + 3];
-    acc_pair(x0, x1, y0, y1, A0, C0, D0);
-    acc_pair(x2, x3, y2, y3, A0, C0, D0);
-    const fe fa0 = fadd(fmul(r0, fsub(x1, x0)), x0), fa1 = fadd(fmul(r0, fsub(x3, x2)), x2);
-    const fe fb0 = fadd(fmul(r0, fsub(y1, y0)), y0), fb1 = fadd(fmul(r0, fsub(y3, y2)), y2);
-    acc_pair(fa0, fa1, fb0, fb1, A1, C1, D1);
-    a4[t] = fadd(fmul(r1, fsub(fa1, fa0)), fa0);
-    b4[t] = fadd(fmul(r1, fsub(fb1, fb0)), fb0);
+    acc_pair(x0, x1, y0, y1, sA0, sC0, sD0);
+    acc_pair(x2, x3, y2, y3, sA0, sC0, sD0);
+    const fe fa0 = ffold(x0, x1, r0), fa1 = ffold(x2, x3, r0), fb0 = ffold(y0, y1, r0), fb1 = ffold(y2, y3, r0);
+    acc_pair(fa0, fa1, fb0, fb1, sA1, sC1, sD1);
+    a4[t] = ffold(fa0, fa1, r1);
+    b4[t] = ffold(fb0, fb1, r1);
   }
+  fe A0 = facc_value(sA0), C0 = facc_value(sC0), D0 = facc_value(sD0);
+  fe A1 = facc_value(sA1), C1 = facc_value(sC1), D1 = facc_value(sD1);
   block_sum3(A0, C0, D0);
   if (threadIdx.x == 0) {
     partial0[3 * blockIdx.x] = A0;
@@ -164,7 +167,7 @@ sc_fold2_kernel(const fe *__restrict__ a, const fe *__restrict__ b, uint64_t m, 
 // A = (e1 - e0)(S1 - S0), C = e0 S0, D = e1 S1 (e_x = eq1(c0, x)), and after
 // the fold by r0 the pair's b is lambda0 eq1(c1, x1) E2[t], lambda0 =
 // eq1(c0, r0); b4 = lambda0 lambda1 E2 (lambda1 = eq1(c1, r1)).
-__global__ void __launch_bounds__(kScThreads)
+__global__ void __launch_bounds__(kScThreads, 2)
 sc_fold2_eq_kernel(const fe *__restrict__ a, const fe *__restrict__ E2, uint64_t m, const fe *c, const fe *chal0,
                    const fe *chal1, fe *__restrict__ a4, fe *__restrict__ b4, fe *partial0, fe *partial1, BStr bs) {
   const uint32_t pb = blockIdx.y;
@@ -181,32 +184,37 @@ sc_fold2_eq_kernel(const fe *__restrict__ a, const fe *__restrict__ E2, uint64_t
   const fe e0 = fsub(fe_one(), c0), f0 = fsub(fe_one(), c1);
   const fe lam0 = fadd(fmul(r0, fsub(c0, e0)), e0), lam1 = fadd(fmul(r1, fsub(c1, f0)), f0);
   const fe lam = fmul(lam0, lam1);
-  fe S0 = fe_zero(), S1 = fe_zero(), T0 = fe_zero(), T1 = fe_zero();
+  facc sS0 = facc_zero(), sS1 = facc_zero(), sT0 = facc_zero(), sT1 = facc_zero();
   const uint64_t stride = (uint64_t)gridDim.x * kScThreads;
   const uint64_t quads = m / 4;
   for (uint64_t t = (uint64_t)blockIdx.x * kScThreads + threadIdx.x; t < quads; t += stride) {
     const fe x0 = a[4 * t], x1 = a[4 * t + 1], x2 = a[4 * t + 2], x3 = a[4 * t + 3];
     const fe E = E2[t];
-    const fe g0 = fmul(f0, E), g1 = fmul(c1, E);
+    const fe g0 = fmul_fold(f0, E), g1 = fmul_fold(c1, E);
     fe fa0, fa1;
     if (!(x0.im | x1.im | x2.im | x3.im)) {
       // base-field entries (the witness of the configurations): products
       // with a base-field factor need two of the four partial products
-      S0 = fadd(S0, fadd(fmul_base(g0, x0.re), fmul_base(g1, x2.re)));
-      S1 = fadd(S1, fadd(fmul_base(g0, x1.re), fmul_base(g1, x3.re)));
-      fa0 = fadd(fmul_base(r0, subp(x1.re, x0.re)), x0);
-      fa1 = fadd(fmul_base(r0, subp(x3.re, x2.re)), x2);
+      facc_mul_base(sS0, g0, x0.re);
+      facc_mul_base(sS0, g1, x2.re);
+      facc_mul_base(sS1, g0, x1.re);
+      facc_mul_base(sS1, g1, x3.re);
+      fa0 = ffold_base(x0.re, x1.re, r0);
+      fa1 = ffold_base(x2.re, x3.re, r0);
     } else {
-      S0 = fadd(S0, fadd(fmul(x0, g0), fmul(x2, g1)));
-      S1 = fadd(S1, fadd(fmul(x1, g0), fmul(x3, g1)));
-      fa0 = fadd(fmul(r0, fsub(x1, x0)), x0);
-      fa1 = fadd(fmul(r0, fsub(x3, x2)), x2);
+      facc_mul(sS0, g0, x0);
+      facc_mul(sS0, g1, x2);
+      facc_mul(sS1, g0, x1);
+      facc_mul(sS1, g1, x3);
+      fa0 = ffold(x0, x1, r0);
+      fa1 = ffold(x2, x3, r0);
     }
-    T0 = fadd(T0, fmul(fa0, E));
-    T1 = fadd(T1, fmul(fa1, E));
-    a4[t] = fadd(fmul(r1, fsub(fa1, fa0)), fa0);
+    facc_mul(sT0, fa0, E);
+    facc_mul(sT1, fa1, E);
+    a4[t] = ffold(fa0, fa1, r1);
     b4[t] = fmul(lam, E);
   }
+  fe S0 = facc_value(sS0), S1 = facc_value(sS1), T0 = facc_value(sT0), T1 = facc_value(sT1);
   fe Z = fe_zero();
   block_sum3(S0, S1, Z);
   if (threadIdx.x == 0) {
@@ -239,18 +247,19 @@ sc_eq_reduce_kernel(const fe *__restrict__ a, const fe *__restrict__ E, uint64_t
   a = badv(a, bs.s[0], pb);
   E = badv(E, bs.s[1], pb);
   partial = badv(partial, bs.s[2], pb);
-  fe S0 = fe_zero(), S1 = fe_zero(), Z = fe_zero();
+  facc sS0 = facc_zero(), sS1 = facc_zero();
   const uint64_t stride = (uint64_t)gridDim.x * kScThreads;
   for (uint64_t j = (uint64_t)blockIdx.x * kScThreads + threadIdx.x; j < pairs; j += stride) {
     const fe e = E[j], w0 = a[2 * j], w1 = a[2 * j + 1];
     if (!(w0.im | w1.im)) {  // base-field entries: two partial products each
-      S0 = fadd(S0, fmul_base(e, w0.re));
-      S1 = fadd(S1, fmul_base(e, w1.re));
+      facc_mul_base(sS0, e, w0.re);
+      facc_mul_base(sS1, e, w1.re);
     } else {
-      S0 = fadd(S0, fmul(w0, e));
-      S1 = fadd(S1, fmul(w1, e));
+      facc_mul(sS0, w0, e);
+      facc_mul(sS1, w1, e);
     }
   }
+  fe S0 = facc_value(sS0), S1 = facc_value(sS1), Z = fe_zero();
   block_sum3(S0, S1, Z);
   if (threadIdx.x == 0) {
     partial[3 * blockIdx.x] = S0;
@@ -272,7 +281,7 @@ sc_eq_fold_kernel(const fe *__restrict__ a, uint64_t m, const fe *chal, fe *__re
   E2 = badv(E2, bs.s[4], pb);
   partial = badv(partial, bs.s[5], pb);
   const fe r = *chal;
-  fe S0 = fe_zero(), S1 = fe_zero(), Z = fe_zero();
+  facc sS0 = facc_zero(), sS1 = facc_zero();
   const uint64_t stride = (uint64_t)gridDim.x * kScThreads;
   const uint64_t quads = m / 4;
   for (uint64_t t = (uint64_t)blockIdx.x * kScThreads + threadIdx.x; t < quads; t += stride) {
@@ -280,23 +289,24 @@ sc_eq_fold_kernel(const fe *__restrict__ a, uint64_t m, const fe *chal, fe *__re
     const fe e0 = E[2 * t], e1 = E[2 * t + 1];
     fe f0, f1;
     if (!(x0.im | x1.im | x2.im | x3.im)) {  // base-field entries (the first fold of the witness)
-      f0 = fadd(fmul_base(r, subp(x1.re, x0.re)), x0);
-      f1 = fadd(fmul_base(r, subp(x3.re, x2.re)), x2);
+      f0 = ffold_base(x0.re, x1.re, r);
+      f1 = ffold_base(x2.re, x3.re, r);
     } else {
-      f0 = fadd(fmul(r, fsub(x1, x0)), x0);
-      f1 = fadd(fmul(r, fsub(x3, x2)), x2);
+      f0 = ffold(x0, x1, r);
+      f1 = ffold(x2, x3, r);
     }
     a2[2 * t] = f0;
     a2[2 * t + 1] = f1;
     const fe e = fadd(e0, e1);
     if (reduce) {
       E2[t] = e;
-      S0 = fadd(S0, fmul(f0, e));
-      S1 = fadd(S1, fmul(f1, e));
+      facc_mul(sS0, f0, e);
+      facc_mul(sS1, f1, e);
     }
   }
   if (m == 2 && blockIdx.x == 0 && threadIdx.x == 0) a2[0] = fadd(fmul(r, fsub(a[1], a[0])), a[0]);
   if (!reduce) return;
+  fe S0 = facc_value(sS0), S1 = facc_value(sS1), Z = fe_zero();
   block_sum3(S0, S1, Z);
   if (threadIdx.x == 0) {
     partial[3 * blockIdx.x] = S0;
@@ -450,18 +460,20 @@ ub_kernel(fe *b, uint64_t nb, const ProofState *st, int l, const fe *pw, BStr bs
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  fe acc[kUbPer];
+  fe acc[kUbPer];  // sums of folded words, folded again after each
 #pragma unroll
   for (int k = 0; k < kUbPer; k++) acc[k] = fe_zero();
   for (int i = warp; i < l; i += kUbWarps) {
     const fe w = s_w[i];
-    fe d = fmul(s_start[i], pw[i * 32 + lane]);
+    fe d = fmul_fold(s_start[i], pw[i * 32 + lane]);
 #pragma unroll
     for (int k = 0; k < kUbPer; k++) {
-      acc[k] = fadd(acc[k], d);
-      d = fmul(d, w);
+      acc[k] = fe_make(fold64(acc[k].re + d.re), fold64(acc[k].im + d.im));
+      if (k + 1 < kUbPer) d = fmul_fold(d, w);
     }
   }
+#pragma unroll
+  for (int k = 0; k < kUbPer; k++) acc[k] = fe_make(canon64(acc[k].re), canon64(acc[k].im));
 #pragma unroll
   for (int k = 0; k < kUbPer; k++) part[warp][lane * kUbPer + k] = acc[k];
   __syncthreads();

@@ -3,6 +3,8 @@
 // vectors, each one streaming pass over HBM.
 #include "gbz_whir_aggr.cuh"
 
+#include <type_traits>
+
 namespace gbz {
 
 namespace {
@@ -24,18 +26,18 @@ __global__ void __launch_bounds__(kThreads) lincomb_kernel(VecList v, const fe *
   __syncthreads();
   const uint64_t stride = (uint64_t)gridDim.x * kThreads;
   for (uint64_t t = (uint64_t)blockIdx.x * kThreads + threadIdx.x; t < n; t += stride) {
-    fe s = acc ? out[t] : fe_zero();
-    for (int i = 0; i < k; i++) s = fadd(s, fmul(c[i], v.p[i][t]));
-    out[t] = s;
+    facc s = facc_zero();
+    for (int i = 0; i < k; i++) facc_mul(s, c[i], v.p[i][t]);
+    const fe x = facc_value(s);
+    out[t] = acc ? fadd(out[t], x) : x;
   }
 }
 
 // Per-CTA partial sums of the TA x TB inner products <a_i, b_j>.
 template <int TA, int TB>
-__global__ void __launch_bounds__(kThreads) multidot_kernel(VecList a, VecList b, uint64_t n, fe *partial) {
-  fe acc[TA * TB];
-#pragma unroll
-  for (int q = 0; q < TA * TB; q++) acc[q] = fe_zero();
+__global__ void __launch_bounds__(kThreads, 2) multidot_kernel(VecList a, VecList b, uint64_t n, fe *partial) {
+  // more than nine 96-bit accumulators would leave one CTA an SM
+  typename std::conditional<(TA * TB > 9), facc64, facc>::type acc[TA * TB] = {};
   const uint64_t stride = (uint64_t)gridDim.x * kThreads;
   for (uint64_t t = (uint64_t)blockIdx.x * kThreads + threadIdx.x; t < n; t += stride) {
     fe x[TA], y[TB];
@@ -46,13 +48,13 @@ __global__ void __launch_bounds__(kThreads) multidot_kernel(VecList a, VecList b
 #pragma unroll
     for (int i = 0; i < TA; i++)
 #pragma unroll
-      for (int j = 0; j < TB; j++) acc[i * TB + j] = fadd(acc[i * TB + j], fmul(x[i], y[j]));
+      for (int j = 0; j < TB; j++) facc_mul(acc[i * TB + j], x[i], y[j]);
   }
   __shared__ fe red[TA * TB][kThreads / 32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int q = 0; q < TA * TB; q++) {
-    fe s = acc[q];
+    fe s = facc_value(acc[q]);
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) s = fadd(s, shfl_down_fe(s, d));
     if (lane == 0) red[q][w] = s;
@@ -159,35 +161,36 @@ aggr_claims_pass_kernel(VecList a, const fe *elo, const fe *ehi, int h, uint64_t
   if (threadIdx.x < TC) sw[threadIdx.x] = bw[threadIdx.x];
   if (aw && threadIdx.x < TA) sw[TC + threadIdx.x] = aw[threadIdx.x];
   __syncthreads();
-  fe acc[TA * TC];
+  facc acc[TA * TC];
 #pragma unroll
-  for (int q = 0; q < TA * TC; q++) acc[q] = fe_zero();
+  for (int q = 0; q < TA * TC; q++) acc[q] = facc_zero();
   const uint64_t stride = (uint64_t)gridDim.x * kThreads, mask = lo_len - 1;
   for (uint64_t t = (uint64_t)blockIdx.x * kThreads + threadIdx.x; t < n; t += stride) {
     fe x[TA];
 #pragma unroll
     for (int i = 0; i < TA; i++) x[i] = a.p[i][t];
-    fe b = first ? fe_zero() : baggr[t];
+    facc bs = facc_zero();
 #pragma unroll
     for (int j = 0; j < TC; j++) {
-      const fe e = fmul(elo[j * lo_len + (t & mask)], ehi[j * hi_len + (t >> h)]);
-      b = fadd(b, fmul(sw[j], e));
+      const fe e = fmul_fold(elo[j * lo_len + (t & mask)], ehi[j * hi_len + (t >> h)]);
+      facc_mul(bs, e, sw[j]);
 #pragma unroll
-      for (int i = 0; i < TA; i++) acc[i * TC + j] = fadd(acc[i * TC + j], fmul(x[i], e));
+      for (int i = 0; i < TA; i++) facc_mul(acc[i * TC + j], e, x[i]);
     }
-    baggr[t] = b;
+    const fe b = facc_value(bs);
+    baggr[t] = first ? b : fadd(baggr[t], b);
     if (aw) {
-      fe v = fe_zero();
+      facc vs = facc_zero();
 #pragma unroll
-      for (int i = 0; i < TA; i++) v = fadd(v, fmul(sw[TC + i], x[i]));
-      arr[t] = v;
+      for (int i = 0; i < TA; i++) facc_mul(vs, x[i], sw[TC + i]);
+      arr[t] = facc_value(vs);
     }
   }
   __shared__ fe red[TA * TC][kThreads / 32];
   const int wq = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int q = 0; q < TA * TC; q++) {
-    fe sum = acc[q];
+    fe sum = facc_value(acc[q]);
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) sum = fadd(sum, shfl_down_fe(sum, d));
     if (lane == 0) red[q][wq] = sum;
