@@ -185,9 +185,10 @@ gbz_status gbz_serve(gbz_ctx *ctx, int count, const double *arrival_s, const uin
  * are the same either way. */
 gbz_status gbz_sched_set_grouping(gbz_ctx *ctx, int on);
 
-/* Frees the scheduler's cached slot plans and the scratch the N-party
+/* Frees the scheduler's cached slot plans, the scratch the N-party
  * calls (gbz_pcs_claim, gbz_pcs_open, gbz_pcs_open_full, gbz_cosumcheck)
- * keep per shape between calls; *cached_bytes (optional) gets the device
+ * keep per shape between calls and the buffers of the last freed commitment
+ * (kept for the next of the same sizes); *cached_bytes (optional) gets the device
  * bytes they held. */
 gbz_status gbz_sched_release(gbz_ctx *ctx, uint64_t *cached_bytes);
 

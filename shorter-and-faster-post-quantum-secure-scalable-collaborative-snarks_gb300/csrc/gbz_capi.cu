@@ -68,8 +68,8 @@ __global__ void geo_prep_kernel(ProofState *st, const int32_t *q, const fe *c, i
 // b[j] += sum_i c_i omega_N^{q_i j} for j < nb (host q, c), in chunks of at
 // most kMaxQueries terms, by the sparse transform or by direct sums.
 static void geometric_update(gbz_ctx *ctx, fe *db, uint64_t nb, const int32_t *hq, const fe *hc, int l, int logN) {
-  if (!ctx->st) GBZ_CUDA(cudaMalloc(&ctx->st, sizeof(ProofState)));
-  if (!ctx->ub_scratch) GBZ_CUDA(cudaMalloc(&ctx->ub_scratch, sizeof(fe) * kUpdateBetasScratch));
+  if (!ctx->st) GBZ_CUDA(device_malloc((void **)&ctx->st, sizeof(ProofState)));
+  if (!ctx->ub_scratch) GBZ_CUDA(device_malloc((void **)&ctx->ub_scratch, sizeof(fe) * kUpdateBetasScratch));
   for (int i0 = 0; i0 < l; i0 += kMaxQueries) {
     const int cnt = std::min(kMaxQueries, l - i0);
     int32_t *dq = (int32_t *)ctx->buf(98, 4ull * kMaxQueries);
@@ -154,6 +154,45 @@ void encode_rows_device(gbz_ctx *ctx, const fe *drows, int nrows, int logrow, in
 
 }  // namespace gbz_api
 
+namespace {
+std::mutex g_spare_mu;
+std::vector<std::weak_ptr<SpareBuffers>> g_spare;
+}  // namespace
+
+std::shared_ptr<SpareBuffers> make_spare_buffers(int device) {
+  std::shared_ptr<SpareBuffers> sp = std::make_shared<SpareBuffers>();
+  size_t fr = 0, tot = 0;
+  GBZ_CUDA(cudaMemGetInfo(&fr, &tot));
+  sp->device = device;
+  sp->limit = tot / 16;
+  std::lock_guard<std::mutex> lk(g_spare_mu);
+  g_spare.erase(std::remove_if(g_spare.begin(), g_spare.end(), [](const auto &w) { return w.expired(); }),
+                g_spare.end());
+  g_spare.push_back(sp);
+  return sp;
+}
+
+namespace gbz {
+
+void release_spare_buffers() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  std::lock_guard<std::mutex> lk(g_spare_mu);
+  for (auto &w : g_spare)
+    if (std::shared_ptr<SpareBuffers> sp = w.lock())
+      if (sp->device == dev) sp->release();
+}
+
+cudaError_t device_malloc(void **p, uint64_t bytes) {
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  release_spare_buffers();
+  return cudaMalloc(p, bytes);
+}
+
+}  // namespace gbz
+
 extern "C" {
 
 gbz_status gbz_create(gbz_ctx **out, int device) {
@@ -186,6 +225,7 @@ void gbz_destroy(gbz_ctx *ctx) {
     for (auto &kv : ctx->scratch) cudaFree(kv.second.first);
     for (auto &kv : ctx->pools)
       for (auto &e : kv.second) cudaFree(e.first);
+    if (ctx->spare) ctx->spare->release(true);
     cudaFree(ctx->st);
     cudaFree(ctx->ub_scratch);
     if (ctx->side.stream) {
@@ -241,7 +281,7 @@ void gbz_host_free(void *ptr) {
 gbz_status gbz_device_alloc(gbz_ctx *ctx, void **ptr, uint64_t bytes) {
   API_BEGIN(ctx)
   need(ptr, "ptr");
-  GBZ_CUDA(cudaMalloc(ptr, bytes ? bytes : 16));
+  GBZ_CUDA(device_malloc(ptr, bytes ? bytes : 16));
   API_END(ctx)
 }
 void gbz_device_free(gbz_ctx *ctx, void *ptr) {
@@ -472,8 +512,8 @@ gbz_status gbz_whir_update_betas(gbz_ctx *ctx, uint64_t *b, uint64_t nb, const i
   if (l && !queries) throw ArgError("null pointer: queries");
   check_pow2(N, "update_betas: N");
   if (ilog2(N) > kMaxLogN) throw ArgError("update_betas: N above 2^28");
-  if (!ctx->st) GBZ_CUDA(cudaMalloc(&ctx->st, sizeof(ProofState)));
-  if (!ctx->ub_scratch) GBZ_CUDA(cudaMalloc(&ctx->ub_scratch, sizeof(fe) * kUpdateBetasScratch));
+  if (!ctx->st) GBZ_CUDA(device_malloc((void **)&ctx->st, sizeof(ProofState)));
+  if (!ctx->ub_scratch) GBZ_CUDA(device_malloc((void **)&ctx->ub_scratch, sizeof(fe) * kUpdateBetasScratch));
   fe *db = dev_view(ctx, 0, (fe *)b, 16 * nb, mem, true);
   const int32_t *dq = dev_view(ctx, 1, queries, 4ull * (l ? l : 1), mem, true);
   ub_prep_kernel<<<1, 256, 0, ctx->stream>>>(ctx->st, dq, l, ilog2(N), fe_make(r[0], r[1]));
@@ -892,6 +932,7 @@ gbz_status gbz_sched_release(gbz_ctx *ctx, uint64_t *cached_bytes) {
       cudaFree(e.first);
     }
   ctx->pools.clear();
+  if (ctx->spare) bytes += ctx->spare->release();
   if (cached_bytes) *cached_bytes = bytes;
   API_END(ctx)
 }
@@ -1196,8 +1237,8 @@ gbz_status gbz_whir_batch_open(gbz_ctx *ctx, int k, const uint64_t *const *array
   }
   const uint64_t L0 = P.cw_len[0];
   const uint8_t *dlv = dev_view(ctx, 610, levels0, 32 * merkle_hashes(L0), mem, true);
-  if (!ctx->st) GBZ_CUDA(cudaMalloc(&ctx->st, sizeof(ProofState)));
-  if (!ctx->ub_scratch) GBZ_CUDA(cudaMalloc(&ctx->ub_scratch, sizeof(fe) * kUpdateBetasScratch));
+  if (!ctx->st) GBZ_CUDA(device_malloc((void **)&ctx->st, sizeof(ProofState)));
+  if (!ctx->ub_scratch) GBZ_CUDA(device_malloc((void **)&ctx->ub_scratch, sizeof(fe) * kUpdateBetasScratch));
   uint8_t *dtr = mem == GBZ_MEM_DEVICE ? transcript : (uint8_t *)ctx->buf(620, P.transcript_bytes);
   BatchResources R;
   R.s = ctx->stream;

@@ -84,6 +84,12 @@ struct ProofState {
   fe whw[kMaxWhirIter][kWhirLogK][3];
 };
 
+// cudaMalloc that, when the device is full, first gives back the commitment
+// buffers that contexts keep between calls (gbz_ctx.cuh) and tries again.
+cudaError_t device_malloc(void **p, uint64_t bytes);
+// Frees those buffers on the current device.
+void release_spare_buffers();
+
 // Error capture for the C-ABI.
 struct Err {
   int code = 0;

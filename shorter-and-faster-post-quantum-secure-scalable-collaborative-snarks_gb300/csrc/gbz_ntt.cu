@@ -561,7 +561,7 @@ void ensure_stages() {
         for (uint32_t k = 0; k < (1u << ns); k++, x = fmul(x, wr)) h[stage_table_offset(ns) + ((r - 1) << ns) + k] = x;
       }
     }
-    GBZ_CUDA(cudaMalloc(&g_stages[dir], sizeof(fe) * h.size()));
+    GBZ_CUDA(device_malloc((void **)&g_stages[dir], sizeof(fe) * h.size()));
     GBZ_CUDA(cudaMemcpy(g_stages[dir], h.data(), sizeof(fe) * h.size(), cudaMemcpyHostToDevice));
   }
   g_stages_device = dev;
@@ -636,7 +636,7 @@ void outer_table_build(int logn, int key_k1) {
     }
     const uint64_t L = 1ull << logn;
     fe *T = nullptr;
-    if (cudaMalloc(&T, sizeof(fe) * L) != cudaSuccess) {
+    if (device_malloc((void **)&T, sizeof(fe) * L) != cudaSuccess) {
       cudaGetLastError();  // no room: the pass keeps the two-level twiddles
       return;
     }
@@ -745,8 +745,8 @@ void ntt_tables_build(NttTables &t, int logn) {
     x = fe_one();
     for (uint64_t i = 0; i < nhi; i++) { hi[i] = x; x = fmul(x, w12); }
     fe **plo = dir ? &t.lo_inv : &t.lo_fwd, **phi = dir ? &t.hi_inv : &t.hi_fwd;
-    GBZ_CUDA(cudaMalloc(plo, sizeof(fe) * nlo));
-    GBZ_CUDA(cudaMalloc(phi, sizeof(fe) * nhi));
+    GBZ_CUDA(device_malloc((void **)plo, sizeof(fe) * nlo));
+    GBZ_CUDA(device_malloc((void **)phi, sizeof(fe) * nhi));
     GBZ_CUDA(cudaMemcpy(*plo, lo.data(), sizeof(fe) * nlo, cudaMemcpyHostToDevice));
     GBZ_CUDA(cudaMemcpy(*phi, hi.data(), sizeof(fe) * nhi, cudaMemcpyHostToDevice));
   }

@@ -11,6 +11,7 @@
 // runs on the device too, in one-CTA kernels, so an opening is a stream of
 // launches with no host round trip.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -919,21 +920,40 @@ struct gbz_pcs {
   fe *cw = nullptr;      // [N][batches][L] codewords
   uint8_t *levels = nullptr;  // [N][2L - 1] column-root trees of distributed_MT
   uint8_t *roots = nullptr;   // [N][32] party roots, then [N][32] the leader root each party derives
-  std::vector<void *> owned;
+  PcsBuffers buf;
+  // Where the buffers go at the end: kept for the committing context's next
+  // commitment when every call on them ran on its stream, else freed.
+  std::shared_ptr<SpareBuffers> spare;
+  mutable std::atomic<bool> keep{false};
+  mutable cudaStream_t stream = nullptr;
 
   ~gbz_pcs() {
     int prev = -1;
     cudaGetDevice(&prev);
     cudaSetDevice(device);
-    for (void *p : owned) cudaFree(p);
+    if (keep) spare->give(buf, stream);
+    else buf.free();
     if (prev >= 0) cudaSetDevice(prev);
   }
-  template <typename T>
-  T *alloc(uint64_t count) {
-    void *p = nullptr;
-    GBZ_CUDA(cudaMalloc(&p, std::max<uint64_t>(count * sizeof(T), 16)));
-    owned.push_back(p);
-    return (T *)p;
+  // cd, cw, levels, roots on the committing context's stream
+  void alloc(gbz_ctx *ctx, uint64_t ncd, uint64_t ncw, uint64_t nlevels, uint64_t nroots) {
+    if (!ctx->spare) ctx->spare = make_spare_buffers(ctx->device);
+    spare = ctx->spare;
+    stream = ctx->stream;
+    const uint64_t n[4] = {16 * ncd, 16 * ncw, nlevels, nroots};
+    for (int i = 0; i < 4; i++) buf.bytes[i] = std::max<uint64_t>(n[i], 16);
+    if (!spare->take(buf, stream))
+      for (int i = 0; i < 4; i++) GBZ_CUDA(device_malloc(&buf.p[i], buf.bytes[i]));
+    cd = (fe *)buf.p[0];
+    cw = (fe *)buf.p[1];
+    levels = (uint8_t *)buf.p[2];
+    roots = (uint8_t *)buf.p[3];
+  }
+  // Called by every entry point that puts work on these buffers.  A context's
+  // stream only changes after a synchronisation (gbz_set_stream).
+  void used_by(const gbz_ctx *ctx) const {
+    if (ctx->spare == spare) stream = ctx->stream;
+    else keep = false;
   }
 };
 
@@ -1300,10 +1320,7 @@ gbz_status gbz_pcs_commit(gbz_ctx *ctx, int N, uint64_t M, int rounds, const int
   // inputs on the device
   const fe *dsh = dev_view(ctx, 0, (const fe *)shares, 16 * S * N, mem, true);
   const fe *drn = dev_view(ctx, 1, (const fe *)random, 16 * R * N, mem, true);
-  pc->cd = pc->alloc<fe>((uint64_t)N * nb * Bs);
-  pc->cw = pc->alloc<fe>((uint64_t)N * nb * L);
-  pc->levels = pc->alloc<uint8_t>(32ull * N * (2 * L - 1));
-  pc->roots = pc->alloc<uint8_t>(64ull * N);
+  pc->alloc(ctx, (uint64_t)N * nb * Bs, (uint64_t)N * nb * L, 32ull * N * (2 * L - 1), 64ull * N);
   // prepare_data: the rows of every party as 2-D copies (height = parties)
   GBZ_CUDA(cudaMemsetAsync(pc->cd, 0, 16ull * N * nb * Bs, s));
   for (const Run &r : runs) {
@@ -1328,6 +1345,7 @@ gbz_status gbz_pcs_commit(gbz_ctx *ctx, int N, uint64_t M, int rounds, const int
     GBZ_CUDA(cudaMemcpyAsync(leader_root, pc->roots + 32ull * N, 32, k, s));
   }
   GBZ_CUDA(cudaStreamSynchronize(s));  // the staged inputs are scratch of the context
+  pc->keep = true;
   *out = pc.release();
   API_END(ctx)
 }
@@ -1356,6 +1374,7 @@ gbz_status gbz_pcs_commit_data(gbz_ctx *ctx, const gbz_pcs *pcs, int party, uint
   if (party < 0 || party >= pcs->sc.N) throw ArgError("pcs: party out of range");
   const cudaMemcpyKind k = mem == GBZ_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
   const uint64_t nb = pcs->batches, Bs = pcs->Bs, L = pcs->L;
+  pcs->used_by(ctx);
   if (rows) GBZ_CUDA(cudaMemcpyAsync(rows, pcs->cd + party * nb * Bs, 16 * nb * Bs, k, ctx->stream));
   if (codewords) GBZ_CUDA(cudaMemcpyAsync(codewords, pcs->cw + party * nb * L, 16 * nb * L, k, ctx->stream));
   if (levels)
@@ -1371,6 +1390,7 @@ gbz_status gbz_pcs_claim(gbz_ctx *ctx, const gbz_pcs *pcs, const uint64_t *r, in
   need(r, "r");
   need(K, "K");
   if (pcs->device != ctx->device) throw ArgError("pcs: committed on another device");
+  pcs->used_by(ctx);
   const int N = pcs->sc.N, nb = pcs->batches, lk = ilog2(N / 4), logBs = ilog2(pcs->Bs);
   if (nr != lk + 5 + logBs) throw ArgError("pcs: the point must have log2(N/4) + 5 + log2(row length) entries");
   cudaStream_t s = ctx->stream;
@@ -1426,6 +1446,7 @@ gbz_status gbz_pcs_claim_piop(gbz_ctx *ctx, const gbz_pcs *pcs, const uint64_t *
   need(b3, "b3");
   need(K, "K");
   if (pcs->device != ctx->device) throw ArgError("pcs: committed on another device");
+  pcs->used_by(ctx);
   const int N = pcs->sc.N, nb = pcs->batches;
   const uint64_t Bs = pcs->Bs, q0 = (uint64_t)pcs->sc.queries[0];
   if (nb1 < 0) throw ArgError("pcs: b1 length");
@@ -1474,6 +1495,7 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
   need(fs, "fs");
   need(transcript, "transcript");
   if (pcs->device != ctx->device) throw ArgError("pcs: committed on another device");
+  pcs->used_by(ctx);
   const PcsSchedule &sc = pcs->sc;
   const int N = sc.N, logN = ilog2(N), nb = pcs->batches;
   const uint64_t Bs = pcs->Bs, L = pcs->L;

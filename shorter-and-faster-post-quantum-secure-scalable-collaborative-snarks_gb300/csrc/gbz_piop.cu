@@ -432,8 +432,8 @@ gbz_status gbz_r1cs_create(gbz_ctx *ctx, int N, uint64_t rows, int logm, const u
         if (ptr[t][g + 1] < ptr[t][g]) throw ArgError("r1cs: row pointers must not decrease");
       for (uint64_t e = 0; e < nnz[t]; e++)
         if (cols[t][e] >= (1ull << logm)) throw ArgError("r1cs: a column is not below 2^logm");
-      GBZ_CUDA(cudaMalloc(&m->ptr[t], 4 * (total + 1)));
-      GBZ_CUDA(cudaMalloc(&m->cols[t], 4 * std::max<uint64_t>(nnz[t], 1)));
+      GBZ_CUDA(device_malloc((void **)&m->ptr[t], 4 * (total + 1)));
+      GBZ_CUDA(device_malloc((void **)&m->cols[t], 4 * std::max<uint64_t>(nnz[t], 1)));
       GBZ_CUDA(cudaMemcpy(m->ptr[t], ptr[t], 4 * (total + 1), cudaMemcpyHostToDevice));
       if (nnz[t]) GBZ_CUDA(cudaMemcpy(m->cols[t], cols[t], 4 * nnz[t], cudaMemcpyHostToDevice));
       m->nnz[t] = nnz[t];

@@ -659,7 +659,7 @@ ProofPlan::~ProofPlan() {
 
 void *ProofPlan::dalloc(uint64_t bytes) {
   void *p = nullptr;
-  GBZ_CUDA(cudaMalloc(&p, bytes ? bytes : 16));
+  GBZ_CUDA(device_malloc(&p, bytes ? bytes : 16));
   allocs.push_back(p);
   return p;
 }

@@ -154,6 +154,9 @@ SlotPlan &Scheduler::plan_for(int slot, int logn, int rate, const SchedOpts &o, 
     size_t fr = 0, tot = 0;
     GBZ_CUDA(cudaMemGetInfo(&fr, &tot));
     if (fr >= need) break;
+    release_spare_buffers();
+    GBZ_CUDA(cudaMemGetInfo(&fr, &tot));
+    if (fr >= need) break;
     if (evict_one_idle(slot, key)) continue;
     bool waited = false;
     for (auto &sl : slots_) {
@@ -270,7 +273,7 @@ void Scheduler::run(const std::vector<ProofJob> &jobs_in, const double *arrival,
     if (dev_errors_) GBZ_CUDA(cudaFree(dev_errors_));
     dev_errors_ = nullptr;
     dev_errors_cap_ = 0;
-    GBZ_CUDA(cudaMalloc(&dev_errors_, sizeof(uint32_t) * nj));
+    GBZ_CUDA(device_malloc((void **)&dev_errors_, sizeof(uint32_t) * nj));
     dev_errors_cap_ = nj;
   }
   for (int l = 0; l < lanes; l++) GBZ_CUDA(cudaStreamSynchronize(slots_[l].s));
