@@ -244,21 +244,32 @@ __device__ __forceinline__ fe pow_table(const fe *lo, const fe *hi, uint64_t e) 
   return fmul(lo[e & 4095u], hi[e >> 12]);
 }
 
+struct UbSlots;
+
+constexpr int kOpenThreads = 128;
+
+// One iteration of the opening on the query stream.
 struct QueryArgs {
   ProofState *st;
-  uint64_t cws, trs;     // per-proof strides of cw and tr in a batch (one CTA per proof)
-  const fe *cw;          // previous codeword
-  uint64_t L;            // its length
-  uint64_t NL;           // new codeword length
-  int l;                 // number of queries
+  uint64_t cws, ps, trs;  // per-proof strides of cw, the partials and tr in a batch (grid.y = proof)
+  const fe *cw;           // the codeword it opens
+  uint64_t L;             // its length
+  int l;                  // number of queries
+  const fe *partial0, *partial1;  // the two round messages' partials
+  int blocks;
   uint8_t *tr;
-  uint64_t off_q, off_rep, off_ans, off_path, off_comb, off_K;
-  // omega_L^{-e} and omega_NL^{e} tables, and per-iteration constants of
+  uint64_t off_poly[kWhirLogK], off_chal[kWhirLogK];
+  uint64_t off_root, off_q, off_rep, off_ans, off_path, off_comb, off_K;
+  const UbSlots *u;       // c_i at slot base + i
+  uint64_t us;
+  int base;
+  // omega_L^{-e} table, and the iteration's constants of
   // get_RS_multifold_segment_tensor for a segment of 4 (coPCS_utils.cpp:333-383)
-  const fe *inv_lo, *inv_hi, *new_lo, *new_hi;
+  const fe *inv_lo, *inv_hi;
   fe step0;    // (omega_L^{-1})^(L/4): advance of inv_omegas at level 0
   fe len_inv;  // 4^{-1}
 };
+
 
 
 // The WHIR randomness of a proof, drawn up front.  Every F::_random() and
@@ -338,103 +349,39 @@ __global__ void __launch_bounds__(256) k_whir_schedule(ProofState *st, SchedArgs
   }
 }
 
-// Preparation of an iteration's update_betas by the round kernel: scaled
-// queries 2 q_i, omega_NL^{2 q_i} and the weights c_i = r^(i+1).
-struct UbPrep {
-  int l;                 // 0: no preparation
-  const fe *lo, *hi;     // omega_NL^e
+// update_betas of every iteration, prepared up front from the drawn query
+// positions: entry base_t + i of an iteration's range holds 2 q_i,
+// omega_NL^{2 q_i}, c_i = r^(i+1) and 32 powers of the root.  The beta
+// updates sit on the chain of folds; with this on it they cost 2.4 us (the
+// powers) and 2 us (roots and weights) more per iteration.
+constexpr int kUbSlots = 1024;  // query slots of a proof (rate 2 at 2^25 uses 619)
+struct UbSlots {
+  fe pw[32 * kUbSlots];
+  fe w[kUbSlots], c[kUbSlots];
+  int32_t q2[kUbSlots];
 };
-// The two WHIR sumcheck rounds of iteration t from the partials of the fused
-// two-round pass, in one launch: each message is recorded (transcript and
-// st->whw for the query chain, which checks it against K) with its challenge
-// drawn up front, and the threads prepare the iteration's update_betas.
-__global__ void k_whir_rounds2_s(const fe *partial0, const fe *partial1, int blocks, ProofState *st, int t,
-                                 uint8_t *tr, uint64_t off_poly0, uint64_t off_chal0, uint64_t off_poly1,
-                                 uint64_t off_chal1, UbPrep u, uint64_t ps, uint64_t trs) {
-  partial0 = badv(partial0, ps, blockIdx.x);
-  partial1 = badv(partial1, ps, blockIdx.x);
-  st += blockIdx.x;
-  tr += trs * blockIdx.x;
-  fe H0[3], H1[3];
-  sum_partials(partial0, blocks, H0);
-  __syncthreads();  // sum_partials' shared scratch is reused
-  sum_partials(partial1, blocks, H1);
-  for (int j = threadIdx.x; j < u.l; j += blockDim.x) {
-    const uint32_t q2 = 2u * (uint32_t)st->wq[t][j];
-    st->q[j] = (int32_t)q2;
-    st->omega_q[j] = pow_table(u.lo, u.hi, q2);
-    st->comb[j] = fpow(st->wrb[t], (uint64_t)j + 1);
-  }
-  if (threadIdx.x) return;
-  for (int k = 0; k < 3; k++) {
-    put_fe(tr, off_poly0 + 16 * k, H0[k]);
-    st->whw[t][0][k] = H0[k];
-    put_fe(tr, off_poly1 + 16 * k, H1[k]);
-    st->whw[t][1][k] = H1[k];
-  }
-  put_fe(tr, off_chal0, st->wr[t][0]);
-  put_fe(tr, off_chal1, st->wr[t][1]);
-}
-
-// whir_query (Whir.cpp:251-314) of iteration t with the drawn positions, and
-// the running claim of whir_sumcheck and update_betas: K is checked against
-// both round messages (K == h(0) + h(1), K = h(r)), then K += sum_i c_i y_i
-// (Whir.cpp:383-384).  Thread i handles query i.
-__global__ void __launch_bounds__(kMaxQueries) k_whir_query_s(QueryArgs a, int t) {
-  __shared__ fe red[kMaxQueries / 32];
-  a.st += blockIdx.x;
-  a.cw = badv(a.cw, a.cws, blockIdx.x);
-  a.tr += a.trs * blockIdx.x;
-  ProofState *st = a.st;
-  const int i = threadIdx.x;
-  fe contrib = fe_zero();
-  if (i < a.l) {
-    const int32_t q = st->wq[t][i];
-    const uint64_t qi = (uint64_t)q;
-    reinterpret_cast<int32_t *>(a.tr + a.off_q)[i] = q;
-    fe seg[kWhirK];
-    for (int j = 0; j < kWhirK; j++) {
-      seg[j] = a.cw[qi + j * (a.L / kWhirK)];
-      put_fe(a.tr, a.off_rep + 16 * (kWhirK * i + j), seg[j]);
-    }
-    // get_RS_multifold_segment_tensor(seg, r, L, qi) with r = the two WHIR
-    // round challenges: level 0 pairs (j, j+2) with omega_L^{-(qi + j L/4)},
-    // level 1 pairs (0, 1) with omega_{L/2}^{-qi} = omega_L^{-2 qi}.
-    const fe one = fe_one(), r0 = st->wr[t][0], r1 = st->wr[t][1];
-    fe inv_om = pow_table(a.inv_lo, a.inv_hi, qi);
-    fe part[2];
-    for (int j = 0; j < 2; j++) {
-      fe s = fadd(seg[j], seg[j + 2]), d = fsub(seg[j], seg[j + 2]);
-      part[j] = fadd(fmul(fsub(one, r0), s), fmul(fmul(r0, inv_om), d));
-      inv_om = fmul(inv_om, a.step0);
-    }
-    fe po = pow_table(a.inv_lo, a.inv_hi, (2 * qi) & (a.L - 1));
-    fe s = fadd(part[0], part[1]), d = fsub(part[0], part[1]);
-    fe y = fmul(a.len_inv, fadd(fmul(fsub(one, r1), s), fmul(r1, fmul(po, d))));
-    put_fe(a.tr, a.off_ans + 16 * i, y);
-    const fe c = fpow(st->wrb[t], (uint64_t)i + 1);
-    put_fe(a.tr, a.off_comb + 16 * i, c);
-    contrib = fmul(c, y);
-  }
-  for (int dd = 16; dd > 0; dd >>= 1) {
-    fe v;
-    v.re = __shfl_down_sync(0xffffffffu, contrib.re, dd);
-    v.im = __shfl_down_sync(0xffffffffu, contrib.im, dd);
-    contrib = fadd(contrib, v);
-  }
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = contrib;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    fe K = st->K;
-    for (int r = 0; r < kWhirLogK; r++) {
-      const fe *h = st->whw[t][r];
-      const fe h01 = fadd(quad_eval(h[0], h[1], h[2], fe_zero()), quad_eval(h[0], h[1], h[2], fe_one()));
-      if (!fe_eq(h01, K)) atomicOr(&st->error, 2u);
-      K = quad_eval(h[0], h[1], h[2], st->wr[t][r]);
-    }
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) K = fadd(K, red[w]);
-    st->K = K;
-    put_fe(a.tr, a.off_K, K);
+static_assert(sizeof(UbSlots) <= sizeof(fe) * kUpdateBetasScratch, "update_betas scratch");
+struct UbPrepArgs {
+  int T;
+  int base[kMaxWhirIter + 1];  // first slot of the iterations; the end
+  int per[kMaxWhirIter];
+  const fe *lo[kMaxWhirIter], *hi[kMaxWhirIter];  // omega_NL^e
+};
+__global__ void __launch_bounds__(128) k_ub_prep(const ProofState *st, UbSlots *u, uint64_t us, UbPrepArgs a) {
+  st += blockIdx.y;
+  u = badv(u, us, blockIdx.y);
+  const int i = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;  // a warp per query
+  if (i >= a.base[a.T]) return;
+  int t = 0;
+  while (i >= a.base[t + 1]) t++;
+  const int j = i - a.base[t];
+  const uint32_t q2 = 2u * (uint32_t)st->wq[t][j];
+  const fe w = pow_table(a.lo[t], a.hi[t], q2);
+  u->pw[32 * i + lane] = fpow(w, (uint64_t)(lane * a.per[t]));
+  if (lane == 0) {
+    u->q2[i] = (int32_t)q2;
+    u->w[i] = w;
+    u->c[i] = fpow(st->wrb[t], (uint64_t)j + 1);
   }
 }
 
@@ -515,20 +462,116 @@ __global__ void k_merkle_root_b(const fe *cw, uint64_t cws, int depth, uint8_t *
 // Authentication paths of the l queries: entry d of query i is the sibling
 // (q >> d) ^ 1 of level d, i.e. G^d(leaf ((q >> d) ^ 1) << d).  One thread
 // per entry, the deepest entries first.
-__global__ void k_whir_paths_chain(const fe *cw, uint64_t leaves, int l, uint8_t *tr, uint64_t off_q,
-                                   uint64_t off_path, uint64_t cws, uint64_t trs) {
-  cw = badv(cw, cws, blockIdx.y);  // a batch: grid.y = proof
-  tr += trs * blockIdx.y;
-  const int depth = 63 - __clzll((long long)leaves);
-  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void path_entry(const fe *cw, int depth, int l, uint64_t t, uint8_t *tr, const int32_t *qs,
+                                           uint64_t off_path) {
   if (t >= (uint64_t)l * depth) return;
   const int d = depth - 1 - (int)(t / l), i = (int)(t % l);
-  const uint64_t q = (uint64_t)(uint32_t)reinterpret_cast<const int32_t *>(tr + off_q)[i];
+  const uint64_t q = (uint64_t)(uint32_t)qs[i];
   uint32_t h[8];
   leaf_hash(cw, ((q >> d) ^ 1ull) << d, h);
   for (int k = 0; k < d; k++) node_hash(h);
   put_hash(tr + off_path + 32ull * ((uint64_t)depth * i + d), h);
 }
+__global__ void k_whir_paths_chain(const fe *cw, uint64_t leaves, int l, uint8_t *tr, uint64_t off_q,
+                                   uint64_t off_path, uint64_t cws, uint64_t trs) {
+  cw = badv(cw, cws, blockIdx.y);  // a batch: grid.y = proof
+  tr += trs * blockIdx.y;
+  path_entry(cw, 63 - __clzll((long long)leaves), l, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, tr,
+             reinterpret_cast<const int32_t *>(tr + off_q), off_path);
+}
+
+namespace {
+
+// whir_query (Whir.cpp:251-314) of iteration t with the drawn positions, its
+// two round messages (recorded with their challenges), and the running claim
+// of whir_sumcheck and update_betas: K is checked against both messages
+// (K == h(0) + h(1), K = h(r)), then K += sum_i c_i y_i (Whir.cpp:383-384).
+__device__ void whir_query_dev(const QueryArgs &a, int t) {
+  __shared__ fe red[kOpenThreads / 32];
+  ProofState *st = a.st;
+  fe H[kWhirLogK][3];
+  sum_partials(a.partial0, a.blocks, H[0]);
+  __syncthreads();  // sum_partials' shared scratch is reused
+  sum_partials(a.partial1, a.blocks, H[1]);
+  const fe one = fe_one(), r0 = st->wr[t][0], r1 = st->wr[t][1];
+  fe contrib = fe_zero();
+  for (int i = threadIdx.x; i < a.l; i += kOpenThreads) {
+    const int32_t q = st->wq[t][i];
+    const uint64_t qi = (uint64_t)q;
+    reinterpret_cast<int32_t *>(a.tr + a.off_q)[i] = q;
+    fe seg[kWhirK];
+    for (int j = 0; j < kWhirK; j++) {
+      seg[j] = a.cw[qi + j * (a.L / kWhirK)];
+      put_fe(a.tr, a.off_rep + 16 * (kWhirK * i + j), seg[j]);
+    }
+    // get_RS_multifold_segment_tensor(seg, r, L, qi) with r = the two WHIR
+    // round challenges: level 0 pairs (j, j+2) with omega_L^{-(qi + j L/4)},
+    // level 1 pairs (0, 1) with omega_{L/2}^{-qi} = omega_L^{-2 qi}.
+    fe inv_om = pow_table(a.inv_lo, a.inv_hi, qi);
+    fe part[2];
+    for (int j = 0; j < 2; j++) {
+      fe s = fadd(seg[j], seg[j + 2]), d = fsub(seg[j], seg[j + 2]);
+      part[j] = fadd(fmul(fsub(one, r0), s), fmul(fmul(r0, inv_om), d));
+      inv_om = fmul(inv_om, a.step0);
+    }
+    fe po = pow_table(a.inv_lo, a.inv_hi, (2 * qi) & (a.L - 1));
+    fe s = fadd(part[0], part[1]), d = fsub(part[0], part[1]);
+    fe y = fmul(a.len_inv, fadd(fmul(fsub(one, r1), s), fmul(r1, fmul(po, d))));
+    put_fe(a.tr, a.off_ans + 16 * i, y);
+    const fe c = a.u->c[a.base + i];
+    put_fe(a.tr, a.off_comb + 16 * i, c);
+    contrib = fadd(contrib, fmul(c, y));
+  }
+  for (int dd = 16; dd > 0; dd >>= 1) {
+    fe v;
+    v.re = __shfl_down_sync(0xffffffffu, contrib.re, dd);
+    v.im = __shfl_down_sync(0xffffffffu, contrib.im, dd);
+    contrib = fadd(contrib, v);
+  }
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = contrib;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    fe K = st->K;
+    for (int r = 0; r < kWhirLogK; r++) {
+      const fe *h = H[r], c = st->wr[t][r];
+      for (int k = 0; k < 3; k++) put_fe(a.tr, a.off_poly[r] + 16 * k, h[k]);
+      put_fe(a.tr, a.off_chal[r], c);
+      const fe h01 = fadd(quad_eval(h[0], h[1], h[2], fe_zero()), quad_eval(h[0], h[1], h[2], fe_one()));
+      if (!fe_eq(h01, K)) atomicOr(&st->error, 2u);
+      K = quad_eval(h[0], h[1], h[2], c);
+    }
+    for (int w = 0; w < kOpenThreads / 32; w++) K = fadd(K, red[w]);
+    st->K = K;
+    put_fe(a.tr, a.off_K, K);
+  }
+}
+
+// An iteration's work on the query stream in one launch: block 0 the root
+// (a chain of depth + 1 compressions), block 1 the round messages and the
+// queries, the others the authentication paths, a thread an entry.  Each is a
+// serial chain of its own, so the launch takes as long as the longest; as
+// three launches behind each other an iteration took 35 us at 2^18, now 13,
+// and bound the opening.  Four warps a block: a compression fills the integer
+// issue slots of an SM's quarter.
+__global__ void __launch_bounds__(kOpenThreads) k_whir_open(QueryArgs a, int t) {
+  a.st += blockIdx.y;
+  a.cw = badv(a.cw, a.cws, blockIdx.y);
+  a.tr += a.trs * blockIdx.y;
+  const int depth = 63 - __clzll((long long)(a.L / 4));
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) merkle_root_dev(a.cw, depth, a.tr, a.off_root);
+  } else if (blockIdx.x == 1) {
+    a.partial0 = badv(a.partial0, a.ps, blockIdx.y);
+    a.partial1 = badv(a.partial1, a.ps, blockIdx.y);
+    a.u = badv(a.u, a.us, blockIdx.y);
+    whir_query_dev(a, t);
+  } else {
+    path_entry(a.cw, depth, a.l, (uint64_t)(blockIdx.x - 2) * kOpenThreads + threadIdx.x, a.tr, a.st->wq[t],
+               a.off_path);
+  }
+}
+
+}  // namespace
 
 // The tree aggregate_commitments builds (Whir.cpp:594-605) has all-zero
 // leaf hashes, so its level-d nodes all equal G^d(0): the root of a tree of
@@ -672,6 +715,14 @@ NttTables &ProofPlan::tables(int lg) {
   return ntt.emplace(lg, t).first->second;
 }
 
+// Partials of the WHIR rounds, two messages of three sums a block, of every
+// iteration: they are read on the query stream while the folds move on.
+static uint64_t whir_partials(uint64_t n) {
+  uint64_t total = 0;
+  for (uint64_t m = n; m > (uint64_t)kWhirK; m /= 4) total += 6 * (uint64_t)sc_blocks(m / 4);
+  return total;
+}
+
 std::unique_ptr<ProofPlan> plan_create(int logn, int rate, int batch) {
   if (logn < 3 || logn > 25) throw ArgError("prover: log2 witness length must be in [3, 25]");
   if (rate < 2 || rate > 64 || !is_pow2((uint64_t)rate)) throw ArgError("prover: rate must be a power of two in [2, 64]");
@@ -694,6 +745,7 @@ std::unique_ptr<ProofPlan> plan_create(int logn, int rate, int batch) {
   p->bs_arr = sizeof(fe) * (n / 2);
   p->bs_beta = sizeof(fe) * n;
   p->bs_part = sizeof(fe) * 3 * (uint64_t)sc_blocks(n / 2);
+  p->bs_wpart = sizeof(fe) * whir_partials(n);
   p->bs_ub = sizeof(fe) * kUpdateBetasScratch;
   p->w = (fe *)p->dalloc(B * p->bs_w);
   p->cw[0] = (fe *)p->dalloc(B * p->bs_cw0);
@@ -716,7 +768,7 @@ std::unique_ptr<ProofPlan> plan_create(int logn, int rate, int batch) {
   p->vb[1] = (fe *)p->dalloc(B * p->bs_v);
   p->beta = (fe *)p->dalloc(B * p->bs_beta);
   p->partial = (fe *)p->dalloc(B * p->bs_part);
-  p->partial2 = (fe *)p->dalloc(B * p->bs_part);
+  p->wpart = (fe *)p->dalloc(B * p->bs_wpart);
   p->ub_scratch = (fe *)p->dalloc(B * p->bs_ub);
   p->st = (ProofState *)p->dalloc(B * sizeof(ProofState));
   GBZ_CUDA(cudaFuncSetAttribute(k_sc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -819,7 +871,9 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
     RUN(PC_PROTOCOL, 1, k_init<<<B, 32, 0, s>>>(st, prng_seed, seed_in_state ? 1 : 0));
   }
   // The opening's randomness, drawn on the query stream while the
-  // commitment and the sumcheck run.
+  // commitment and the sumcheck run, and the beta updates' powers.
+  UbSlots *slots = reinterpret_cast<UbSlots *>(p.ub_scratch);
+  UbPrepArgs ua{};
   {
     SchedArgs sa{};
     uint64_t mm = p.n, LL = p.L, cc = (uint64_t)p.rate;
@@ -840,6 +894,22 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
       GBZ_CUDA(cudaStreamWaitEvent(q, p.ev_init, 0));
     }
     RUN_ON(q, PC_PROTOCOL, 1, k_whir_schedule<<<B, 256, 0, q>>>(st, sa));
+    ua.T = sa.T;
+    LL = p.L;
+    mm = p.n;
+    for (int t = 0; t < sa.T; t++) {
+      LL /= 2;
+      mm /= 4;
+      ua.base[t + 1] = ua.base[t] + sa.l[t];
+      ua.per[t] = update_betas_per(mm, B);
+      if (dry) continue;
+      const NttTables &tnew = p.tables(ilog2(LL));
+      ua.lo[t] = tnew.lo_fwd;
+      ua.hi[t] = tnew.hi_fwd;
+    }
+    if (ua.base[sa.T] > kUbSlots) throw ArgError("prover: too many queries");
+    RUN_ON(q, PC_UPDATE_BETAS, 1,
+           k_ub_prep<<<dim3((unsigned)(ua.base[sa.T] + 3) / 4, B), 128, 0, q>>>(st, slots, p.bs_ub, ua));
     if (!dry) GBZ_CUDA(cudaEventRecord(p.ev_sched, q));
   }
 
@@ -989,7 +1059,7 @@ opening:
   uint64_t ast = p.bs_w, bst = p.bs_beta;  // per-proof strides of a and b
   m = p.n;
   uint64_t cur = (uint64_t)p.rate;
-  fe *arr_next = p.arr;
+  fe *arr_next = p.arr, *wpart = p.wpart;
   for (;;) {
     if (iter >= ProofPlan::kMaxIter) throw ArgError("prover: too many WHIR iterations");
     const int l = whir_query_count((int)cur);
@@ -1002,6 +1072,8 @@ opening:
     const uint64_t op1 = lay.rec(T_WHIR_POLY, 3, 16), oc1 = lay.rec(T_WHIR_CHALLENGE, 1, 16);
     fe *bd = p.vb[(iter + 1) & 1];
     const int blocks = sc_blocks(m / 4);
+    fe *part0 = wpart, *part1 = wpart + 3 * blocks;
+    wpart += 6 * blocks;
     if (iter == 0 && eq_first) {
       BStr fb;  // (a, E2, c, chal0, chal1, a4, b4, partial0, partial1)
       fb.s[0] = ast;
@@ -1011,11 +1083,11 @@ opening:
       fb.s[4] = sts;
       fb.s[5] = p.bs_arr;
       fb.s[6] = p.bs_v;
-      fb.s[7] = p.bs_part;
-      fb.s[8] = p.bs_part;
+      fb.s[7] = p.bs_wpart;
+      fb.s[8] = p.bs_wpart;
       RUN(PC_SUMCHECK, 1,
-          sc_fold2_eq_launch(a, b, m, st->chal, &st->wr[iter][0], &st->wr[iter][1], arr_next, bd, p.partial,
-                             p.partial2, blocks, s, B, fb));
+          sc_fold2_eq_launch(a, b, m, st->chal, &st->wr[iter][0], &st->wr[iter][1], arr_next, bd, part0, part1,
+                             blocks, s, B, fb));
     } else {
       BStr fb;  // (a, b, chal0, chal1, a4, b4, partial0, partial1)
       fb.s[0] = ast;
@@ -1024,24 +1096,11 @@ opening:
       fb.s[3] = sts;
       fb.s[4] = p.bs_arr;
       fb.s[5] = p.bs_v;
-      fb.s[6] = p.bs_part;
-      fb.s[7] = p.bs_part;
+      fb.s[6] = p.bs_wpart;
+      fb.s[7] = p.bs_wpart;
       RUN(PC_SUMCHECK, 1,
-          sc_fold2_launch(a, b, m, &st->wr[iter][0], &st->wr[iter][1], arr_next, bd, p.partial, p.partial2, blocks,
-                          s, B, fb));
-    }
-    {
-      // both round messages; the kernel also prepares this iteration's beta update
-      UbPrep u{};
-      if (!dry) {
-        const NttTables &tnew = p.tables(ilog2(NL));
-        u.l = l;
-        u.lo = tnew.lo_fwd;
-        u.hi = tnew.hi_fwd;
-      }
-      RUN(PC_PROTOCOL, 1,
-          k_whir_rounds2_s<<<B, 256, 0, s>>>(p.partial, p.partial2, blocks, st, iter, tr, op, oc, op1, oc1, u,
-                                             p.bs_part, trs));
+          sc_fold2_launch(a, b, m, &st->wr[iter][0], &st->wr[iter][1], arr_next, bd, part0, part1, blocks, s, B,
+                          fb));
     }
     a = arr_next;
     b = bd;
@@ -1067,18 +1126,29 @@ opening:
     }
     off_root[iter + 1] = off;
     if (!dry) GBZ_CUDA(cudaEventRecord(p.ev_commit[iter + 1], c));
-    // queries of iteration t on q: they open the codeword of commit t and
-    // check K against this iteration's round messages
+    // queries of iteration t on q: they open the codeword of commit t,
+    // record this iteration's round messages and check K against them
     const int depth = ilog2(L / 4);
-    QueryArgs qa;
+    QueryArgs qa{};
     qa.st = st;
     qa.cws = cw_s[cwi];
+    qa.ps = p.bs_wpart;
     qa.trs = trs;
     qa.cw = p.cw[cwi];
     qa.L = L;
-    qa.NL = NL;
     qa.l = l;
+    qa.partial0 = part0;
+    qa.partial1 = part1;
+    qa.blocks = blocks;
     qa.tr = tr;
+    qa.off_poly[0] = op;
+    qa.off_chal[0] = oc;
+    qa.off_poly[1] = op1;
+    qa.off_chal[1] = oc1;
+    qa.off_root = off_root[iter];
+    qa.u = slots;
+    qa.us = p.bs_ub;
+    qa.base = ua.base[iter];
     qa.off_q = lay.rec(T_WHIR_QUERIES, l, 4);
     qa.off_rep = lay.rec(T_WHIR_REPLIES, l * kWhirK, 16);
     qa.off_ans = lay.rec(T_WHIR_ANSWERS, l, 16);
@@ -1089,8 +1159,6 @@ opening:
       const NttTables &told = p.tables(ilog2(L));
       qa.inv_lo = told.lo_inv;
       qa.inv_hi = told.hi_inv;
-      qa.new_lo = nullptr;
-      qa.new_hi = nullptr;
       const fe om_inv = finv(root_of_unity(ilog2(L)));
       qa.step0 = fpow(om_inv, L / kWhirK);
       qa.len_inv = finv(fe_make(kWhirK, 0));
@@ -1099,15 +1167,12 @@ opening:
       GBZ_CUDA(cudaStreamWaitEvent(q, p.ev_commit[iter], 0));
       GBZ_CUDA(cudaStreamWaitEvent(q, p.ev_fold[iter], 0));
     }
-    RUN_ON(q, PC_MERKLE, 1, k_merkle_root_b<<<B, 32, 0, q>>>(qa.cw, qa.cws, depth, tr, trs, off_root[iter]));
-    RUN_ON(q, PC_QUERY, 1, k_whir_query_s<<<B, kMaxQueries, 0, q>>>(qa, iter));
-    {
-      const uint64_t hashes = (uint64_t)l * depth;  // depth >= 2: every queried codeword has 16+ entries
-      RUN_ON(q, PC_QUERY, 1,
-             k_whir_paths_chain<<<dim3((unsigned)((hashes + 127) / 128), B), 128, 0, q>>>(
-                 qa.cw, L / 4, l, tr, qa.off_q, qa.off_path, qa.cws, trs));
-      if (!dry && hashes == 0) throw ArgError("prover: empty authentication paths");
-    }
+    // depth >= 2: every queried codeword has 16+ entries
+    const uint64_t hashes = (uint64_t)l * depth;
+    if (hashes == 0) throw ArgError("prover: empty authentication paths");
+    RUN_ON(q, PC_QUERY, 1,
+           k_whir_open<<<dim3((unsigned)(2 + (hashes + kOpenThreads - 1) / kOpenThreads), B), kOpenThreads, 0, q>>>(
+               qa, iter));
     if (!dry) GBZ_CUDA(cudaEventRecord(p.ev_query[iter], q));
     // update_betas on s: b[j] += sum_i c_i omega_NL^{q_i j} is the forward
     // transform of a vector with l nonzeros.  When l * |b| exceeds a few
@@ -1119,12 +1184,15 @@ opening:
     if (update_betas_by_transform(l, m, NL / 2)) {
       // one sparse transform per proof of a batch
       RUN(PC_UPDATE_BETAS, 2 * B, for (int pb = 0; pb < B; pb++) {
-        ntt_sparse_accumulate(p.tables(ilog2(NL) - 1), st[pb].q, st[pb].comb, l,
+        const UbSlots *u = reinterpret_cast<const UbSlots *>(reinterpret_cast<const char *>(slots) + p.bs_ub * pb);
+        ntt_sparse_accumulate(p.tables(ilog2(NL) - 1), u->q2 + ua.base[iter], u->c + ua.base[iter], l,
                               reinterpret_cast<fe *>(reinterpret_cast<char *>(bd) + p.bs_v * pb), m,
                               reinterpret_cast<fe *>(reinterpret_cast<char *>(p.tmp2) + p.bs_tmp2 * pb), s, 1);
       });
     } else {
-      RUN(PC_UPDATE_BETAS, 2, update_betas_launch(bd, m, st, l, p.ub_scratch, s, B, p.bs_v, p.bs_ub));
+      RUN(PC_UPDATE_BETAS, 1,
+          update_betas_powers_launch(bd, m, slots->w + ua.base[iter], slots->c + ua.base[iter], l,
+                                     slots->pw + 32 * ua.base[iter], s, B, p.bs_v, p.bs_ub));
     }
     cwi = nci;
     L = NL;
@@ -1290,7 +1358,7 @@ void launch_proof_graph(ProofPlan &p, const fe *w, uint32_t prng_seed, cudaStrea
 uint64_t plan_bytes(int logn, int rate, int batch) {
   const uint64_t n = 1ull << logn, L = n * (uint64_t)rate;
   uint64_t b = sizeof(fe) * (n + L + L / 2 + L + L / 2 + 5 * (n / 2) + n);
-  b += sizeof(fe) * (6 * (uint64_t)sc_blocks(n / 2) + kUpdateBetasScratch) + sizeof(ProofState);
+  b += sizeof(fe) * (3 * (uint64_t)sc_blocks(n / 2) + whir_partials(n) + kUpdateBetasScratch) + sizeof(ProofState);
   b *= (uint64_t)batch;
   b += 64ull << 20;  // transcripts, twiddle tables and allocation granularity (upper bound)
   b += (uint64_t)batch << 20;

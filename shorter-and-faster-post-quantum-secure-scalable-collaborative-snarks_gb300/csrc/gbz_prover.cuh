@@ -60,15 +60,16 @@ struct ProofPlan {
   uint64_t n = 0, L = 0;
   int B = 1;
   uint64_t bs_w = 0, bs_cw0 = 0, bs_cw1 = 0, bs_tmp = 0, bs_tmp2 = 0, bs_v = 0, bs_arr = 0, bs_beta = 0,
-           bs_part = 0, bs_ub = 0;
+           bs_part = 0, bs_wpart = 0, bs_ub = 0;
   fe *w = nullptr;                // witness staging (host-input proofs)
   fe *cw[2] = {nullptr, nullptr}; // codeword ping-pong (L, L/2)
   fe *tmp = nullptr;              // NTT intermediate of the commits (L)
   fe *tmp2 = nullptr;             // NTT intermediate of the sparse beta updates (L/2)
   // The opening runs as three chains joined by events: folds and beta
-  // updates on the caller's stream, commits (NTT + Merkle) on s2, queries
-  // (replies, answers, paths, the running claim K) on s3.  Each waits only
-  // for the data it reads; the WHIR randomness is drawn up front on s3.
+  // updates on the caller's stream, commits (NTT) on s2, queries (round
+  // messages, replies, answers, paths, roots, the running claim K) on s3.
+  // Each waits only for the data it reads; the WHIR randomness is drawn, and
+  // the beta updates' powers are formed, up front on s3.
   cudaStream_t s2 = nullptr, s3 = nullptr;
   static constexpr int kMaxIter = kMaxWhirIter;
   cudaEvent_t ev_in = nullptr, ev_init = nullptr, ev_sched = nullptr, ev_fold[kMaxIter] = {}, ev_commit[kMaxIter + 1] = {},
@@ -78,8 +79,8 @@ struct ProofPlan {
   fe *vb[2] = {nullptr, nullptr}; // folded second vector ping-pong
   fe *beta = nullptr;             // eq table (n)
   fe *partial = nullptr;          // per-CTA round-message partials
-  fe *partial2 = nullptr;         // the second round's, when two rounds share a pass
-  fe *ub_scratch = nullptr;       // update_betas power tables
+  fe *wpart = nullptr;            // the WHIR rounds' partials, of every iteration (read by the queries)
+  fe *ub_scratch = nullptr;       // update_betas roots, weights and powers of every iteration (UbSlots)
   ProofState *st = nullptr;
   uint8_t *transcript = nullptr;
   uint64_t transcript_bytes = 0;

@@ -424,62 +424,59 @@ __global__ void __launch_bounds__(256) beta_tensor_kernel(const fe *r, int nr, i
   }
 }
 
-// update_betas: b[j] += sum_i c_i * w_i^j.  A CTA owns kUbSpan = 256
-// consecutive entries: lane L of every warp owns the kUbPer = 8 entries
-// starting at cta0 + 8L, and warp g takes the queries i = g (mod 8), so the
-// l * 256 multiply-adds of a CTA are spread over all its threads; the eight
-// warps' partial sums are added in shared memory.  A thread starts each of
-// its queries' geometric runs from s_i * pw_i[L] (s_i = c_i w_i^{cta0},
-// pw_i[L] = w_i^{8L}) and steps it by w_i.
+// update_betas: b[j] += sum_i c_i * w_i^j.  A CTA owns 32 PER consecutive
+// entries: lane L of every warp owns the PER entries starting at cta0 + PER L,
+// and warp g takes the queries i = g (mod 8), so the l * 32 PER multiply-adds
+// of a CTA are spread over all its threads; the eight warps' partial sums are
+// added in shared memory.  A thread starts each of its queries' geometric runs
+// from s_i * pw_i[L] (s_i = c_i w_i^{cta0}, pw_i[L] = w_i^{PER L}) and steps
+// it by w_i.
 constexpr int kUbThreads = 256;
 constexpr int kUbWarps = kUbThreads / 32;
-constexpr int kUbPer = 8;
-constexpr int kUbSpan = 32 * kUbPer;
 
-__global__ void __launch_bounds__(kUbThreads) ub_table_kernel(const ProofState *st, int l, fe *pw, BStr bs) {
-  // pw[i*32 + L] = w_i^(L * kUbPer)
-  st = badv(st, bs.s[0], blockIdx.y);
-  pw = badv(pw, bs.s[1], blockIdx.y);
+// pw[i*32 + L] = w_i^(L * per)
+__global__ void __launch_bounds__(32) ub_table_kernel(const fe *w, int per, fe *pw) {
   const int i = blockIdx.x, t = threadIdx.x;
-  if (i >= l || t >= 32) return;
-  pw[i * 32 + t] = fpow(st->omega_q[i], (uint64_t)t * kUbPer);
+  pw[i * 32 + t] = fpow(w[i], (uint64_t)t * per);
 }
 
+template <int PER>
 __global__ void __launch_bounds__(kUbThreads)
-ub_kernel(fe *b, uint64_t nb, const ProofState *st, int l, const fe *pw, BStr bs) {
+ub_kernel(fe *b, uint64_t nb, const fe *w, const fe *c, int l, const fe *pw, uint64_t b_stride, uint64_t u_stride) {
+  constexpr int SPAN = 32 * PER;
   __shared__ fe s_start[kMaxQueries], s_w[kMaxQueries];
-  b = badv(b, bs.s[0], blockIdx.y);
-  st = badv(st, bs.s[1], blockIdx.y);
-  pw = badv(pw, bs.s[2], blockIdx.y);
-  __shared__ fe part[kUbWarps][kUbSpan];
-  const uint64_t cta0 = (uint64_t)blockIdx.x * kUbSpan;
+  __shared__ fe part[kUbWarps][SPAN];
+  b = badv(b, b_stride, blockIdx.y);
+  w = badv(w, u_stride, blockIdx.y);
+  c = badv(c, u_stride, blockIdx.y);
+  pw = badv(pw, u_stride, blockIdx.y);
+  const uint64_t cta0 = (uint64_t)blockIdx.x * SPAN;
   for (int i = threadIdx.x; i < l; i += kUbThreads) {
-    const fe w = st->omega_q[i];
-    s_w[i] = w;
-    s_start[i] = fmul(st->comb[i], fpow(w, cta0));
+    const fe wi = w[i];
+    s_w[i] = wi;
+    s_start[i] = fmul(c[i], fpow(wi, cta0));
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  fe acc[kUbPer];  // sums of folded words, folded again after each
+  fe acc[PER];  // sums of folded words, folded again after each
 #pragma unroll
-  for (int k = 0; k < kUbPer; k++) acc[k] = fe_zero();
+  for (int k = 0; k < PER; k++) acc[k] = fe_zero();
+#pragma unroll(PER == 1 ? 4 : 1)
   for (int i = warp; i < l; i += kUbWarps) {
-    const fe w = s_w[i];
+    const fe wi = s_w[i];
     fe d = fmul_fold(s_start[i], pw[i * 32 + lane]);
 #pragma unroll
-    for (int k = 0; k < kUbPer; k++) {
+    for (int k = 0; k < PER; k++) {
       acc[k] = fe_make(fold64(acc[k].re + d.re), fold64(acc[k].im + d.im));
-      if (k + 1 < kUbPer) d = fmul_fold(d, w);
+      if (k + 1 < PER) d = fmul_fold(d, wi);
     }
   }
 #pragma unroll
-  for (int k = 0; k < kUbPer; k++) acc[k] = fe_make(canon64(acc[k].re), canon64(acc[k].im));
-#pragma unroll
-  for (int k = 0; k < kUbPer; k++) part[warp][lane * kUbPer + k] = acc[k];
+  for (int k = 0; k < PER; k++) part[warp][lane * PER + k] = fe_make(canon64(acc[k].re), canon64(acc[k].im));
   __syncthreads();
   // thread t finishes entry cta0 + t
   const uint64_t j = cta0 + threadIdx.x;
-  if (j >= nb) return;
+  if (threadIdx.x >= SPAN || j >= nb) return;
   fe sum = part[0][threadIdx.x];
 #pragma unroll
   for (int g = 1; g < kUbWarps; g++) sum = fadd(sum, part[g][threadIdx.x]);
@@ -565,21 +562,30 @@ void beta_launch(const fe *r, int nr, fe *B, cudaStream_t s, int batch, uint64_t
   GBZ_CUDA(cudaGetLastError());
 }
 
-void update_betas_launch(fe *b, uint64_t nb, const ProofState *st, int l, fe *pw_scratch, cudaStream_t s, int batch,
-                         uint64_t b_stride, uint64_t pw_stride) {
+int update_betas_per(uint64_t nb, int batch) {
+  const uint64_t entries = nb * (uint64_t)batch;
+  return entries >= (1ull << 15) ? 8 : entries >= (1ull << 13) ? 2 : 1;
+}
+
+void update_betas_powers_launch(fe *b, uint64_t nb, const fe *w, const fe *c, int l, const fe *pw, cudaStream_t s,
+                                int batch, uint64_t b_stride, uint64_t u_stride) {
   if (l <= 0) return;
   if (l > kMaxQueries) throw ArgError("update_betas: too many queries");
-  BStr t, u;
-  t.s[0] = sizeof(ProofState);
-  t.s[1] = pw_stride;
-  u.s[0] = b_stride;
-  u.s[1] = sizeof(ProofState);
-  u.s[2] = pw_stride;
-  if (batch == 1) t = u = BStr();
-  ub_table_kernel<<<dim3(l, batch), 32, 0, s>>>(st, l, pw_scratch, t);
+  const int per = update_betas_per(nb, batch), span = 32 * per;
+  const dim3 grid((unsigned)((nb + span - 1) / span), batch);
+  if (!grid.x) return;
+  if (per == 8) ub_kernel<8><<<grid, kUbThreads, 0, s>>>(b, nb, w, c, l, pw, b_stride, u_stride);
+  else if (per == 2) ub_kernel<2><<<grid, kUbThreads, 0, s>>>(b, nb, w, c, l, pw, b_stride, u_stride);
+  else ub_kernel<1><<<grid, kUbThreads, 0, s>>>(b, nb, w, c, l, pw, b_stride, u_stride);
   GBZ_CUDA(cudaGetLastError());
-  ub_kernel<<<dim3((unsigned)((nb + kUbSpan - 1) / kUbSpan), batch), kUbThreads, 0, s>>>(b, nb, st, l, pw_scratch, u);
+}
+
+void update_betas_launch(fe *b, uint64_t nb, const ProofState *st, int l, fe *pw_scratch, cudaStream_t s) {
+  if (l <= 0) return;
+  if (l > kMaxQueries) throw ArgError("update_betas: too many queries");
+  ub_table_kernel<<<l, 32, 0, s>>>(st->omega_q, update_betas_per(nb, 1), pw_scratch);
   GBZ_CUDA(cudaGetLastError());
+  update_betas_powers_launch(b, nb, st->omega_q, st->comb, l, pw_scratch, s, 1, 0, 0);
 }
 
 }  // namespace gbz
