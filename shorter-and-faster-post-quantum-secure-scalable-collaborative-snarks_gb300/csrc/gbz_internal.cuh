@@ -228,8 +228,8 @@ void sc_step_launch(const fe *a, const fe *b, uint64_t m, const fe *chal, fe *a2
 // m/4, the fold by *chal0 then *chal1.  m >= 4.
 // batch > 1: grid.y = proof, bs the strides of (a, b, chal0, chal1, a4, b4,
 // partial0, partial1) (sc_fold2) / (a, E2, c, chal0, chal1, a4, b4,
-// partial0, partial1) (sc_fold2_eq) / (a, E, chal, a2, E2, partial)
-// (sc_eq_step).
+// partial0, partial1) (sc_fold2_eq) / (a, E, partial) (sc_eq_reduce) /
+// (a, chal, a4, E, E4, partial) (sc_eq_fold).
 void sc_fold2_launch(const fe *a, const fe *b, uint64_t m, const fe *chal0, const fe *chal1, fe *a4, fe *b4,
                      fe *partial0, fe *partial1, int blocks, cudaStream_t s, int batch = 1, const BStr &bs = BStr());
 // The same with b = precompute_beta(c) given by E2, the eq table of c[2..]
@@ -237,13 +237,16 @@ void sc_fold2_launch(const fe *a, const fe *b, uint64_t m, const fe *chal0, cons
 void sc_fold2_eq_launch(const fe *a, const fe *E2, uint64_t m, const fe *c, const fe *chal0, const fe *chal1, fe *a4,
                         fe *b4, fe *partial0, fe *partial1, int blocks, cudaStream_t s, int batch = 1,
                         const BStr &bs = BStr());
-// The same steps for the sumcheck of sum_x w(x) eq(z, x) with the eq vector
-// kept as the shrinking table E_i of z_{i+1..}: chal == nullptr gives the
-// sums S(0), S(1) of (a, E); otherwise a is folded by *chal into a2 (m/2),
-// E2 = pairwise sums of E (m/4) and, when reduce, the sums of (a2, E2).
-// Partials are (S0, S1, 0) per block.
-void sc_eq_step_launch(const fe *a, const fe *E, uint64_t m, const fe *chal, fe *a2, fe *E2, bool reduce,
-                       fe *partial, int blocks, cudaStream_t s, int batch = 1, const BStr &bs = BStr());
+// The sumcheck of sum_x w(x) eq(z, x), two rounds a pass, with the eq vector
+// kept as a shrinking table (E of m/4 entries for w of m entries): the four
+// sums T_k = sum_j a[4j + k] E[j] of both rounds (m a multiple of 4), and the
+// fold of a by chal[0], chal[1] into a4 (m/4, m a multiple of 128) with
+// E4 = sums of four of E (m/16) and, when reduce, the T sums of (a4, E4).
+// Partials are (T0, T1, T2, T3) per block.
+void sc_eq_reduce_launch(const fe *a, const fe *E, uint64_t m, fe *partial, int blocks, cudaStream_t s,
+                         int batch = 1, const BStr &bs = BStr());
+void sc_eq_fold_launch(const fe *a, const fe *E, uint64_t m, const fe *chal, fe *a4, fe *E4, bool reduce, fe *partial,
+                       int blocks, cudaStream_t s, int batch = 1, const BStr &bs = BStr());
 // Round-message reduction of `blocks` partials into out[3].
 void sc_sum_launch(const fe *partial, int blocks, fe *out3, cudaStream_t s);
 
@@ -258,7 +261,7 @@ constexpr uint64_t kUpdateBetasScratch = (uint64_t)kMaxQueries * 256;
 void update_betas_launch(fe *b, uint64_t nb, const ProofState *st, int l, fe *pw_scratch, cudaStream_t s);
 // Entries a lane of the update owns: fewer where the vectors are too short to
 // give every SM a CTA of 32 x 8 entries (256 entries by 100 queries: 16.2 us
-// in one CTA, 4.9 us in eight).
+// in one CTA, 5.9 us in eight).
 int update_betas_per(uint64_t nb, int batch);
 // The same update from roots w_i, weights c_i and the powers
 // pw[32 i + L] = w_i^(L update_betas_per(nb, batch)) that are there already.

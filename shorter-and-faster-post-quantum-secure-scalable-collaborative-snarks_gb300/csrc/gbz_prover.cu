@@ -27,22 +27,11 @@ namespace {
 // ------------------------------------------------------------ kernels
 
 
-// The glibc generator state is worked on in shared memory by one thread and
-// written back: its table is indexed dynamically, and hundreds of draws on
-// the global copy would each pay a memory round trip.
-__global__ void k_init(ProofState *st, uint32_t seed, int seed_in_state) {
-  __shared__ glibc_prng g;
-  st += blockIdx.x;  // a batch: one CTA per proof
-  if (threadIdx.x) return;
-  st->fs = fe_zero();
-  prng_seed(g, seed_in_state ? st->seed_in : seed);
-  st->prng = g;
-  st->y = fe_zero();
-  st->K = fe_zero();
-  st->error = 0;
+// The generator of a proof (a batch: one CTA per proof).
+__global__ void __launch_bounds__(32) k_init(ProofState *st, uint32_t seed, int seed_in_state) {
+  st += blockIdx.x;
+  prng_warp_seed(st->prng, seed_in_state ? st->seed_in : seed, threadIdx.x);
 }
-
-// The state of an opening alone: the caller's generator, point and claim.
 __global__ void k_init_open(ProofState *st, glibc_prng g, const fe *point, int logn, fe K) {
   if (threadIdx.x == 0) {
     st->fs = fe_zero();
@@ -55,11 +44,16 @@ __global__ void k_init_open(ProofState *st, glibc_prng g, const fe *point, int l
 }
 
 // z_i = hash_to_field({0}) for i < logn.
+// The start of a proof's protocol state and its evaluation point.
 __global__ void k_point(ProofState *st, int logn, uint8_t *tr, uint64_t off, uint64_t trs) {
   st += blockIdx.x;
   tr += trs * blockIdx.x;
   if (threadIdx.x) return;
-  fe s = st->fs;
+  st->y = fe_zero();
+  st->K = fe_zero();
+  st->error = 0;
+  fe s = fe_zero();
+#pragma unroll 1
   for (int i = 0; i < logn; i++) {
     s = hash_F(s, fe_zero());
     st->z[i] = s;
@@ -98,146 +92,180 @@ __device__ void sum_partials(const fe *partial, int blocks, fe out[3]) {
   }
 }
 
-// Round i of the sumcheck of sum w(x) eq(z, x) from the S(0), S(1) sums:
-// H(X) = epre * eq1(z_i, X) * (S0 + X (S1 - S0)) (the reference's round
-// message of the pairs of w and the folded eq vector); claim check; the
-// Fiat-Shamir challenge hash_to_field({H.a, H.b, H.c}); y = H(c); and
-// epre *= eq1(z_i, c).
-__device__ fe sc_round_eq_apply(const fe SS[3], ProofState *st, int round, uint8_t *tr, int64_t off_claim,
-                                uint64_t off_poly, uint64_t off_chal) {
-  if (round == 0) st->epre = fe_one();
-  const fe z = st->z[round], ep = st->epre;
-  const fe a1 = fsub(fadd(z, z), fe_one()), b1 = fsub(fe_one(), z);
-  const fe a2 = fsub(SS[2], SS[0]), b2 = SS[0];
-  fe H[3];
-  H[0] = fmul(ep, fmul(a1, a2));
-  H[1] = fmul(ep, fadd(fmul(a1, b2), fmul(b1, a2)));
-  H[2] = fmul(ep, fmul(b1, b2));
-  fe h01 = fadd(quad_eval(H[0], H[1], H[2], fe_zero()), quad_eval(H[0], H[1], H[2], fe_one()));
-  if (off_claim >= 0) {
-    st->y = h01;
-    put_fe(tr, (uint64_t)off_claim, h01);
-  } else if (!fe_eq(h01, st->y)) {
-    atomicOr(&st->error, 1u);
-  }
-  for (int k = 0; k < 3; k++) put_fe(tr, off_poly + 16 * k, H[k]);
-  fe s = st->fs;
-  for (int k = 0; k < 3; k++) s = hash_F(s, H[k]);
-  st->fs = s;
-  st->chal[round] = s;
-  put_fe(tr, off_chal, s);
-  st->y = quad_eval(H[0], H[1], H[2], s);
-  st->epre = fmul(ep, fadd(b1, fmul(a1, s)));
-  return s;
-}
-
-__global__ void k_sc_round_eq(const fe *partial, int blocks, ProofState *st, int round, uint8_t *tr,
-                              int64_t off_claim, uint64_t off_poly, uint64_t off_chal, uint64_t ps, uint64_t trs) {
-  partial = badv(partial, ps, blockIdx.x);
-  st += blockIdx.x;
-  tr += trs * blockIdx.x;
-  fe SS[3];
-  sum_partials(partial, blocks, SS);  // (S0, -S0-S1, S1)
-  if (threadIdx.x) return;
-  (void)sc_round_eq_apply(SS, st, round, tr, off_claim, off_poly, off_chal);
-}
-
-// The last rounds of the same sumcheck in one CTA, once w (m entries) and
-// its eq table E (m / 2) fit in shared memory: per round r the fold of w by
-// chal[r-1], the pairwise sums of E, the sums S(0), S(1) and the round
-// itself (thread 0), with no launch or global round trip between rounds;
-// then the final fold and the SC_FINAL record.  Round r's SC_POLY payload
-// is at off_poly0 + 80 (r - round0), its SC_CHALLENGE 56 bytes after it.
-constexpr int kScTailMax = 4096;
 // Batched plans: codewords of 2^kBatchRealLog entries or more are committed
 // proof by proof with the real-input transform, shorter ones in one batched
 // general transform.
 constexpr int kBatchRealLog = 18;
-constexpr int kScTailThreads = 1024;
+
+// The Fiat-Shamir state of the sumcheck of sum w(x) eq(z, x): the hash chain,
+// the running claim, prod_{k < i} eq1(z_k, chal_k) and the verdict.
+struct ScChain {
+  fe fs, y, ep;
+  uint32_t bad;
+};
+
+// Round i of that sumcheck from S(0), S(1):
+// H(X) = epre * eq1(z_i, X) * (S0 + X (S1 - S0)) (the reference's round
+// message of the pairs of w and the folded eq vector); claim check (the first
+// round records it); the challenge hash_to_field({H.a, H.b, H.c}); y = H(c);
+// and epre *= eq1(z_i, c).  Payload of the message at off_poly, the challenge
+// 56 bytes after it.
+__device__ __forceinline__ fe sc_round_eq(ScChain &v, fe S0, fe S1, fe z, fe *chal, uint8_t *tr, int64_t off_claim,
+                                          uint64_t off_poly) {
+  const fe a1 = fsub(fadd(z, z), fe_one()), b1 = fsub(fe_one(), z), d = fsub(S1, S0);
+  const fe A = fmul(v.ep, a1), B = fmul(v.ep, b1);
+  const fe h0 = fmul(A, d), h1 = fadd(fmul(A, S0), fmul(B, d)), h2 = fmul(B, S0);
+  const fe h01 = fadd(h2, fadd(fadd(h0, h1), h2));  // H(0) + H(1)
+  if (off_claim >= 0) put_fe(tr, (uint64_t)off_claim, h01);
+  else if (!fe_eq(h01, v.y)) v.bad = 1;
+  put_fe(tr, off_poly, h0);
+  put_fe(tr, off_poly + 16, h1);
+  put_fe(tr, off_poly + 32, h2);
+  fe s = v.fs;
+#pragma unroll 1
+  for (int k = 0; k < 3; k++) s = hash_F(s, k == 0 ? h0 : k == 1 ? h1 : h2);
+  v.fs = s;
+  *chal = s;
+  put_fe(tr, off_poly + 56, s);
+  v.y = fadd(fmul(fadd(fmul(h0, s), h1), s), h2);
+  v.ep = fadd(fmul(A, s), B);
+  return s;
+}
+
+__device__ __forceinline__ fe shfl_xor_fe(fe x, int d) {
+  return fe_make(__shfl_xor_sync(0xffffffffu, x.re, d), __shfl_xor_sync(0xffffffffu, x.im, d));
+}
+
+// Rounds i and i + 1 from the T sums of a pass (gbz_sumcheck.cu): the sum of
+// the partials, then thread 0 alone through both rounds' hash chains (3.4 us
+// of the 5 a launch takes).
+__global__ void __launch_bounds__(256)
+k_sc_rounds_eq(const fe *partial, int blocks, ProofState *st, int round, uint8_t *tr, int64_t off_claim,
+               uint64_t off_poly, uint64_t ps, uint64_t trs) {
+  __shared__ fe red[8][4];
+  partial = badv(partial, ps, blockIdx.x);
+  st += blockIdx.x;
+  tr += trs * blockIdx.x;
+  const fe z0 = st->z[round], z1 = st->z[round + 1];
+  ScChain v{st->fs, st->y, round ? st->epre : fe_one(), 0};
+  fe x = fe_zero();
+  for (int i = threadIdx.x; i < 4 * blocks; i += 256) x = fadd(x, partial[i]);
+  for (int d = 4; d < 32; d *= 2) x = fadd(x, shfl_xor_fe(x, d));
+  if ((threadIdx.x & 31) < 4) red[threadIdx.x >> 5][threadIdx.x & 3] = x;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  x = red[threadIdx.x >> 2][threadIdx.x & 3];
+  for (int d = 4; d < 32; d *= 2) x = fadd(x, shfl_xor_fe(x, d));
+  if (threadIdx.x < 4) red[0][threadIdx.x] = x;
+  __syncwarp();
+  if (threadIdx.x) return;
+  const fe T0 = red[0][0], T1 = red[0][1], T2 = red[0][2], T3 = red[0][3];
+  const fe c = sc_round_eq(v, fadd(T0, fmul(z1, fsub(T2, T0))), fadd(T1, fmul(z1, fsub(T3, T1))), z0,
+                           &st->chal[round], tr, off_claim, off_poly);
+  (void)sc_round_eq(v, fadd(T0, fmul(c, fsub(T1, T0))), fadd(T2, fmul(c, fsub(T3, T2))), z1, &st->chal[round + 1],
+                    tr, -1, off_poly + 80);
+  st->fs = v.fs;
+  st->y = v.y;
+  st->epre = v.ep;
+  if (v.bad) atomicOr(&st->error, 1u);
+}
+
+// The last rounds of the same sumcheck in one CTA, from w of m <= kScTailMax
+// entries and its table E (m / 4) on, then the final fold and the SC_FINAL
+// record.  The hash chain of a round is serial (1.7 us); everything else runs
+// beside it: with the T sums of w_r in hand, thread 0 knows round r + 1's
+// message as soon as it has challenge r, and while it hashes it the workers
+// fold w by challenge r and form the next T sums.  (The fold, the sums and
+// the reductions in turn with the hashes took 7 us a round, 63 us for 2^10.)
+// The workers are the warps outside the first one's quarter of the SM, whose
+// issue slots the compressions fill.  Round r's SC_POLY payload is at
+// off_poly0 + 80 (r - round0), its SC_CHALLENGE 56 bytes after it.
+constexpr int kScTailMax = 4096;
+constexpr int kScTailThreads = 1024, kScTailWorkers = kScTailThreads / 4 * 3;
+constexpr size_t kScTailShared = sizeof(fe) * (kScTailMax / 2 + kScTailMax / 4 + kScTailMax / 8 + kScTailMax / 16);
 __global__ void __launch_bounds__(kScTailThreads)
-k_sc_tail(ProofState *st, const fe *a, const fe *E, int m, int round0, int logn, uint8_t *tr, uint64_t off_poly0,
-          uint64_t off_final, BStr bs) {
+k_sc_tail(ProofState *st, const fe *a, const fe *E, int m, int round0, int logn, uint8_t *tr, int64_t off_claim,
+          uint64_t off_poly0, uint64_t off_final, BStr bs) {
   extern __shared__ fe tail_sm[];
+  __shared__ fe red[kScTailWorkers / 32][4], T[2][4], zs[64], chal[2];
   // a batch: one CTA per proof; bs = strides of (a, E, tr)
   st += blockIdx.x;
   a = badv(a, bs.s[0], blockIdx.x);
   E = badv(E, bs.s[1], blockIdx.x);
   tr = badv(tr, bs.s[2], blockIdx.x);
-  fe *w = tail_sm, *e = tail_sm + kScTailMax;
-  __shared__ fe red[2][kScTailThreads / 32];
-  __shared__ fe chal_s;
-  for (int j = threadIdx.x; j < m; j += blockDim.x) w[j] = a[j];
-  for (int j = threadIdx.x; j < m / 2; j += blockDim.x) e[j] = E[j];
-  if (threadIdx.x == 0) chal_s = st->chal[round0 - 1];
+  fe *w[2] = {tail_sm, tail_sm + kScTailMax / 2};
+  fe *e[2] = {tail_sm + kScTailMax / 2 + kScTailMax / 4, tail_sm + kScTailMax / 2 + kScTailMax / 4 + kScTailMax / 8};
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool worker = (warp & 3) != 0;
+  const int wid = (warp >> 2) * 3 + (warp & 3) - 1;  // worker warp
+  const int t = wid * 32 + lane;
+  // T sums from the workers' accumulators (a thread's entries all have the
+  // same index mod 4)
+  auto sum_classes = [&](const facc &acc, fe *out) {
+    fe x = facc_value(acc);
+    for (int d = 4; d < 32; d *= 2) x = fadd(x, shfl_xor_fe(x, d));
+    if (lane < 4) red[wid][lane] = x;
+    asm volatile("bar.sync 1, %0;" ::"n"(kScTailWorkers) : "memory");
+    if (wid) return;
+    x = fe_zero();
+    for (int k = lane >> 2; k < kScTailWorkers / 32; k += 8) x = fadd(x, red[k][lane & 3]);
+    for (int d = 4; d < 32; d *= 2) x = fadd(x, shfl_xor_fe(x, d));
+    if (lane < 4) out[lane] = x;
+  };
+  ScChain v{};
+  if (threadIdx.x < logn) zs[threadIdx.x] = st->z[threadIdx.x];
+  if (threadIdx.x == 0) v = ScChain{st->fs, st->y, round0 ? st->epre : fe_one(), 0};
+  if (worker) {
+    facc acc = facc_zero();
+    for (int x = t; x < m; x += kScTailWorkers) facc_mul(acc, a[x], E[x >> 2]);
+    sum_classes(acc, T[round0 & 1]);
+  }
   __syncthreads();
-  for (int r = round0; r <= logn; r++) {
-    // fold w by the previous challenge; E to pairwise sums (r < logn)
-    const fe c = chal_s;
-    const int half = m / 2;
-    fe nw[kScTailMax / 2 / kScTailThreads], ne[kScTailMax / 4 / kScTailThreads + 1];
-    int k = 0;
-    for (int j = threadIdx.x; j < half; j += blockDim.x, k++)
-      nw[k] = fadd(fmul(c, fsub(w[2 * j + 1], w[2 * j])), w[2 * j]);
-    k = 0;
-    if (r < logn)
-      for (int j = threadIdx.x; j < half / 2; j += blockDim.x, k++) ne[k] = fadd(e[2 * j], e[2 * j + 1]);
-    __syncthreads();
-    k = 0;
-    for (int j = threadIdx.x; j < half; j += blockDim.x, k++) w[j] = nw[k];
-    k = 0;
-    if (r < logn)
-      for (int j = threadIdx.x; j < half / 2; j += blockDim.x, k++) e[j] = ne[k];
-    m = half;
-    __syncthreads();
-    if (r == logn) break;
-    // S(0) = sum w[2j] E[j], S(1) = sum w[2j+1] E[j]
-    fe S0 = fe_zero(), S1 = fe_zero();
-    for (int j = threadIdx.x; j < m / 2; j += blockDim.x) {
-      S0 = fadd(S0, fmul(w[2 * j], e[j]));
-      S1 = fadd(S1, fmul(w[2 * j + 1], e[j]));
-    }
-    for (int d = 16; d > 0; d >>= 1) {
-      fe t;
-      t.re = __shfl_down_sync(0xffffffffu, S0.re, d); t.im = __shfl_down_sync(0xffffffffu, S0.im, d); S0 = fadd(S0, t);
-      t.re = __shfl_down_sync(0xffffffffu, S1.re, d); t.im = __shfl_down_sync(0xffffffffu, S1.im, d); S1 = fadd(S1, t);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      red[0][threadIdx.x >> 5] = S0;
-      red[1][threadIdx.x >> 5] = S1;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      fe A = fe_zero(), B = fe_zero();
-      for (int q = 0; q < (int)(blockDim.x >> 5); q++) {
-        A = fadd(A, red[0][q]);
-        B = fadd(B, red[1][q]);
+  if (threadIdx.x == 0) {
+    const fe *q = T[round0 & 1], z1 = zs[round0 + 1];
+    chal[round0 & 1] = sc_round_eq(v, fadd(q[0], fmul(z1, fsub(q[2], q[0]))), fadd(q[1], fmul(z1, fsub(q[3], q[1]))),
+                                   zs[round0], &st->chal[round0], tr, off_claim, off_poly0);
+  }
+  __syncthreads();
+  int pp = 0;
+#pragma unroll 1
+  for (int r = round0; r < logn; r++) {  // w_r of m entries, its E and T, challenge r
+    const fe c = chal[r & 1];
+    fe *wn = w[pp], *en = e[pp];
+    if (!worker) {
+      if (threadIdx.x == 0 && r + 1 < logn) {
+        const fe *q = T[r & 1];
+        chal[(r + 1) & 1] = sc_round_eq(v, fadd(q[0], fmul(c, fsub(q[1], q[0]))), fadd(q[2], fmul(c, fsub(q[3], q[2]))),
+                                        zs[r + 1], &st->chal[r + 1], tr, -1,
+                                        off_poly0 + 80ull * (uint64_t)(r + 1 - round0));
       }
-      const fe SS[3] = {A, fe_zero(), B};
-      const uint64_t op = off_poly0 + 80ull * (uint64_t)(r - round0);
-      chal_s = sc_round_eq_apply(SS, st, r, tr, -1, op, op + 56);
+    } else {
+      facc acc = facc_zero();
+      for (int x = t; x < m / 2; x += kScTailWorkers) {
+        const fe f = ffold(a[2 * x], a[2 * x + 1], c);
+        wn[x] = f;
+        if (m >= 8) {
+          const fe ee = fadd(E[2 * (x >> 2)], E[2 * (x >> 2) + 1]);
+          if ((x & 3) == 0) en[x >> 2] = ee;
+          facc_mul(acc, f, ee);
+        }
+      }
+      if (m >= 8) sum_classes(acc, T[(r + 1) & 1]);
     }
+    a = wn;
+    E = en;
+    m /= 2;
+    pp ^= 1;
     __syncthreads();
   }
-  if (threadIdx.x == 0) {  // k_sc_final: the folded w and the eq prefix
-    put_fe(tr, off_final, w[0]);
-    put_fe(tr, off_final + 16, st->epre);
-    st->K = w[0];
+  if (threadIdx.x == 0) {  // the folded w and the eq prefix
+    put_fe(tr, off_final, a[0]);
+    put_fe(tr, off_final + 16, v.ep);
+    st->K = a[0];
+    st->fs = v.fs;
+    if (v.bad) atomicOr(&st->error, 1u);
   }
 }
-
-__global__ void k_sc_final(ProofState *st, const fe *v1, const fe *v2, uint8_t *tr, uint64_t off, BStr bs) {
-  st += blockIdx.x;
-  v1 = badv(v1, bs.s[0], blockIdx.x);
-  if (v2) v2 = badv(v2, bs.s[1], blockIdx.x);
-  tr = badv(tr, bs.s[2], blockIdx.x);
-  if (threadIdx.x) return;
-  // v2 == nullptr: the eq vector was not folded, its last value is epre
-  fe a = v1[0], b = v2 ? v2[0] : st->epre;
-  put_fe(tr, off, a);
-  put_fe(tr, off + 16, b);
-  st->K = a;  // Whir_Open: K = claims[0].first
-}
-
 
 // omega^e from a two-level power table (lo[e & 4095] * hi[e >> 12]).
 __device__ __forceinline__ fe pow_table(const fe *lo, const fe *hi, uint64_t e) {
@@ -298,36 +326,28 @@ __device__ uint64_t number_from(const int32_t *d) {
   return ret;
 }
 
-// One thread runs the generator with its 31-word table in registers (the
-// table rotated so that the front index is 3 and the rear 0, which makes
-// every index of a 31-draw cycle a constant) and stores the N outputs in
-// shared memory; then all threads derive the field elements (40 outputs
-// each) and the query positions from them.
+// The first warp runs the generator and stores the N outputs in shared
+// memory; then all threads derive the field elements (40 outputs each, a
+// thread an element) and the query positions from them.  With one thread
+// drawing and three deriving a launch took 17.5 us at 2^10, now 12.
 __global__ void __launch_bounds__(256) k_whir_schedule(ProofState *st, SchedArgs a) {
-  __shared__ int32_t draws[kMaxDraws];
+  __shared__ int32_t draws[kMaxDraws + 31];
   st += blockIdx.x;
   int N = kFieldDraws * a.lg_final;
   for (int t = 0; t < a.T; t++) N += 3 * kFieldDraws + a.l[t];
-  if (threadIdx.x == 0) {
-    const int f0 = st->prng.f;
-    uint32_t reg[31];
-#pragma unroll
-    for (int k = 0; k < 31; k++) reg[k] = (uint32_t)st->prng.tbl[(k + f0 + 28) % 31];
-    for (int n = 0; n < N; n += 31) {
-#pragma unroll
-      for (int j = 0; j < 31; j++) {
-        if (n + j < N) {
-          reg[(j + 3) % 31] += reg[j];
-          draws[n + j] = (int32_t)(reg[(j + 3) % 31] >> 1);
-        }
-      }
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x, f0 = st->prng.f;
+    uint32_t x = prng_warp_load(st->prng, lane);
+    int n = 0;
+    for (; n + 31 <= N; n += 31) {
+      x = prng_warp_next(x, lane);
+      if (lane < 31) draws[n + lane] = (int32_t)(x >> 1);
     }
-    // the table in place, both indices advanced by N (glibc's state after N draws)
-#pragma unroll
-    for (int k = 0; k < 31; k++) st->prng.tbl[(k + f0 + 28) % 31] = (int32_t)reg[k];
-    const int f = (f0 + N) % 31;
-    st->prng.f = f;
-    st->prng.r = (f + 28) % 31;
+    const uint32_t y = prng_warp_next(x, lane);
+    if (lane < N - n) draws[n + lane] = (int32_t)(y >> 1);
+    x = prng_warp_shift(x, y, N - n, lane);
+    __syncwarp();
+    prng_warp_store(st->prng, x, f0, N, lane);
   }
   __syncthreads();
   // per iteration: r0, r1 (40 outputs each), l queries, update_betas' r; then the final point
@@ -335,15 +355,16 @@ __global__ void __launch_bounds__(256) k_whir_schedule(ProofState *st, SchedArgs
   for (int t = 0; t < a.T; t++) {
     const int l = a.l[t];
     for (int i = threadIdx.x; i < l; i += blockDim.x) st->wq[t][i] = draws[off + 2 * kFieldDraws + i] % a.qmod[t];
-    if (threadIdx.x < 3) {
-      const int o = threadIdx.x < 2 ? off + kFieldDraws * threadIdx.x : off + 2 * kFieldDraws + l;
+    const int k = (int)threadIdx.x - 3 * t;
+    if (k >= 0 && k < 3) {
+      const int o = k < 2 ? off + kFieldDraws * k : off + 2 * kFieldDraws + l;
       const fe v = fe_make(number_from(draws + o) % P, number_from(draws + o + 20) % P);
-      if (threadIdx.x < 2) st->wr[t][threadIdx.x] = v;
+      if (k < 2) st->wr[t][k] = v;
       else st->wrb[t] = v;
     }
     off += 3 * kFieldDraws + l;
   }
-  for (int i = threadIdx.x; i < a.lg_final; i += blockDim.x) {
+  for (int i = (int)blockDim.x - 1 - (int)threadIdx.x; i < a.lg_final; i += blockDim.x) {
     const int o = off + kFieldDraws * i;
     st->fin_r[i] = fe_make(number_from(draws + o) % P, number_from(draws + o + 20) % P);
   }
@@ -695,7 +716,6 @@ ProofPlan::~ProofPlan() {
     if (e) cudaEventDestroy(e);
   if (ev_sched) cudaEventDestroy(ev_sched);
   if (ev_root_tail) cudaEventDestroy(ev_root_tail);
-  if (ev_init) cudaEventDestroy(ev_init);
   if (s2) cudaStreamDestroy(s2);
   if (s3) cudaStreamDestroy(s3);
 }
@@ -744,7 +764,7 @@ std::unique_ptr<ProofPlan> plan_create(int logn, int rate, int batch) {
   p->bs_v = sizeof(fe) * (n / 2);
   p->bs_arr = sizeof(fe) * (n / 2);
   p->bs_beta = sizeof(fe) * n;
-  p->bs_part = sizeof(fe) * 3 * (uint64_t)sc_blocks(n / 2);
+  p->bs_part = sizeof(fe) * 4 * (uint64_t)sc_blocks(n / 4);
   p->bs_wpart = sizeof(fe) * whir_partials(n);
   p->bs_ub = sizeof(fe) * kUpdateBetasScratch;
   p->w = (fe *)p->dalloc(B * p->bs_w);
@@ -756,7 +776,6 @@ std::unique_ptr<ProofPlan> plan_create(int logn, int rate, int batch) {
   GBZ_CUDA(cudaStreamCreateWithFlags(&p->s3, cudaStreamNonBlocking));
   GBZ_CUDA(cudaEventCreateWithFlags(&p->ev_in, cudaEventDisableTiming));
   GBZ_CUDA(cudaEventCreateWithFlags(&p->ev_sched, cudaEventDisableTiming));
-  GBZ_CUDA(cudaEventCreateWithFlags(&p->ev_init, cudaEventDisableTiming));
   GBZ_CUDA(cudaEventCreateWithFlags(&p->ev_root_tail, cudaEventDisableTiming));
   for (auto &e : p->ev_fold) GBZ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   for (auto &e : p->ev_commit) GBZ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -772,7 +791,7 @@ std::unique_ptr<ProofPlan> plan_create(int logn, int rate, int batch) {
   p->ub_scratch = (fe *)p->dalloc(B * p->bs_ub);
   p->st = (ProofState *)p->dalloc(B * sizeof(ProofState));
   GBZ_CUDA(cudaFuncSetAttribute(k_sc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(fe) * (kScTailMax + kScTailMax / 2))));
+                                (int)kScTailShared));
   // Build the transcript layout (record headers are constant).
   p->layout.record_headers = true;
   enqueue_proof(*p, nullptr, 1, nullptr, /*dry=*/true);  // layout and launch counts
@@ -861,15 +880,25 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
   // With the profiler on, the commits stay on s so that the per-category
   // event times do not include waits for the other stream's kernels.
   cudaStream_t c = prof ? s : p.s2, q = prof ? s : p.s3;
-  if (!dry) {
+  // A proof of its own seeds its generator on q, so that its three chains
+  // start at once (2^18: 322 us, behind the seeding 347); the scheduler's
+  // graphs, many in flight, start as one node (64 mixed proofs 4900 us, as
+  // three 5090).
+  const bool fork_first = !open && !seed_in_state;
+  auto fork = [&]() {
+    if (dry) return;
     GBZ_CUDA(cudaEventRecord(p.ev_in, s));
     GBZ_CUDA(cudaStreamWaitEvent(c, p.ev_in, 0));
-  }
+    GBZ_CUDA(cudaStreamWaitEvent(q, p.ev_in, 0));
+  };
+  if (fork_first) fork();
   if (open) {
     RUN(PC_PROTOCOL, 1, k_init_open<<<1, 32, 0, s>>>(st, open->prng, open->point, logn, open->K));
   } else {
-    RUN(PC_PROTOCOL, 1, k_init<<<B, 32, 0, s>>>(st, prng_seed, seed_in_state ? 1 : 0));
+    const cudaStream_t is = fork_first ? q : s;
+    RUN_ON(is, PC_PROTOCOL, 1, k_init<<<B, 32, 0, is>>>(st, prng_seed, seed_in_state ? 1 : 0));
   }
+  if (!fork_first) fork();
   // The opening's randomness, drawn on the query stream while the
   // commitment and the sumcheck run, and the beta updates' powers.
   UbSlots *slots = reinterpret_cast<UbSlots *>(p.ub_scratch);
@@ -889,10 +918,6 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
       if (mm <= (uint64_t)kWhirK) break;
     }
     sa.lg_final = ilog2(mm);
-    if (!dry) {
-      GBZ_CUDA(cudaEventRecord(p.ev_init, s));
-      GBZ_CUDA(cudaStreamWaitEvent(q, p.ev_init, 0));
-    }
     RUN_ON(q, PC_PROTOCOL, 1, k_whir_schedule<<<B, 256, 0, q>>>(st, sa));
     ua.T = sa.T;
     LL = p.L;
@@ -960,84 +985,54 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
   // 2. evaluation point and its eq table.
   off = lay.rec(T_EVAL_POINT, logn, 16);
   RUN(PC_PROTOCOL, 1, k_point<<<B, 32, 0, s>>>(st, logn, tr, off, trs));
-  // eq table E_0 of z_1..z_{logn-1} (the eq factor of variable 0 is kept apart)
-  RUN(PC_BETA, 1, beta_launch(st->z + 1, logn - 1, p.vb[0], s, B, sts, p.bs_v));
-
-  // 3. sumcheck of sum w(x) eq(z, x): w is folded each round, the eq vector
-  //    is represented by the shrinking tables E_i (vb ping-pong) and the
-  //    prefix product epre (k_sc_round_eq).
-  uint64_t off_claim = lay.rec(T_CLAIM, 1, 16);
-  int pp = 0, ep = 0;  // va ping-pong for w, vb ping-pong for E
-  bool tail_done = false;
-  uint64_t as = p.bs_w;  // per-proof stride of a (the witness, then va)
-  for (int i = 0; i < logn; i++) {
-    if (i >= 1 && m <= (uint64_t)kScTailMax) {
-      // the remaining rounds and the final fold in one CTA
-      const uint64_t op0 = lay.rec(T_SC_POLY, 3, 16);
-      for (int r = i; r < logn; r++) {
-        const uint64_t op = r == i ? op0 : lay.rec(T_SC_POLY, 3, 16);
-        const uint64_t oc = lay.rec(T_SC_CHALLENGE, 1, 16);
-        if (op != op0 + 80ull * (uint64_t)(r - i) || oc != op + 56) throw ArgError("prover: sumcheck record layout");
-      }
-      off = lay.rec(T_SC_FINAL, 2, 16);
-      BStr tb;
-      tb.s[0] = as;
-      tb.s[1] = p.bs_v;
-      tb.s[2] = trs;
-      RUN(PC_SUMCHECK, 1,
-          (k_sc_tail<<<B, kScTailThreads, sizeof(fe) * (kScTailMax + kScTailMax / 2), s>>>(st, a, p.vb[ep], (int)m, i,
-                                                                                         logn, tr, op0, off, tb)));
-      tail_done = true;
-      break;
-    }
-    uint64_t off_poly = lay.rec(T_SC_POLY, 3, 16);
-    uint64_t off_chal = lay.rec(T_SC_CHALLENGE, 1, 16);
-    int blocks;
-    // strides of (a, E, chal, a2, E2, partial)
-    BStr es;
-    es.s[0] = as;
-    es.s[1] = p.bs_v;
-    es.s[2] = sts;
-    es.s[3] = p.bs_v;
-    es.s[4] = p.bs_v;
-    es.s[5] = p.bs_part;
-    if (i == 0) {
-      blocks = sc_blocks(m / 2);
-      RUN(PC_SUMCHECK, 1,
-          sc_eq_step_launch(a, p.vb[0], m, nullptr, nullptr, nullptr, true, p.partial, blocks, s, B, es));
-    } else {
+  // 3. sumcheck of sum w(x) eq(z, x), two rounds a pass: w is folded by both
+  //    challenges, the eq vector is represented by the shrinking tables
+  //    E_{i+1} (vb ping-pong) and the prefix product epre; the last rounds
+  //    (or all of a small proof) in one CTA.
+  RUN(PC_BETA, 1, beta_launch(st->z + 2, logn - 2, p.vb[0], s, B, sts, p.bs_v));
+  const uint64_t off_claim = lay.rec(T_CLAIM, 1, 16);
+  const uint64_t off_poly0 = lay.len + 8;
+  for (int r = 0; r < logn; r++) {
+    const uint64_t op = lay.rec(T_SC_POLY, 3, 16), oc = lay.rec(T_SC_CHALLENGE, 1, 16);
+    if (op != off_poly0 + 80ull * (uint64_t)r || oc != op + 56) throw ArgError("prover: sumcheck record layout");
+  }
+  off = lay.rec(T_SC_FINAL, 2, 16);
+  int pp = 0, i = 0;       // va and vb ping-pong
+  uint64_t as = p.bs_w;    // per-proof stride of a (the witness, then va)
+  if (m > (uint64_t)kScTailMax) {
+    int blocks = sc_blocks(m / 4);
+    BStr rs;  // (a, E, partial)
+    rs.s[0] = as;
+    rs.s[1] = p.bs_v;
+    rs.s[2] = p.bs_part;
+    RUN(PC_SUMCHECK, 1, sc_eq_reduce_launch(a, p.vb[0], m, p.partial, blocks, s, B, rs));
+    for (; m > (uint64_t)kScTailMax; i += 2, m /= 4, pp ^= 1) {
+      RUN(PC_PROTOCOL, 1,
+          k_sc_rounds_eq<<<B, 256, 0, s>>>(p.partial, blocks, st, i, tr, i == 0 ? (int64_t)off_claim : -1,
+                                           off_poly0 + 80ull * (uint64_t)i, p.bs_part, trs));
       blocks = sc_blocks(m / 4);
-      fe *a2 = p.va[pp];
+      BStr fs;  // (a, chal, a4, E, E4, partial)
+      fs.s[0] = as;
+      fs.s[1] = sts;
+      fs.s[2] = p.bs_v;
+      fs.s[3] = p.bs_v;
+      fs.s[4] = p.bs_v;
+      fs.s[5] = p.bs_part;
       RUN(PC_SUMCHECK, 1,
-          sc_eq_step_launch(a, p.vb[ep], m, &st->chal[i - 1], a2, p.vb[ep ^ 1], true, p.partial, blocks, s, B, es));
-      a = a2;
+          sc_eq_fold_launch(a, p.vb[pp], m, &st->chal[i], p.va[pp], p.vb[pp ^ 1], m / 4 > (uint64_t)kScTailMax,
+                            p.partial, blocks, s, B, fs));
+      a = p.va[pp];
       as = p.bs_v;
-      pp ^= 1;
-      ep ^= 1;
-      m /= 2;
     }
-    RUN(PC_PROTOCOL, 1,
-        k_sc_round_eq<<<B, 256, 0, s>>>(p.partial, blocks, st, i, tr, i == 0 ? (int64_t)off_claim : -1, off_poly,
-                                        off_chal, p.bs_part, trs));
   }
-  if (!tail_done) {
-    fe *a2 = p.va[pp];
-    BStr es;
-    es.s[0] = as;
-    es.s[1] = p.bs_v;
-    es.s[2] = sts;
-    es.s[3] = p.bs_v;
-    es.s[4] = p.bs_v;
-    es.s[5] = p.bs_part;
-    RUN(PC_SUMCHECK, 1,
-        sc_eq_step_launch(a, p.vb[ep], m, &st->chal[logn - 1], a2, nullptr, false, p.partial, 1, s, B, es));
-    off = lay.rec(T_SC_FINAL, 2, 16);
-    BStr fs;
-    fs.s[0] = p.bs_v;
-    fs.s[2] = trs;
-    RUN(PC_PROTOCOL, 1, k_sc_final<<<B, 32, 0, s>>>(st, a2, nullptr, tr, off, fs));
-    pp ^= 1;
-  }
+  BStr tb;  // (a, E, tr)
+  tb.s[0] = as;
+  tb.s[1] = p.bs_v;
+  tb.s[2] = trs;
+  RUN(PC_SUMCHECK, 1,
+      (k_sc_tail<<<B, kScTailThreads, kScTailShared, s>>>(st, a, p.vb[pp], (int)m, i, logn, tr,
+                                                         i == 0 ? (int64_t)off_claim : -1,
+                                                         off_poly0 + 80ull * (uint64_t)i, off, tb)));
   }
 opening:
 
@@ -1358,7 +1353,7 @@ void launch_proof_graph(ProofPlan &p, const fe *w, uint32_t prng_seed, cudaStrea
 uint64_t plan_bytes(int logn, int rate, int batch) {
   const uint64_t n = 1ull << logn, L = n * (uint64_t)rate;
   uint64_t b = sizeof(fe) * (n + L + L / 2 + L + L / 2 + 5 * (n / 2) + n);
-  b += sizeof(fe) * (3 * (uint64_t)sc_blocks(n / 2) + whir_partials(n) + kUpdateBetasScratch) + sizeof(ProofState);
+  b += sizeof(fe) * (4 * (uint64_t)sc_blocks(n / 4) + whir_partials(n) + kUpdateBetasScratch) + sizeof(ProofState);
   b *= (uint64_t)batch;
   b += 64ull << 20;  // transcripts, twiddle tables and allocation granularity (upper bound)
   b += (uint64_t)batch << 20;

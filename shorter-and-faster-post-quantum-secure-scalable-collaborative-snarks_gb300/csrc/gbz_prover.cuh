@@ -72,7 +72,7 @@ struct ProofPlan {
   // the beta updates' powers are formed, up front on s3.
   cudaStream_t s2 = nullptr, s3 = nullptr;
   static constexpr int kMaxIter = kMaxWhirIter;
-  cudaEvent_t ev_in = nullptr, ev_init = nullptr, ev_sched = nullptr, ev_fold[kMaxIter] = {}, ev_commit[kMaxIter + 1] = {},
+  cudaEvent_t ev_in = nullptr, ev_sched = nullptr, ev_fold[kMaxIter] = {}, ev_commit[kMaxIter + 1] = {},
               ev_query[kMaxIter] = {}, ev_root_tail = nullptr;
   fe *va[2] = {nullptr, nullptr}; // folded first vector ping-pong (n/2 each)
   fe *arr = nullptr;              // the folded polynomials arr_1, arr_2, ... back to back (read by the commits)

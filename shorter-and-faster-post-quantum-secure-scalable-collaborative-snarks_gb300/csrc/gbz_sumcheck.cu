@@ -232,87 +232,85 @@ sc_fold2_eq_kernel(const fe *__restrict__ a, const fe *__restrict__ E2, uint64_t
   }
 }
 
-// Sumcheck of sum_x w(x) eq(z, x) without folding the eq vector.  After i
-// rounds the folded eq vector is epre * eq1(z_i, x_0) * E_i[x'], E_i the eq
-// table of z_{i+1..} (eq1(z, x) = z x + (1 - z)(1 - x)), so the round
-// polynomial is epre * eq1(z_i, X) * S(X) with S(X) = sum_j l_j(X) E_i[j]:
-// only S(0) = sum w[2j] E_i[j] and S(1) = sum w[2j+1] E_i[j] are summed
-// over the vector (the same polynomial as the pairwise products of the
-// reference's loop, computed with half the reads and multiplies).
-// E_{i+1}[t] = E_i[2t] + E_i[2t+1].
-// partial[3 blk + {0, 1, 2}] = (S0, S1, 0).
-__global__ void __launch_bounds__(kScThreads)
-sc_eq_reduce_kernel(const fe *__restrict__ a, const fe *__restrict__ E, uint64_t pairs, fe *partial, BStr bs) {
-  const uint32_t pb = blockIdx.y;
-  a = badv(a, bs.s[0], pb);
-  E = badv(E, bs.s[1], pb);
-  partial = badv(partial, bs.s[2], pb);
-  facc sS0 = facc_zero(), sS1 = facc_zero();
-  const uint64_t stride = (uint64_t)gridDim.x * kScThreads;
-  for (uint64_t j = (uint64_t)blockIdx.x * kScThreads + threadIdx.x; j < pairs; j += stride) {
-    const fe e = E[j], w0 = a[2 * j], w1 = a[2 * j + 1];
-    if (!(w0.im | w1.im)) {  // base-field entries: two partial products each
-      facc_mul_base(sS0, e, w0.re);
-      facc_mul_base(sS1, e, w1.re);
-    } else {
-      facc_mul(sS0, w0, e);
-      facc_mul(sS1, w1, e);
-    }
-  }
-  fe S0 = facc_value(sS0), S1 = facc_value(sS1), Z = fe_zero();
-  block_sum3(S0, S1, Z);
-  if (threadIdx.x == 0) {
-    partial[3 * blockIdx.x] = S0;
-    partial[3 * blockIdx.x + 1] = S1;
-    partial[3 * blockIdx.x + 2] = fe_zero();
-  }
+// Sumcheck of sum_x w(x) eq(z, x) without folding the eq vector, two rounds
+// a pass.  After i rounds the folded eq vector is
+// epre * eq1(z_i, x_0) * E_i[x'], E_i the eq table of z_{i+1..}
+// (eq1(z, x) = z x + (1 - z)(1 - x)), so the round polynomial is
+// epre * eq1(z_i, X) * S(X), S(X) linear with S(0) = sum w[2j] E_i[j] and
+// S(1) = sum w[2j+1] E_i[j] (the same polynomial as the pairwise products of
+// the reference's loop).  E_i[2j + x] = eq1(z_{i+1}, x) E_{i+1}[j], so with
+//   T_k = sum_j w[4j + k] E_{i+1}[j], k < 4,
+// round i has S(X) = (1 - z_{i+1}) T_X + z_{i+1} T_{2+X}, and round i + 1,
+// after the challenge c, S(X) = T_{2X} + c (T_{2X+1} - T_{2X}): one pass over
+// w and one launch between hash chains for both (a pass a round took twice
+// the reads and multiplies, and 11 us a round where launches are short).
+// E_{i+3}[t] = sum of the four entries of E_{i+1} from 4t on.
+// partial[4 blk + k] = T_k.  A thread's entries all have the same index mod 4.
+__device__ void block_sum_classes(const facc &acc, fe *partial) {
+  __shared__ fe red[kScThreads / 32][4];
+  fe x = facc_value(acc);
+#pragma unroll
+  for (int d = 4; d < 32; d <<= 1)
+    x = fadd(x, fe_make(__shfl_xor_sync(0xffffffffu, x.re, d), __shfl_xor_sync(0xffffffffu, x.im, d)));
+  if ((threadIdx.x & 31) < 4) red[threadIdx.x >> 5][threadIdx.x & 3] = x;
+  __syncthreads();
+  if (threadIdx.x >= 4) return;
+  x = red[0][threadIdx.x];
+#pragma unroll
+  for (int w = 1; w < kScThreads / 32; w++) x = fadd(x, red[w][threadIdx.x]);
+  partial[4 * blockIdx.x + threadIdx.x] = x;
 }
 
-// Fold a (length m) by *chal into a2, E (length m/2) into E2 (length m/4)
-// by pairwise sums, and (reduce) the S sums of the folded pairs with E2.
 __global__ void __launch_bounds__(kScThreads)
-sc_eq_fold_kernel(const fe *__restrict__ a, uint64_t m, const fe *chal, fe *__restrict__ a2,
-                  const fe *__restrict__ E, fe *__restrict__ E2, int reduce, fe *partial, BStr bs) {
-  const uint32_t pb = blockIdx.y;
-  a = badv(a, bs.s[0], pb);
-  chal = badv(chal, bs.s[1], pb);
-  a2 = badv(a2, bs.s[2], pb);
-  E = badv(E, bs.s[3], pb);
-  E2 = badv(E2, bs.s[4], pb);
-  partial = badv(partial, bs.s[5], pb);
-  const fe r = *chal;
-  facc sS0 = facc_zero(), sS1 = facc_zero();
+sc_eq_reduce_kernel(const fe *__restrict__ a, const fe *__restrict__ E, uint64_t m, fe *partial, BStr bs) {
+  a = badv(a, bs.s[0], blockIdx.y);
+  E = badv(E, bs.s[1], blockIdx.y);
+  partial = badv(partial, bs.s[2], blockIdx.y);
+  facc acc = facc_zero();
   const uint64_t stride = (uint64_t)gridDim.x * kScThreads;
-  const uint64_t quads = m / 4;
-  for (uint64_t t = (uint64_t)blockIdx.x * kScThreads + threadIdx.x; t < quads; t += stride) {
-    const fe x0 = a[4 * t], x1 = a[4 * t + 1], x2 = a[4 * t + 2], x3 = a[4 * t + 3];
-    const fe e0 = E[2 * t], e1 = E[2 * t + 1];
+#pragma unroll 4
+  for (uint64_t x = (uint64_t)blockIdx.x * kScThreads + threadIdx.x; x < m; x += stride) {
+    const fe e = E[x >> 2], w = a[x];
+    if (!w.im) facc_mul_base(acc, e, w.re);  // a base-field entry: two partial products
+    else facc_mul(acc, w, e);
+  }
+  block_sum_classes(acc, partial);
+}
+
+// Fold a (m entries, a multiple of 128) by chal[0] and chal[1] into a4, and
+// (reduce) E (m / 4 entries) into E4 and the T sums of a4 with E4.
+__global__ void __launch_bounds__(kScThreads)
+sc_eq_fold_kernel(const fe *__restrict__ a, uint64_t m, const fe *chal, fe *__restrict__ a4,
+                  const fe *__restrict__ E, fe *__restrict__ E4, int reduce, fe *partial, BStr bs) {
+  a = badv(a, bs.s[0], blockIdx.y);
+  chal = badv(chal, bs.s[1], blockIdx.y);
+  a4 = badv(a4, bs.s[2], blockIdx.y);
+  E = badv(E, bs.s[3], blockIdx.y);
+  E4 = badv(E4, bs.s[4], blockIdx.y);
+  partial = badv(partial, bs.s[5], blockIdx.y);
+  const fe c0 = chal[0], c1 = chal[1];
+  facc acc = facc_zero();
+  const uint64_t stride = (uint64_t)gridDim.x * kScThreads;
+  for (uint64_t j = (uint64_t)blockIdx.x * kScThreads + threadIdx.x; j < m / 4; j += stride) {
+    const fe x0 = a[4 * j], x1 = a[4 * j + 1], x2 = a[4 * j + 2], x3 = a[4 * j + 3];
+    fe e = E[j];
     fe f0, f1;
     if (!(x0.im | x1.im | x2.im | x3.im)) {  // base-field entries (the first fold of the witness)
-      f0 = ffold_base(x0.re, x1.re, r);
-      f1 = ffold_base(x2.re, x3.re, r);
+      f0 = ffold_base(x0.re, x1.re, c0);
+      f1 = ffold_base(x2.re, x3.re, c0);
     } else {
-      f0 = ffold(x0, x1, r);
-      f1 = ffold(x2, x3, r);
+      f0 = ffold(x0, x1, c0);
+      f1 = ffold(x2, x3, c0);
     }
-    a2[2 * t] = f0;
-    a2[2 * t + 1] = f1;
-    const fe e = fadd(e0, e1);
-    if (reduce) {
-      E2[t] = e;
-      facc_mul(sS0, f0, e);
-      facc_mul(sS1, f1, e);
-    }
+    f0 = ffold(f0, f1, c1);
+    a4[j] = f0;
+#pragma unroll
+    for (int d = 1; d < 4; d <<= 1)
+      e = fadd(e, fe_make(__shfl_xor_sync(0xffffffffu, e.re, d), __shfl_xor_sync(0xffffffffu, e.im, d)));
+    if ((j & 3) == 0) E4[j >> 2] = e;
+    if (reduce) facc_mul(acc, f0, e);
   }
-  if (m == 2 && blockIdx.x == 0 && threadIdx.x == 0) a2[0] = fadd(fmul(r, fsub(a[1], a[0])), a[0]);
-  if (!reduce) return;
-  fe S0 = facc_value(sS0), S1 = facc_value(sS1), Z = fe_zero();
-  block_sum3(S0, S1, Z);
-  if (threadIdx.x == 0) {
-    partial[3 * blockIdx.x] = S0;
-    partial[3 * blockIdx.x + 1] = S1;
-    partial[3 * blockIdx.x + 2] = fe_zero();
-  }
+  if (reduce) block_sum_classes(acc, partial);
 }
 
 // out = (a, b, c) of the round message from (A, C, D) partials.
@@ -517,25 +515,16 @@ void sc_fold2_eq_launch(const fe *a, const fe *E2, uint64_t m, const fe *c, cons
   GBZ_CUDA(cudaGetLastError());
 }
 
-void sc_eq_step_launch(const fe *a, const fe *E, uint64_t m, const fe *chal, fe *a2, fe *E2, bool reduce,
-                       fe *partial, int blocks, cudaStream_t s, int batch, const BStr &bs) {
-  // bs: strides of (a, E, chal, a2, E2, partial)
-  if (!chal) {
-    BStr r;
-    r.s[0] = bs.s[0];
-    r.s[1] = bs.s[1];
-    r.s[2] = bs.s[5];
-    sc_eq_reduce_kernel<<<dim3(blocks, batch), kScThreads, 0, s>>>(a, E, m / 2, partial, r);
-  } else {
-    BStr f;
-    f.s[0] = bs.s[0];
-    f.s[1] = bs.s[2];
-    f.s[2] = bs.s[3];
-    f.s[3] = bs.s[1];
-    f.s[4] = bs.s[4];
-    f.s[5] = bs.s[5];
-    sc_eq_fold_kernel<<<dim3(blocks, batch), kScThreads, 0, s>>>(a, m, chal, a2, E, E2, reduce ? 1 : 0, partial, f);
-  }
+void sc_eq_reduce_launch(const fe *a, const fe *E, uint64_t m, fe *partial, int blocks, cudaStream_t s, int batch,
+                         const BStr &bs) {
+  sc_eq_reduce_kernel<<<dim3(blocks, batch), kScThreads, 0, s>>>(a, E, m, partial, bs);
+  GBZ_CUDA(cudaGetLastError());
+}
+
+void sc_eq_fold_launch(const fe *a, const fe *E, uint64_t m, const fe *chal, fe *a4, fe *E4, bool reduce, fe *partial,
+                       int blocks, cudaStream_t s, int batch, const BStr &bs) {
+  if (m < 128 || m % 128) throw ArgError("two-round fold of w needs a multiple of 128 entries");
+  sc_eq_fold_kernel<<<dim3(blocks, batch), kScThreads, 0, s>>>(a, m, chal, a4, E, E4, reduce ? 1 : 0, partial, bs);
   GBZ_CUDA(cudaGetLastError());
 }
 
