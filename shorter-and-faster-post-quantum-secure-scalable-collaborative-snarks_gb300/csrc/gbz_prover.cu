@@ -698,13 +698,13 @@ uint64_t Layout::rec(uint32_t tag, uint32_t count, uint32_t unit) {
   return off + 8;
 }
 
+namespace {
+void graph_free(ProofGraph &g);
+}
 ProofPlan::~ProofPlan() {
   if (s2) cudaStreamSynchronize(s2);
   if (s3) cudaStreamSynchronize(s3);
-  for (auto &g : graphs) {
-    if (g.exec) cudaGraphExecDestroy(g.exec);
-    if (g.graph) cudaGraphDestroy(g.graph);
-  }
+  for (auto &g : graphs) graph_free(g);
   for (auto &kv : ntt) ntt_tables_free(kv.second);
   for (void *p : allocs) cudaFree(p);
   if (ev_in) cudaEventDestroy(ev_in);
@@ -842,7 +842,7 @@ void plan_prepare_open(ProofPlan &p) {
 // The dry run (dry = true) launches nothing; it fixes the transcript layout
 // and counts the launches per category.
 void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStream_t s, bool dry, bool seed_in_state,
-                   const OpenOnly *open) {
+                   const OpenOnly *open, ProofPart part) {
   Layout &lay = p.layout;
   lay.len = 0;
   if (dry) {
@@ -859,6 +859,9 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
   const uint64_t trs = p.transcript_bytes, sts = sizeof(ProofState);
   const uint64_t cw_s[2] = {p.bs_cw0, p.bs_cw1};
   Profiler *prof = (!dry && p.prof && p.prof->enabled) ? p.prof : nullptr;
+  // Whether what comes next is enqueued: not in the dry run, and not what
+  // another part holds.
+  bool go = !dry && part != PART_OPENING;
   // RUN(category, kernel launches, statement): counts in the dry run, else
   // runs the statement (bracketed by profiler events when enabled).
 #define RUN_ON(strm, cat, nlaunch, ...)        \
@@ -866,7 +869,7 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
     if (dry) {                                 \
       p.launches += (nlaunch);                 \
       p.cat_launches[cat] += (nlaunch);        \
-    } else {                                   \
+    } else if (go) {                           \
       if (prof) prof->begin(cat, strm);        \
       __VA_ARGS__;                             \
       GBZ_CUDA(cudaGetLastError());            \
@@ -886,7 +889,7 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
   // three 5090).
   const bool fork_first = !open && !seed_in_state;
   auto fork = [&]() {
-    if (dry) return;
+    if (!go) return;
     GBZ_CUDA(cudaEventRecord(p.ev_in, s));
     GBZ_CUDA(cudaStreamWaitEvent(c, p.ev_in, 0));
     GBZ_CUDA(cudaStreamWaitEvent(q, p.ev_in, 0));
@@ -899,93 +902,19 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
     RUN_ON(is, PC_PROTOCOL, 1, k_init<<<B, 32, 0, is>>>(st, prng_seed, seed_in_state ? 1 : 0));
   }
   if (!fork_first) fork();
-  // The opening's randomness, drawn on the query stream while the
-  // commitment and the sumcheck run, and the beta updates' powers.
-  UbSlots *slots = reinterpret_cast<UbSlots *>(p.ub_scratch);
-  UbPrepArgs ua{};
-  {
-    SchedArgs sa{};
-    uint64_t mm = p.n, LL = p.L, cc = (uint64_t)p.rate;
-    for (;;) {
-      if (sa.T >= kMaxWhirIter) throw ArgError("prover: too many WHIR iterations");
-      mm /= 4;
-      sa.l[sa.T] = whir_query_count((int)cc);
-      sa.qmod[sa.T] = (int32_t)(LL / 4);
-      if (sa.l[sa.T] < 1 || sa.l[sa.T] > kMaxQueries) throw ArgError("prover: query count out of range");
-      sa.T++;
-      LL = 2 * cc * mm;
-      cc *= 2;
-      if (mm <= (uint64_t)kWhirK) break;
-    }
-    sa.lg_final = ilog2(mm);
-    RUN_ON(q, PC_PROTOCOL, 1, k_whir_schedule<<<B, 256, 0, q>>>(st, sa));
-    ua.T = sa.T;
-    LL = p.L;
-    mm = p.n;
-    for (int t = 0; t < sa.T; t++) {
-      LL /= 2;
-      mm /= 4;
-      ua.base[t + 1] = ua.base[t] + sa.l[t];
-      ua.per[t] = update_betas_per(mm, B);
-      if (dry) continue;
-      const NttTables &tnew = p.tables(ilog2(LL));
-      ua.lo[t] = tnew.lo_fwd;
-      ua.hi[t] = tnew.hi_fwd;
-    }
-    if (ua.base[sa.T] > kUbSlots) throw ArgError("prover: too many queries");
-    RUN_ON(q, PC_UPDATE_BETAS, 1,
-           k_ub_prep<<<dim3((unsigned)(ua.base[sa.T] + 3) / 4, B), 128, 0, q>>>(st, slots, p.bs_ub, ua));
-    if (!dry) GBZ_CUDA(cudaEventRecord(p.ev_sched, q));
-  }
-
-  // 1. commitment: codeword = NTT(w padded to rate*n), Merkle tree.
-  uint64_t L = p.L;
-  int cwi = 0;
-  uint64_t off = lay.rec(T_COMMIT_ROOT, 1, 32);
-  // The witness is expected in the base field (the imaginary words zero):
-  // its transform is then a half-length transform of packed pairs
-  // (ntt_launch_real); any other witness takes the general transform.
-  if (open) {
-    if (!dry && open->codeword != p.cw[0])
-      GBZ_CUDA(cudaMemcpyAsync(p.cw[0], open->codeword, 16 * L, cudaMemcpyDeviceToDevice, c));
-  } else if (B > 1 && ilog2(L) < kBatchRealLog) {
-    // short codewords (launch bound): the batch's codewords as one batched
-    // transform (the same values as the real-input path of a single proof)
-    RUN_ON(c, PC_NTT, ntt_launch_count(ilog2(L)),
-           ntt_launch_rows(p.tables(ilog2(L)), w, p.n, p.bs_w / sizeof(fe), p.cw[0], p.bs_cw0 / sizeof(fe), B, p.tmp,
-                           false, c));
-  } else if (B > 1) {
-    // long codewords (integer-pipe bound): the real-input transform of each
-    // proof, half the multiplies of the general one
-    for (int pb = 0; pb < B; pb++) {
-      if (!dry) GBZ_CUDA(cudaMemsetAsync(&st[pb].nonreal, 0, sizeof(uint32_t), c));
-      RUN_ON(c, PC_NTT, ntt_launch_real_count(ilog2(L)),
-             ntt_launch_real(p.tables(ilog2(L) - 1), p.tables(ilog2(L)),
-                             reinterpret_cast<const fe *>(reinterpret_cast<const char *>(w) + p.bs_w * pb), p.n,
-                             reinterpret_cast<fe *>(reinterpret_cast<char *>(p.cw[0]) + p.bs_cw0 * pb),
-                             reinterpret_cast<fe *>(reinterpret_cast<char *>(p.tmp) + p.bs_tmp * pb), &st[pb].nonreal,
-                             c));
-    }
-  } else {
-    if (!dry) GBZ_CUDA(cudaMemsetAsync(&st->nonreal, 0, sizeof(uint32_t), c));
-    RUN_ON(c, PC_NTT, ntt_launch_real_count(ilog2(L)),
-           ntt_launch_real(p.tables(ilog2(L) - 1), p.tables(ilog2(L)), w, p.n, p.cw[0], p.tmp, &st->nonreal, c));
-  }
-  // The root (a chain of compressions from leaf 0) is computed on the query
-  // stream once the codeword exists, off the chain of commits.
+  // The records before the opening; the root's payload is written by its
+  // first queries.
   uint64_t off_root[kMaxWhirIter + 1];
-  off_root[0] = off;
-  if (!dry) GBZ_CUDA(cudaEventRecord(p.ev_commit[0], c));
-  int iter = 0;
-
-  uint64_t m = p.n;
+  off_root[0] = lay.rec(T_COMMIT_ROOT, 1, 32);
+  uint64_t off = 0, m = p.n, L = p.L;
   const fe *a = w;
-  if (open) goto opening;
-  {
-  // 2. evaluation point and its eq table.
+  int cwi = 0, iter = 0;
+
+  auto sumcheck = [&]() {
+  // 1. evaluation point and its eq table.
   off = lay.rec(T_EVAL_POINT, logn, 16);
   RUN(PC_PROTOCOL, 1, k_point<<<B, 32, 0, s>>>(st, logn, tr, off, trs));
-  // 3. sumcheck of sum w(x) eq(z, x), two rounds a pass: w is folded by both
+  // 2. sumcheck of sum w(x) eq(z, x), two rounds a pass: w is folded by both
   //    challenges, the eq vector is represented by the shrinking tables
   //    E_{i+1} (vb ping-pong) and the prefix product epre; the last rounds
   //    (or all of a small proof) in one CTA.
@@ -1033,8 +962,104 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
       (k_sc_tail<<<B, kScTailThreads, kScTailShared, s>>>(st, a, p.vb[pp], (int)m, i, logn, tr,
                                                          i == 0 ? (int64_t)off_claim : -1,
                                                          off_poly0 + 80ull * (uint64_t)i, off, tb)));
+  };
+
+  // The opening's randomness, drawn on the query stream while the
+  // commitment and the sumcheck run, and the beta updates' powers.
+  UbSlots *slots = reinterpret_cast<UbSlots *>(p.ub_scratch);
+  UbPrepArgs ua{};
+  auto draws = [&]() {
+    SchedArgs sa{};
+    uint64_t mm = p.n, LL = p.L, cc = (uint64_t)p.rate;
+    for (;;) {
+      if (sa.T >= kMaxWhirIter) throw ArgError("prover: too many WHIR iterations");
+      mm /= 4;
+      sa.l[sa.T] = whir_query_count((int)cc);
+      sa.qmod[sa.T] = (int32_t)(LL / 4);
+      if (sa.l[sa.T] < 1 || sa.l[sa.T] > kMaxQueries) throw ArgError("prover: query count out of range");
+      sa.T++;
+      LL = 2 * cc * mm;
+      cc *= 2;
+      if (mm <= (uint64_t)kWhirK) break;
+    }
+    sa.lg_final = ilog2(mm);
+    RUN_ON(q, PC_PROTOCOL, 1, k_whir_schedule<<<B, 256, 0, q>>>(st, sa));
+    ua.T = sa.T;
+    LL = p.L;
+    mm = p.n;
+    for (int t = 0; t < sa.T; t++) {
+      LL /= 2;
+      mm /= 4;
+      ua.base[t + 1] = ua.base[t] + sa.l[t];
+      ua.per[t] = update_betas_per(mm, B);
+      if (!go) continue;
+      const NttTables &tnew = p.tables(ilog2(LL));
+      ua.lo[t] = tnew.lo_fwd;
+      ua.hi[t] = tnew.hi_fwd;
+    }
+    if (ua.base[sa.T] > kUbSlots) throw ArgError("prover: too many queries");
+    RUN_ON(q, PC_UPDATE_BETAS, 1,
+           k_ub_prep<<<dim3((unsigned)(ua.base[sa.T] + 3) / 4, B), 128, 0, q>>>(st, slots, p.bs_ub, ua));
+    if (go) GBZ_CUDA(cudaEventRecord(p.ev_sched, q));
+  };
+
+  // 3. commitment: codeword = NTT(w padded to rate*n), Merkle tree.
+  auto commit = [&]() {
+  // The witness is expected in the base field (the imaginary words zero):
+  // its transform is then a half-length transform of packed pairs
+  // (ntt_launch_real); any other witness takes the general transform.
+  if (open) {
+    if (go && open->codeword != p.cw[0])
+      GBZ_CUDA(cudaMemcpyAsync(p.cw[0], open->codeword, 16 * L, cudaMemcpyDeviceToDevice, c));
+  } else if (B > 1 && ilog2(L) < kBatchRealLog) {
+    // short codewords (launch bound): the batch's codewords as one batched
+    // transform (the same values as the real-input path of a single proof)
+    RUN_ON(c, PC_NTT, ntt_launch_count(ilog2(L)),
+           ntt_launch_rows(p.tables(ilog2(L)), w, p.n, p.bs_w / sizeof(fe), p.cw[0], p.bs_cw0 / sizeof(fe), B, p.tmp,
+                           false, c));
+  } else if (B > 1) {
+    // long codewords (integer-pipe bound): the real-input transform of each
+    // proof, half the multiplies of the general one
+    for (int pb = 0; pb < B; pb++) {
+      if (go) GBZ_CUDA(cudaMemsetAsync(&st[pb].nonreal, 0, sizeof(uint32_t), c));
+      RUN_ON(c, PC_NTT, ntt_launch_real_count(ilog2(L)),
+             ntt_launch_real(p.tables(ilog2(L) - 1), p.tables(ilog2(L)),
+                             reinterpret_cast<const fe *>(reinterpret_cast<const char *>(w) + p.bs_w * pb), p.n,
+                             reinterpret_cast<fe *>(reinterpret_cast<char *>(p.cw[0]) + p.bs_cw0 * pb),
+                             reinterpret_cast<fe *>(reinterpret_cast<char *>(p.tmp) + p.bs_tmp * pb), &st[pb].nonreal,
+                             c));
+    }
+  } else {
+    if (go) GBZ_CUDA(cudaMemsetAsync(&st->nonreal, 0, sizeof(uint32_t), c));
+    RUN_ON(c, PC_NTT, ntt_launch_real_count(ilog2(L)),
+           ntt_launch_real(p.tables(ilog2(L) - 1), p.tables(ilog2(L)), w, p.n, p.cw[0], p.tmp, &st->nonreal, c));
   }
-opening:
+  if (go) GBZ_CUDA(cudaEventRecord(p.ev_commit[0], c));
+  };
+
+  // On one stream the order of the launches, across them the order in which a
+  // graph gets going: the start alone with the sumcheck first, a whole proof
+  // with its commitment first (2^24 2641 us, the sumcheck first 2705).
+  if (part == PART_START) {
+    sumcheck();
+    draws();
+    commit();
+  } else {
+    draws();
+    commit();
+    if (!open) sumcheck();
+  }
+
+  if (part == PART_START) {  // s joins the commitment and the draws
+    GBZ_CUDA(cudaStreamWaitEvent(s, p.ev_commit[0], 0));
+    GBZ_CUDA(cudaStreamWaitEvent(s, p.ev_sched, 0));
+    lay.len = p.transcript_bytes;
+    return;
+  }
+  if (part == PART_OPENING) {
+    go = true;
+    fork();
+  }
 
   // 4. WHIR open of (v1[0], chal): b = precompute_beta(chal), arr = w.
   //    Three chains: folds and beta updates on s, commits on c, queries
@@ -1048,7 +1073,7 @@ opening:
   RUN(PC_BETA, 1,
       eq_first ? beta_launch(st->chal + 2, logn - 2, p.beta, s, B, sts, p.bs_beta)
                : beta_launch(st->chal, logn, p.beta, s, B, sts, p.bs_beta));
-  if (!dry) GBZ_CUDA(cudaStreamWaitEvent(s, p.ev_sched, 0));  // round challenges
+  if (go && part == PART_ALL) GBZ_CUDA(cudaStreamWaitEvent(s, p.ev_sched, 0));  // round challenges
   a = w;
   const fe *b = p.beta;
   uint64_t ast = p.bs_w, bst = p.bs_beta;  // per-proof strides of a and b
@@ -1103,12 +1128,12 @@ opening:
     bst = p.bs_v;
     m /= 4;
     arr_next += m;
-    if (!dry) GBZ_CUDA(cudaEventRecord(p.ev_fold[iter], s));
+    if (go) GBZ_CUDA(cudaEventRecord(p.ev_fold[iter], s));
     // commit arr_{t+1} at rate 2*cur on c, once the query that opened the
     // buffer's previous codeword (iteration t-1) is done
     const int nci = cwi ^ 1;
     off = lay.rec(T_WHIR_ROOT, 1, 32);
-    if (!dry) {
+    if (go) {
       GBZ_CUDA(cudaStreamWaitEvent(c, p.ev_fold[iter], 0));
       if (iter > 0) GBZ_CUDA(cudaStreamWaitEvent(c, p.ev_query[iter - 1], 0));
     }
@@ -1120,7 +1145,7 @@ opening:
       RUN_ON(c, PC_NTT, ntt_launch_count(ilog2(NL)), ntt_launch(p.tables(ilog2(NL)), a, m, p.cw[nci], p.tmp, false, c));
     }
     off_root[iter + 1] = off;
-    if (!dry) GBZ_CUDA(cudaEventRecord(p.ev_commit[iter + 1], c));
+    if (go) GBZ_CUDA(cudaEventRecord(p.ev_commit[iter + 1], c));
     // queries of iteration t on q: they open the codeword of commit t,
     // record this iteration's round messages and check K against them
     const int depth = ilog2(L / 4);
@@ -1150,7 +1175,7 @@ opening:
     qa.off_path = lay.rec(T_WHIR_PATHS, l * depth, 32);
     qa.off_comb = lay.rec(T_WHIR_COMBINE, l, 16);
     qa.off_K = lay.rec(T_WHIR_K, 1, 16);
-    if (!dry) {
+    if (go) {
       const NttTables &told = p.tables(ilog2(L));
       qa.inv_lo = told.lo_inv;
       qa.inv_hi = told.hi_inv;
@@ -1159,7 +1184,7 @@ opening:
       qa.len_inv = finv(fe_make(kWhirK, 0));
       // the codeword it opens, and this iteration's round messages (for
       // iteration 0 also K = v1[0], set before on s)
-      GBZ_CUDA(cudaStreamWaitEvent(q, p.ev_commit[iter], 0));
+      if (iter > 0 || part == PART_ALL) GBZ_CUDA(cudaStreamWaitEvent(q, p.ev_commit[iter], 0));
       GBZ_CUDA(cudaStreamWaitEvent(q, p.ev_fold[iter], 0));
     }
     // depth >= 2: every queried codeword has 16+ entries
@@ -1168,7 +1193,7 @@ opening:
     RUN_ON(q, PC_QUERY, 1,
            k_whir_open<<<dim3((unsigned)(2 + (hashes + kOpenThreads - 1) / kOpenThreads), B), kOpenThreads, 0, q>>>(
                qa, iter));
-    if (!dry) GBZ_CUDA(cudaEventRecord(p.ev_query[iter], q));
+    if (go) GBZ_CUDA(cudaEventRecord(p.ev_query[iter], q));
     // update_betas on s: b[j] += sum_i c_i omega_NL^{q_i j} is the forward
     // transform of a vector with l nonzeros.  When l * |b| exceeds a few
     // transform lengths, the sparse transform is cheaper than the direct
@@ -1206,10 +1231,10 @@ opening:
     RUN(PC_PROTOCOL, 1, k_final_b<<<B, 32, 0, s>>>(st, a, b, (int)m, tr, off_poly, off_point, off_eval, fb));
   }
   // root of the last commitment (never opened) on the query stream
-  if (!dry) GBZ_CUDA(cudaStreamWaitEvent(q, p.ev_commit[iter], 0));
+  if (go) GBZ_CUDA(cudaStreamWaitEvent(q, p.ev_commit[iter], 0));
   RUN_ON(q, PC_MERKLE, 1,
          k_merkle_root_b<<<B, 32, 0, q>>>(p.cw[cwi], cw_s[cwi], ilog2(L / 4), tr, trs, off_root[iter]));
-  if (!dry) {  // join the commit and query chains
+  if (go) {  // join the commit and query chains
     GBZ_CUDA(cudaEventRecord(p.ev_root_tail, q));
     GBZ_CUDA(cudaStreamWaitEvent(s, p.ev_commit[iter], 0));
     GBZ_CUDA(cudaStreamWaitEvent(s, p.ev_root_tail, 0));
@@ -1286,6 +1311,38 @@ void set_seeds_launch(ProofPlan &p, const uint32_t *seeds, int count, cudaStream
   }
 }
 
+namespace {
+// Captures one part of a proof on s.
+cudaGraph_t capture_part(ProofPlan &p, const fe *w, uint32_t prng_seed, cudaStream_t s, ProofPart part) {
+  GBZ_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+  cudaGraph_t g = nullptr;
+  try {
+    enqueue_proof(p, w, prng_seed, s, false, false, nullptr, part);
+  } catch (...) {
+    cudaStreamEndCapture(s, &g);
+    if (g) cudaGraphDestroy(g);
+    throw;
+  }
+  GBZ_CUDA(cudaStreamEndCapture(s, &g));
+  return g;
+}
+
+void graph_free(ProofGraph &g) {
+  for (cudaGraphExec_t e : g.exec)
+    if (e) cudaGraphExecDestroy(e);
+  for (cudaGraph_t x : g.graph)
+    if (x) cudaGraphDestroy(x);
+}
+}  // namespace
+
+// A launch of a graph takes about 1 us a node before its critical chain gets
+// going (63 nodes at 2^18, the evaluation point 45 us late).  Up to codewords
+// of 2^kSplitLog the opening is a second graph, submitted while the sumcheck
+// runs (2^10 124 -> 122 us, 2^18 324 -> 313, 2^20 equal); above, where the
+// commitment outlasts the sumcheck, the opening's folds would wait for it
+// (2^24 2641 -> 2670).
+constexpr int kSplitLog = 22;
+
 void launch_proof_graph(ProofPlan &p, const fe *w, uint32_t prng_seed, cudaStream_t s) {
   ProofGraph *g = nullptr;
   for (auto &e : p.graphs)
@@ -1297,44 +1354,39 @@ void launch_proof_graph(ProofPlan &p, const fe *w, uint32_t prng_seed, cudaStrea
       for (size_t i = 1; i < p.graphs.size(); i++)
         if (p.graphs[i].last_use < p.graphs[lru].last_use) lru = i;
       GBZ_CUDA(cudaStreamSynchronize(s));
-      cudaGraphExecDestroy(p.graphs[lru].exec);
-      cudaGraphDestroy(p.graphs[lru].graph);
+      graph_free(p.graphs[lru]);
       p.graphs.erase(p.graphs.begin() + lru);
     }
+    const bool split = ilog2(p.L) <= kSplitLog;
     ProofGraph ng;
     ng.w = w;
-    GBZ_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     try {
-      enqueue_proof(p, w, prng_seed, s, false, false);
+      ng.graph[0] = capture_part(p, w, prng_seed, s, split ? PART_START : PART_ALL);
+      if (split) ng.graph[1] = capture_part(p, w, prng_seed, s, PART_OPENING);
+      // the k_init node carries the seed
+      size_t count = 0;
+      GBZ_CUDA(cudaGraphGetNodes(ng.graph[0], nullptr, &count));
+      std::vector<cudaGraphNode_t> nodes(count);
+      GBZ_CUDA(cudaGraphGetNodes(ng.graph[0], nodes.data(), &count));
+      for (auto nd : nodes) {
+        cudaGraphNodeType ty;
+        GBZ_CUDA(cudaGraphNodeGetType(nd, &ty));
+        if (ty != cudaGraphNodeTypeKernel) continue;
+        cudaKernelNodeParams kp{};
+        GBZ_CUDA(cudaGraphKernelNodeGetParams(nd, &kp));
+        if (kp.func == reinterpret_cast<void *>(k_init)) {
+          ng.init_node = nd;
+          ng.init_params = kp;
+          break;
+        }
+      }
+      if (!ng.init_node) throw ArgError("prover graph: initial node not found");
+      for (int k = 0; k < 2; k++)
+        if (ng.graph[k]) GBZ_CUDA(cudaGraphInstantiate(&ng.exec[k], ng.graph[k], 0));
     } catch (...) {
-      cudaGraph_t tmp = nullptr;
-      cudaStreamEndCapture(s, &tmp);
-      if (tmp) cudaGraphDestroy(tmp);
+      graph_free(ng);
       throw;
     }
-    GBZ_CUDA(cudaStreamEndCapture(s, &ng.graph));
-    // the k_init node carries the seed
-    size_t count = 0;
-    GBZ_CUDA(cudaGraphGetNodes(ng.graph, nullptr, &count));
-    std::vector<cudaGraphNode_t> nodes(count);
-    GBZ_CUDA(cudaGraphGetNodes(ng.graph, nodes.data(), &count));
-    for (auto nd : nodes) {
-      cudaGraphNodeType ty;
-      GBZ_CUDA(cudaGraphNodeGetType(nd, &ty));
-      if (ty != cudaGraphNodeTypeKernel) continue;
-      cudaKernelNodeParams kp{};
-      GBZ_CUDA(cudaGraphKernelNodeGetParams(nd, &kp));
-      if (kp.func == reinterpret_cast<void *>(k_init)) {
-        ng.init_node = nd;
-        ng.init_params = kp;
-        break;
-      }
-    }
-    if (!ng.init_node) {
-      cudaGraphDestroy(ng.graph);
-      throw ArgError("prover graph: initial node not found");
-    }
-    GBZ_CUDA(cudaGraphInstantiate(&ng.exec, ng.graph, 0));
     p.graphs.push_back(ng);
     g = &p.graphs.back();
   }
@@ -1346,8 +1398,9 @@ void launch_proof_graph(ProofPlan &p, const fe *w, uint32_t prng_seed, cudaStrea
   cudaKernelNodeParams kp = g->init_params;
   kp.kernelParams = args;
   kp.extra = nullptr;
-  GBZ_CUDA(cudaGraphExecKernelNodeSetParams(g->exec, g->init_node, &kp));
-  GBZ_CUDA(cudaGraphLaunch(g->exec, s));
+  GBZ_CUDA(cudaGraphExecKernelNodeSetParams(g->exec[0], g->init_node, &kp));
+  GBZ_CUDA(cudaGraphLaunch(g->exec[0], s));
+  if (g->exec[1]) GBZ_CUDA(cudaGraphLaunch(g->exec[1], s));
 }
 
 uint64_t plan_bytes(int logn, int rate, int batch) {

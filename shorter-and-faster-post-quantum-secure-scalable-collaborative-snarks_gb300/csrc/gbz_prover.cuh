@@ -39,12 +39,13 @@ struct Profiler {
   ~Profiler();
 };
 
-// A proof captured as a CUDA graph for one witness address; the PRNG seed
-// is a parameter of the captured k_init node, updated before each launch.
+// A proof captured as one or two CUDA graphs for one witness address; the
+// PRNG seed is a parameter of the captured k_init node, updated before each
+// launch.
 struct ProofGraph {
   const fe *w = nullptr;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  cudaGraph_t graph[2] = {nullptr, nullptr};
+  cudaGraphExec_t exec[2] = {nullptr, nullptr};
   cudaGraphNode_t init_node = nullptr;
   cudaKernelNodeParams init_params{};
   uint64_t last_use = 0;
@@ -146,12 +147,15 @@ void plan_prepare_open(ProofPlan &p);
 // With `open`, only the opening of (witness, open->codeword) at the given
 // claim is enqueued: the commitment root of the codeword, then the WHIR
 // records (no evaluation point, claim or sumcheck records).
+// PART_START: everything before the opening; PART_OPENING: the opening of the
+// proof whose start is before it on s.
+enum ProofPart { PART_ALL, PART_START, PART_OPENING };
 void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStream_t s, bool dry,
-                   bool seed_in_state = false, const OpenOnly *open = nullptr);
+                   bool seed_in_state = false, const OpenOnly *open = nullptr, ProofPart part = PART_ALL);
 void set_seed_launch(ProofPlan &p, uint32_t seed, cudaStream_t s);
 // The seeds of the first count proofs of a batched plan (passed by value).
 void set_seeds_launch(ProofPlan &p, const uint32_t *seeds, int count, cudaStream_t s);
-// Enqueues one proof of the witness at w by replaying a captured graph
+// Enqueues one proof of the witness at w by replaying captured graphs
 // (captured on first use of this address; s must be a capturable stream).
 void launch_proof_graph(ProofPlan &p, const fe *w, uint32_t prng_seed, cudaStream_t s);
 // Device bytes a plan of this shape allocates (an upper bound).

@@ -32,3 +32,14 @@ def test_lengths(ctx, oracle, logn, fill):
 def test_seeds(ctx, oracle, seed):
     w = witness(5, "base")
     assert ctx.prove(w, 5, 4, seed).tobytes() == bytes(oracle.prove(w, 5, 4, seed))
+
+
+@pytest.mark.parametrize("logn,rate", [(3, 2), (12, 4), (21, 2), (21, 4)])
+def test_graphs_on_both_sides_of_the_split(gbz, logn, rate):
+    c = gbz.Context(0)
+    w = witness(logn, "base")
+    c.set_graphs(False)
+    want = [c.prove(w, logn, rate, s).tobytes() for s in (1, 2)]
+    c.set_graphs(True)
+    assert [c.prove(w, logn, rate, s).tobytes() for s in (1, 2, 1)] == want + want[:1]
+    c.close()
