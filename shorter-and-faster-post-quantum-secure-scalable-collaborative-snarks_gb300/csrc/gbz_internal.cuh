@@ -149,7 +149,7 @@ void ntt_launch(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
 // holds N entries; n_valid is even.
 void ntt_launch_real(const NttTables &t_half, const NttTables &t_full, const fe *in, uint64_t n_valid, fe *out,
                      fe *tmp, uint32_t *nonreal, cudaStream_t s);
-int ntt_launch_real_count(int logn);
+int ntt_launch_real_count(int logn, uint64_t n_valid);
 // `rows` transforms of the same length in the same launches: row r reads
 // in + r in_stride (n_valid entries, zero beyond) and writes out + r
 // out_stride, output k at out_elem_stride * k within the row; tmp holds
@@ -167,7 +167,7 @@ void ntt_launch_rows(const NttTables &t, const fe *in, uint64_t n_valid, uint64_
 void ntt_sparse_accumulate(const NttTables &t, const int32_t *q, const fe *c, int l, fe *acc, uint64_t nacc,
                            fe *tmp, cudaStream_t s, int q_shift = 0);
 void ntt_tables_build(NttTables &t, int logn);
-int ntt_launch_count(int logn);
+int ntt_launch_count(int logn, uint64_t n_valid = 0, int rows = 1);
 // count independent transforms of length 2^t.logn (<= 2^13): transform g
 // reads in[g * in_stride + j] for j < j_valid (zero beyond) and writes
 // out[g * 2^logn + k].

@@ -38,6 +38,8 @@ constexpr int kSubLog = 13;          // largest sub-transform held in shared mem
 constexpr int kTwLoBits = 12;        // outer twiddle table split
 constexpr int kMaxThreads = 1024;
 constexpr int kCtaElems = 1 << kSubLog;  // most elements staged per CTA
+constexpr int kSmallLog = 10;        // longest sub-transform of the small kernel
+constexpr int kCosetLog = 10;        // longest transform taken in cosets
 constexpr int kPerThread = 8;            // elements per thread (CTA = max(32, E/8) threads)
 
 // Two-pass shape of a length set by ntt_set_shape (the autotuner): k1 = log2
@@ -79,6 +81,10 @@ struct PassArgs {
   int acc;
   // Every entry is present: n_valid and j_valid need no test (set at launch).
   int dense;
+  // Coset form of a padded transform (the small kernel): entry j of
+  // sub-transform l is multiplied by omega_L^{l j} (in_lo, in_hi as tw_lo,
+  // tw_hi) when it is loaded.
+  const fe *in_lo, *in_hi;
   // Entries j >= j_valid of every sub-transform are zero (per-transform
   // padding of batched transforms; S when unused).
   uint32_t j_valid;
@@ -496,6 +502,72 @@ __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs
   }
 }
 
+// A launch of few short transforms is over before a pass kernel's 20 to 60 KB
+// of unrolled butterflies have come in, each run through once: 8 to 12 us for
+// transforms of 2^4 to 2^10.  Here a thread takes one radix-2 butterfly a
+// level, in a loop of 2 KB that every length and both directions share, with
+// the half table of omega_n in shared memory: half as much arithmetic again,
+// which such a launch does not notice (2^6 to 2^10 by 4 cosets 10.4 -> 3.7 us,
+// 2^8 to 2^15 by 128 13.3 -> 5.0, 2^10 to 2^16 by 64 14.8 -> 8.9; one
+// transform of 2^11 gains nothing).
+// half_tw: omega_{2^kSmallLog}^k of the direction, k < 2^(kSmallLog - 1).
+__global__ void __launch_bounds__(1 << (kSmallLog - 1)) ntt_small_kernel(const PassArgs a, const fe *half_tw) {
+  if (a.run_if && *a.run_if == 0) return;
+  extern __shared__ fe smem[];
+  const int logS = a.logS, logB = a.logB;
+  const uint32_t half = 1u << (logS - 1), total = 2u << (logS - 1 + logB), tid = threadIdx.x;
+  const uint32_t b = tid >> (logS - 1), j = tid & (half - 1);
+  const uint64_t l = ((uint64_t)blockIdx.x << logB) + b;
+  const fe *in = a.in + blockIdx.y * a.row_in;
+  fe *out = a.out + blockIdx.y * a.row_out;
+  fe *tw = smem, *buf[2] = {smem + half, smem + half + total};
+  fe x[2];
+#pragma unroll 1
+  for (int r = 0; r < 2; r++) {
+    const uint32_t jj = j + r * half;
+    const uint64_t addr = l * a.in_gstride + (uint64_t)jj * a.in_jstride;
+    const bool ok = addr < a.n_valid && jj < a.j_valid;
+    fe v = fe_zero();
+    if (a.pack_real) {
+      if (ok) {
+        const fe e0 = in[2 * addr], e1 = in[2 * addr + 1];
+        if (e0.im | e1.im) atomicOr(a.nonreal, 1u);
+        v = fe_make(e0.re, e1.re);
+      }
+    } else if (ok) {
+      v = in[addr];
+      if (a.in_lo) {
+        const uint64_t ex = l * jj;
+        fe w = a.in_lo[ex & ((1u << kTwLoBits) - 1)];
+        if (ex >> kTwLoBits) w = fmul(w, a.in_hi[ex >> kTwLoBits]);
+        v = fmul(v, w);
+      }
+    }
+    if (r) x[1] = v;
+    else x[0] = v;
+  }
+  for (uint32_t t = tid; t < half; t += blockDim.x) tw[t] = half_tw[t << (kSmallLog - logS)];
+  fe y0 = fadd(x[0], x[1]), y1 = fsub(x[0], x[1]);
+#pragma unroll 1
+  for (int s = 1; s < logS; s++) {  // x'[(j / Ns) 2 Ns + j mod Ns (+ Ns)], Ns = 2^(s-1), then the next level
+    fe *o = buf[s & 1] + (b << logS);
+    const uint32_t low = j & ((1u << (s - 1)) - 1), at = ((j - low) << 1) + low;
+    o[at] = y0;
+    o[at + (1u << (s - 1))] = y1;
+    __syncthreads();
+    const fe u = o[j], t = fmul(o[j + half], tw[(j & ((1u << s) - 1)) << (logS - 1 - s)]);
+    y0 = fadd(u, t);
+    y1 = fsub(u, t);
+  }
+  if (a.has_scale) {
+    y0 = fmul(y0, a.scale);
+    y1 = fmul(y1, a.scale);
+  }
+  fe *o = out + l * a.out_gstride + j * a.out_kstride;
+  *o = y0;
+  o[half * a.out_kstride] = y1;
+}
+
 // Column chains of a sparse input: next[t] = the next entry with the same
 // column ((q >> shift) & colmask), -1 at the end; lead[t] = 1 for the first
 // entry of each column.  One thread per entry (l <= kMaxQueries).
@@ -544,6 +616,7 @@ PassKernel pass_kernel(int logS, bool inverse, bool pack) {
 
 // Stage twiddle tables per direction, shared by every length.
 fe *g_stages[2] = {nullptr, nullptr};
+fe *g_half_tw[2] = {nullptr, nullptr};  // the small kernel's
 int g_stages_device = -1;
 
 void ensure_stages() {
@@ -564,6 +637,16 @@ void ensure_stages() {
     GBZ_CUDA(device_malloc((void **)&g_stages[dir], sizeof(fe) * h.size()));
     GBZ_CUDA(cudaMemcpy(g_stages[dir], h.data(), sizeof(fe) * h.size(), cudaMemcpyHostToDevice));
   }
+  for (int dir = 0; dir < 2; dir++) {
+    fe w = root_of_unity(kSmallLog);
+    if (dir) w = finv(w);
+    std::vector<fe> t(1u << (kSmallLog - 1), fe_one());
+    for (size_t k = 1; k < t.size(); k++) t[k] = fmul(t[k - 1], w);
+    GBZ_CUDA(device_malloc((void **)&g_half_tw[dir], sizeof(fe) * t.size()));
+    GBZ_CUDA(cudaMemcpy(g_half_tw[dir], t.data(), sizeof(fe) * t.size(), cudaMemcpyHostToDevice));
+  }
+  GBZ_CUDA(cudaFuncSetAttribute(ntt_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(sizeof(fe) * (5u << (kSmallLog - 1)))));
   g_stages_device = dev;
   for (int logS = 0; logS <= kSubLog; logS++)
     for (int kind = 0; kind < 3; kind++)
@@ -571,12 +654,32 @@ void ensure_stages() {
                                     (int)(sizeof(fe) * kCtaElems)));
 }
 
+// Launches of up to 2^kSmallTotal elements in sub-transforms of up to
+// 2^kSmallLog take the small kernel, cosets up to 2^kCosetTotal (below).  The
+// proofs and openings that were timed do not tell 2^13 from 2^17 for the
+// first, nor 2^16 from 2^19 for the second.
+constexpr int kSmallTotal = 16, kCosetTotal = 18;
+
+bool small_launch(const PassArgs &a, uint64_t groups, int rows) {
+  return a.in_lo || (a.logS >= 1 && a.logS <= kSmallLog && a.logG == 0 && !a.tw_lo && !a.sp_l && !a.acc &&
+                     ((groups * (uint64_t)rows) << a.logS) <= (1ull << kSmallTotal));
+}
+
 void launch_pass(PassArgs a, uint64_t groups, cudaStream_t s, int rows = 1) {
+  if (rows < 1 || rows > 65535) throw ArgError("transform: 1..65535 rows per launch");
+  if (small_launch(a, groups, rows)) {
+    // a warp of butterflies a CTA at least
+    a.logB = std::min(std::max(0, 6 - a.logS), ilog2(groups & (~groups + 1)));
+    const uint32_t threads = 1u << (a.logS - 1 + a.logB);
+    ntt_small_kernel<<<dim3((unsigned)(groups >> a.logB), (unsigned)rows), threads, sizeof(fe) * 5 * threads, s>>>(
+        a, g_half_tw[a.inverse ? 1 : 0]);
+    GBZ_CUDA(cudaGetLastError());
+    return;
+  }
   const uint64_t tiles = groups >> a.logB;
   const uint32_t E = 1u << (a.logS + a.logB);
   const size_t smem = a.logS > 3 || a.sp_l > 0 ? sizeof(fe) * E : 0;
   const unsigned threads = E / kPerThread > 32 ? E / kPerThread : 32;
-  if (rows < 1 || rows > 65535) throw ArgError("transform: 1..65535 rows per launch");
   if (a.logG == 0) a.logG = 40;  // every g is a column of its own
   const uint64_t last = (groups - 1) * a.in_gstride + ((1ull << a.logS) - 1) * a.in_jstride;
   a.dense = a.j_valid >= (1u << a.logS) && (a.n_valid == ~0ull || last < a.n_valid);
@@ -761,7 +864,22 @@ void ntt_tables_build(NttTables &t, int logn) {
   }
 }
 
-int ntt_launch_count(int logn) {
+namespace {
+// A transform of n <= 2^kCosetLog entries padded to L >= 8 n is L / n
+// transforms of length n: X[k + (L/n) m] = DFT_n(x_j omega_L^{jk})[m], log n
+// levels and a product instead of log L levels in one or two passes, and L / n
+// or so CTAs where a whole transform in one CTA leaves the chip idle (2^4 to
+// 2^13 28.3 us in one CTA, 3.5 in cosets; 2^8 to 2^15 15.6 us in two passes,
+// 5.0).  Longer launches (above 2^kCosetTotal elements) keep the passes, which
+// issue less.
+bool coset_form(int logn, uint64_t n_valid, int rows) {
+  return n_valid > 1 && n_valid <= (1u << kCosetLog) && logn >= 3 + ilog2(2 * n_valid - 1) &&
+         ((uint64_t)rows << logn) <= (1ull << kCosetTotal);
+}
+}  // namespace
+
+int ntt_launch_count(int logn, uint64_t n_valid, int rows) {
+  if (coset_form(logn, n_valid, rows)) return 1;
   if (logn <= kSubLog) return 1;
   return g_shape[logn].k1 > 0 ? 2 : schedule(logn).passes;
 }
@@ -856,6 +974,24 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
   a.scale = t.inv_len;
   a.inverse = inverse ? 1 : 0;
   a.j_valid = 1u << kSubLog;
+  const int logv = n_valid ? ilog2(2 * n_valid - 1) : 0;  // 2^logv >= n_valid
+  const fe *in_end = in + (uint64_t)(rows - 1) * row_in + n_valid;
+  const fe *out_end = out + (uint64_t)(rows - 1) * row_out + ((L - 1) * out_elem_stride + 1);
+  if (!gate.pack_real && coset_form(logn, n_valid, rows) && (in_end <= out || out_end <= in)) {
+    a.in = in;
+    a.out = out;
+    a.n_valid = n_valid;
+    a.in_gstride = 0;
+    a.in_jstride = 1;
+    a.in_lo = inverse ? t.lo_inv : t.lo_fwd;
+    a.in_hi = inverse ? t.hi_inv : t.hi_fwd;
+    a.out_gstride = out_elem_stride;
+    a.out_kstride = out_elem_stride << (logn - logv);
+    a.logS = logv;
+    a.has_scale = inverse;
+    launch_pass(a, 1ull << (logn - logv), s, rows);
+    return;
+  }
   if (logn <= kSubLog) {
     a.in = in;
     a.out = out;
@@ -990,7 +1126,9 @@ void ntt_launch_real(const NttTables &t_half, const NttTables &t_full, const fe 
   ntt_passes(t_full, in, n_valid, out, tmp, false, s, 1, 0, 0, f);
 }
 
-int ntt_launch_real_count(int logn) { return ntt_launch_count(logn - 1) + 1 + ntt_launch_count(logn); }
+int ntt_launch_real_count(int logn, uint64_t n_valid) {
+  return ntt_launch_count(logn - 1) + 1 + ntt_launch_count(logn, n_valid);
+}
 
 void ntt_launch_rows(const NttTables &t, const fe *in, uint64_t n_valid, uint64_t in_stride, fe *out,
                      uint64_t out_stride, int rows, fe *tmp, bool inverse, cudaStream_t s, uint64_t out_elem_stride) {

@@ -1014,7 +1014,7 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
   } else if (B > 1 && ilog2(L) < kBatchRealLog) {
     // short codewords (launch bound): the batch's codewords as one batched
     // transform (the same values as the real-input path of a single proof)
-    RUN_ON(c, PC_NTT, ntt_launch_count(ilog2(L)),
+    RUN_ON(c, PC_NTT, ntt_launch_count(ilog2(L), p.n, B),
            ntt_launch_rows(p.tables(ilog2(L)), w, p.n, p.bs_w / sizeof(fe), p.cw[0], p.bs_cw0 / sizeof(fe), B, p.tmp,
                            false, c));
   } else if (B > 1) {
@@ -1022,7 +1022,7 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
     // proof, half the multiplies of the general one
     for (int pb = 0; pb < B; pb++) {
       if (go) GBZ_CUDA(cudaMemsetAsync(&st[pb].nonreal, 0, sizeof(uint32_t), c));
-      RUN_ON(c, PC_NTT, ntt_launch_real_count(ilog2(L)),
+      RUN_ON(c, PC_NTT, ntt_launch_real_count(ilog2(L), p.n),
              ntt_launch_real(p.tables(ilog2(L) - 1), p.tables(ilog2(L)),
                              reinterpret_cast<const fe *>(reinterpret_cast<const char *>(w) + p.bs_w * pb), p.n,
                              reinterpret_cast<fe *>(reinterpret_cast<char *>(p.cw[0]) + p.bs_cw0 * pb),
@@ -1031,7 +1031,7 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
     }
   } else {
     if (go) GBZ_CUDA(cudaMemsetAsync(&st->nonreal, 0, sizeof(uint32_t), c));
-    RUN_ON(c, PC_NTT, ntt_launch_real_count(ilog2(L)),
+    RUN_ON(c, PC_NTT, ntt_launch_real_count(ilog2(L), p.n),
            ntt_launch_real(p.tables(ilog2(L) - 1), p.tables(ilog2(L)), w, p.n, p.cw[0], p.tmp, &st->nonreal, c));
   }
   if (go) GBZ_CUDA(cudaEventRecord(p.ev_commit[0], c));
@@ -1138,11 +1138,11 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
       if (iter > 0) GBZ_CUDA(cudaStreamWaitEvent(c, p.ev_query[iter - 1], 0));
     }
     if (B > 1) {
-      RUN_ON(c, PC_NTT, ntt_launch_count(ilog2(NL)),
+      RUN_ON(c, PC_NTT, ntt_launch_count(ilog2(NL), m, B),
              ntt_launch_rows(p.tables(ilog2(NL)), a, m, p.bs_arr / sizeof(fe), p.cw[nci], cw_s[nci] / sizeof(fe), B,
                              p.tmp, false, c));
     } else {
-      RUN_ON(c, PC_NTT, ntt_launch_count(ilog2(NL)), ntt_launch(p.tables(ilog2(NL)), a, m, p.cw[nci], p.tmp, false, c));
+      RUN_ON(c, PC_NTT, ntt_launch_count(ilog2(NL), m), ntt_launch(p.tables(ilog2(NL)), a, m, p.cw[nci], p.tmp, false, c));
     }
     off_root[iter + 1] = off;
     if (go) GBZ_CUDA(cudaEventRecord(p.ev_commit[iter + 1], c));
