@@ -275,58 +275,111 @@ __global__ void k_indexes(PcsDev *st, int l, int N, uint32_t Mq, int32_t *qp, in
   }
 }
 
+// 1 / x = conj(x) / (re^2 + im^2) for x != 0 (the norm vanishes for x = 0
+// only, p = 3 mod 4), the norm inverted as N^(p - 2), p - 2 = 2^61 - 3:
+// x_k = N^(2^k - 1) up to k = 59, then N^(4 (2^59 - 1) + 1).
+__device__ __forceinline__ uint64_t mulp1(uint64_t a, uint64_t b) { return redp(mulp_lazy(a, b)); }
+__device__ fe inverse_dev(fe x) {
+  const uint64_t n = addp(mulp1(x.re, x.re), mulp1(x.im, x.im));
+  uint64_t r = n;  // n^(2^k - 1)
+  int k = 1;
+#pragma unroll 1
+  for (int bit = 4; bit >= 0; bit--) {  // 59 = 111011 in binary
+    uint64_t t = r;
+    for (int q = 0; q < k; q++) t = mulp1(t, t);
+    r = mulp1(t, r);
+    k *= 2;
+    if ((59 >> bit) & 1) {
+      r = mulp1(mulp1(r, r), n);
+      k++;
+    }
+  }
+  r = mulp1(r, r);
+  r = mulp1(mulp1(r, r), n);
+  return fe_make(mulp1(x.re, r), mulp1(x.im ? P - x.im : 0, r));
+}
+
+// The Lagrange weights at c over the D = 2^logD points w^k and over the d =
+// D >> ext points w^(k << ext) (compute_lagrange_coeff, utils.cpp:169-197: the
+// inverse transform of the powers of c), and the value of the polynomial with
+// evaluations poly there (valid in thread 0).  The geometric sum in closed
+// form, L[k] = (c^D - 1) / (D (c w^-k - 1)) (1 where c w^-k = 1, and then 0
+// elsewhere): an inverse a point, 1.7 us, where the sums took D^2 products in
+// one CTA, 94 us for 512 points.  wp: the powers of w^-1.  256 threads.
+__device__ fe lagrange_dev(fe c, int logD, int ext, const fe *wp, const fe *poly, fe invD, fe invd, fe *LD, fe *Ld) {
+  __shared__ fe red[8];
+  const int D = 1 << logD;
+  fe cd = c, cD;
+  for (int i = 0; i < logD - ext; i++) cd = fmul(cd, cd);
+  cD = cd;
+  for (int i = 0; i < ext; i++) cD = fmul(cD, cD);
+  cD = fmul(fsub(cD, fe_one()), invD);
+  cd = fmul(fsub(cd, fe_one()), invd);
+  facc acc = facc_zero();
+  for (int k = threadIdx.x; k < D; k += 256) {
+    const fe den = fsub(fmul(c, wp[k]), fe_one());
+    const bool hit = !(den.re | den.im);
+    const fe inv = inverse_dev(den);
+    const fe l = hit ? fe_one() : fmul(cD, inv);
+    if (LD) LD[k] = l;
+    facc_mul(acc, poly[k], l);
+    if ((k & ((1 << ext) - 1)) == 0) Ld[k >> ext] = hit ? fe_one() : fmul(cd, inv);
+  }
+  fe x = facc_value(acc);
+#pragma unroll
+  for (int m = 16; m > 0; m >>= 1)
+    x = fadd(x, fe_make(__shfl_xor_sync(0xffffffffu, x.re, m), __shfl_xor_sync(0xffffffffu, x.im, m)));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int w = 1; w < 8; w++) x = fadd(x, red[w]);
+  return x;
+}
+
+// The hash chain over n field elements, the next one on its way while one is
+// hashed.
+__device__ fe hash_chain(fe fs, const fe *x, int n) {
+  fe next = x[0];
+#pragma unroll 1
+  for (int k = 0; k < n; k++) {
+    const fe v = next;
+    if (k + 1 < n) next = x[k + 1];
+    fs = hash_F(fs, v);
+  }
+  return fs;
+}
+
 // The leader's check of round i and its challenge (coPCS.cpp:1463-1483):
 // sum_j poly[2j] = K, c = hash_to_field(poly), K = sum_k poly[k] L2[k] with
 // L2 = compute_lagrange_coeff(c, 2d), and the fold weights L = the same at
 // length d (utils.cpp:169-197: the inverse transform of the powers of c).
-// scratch: 2 * 2d entries.
+// The chain of 2d hashes is what takes the time (0.55 us each); scratch: 2d
+// entries.
 __global__ void __launch_bounds__(256)
 k_round_verify(PcsDev *st, const fe *poly, int logd, fe wi, fe invD, fe invd, fe *L, fe *scratch, uint8_t *tr,
                uint64_t off_poly, uint64_t off_chal) {
-  __shared__ fe red[256];
   __shared__ fe chal;
-  __shared__ fe sh_cw[2 * 1024];  // the powers of c and of w^-1 (global scratch beyond 1024 points)
   const int d = 1 << logd, D = 2 * d;
-  fe *cp = D <= 1024 ? sh_cw : scratch, *wp = D <= 1024 ? sh_cw + D : scratch + D;
   // (wi = omega_D^-1, invD, invd: constants of the shape, formed on the host)
   for (int k = threadIdx.x; k < D; k += blockDim.x) {
-    wp[k] = fpow(wi, (uint64_t)k);
+    scratch[k] = fpow(wi, (uint64_t)k);
     put_fe(tr, off_poly + 16ull * k, poly[k]);
   }
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 32) {
     fe ev = fe_zero();
     for (int j = 0; j < d; j++) ev = fadd(ev, poly[2 * j]);
     if (!fe_eq(ev, st->K)) st->error |= 1;
-    fe fs = st->fs;
-    for (int k = 0; k < D; k++) fs = hash_F(fs, poly[k]);
+  }
+  if (threadIdx.x == 0) {
+    const fe fs = hash_chain(st->fs, poly, D);
     st->fs = fs;
     st->c = fs;
     put_fe(tr, off_chal, fs);
     chal = fs;
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < D; k += blockDim.x) cp[k] = fpow(chal, (uint64_t)k);
-  __syncthreads();
-  // L2[k] = (1/D) sum_j c^j w^{-jk}; K' = sum_k poly[k] L2[k]
-  fe acc = fe_zero();
-  for (int k = threadIdx.x; k < D; k += blockDim.x) {
-    fe s = fe_zero();
-    for (int j = 0; j < D; j++) s = fadd(s, fmul(cp[j], wp[((uint64_t)j * k) & (D - 1)]));
-    acc = fadd(acc, fmul(poly[k], fmul(s, invD)));
-  }
-  // L[k] = (1/d) sum_{j<d} c^j w_d^{-jk}, w_d^{-1} = (w_D^{-1})^2
-  for (int k = threadIdx.x; k < d; k += blockDim.x) {
-    fe s = fe_zero();
-    for (int j = 0; j < d; j++) s = fadd(s, fmul(cp[j], wp[(2ull * j * k) & (D - 1)]));
-    L[k] = fmul(s, invd);
-  }
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] = fadd(red[threadIdx.x], red[threadIdx.x + s]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) st->K = red[0];
+  const fe K = lagrange_dev(chal, logd + 1, 1, scratch, poly, invD, invd, nullptr, L);
+  if (threadIdx.x == 0) st->K = K;
 }
 
 // delegate_checks (coPCS.cpp:753-763): per query j (party a, position q),
@@ -538,24 +591,26 @@ struct ROffs {
 
 // H_p += c H_r with H_r = R_p[iter], H_r[0] += sum_{j > iter} sum_k R_p[j][step k]
 // (coSumcheck.cpp:47-60, 181-193).  One CTA per party.
-__global__ void k_cosc_add_hr(fe *H, int D, const fe *R, uint64_t rstride, ROffs ro, int iter, int step,
-                              const CoscDev *st) {
+__global__ void __launch_bounds__(256)
+k_cosc_add_hr(fe *H, int D, const fe *R, uint64_t rstride, ROffs ro, int iter, int step, const CoscDev *st) {
   const uint64_t p = blockIdx.x;
   const fe *Rp = R + p * rstride;
-  __shared__ fe extra;
-  if (threadIdx.x == 0) {
-    fe e = fe_zero();
-    for (int j = iter + 1; j < ro.n; j++) {
-      const int len = (int)(ro.off[j + 1] - ro.off[j]);
-      for (int k = 0; k < len / step; k++) e = fadd(e, Rp[ro.off[j] + step * k]);
-    }
-    extra = e;
+  __shared__ fe red[8];
+  fe e = fe_zero();
+  for (int j = iter + 1; j < ro.n; j++) {
+    const int len = (int)(ro.off[j + 1] - ro.off[j]);
+    for (int k = threadIdx.x; k < len / step; k += 256) e = fadd(e, Rp[ro.off[j] + step * k]);
   }
+#pragma unroll
+  for (int m = 16; m > 0; m >>= 1)
+    e = fadd(e, fe_make(__shfl_xor_sync(0xffffffffu, e.re, m), __shfl_xor_sync(0xffffffffu, e.im, m)));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = e;
   __syncthreads();
   const fe c = st->c;
   for (int k = threadIdx.x; k < D; k += blockDim.x) {
     fe hr = Rp[ro.off[iter] + k];
-    if (k == 0) hr = fadd(hr, extra);
+    if (k == 0)
+      for (int w = 0; w < 8; w++) hr = fadd(hr, red[w]);
     H[p * D + k] = fadd(H[p * D + k], fmul(c, hr));
   }
 }
@@ -563,54 +618,32 @@ __global__ void k_cosc_add_hr(fe *H, int D, const fe *R, uint64_t rstride, ROffs
 // The leader's round: sum_{j<d} H[j << ext] = K (flag otherwise), r =
 // hash_to_field(H), LD = compute_lagrange_coeff(r, D = d << ext), K = sum
 // H LD, Ld = compute_lagrange_coeff(r, d) (coSumcheck.cpp:258-293,
-// 362-396).  scratch: 2 D entries.
+// 362-396).  As k_round_verify (512 points 457 us, now 300); scratch: D entries.
 __global__ void __launch_bounds__(256)
 k_cosc_verify(CoscDev *st, const fe *poly, int logd, int ext, int round, fe wi, fe invD, fe invd, fe *LD, fe *Ld,
               fe *scratch, uint8_t *tr, uint64_t off_poly, uint64_t off_chal) {
-  __shared__ fe red[256];
   __shared__ fe chal;
-  __shared__ fe sh_cw[2 * 1024];  // the powers of c and of w^-1 (global scratch beyond 1024 points)
   const int d = 1 << logd, D = d << ext;
-  fe *cp = D <= 1024 ? sh_cw : scratch, *wp = D <= 1024 ? sh_cw + D : scratch + D;
   // (wi = omega_D^-1, invD, invd: constants of the shape, formed on the host)
   for (int k = threadIdx.x; k < D; k += blockDim.x) {
-    wp[k] = fpow(wi, (uint64_t)k);
+    scratch[k] = fpow(wi, (uint64_t)k);
     put_fe(tr, off_poly + 16ull * k, poly[k]);
   }
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 32) {
     fe ev = fe_zero();
     for (int j = 0; j < d; j++) ev = fadd(ev, poly[j << ext]);
     if (!fe_eq(ev, st->K)) st->flags |= 1u << round;
-    fe fs = st->fs;
-    for (int k = 0; k < D; k++) fs = hash_F(fs, poly[k]);
+  }
+  if (threadIdx.x == 0) {
+    const fe fs = hash_chain(st->fs, poly, D);
     st->fs = fs;
     st->r[round] = fs;
     put_fe(tr, off_chal, fs);
     chal = fs;
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < D; k += blockDim.x) cp[k] = fpow(chal, (uint64_t)k);
-  __syncthreads();
-  fe acc = fe_zero();
-  for (int k = threadIdx.x; k < D; k += blockDim.x) {
-    fe s = fe_zero();
-    for (int j = 0; j < D; j++) s = fadd(s, fmul(cp[j], wp[((uint64_t)j * k) & (D - 1)]));
-    s = fmul(s, invD);
-    LD[k] = s;
-    acc = fadd(acc, fmul(poly[k], s));
-  }
-  for (int k = threadIdx.x; k < d; k += blockDim.x) {
-    fe s = fe_zero();
-    for (int j = 0; j < d; j++) s = fadd(s, fmul(cp[j], wp[(((uint64_t)j * k) << ext) & (D - 1)]));
-    Ld[k] = fmul(s, invd);
-  }
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] = fadd(red[threadIdx.x], red[threadIdx.x + s]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) st->K = red[0];
+  const fe K = lagrange_dev(chal, logd + ext, ext, scratch, poly, invD, invd, LD, Ld);
+  if (threadIdx.x == 0) st->K = K;
 }
 
 // quadratic_coSumcheck_phase2_sparse (coSumcheck.cpp:215-228) for every party:
@@ -654,14 +687,16 @@ __global__ void k_cosc_ip(const fe *LD, ROffs ro, fe *ip) {
 // N/2 x N map U), its check, the last challenge, the Lagrange weights over
 // N/4 points and the claims; for the cubic form also the check of b1[0]
 // against the round weights.  One CTA of kCoscThreads: the parties' values,
-// the unpack and the check's terms in parallel, the Fiat-Shamir chain and
-// the claims on thread 0.
+// the unpack, the check's terms and the weights in parallel, the check beside
+// the Fiat-Shamir chain (24 or 40 hashes at 16 parties; all of it on thread 0
+// with two inverses by 300 products took 110 us, now 29).
 __global__ void k_cosc_final(CoscDev *st, int cubic, int N, const fe *p1, const fe *p2, const fe *p3, const fe *b1,
                              uint64_t mstride, const fe *U, const fe *b2, const fe *Ld_hist, const int *logd_hist,
-                             int nrounds, const fe *r1, fe *claims, uint8_t *tr, uint64_t off_shares,
+                             int nrounds, const fe *r1, fe wi, fe iq, fe *claims, uint8_t *tr, uint64_t off_shares,
                              uint64_t off_unpacked, uint64_t off_r, uint64_t off_claims) {
   const int rows = cubic ? 4 : 5, half = N / 2, quarter = N / 4;
   __shared__ fe H[kCoscMaxRows][kPcsMaxParties / 2];
+  __shared__ fe L[kPcsMaxParties / 4], r;
   __shared__ fe S[kPcsMaxParties][kCoscMaxRows];
   __shared__ fe red[kCoscThreads];
   // the parties' final values (thread p), then the unpack (thread (i, j))
@@ -704,61 +739,59 @@ __global__ void k_cosc_final(CoscDev *st, int cubic, int N, const fe *p1, const 
         for (int t = 0; t < ld; t++) b = fmul(b, ((j >> t) & 1) ? r1[ctr + t] : fsub(fe_one(), r1[ctr + t]));
         acc = fadd(acc, fmul(b, Ld_hist[at + j]));
       }
-      red[threadIdx.x] = acc;
+#pragma unroll
+      for (int m = 16; m > 0; m >>= 1)
+        acc = fadd(acc, fe_make(__shfl_xor_sync(0xffffffffu, acc.re, m), __shfl_xor_sync(0xffffffffu, acc.im, m)));
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
       __syncthreads();
       if (threadIdx.x == 0) {
-        fe a = fe_zero();
-        for (int t = 0; t < (int)blockDim.x; t++) a = fadd(a, red[t]);
-        y = fmul(y, a);
+        for (int t = 1; t < kCoscThreads / 32; t++) acc = fadd(acc, red[t]);
+        y = fmul(y, acc);
       }
       __syncthreads();
       ctr += ld;
       at += d;
     }
   }
-  if (threadIdx.x) return;
-  fe K = st->K;
-  const fe c = st->c;
-  for (int i = 0; i < quarter; i++) {
-    fe t;
-    if (cubic) t = fmul(b2[i], fadd(fmul(b1[0], fsub(fmul(H[0][i], H[1][i]), H[2][i])), fmul(c, H[3][i])));
-    else t = fadd(fadd(fmul(H[0][i], H[1][i]), fmul(H[2][i], H[3][i])), fmul(c, H[4][i]));
-    K = fsub(K, t);
-  }
-  if (!fe_eq(K, fe_zero())) st->flags |= 1u << 29;
-  fe fs = st->fs;
-  const int hashed = cubic ? 3 : rows;
-  for (int i = 0; i < hashed; i++)
-    for (int j = 0; j < half; j++) fs = hash_F(fs, H[i][j]);
-  st->fs = fs;
-  put_fe(tr, off_r, fs);
-  // L over N/4 points: compute_lagrange_coeff(r, N/4), or {1} for one point
-  fe L[kPcsMaxParties / 4];
-  if (quarter == 1) {
-    L[0] = fe_one();
-  } else {
-    int lq = 0;
-    while ((1 << lq) < quarter) lq++;
-    const fe wi = finv(root_of_unity(lq)), iq = finv(fe_make((uint64_t)quarter, 0));
-    for (int k = 0; k < quarter; k++) {
-      fe acc = fe_zero(), x = fe_one();
-      const fe step = fpow(wi, (uint64_t)k);
-      fe w = fe_one();
-      for (int j = 0; j < quarter; j++) {
-        acc = fadd(acc, fmul(x, w));
-        x = fmul(x, fs);
-        w = fmul(w, step);
-      }
-      L[k] = fmul(acc, iq);
+  if (threadIdx.x == 0) {
+    fe fs = st->fs;
+    const int hashed = cubic ? 3 : rows;
+    for (int i = 0; i < hashed; i++) fs = hash_chain(fs, H[i], half);
+    st->fs = fs;
+    put_fe(tr, off_r, fs);
+    r = fs;
+    if (cubic && !fe_eq(y, b1[0])) atomicOr(&st->flags, 1u << 30);
+  } else if (threadIdx.x == 32) {
+    fe K = st->K;
+    const fe c = st->c;
+    for (int i = 0; i < quarter; i++) {
+      fe t;
+      if (cubic) t = fmul(b2[i], fadd(fmul(b1[0], fsub(fmul(H[0][i], H[1][i]), H[2][i])), fmul(c, H[3][i])));
+      else t = fadd(fadd(fmul(H[0][i], H[1][i]), fmul(H[2][i], H[3][i])), fmul(c, H[4][i]));
+      K = fsub(K, t);
     }
+    if (!fe_eq(K, fe_zero())) atomicOr(&st->flags, 1u << 29);
   }
-  for (int i = 0; i < rows; i++) {
+  __syncthreads();
+  // L over N/4 points: compute_lagrange_coeff(r, N/4), or {1} for one point
+  // (wi = omega_{N/4}^-1 and iq = 4 / N from the host)
+  for (int k = threadIdx.x; k < quarter; k += blockDim.x) {
+    fe acc = fe_zero(), x = fe_one();
+    const fe step = fmul(r, fpow(wi, (uint64_t)k));
+    for (int j = 0; j < quarter; j++) {
+      acc = fadd(acc, x);
+      x = fmul(x, step);
+    }
+    L[k] = quarter == 1 ? fe_one() : fmul(acc, iq);
+  }
+  __syncthreads();
+  if (threadIdx.x < rows) {
+    const int i = threadIdx.x;
     fe e = fe_zero();
     for (int j = 0; j < quarter; j++) e = fadd(e, fmul(L[j], H[i][j]));
     claims[i] = e;
     put_fe(tr, off_claims + 16ull * i, e);
   }
-  if (cubic && !fe_eq(y, b1[0])) st->flags |= 1u << 30;
 }
 
 }  // namespace
@@ -1227,8 +1260,9 @@ CoscOut cosumcheck_run(gbz_ctx *ctx, int form, int N, uint64_t n, const fe *p1, 
     at += d;
   }
   fe *dcl = ob.alloc<fe>(rows);
-  k_cosc_final<<<1, kCoscThreads, 0, s>>>(st, cubic ? 1 : 0, N, v1, v2, v3, vb, m, dU, db2, Ldh, dlog, ndeg, dr1, dcl, tr,
-                                off_sh, off_un, off_r, off_cl);
+  const fe wq = N > 4 ? finv(root_of_unity(ilog2(N / 4))) : fe_one();
+  k_cosc_final<<<1, kCoscThreads, 0, s>>>(st, cubic ? 1 : 0, N, v1, v2, v3, vb, m, dU, db2, Ldh, dlog, ndeg, dr1, wq,
+                                          finv(fe_make((uint64_t)(N / 4), 0)), dcl, tr, off_sh, off_un, off_r, off_cl);
   GBZ_CUDA(cudaGetLastError());
   if (ip) {
     k_cosc_ip<<<ndeg, 256, 0, s>>>(LDall, ro, ip);
