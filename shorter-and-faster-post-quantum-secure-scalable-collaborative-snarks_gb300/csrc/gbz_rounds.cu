@@ -42,7 +42,7 @@ __device__ __forceinline__ uint64_t halfp(uint64_t x) { return (x & 1) ? (x + P)
 __device__ __forceinline__ fe fhalf(fe x) { return fe_make(halfp(x.re), halfp(x.im)); }
 
 // The cubic form accumulates, per thread, the sums of its products at 0, 1,
-// -1 and the leading coefficient (8 products a pair instead of 9); this
+// -1 and the leading coefficient (7 products a pair instead of 9); this
 // turns them into the coefficients (x^3, x^2, x, 1) before the sums are
 // combined across threads.  The map is linear and exact, so the messages
 // are the coefficient sums the reference forms pair by pair.
@@ -95,11 +95,14 @@ __device__ __forceinline__ void accumulate(const Line *l, fe b, typename Sums<FO
     facc_mul(acc[1], l[0].h, l[1].h);
     facc_mul(acc[2], l[0].b, l[1].b);
   } else if constexpr (FORM == SC_CUBIC) {
-    const fe m0 = fsub_lazy(l[0].b, l[0].a), m1 = fsub(l[1].b, l[1].a), m2 = fsub(l[2].b, l[2].a);
-    facc_mul(acc[0], fmul_fold(l[0].a, l[1].a), l[2].a);
-    facc_mul(acc[1], fmul_fold(l[0].h, l[1].h), l[2].h);
-    facc_mul(acc[2], fmul_fold(m0, m1), m2);
-    facc_mul(acc[3], fmul_fold(l[0].b, l[1].b), l[2].b);
+    // the first two lines' product at the leading coefficient, 1 and 0 gives
+    // its value at -1: 2 (q_inf + q_0) - q_1, with 2p to stay positive
+    const fe qi = fmul_fold(l[0].a, l[1].a), q1 = fmul_fold(l[0].h, l[1].h), q0 = fmul_fold(l[0].b, l[1].b);
+    const fe qm = fe_make(fold64(2 * (qi.re + q0.re) + (2 * P - q1.re)), fold64(2 * (qi.im + q0.im) + (2 * P - q1.im)));
+    facc_mul(acc[0], qi, l[2].a);
+    facc_mul(acc[1], q1, l[2].h);
+    facc_mul(acc[2], qm, fsub(l[2].b, l[2].a));
+    facc_mul(acc[3], q0, l[2].b);
   } else if constexpr (FORM == SC_QUADRUPLE) {
     // ((l1 l2) l3) l4 as the reference multiplies them (polynomial.cpp:91-101)
     lmul(l[0], l[1], q);
