@@ -132,6 +132,16 @@ GBZ_HD void prng_seed(glibc_prng &g, uint32_t seed) {
   for (int i = 0; i < 310; i++) (void)prng_next(g);
 }
 
+// randomNumber (fieldElement.cpp:363-368) from 20 consecutive outputs.
+GBZ_HD uint64_t prng_number_from(const int32_t *d) {
+  uint64_t ret = (uint64_t)(d[0] % 10);
+  for (int i = 1; i < 20; i++) {
+    ret = ret * 10ull + (uint64_t)(d[i] % 10);
+    ret = ret >= P ? ret % P : ret;
+  }
+  return ret;
+}
+
 #ifdef __CUDACC__
 // The same generator by a warp, 31 outputs at a time: lane j < 31 holds the
 // j-th oldest of the last 31 values x, and x[n] = x[n-31] + x[n-3] makes the

@@ -118,35 +118,6 @@ __global__ void k_tail_init(ProofState *st, glibc_prng g, uint32_t *flags) {
 }
 
 // ---- the delegation sumchecks ------------------------------------------------
-// Round message H of the partials, the check H(0) + H(1) = y (flag `bit`),
-// the challenge drawn ahead, y = H(challenge).
-__global__ void k_sc_finish(const fe *partial, int blocks, int nc, fe *y, const fe *draw, fe *ch, int round,
-                            uint32_t *flags, uint32_t bit, uint8_t *tr, uint64_t off_polys) {
-  __shared__ fe red[kMaxFormCoeffs][kT];
-  fe acc[kMaxFormCoeffs];
-  for (int k = 0; k < kMaxFormCoeffs; k++) acc[k] = fe_zero();
-  for (int i = threadIdx.x; i < blocks; i += kT)
-    for (int k = 0; k < nc; k++) acc[k] = fadd(acc[k], partial[(uint64_t)i * nc + k]);
-  for (int k = 0; k < kMaxFormCoeffs; k++) red[k][threadIdx.x] = acc[k];
-  __syncthreads();
-  for (int w = kT / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w)
-      for (int k = 0; k < kMaxFormCoeffs; k++) red[k][threadIdx.x] = fadd(red[k][threadIdx.x], red[k][threadIdx.x + w]);
-    __syncthreads();
-  }
-  if (threadIdx.x) return;
-  // coefficients highest degree first: H(0) + H(1) = 2 c_last + the others
-  fe s = red[nc - 1][0];
-  for (int k = 0; k < nc; k++) s = fadd(s, red[k][0]);
-  if (bit && !fe_eq(s, *y)) atomicOr(flags, bit);
-  for (int k = 0; k < nc; k++) put_fe(tr, off_polys + 16ull * ((uint64_t)round * nc + k), red[k][0]);
-  const fe c = *draw;
-  ch[round] = c;
-  fe v = red[0][0];
-  for (int k = 1; k < nc; k++) v = fadd(fmul(v, c), red[k][0]);
-  *y = v;
-}
-
 __global__ void k_set(fe *dst, const fe *src) {
   if (threadIdx.x == 0) *dst = *src;
 }
@@ -729,41 +700,31 @@ struct Tail {
     if (n < 2 || !is_pow2(n)) throw ArgError("pcs leader: sumcheck length must be a power of two >= 2");
     const uint64_t op = lay.rec(T_D_POLYS, (uint32_t)(rounds * nc), 16), of = lay.rec(T_D_FINAL, (uint32_t)nv, 16);
     if (dry) return;
-    const int pb = round_blocks(n / 2);
-    fe *partial = alloc<fe>((uint64_t)pb * nc);
+    // The challenges are known: the rounds with more than 2^kDrawnTailLog
+    // entries entering them are launched one behind the other, the others and
+    // all messages follow in one CTA (form_tail_drawn_kernel).
+    const int i0 = std::max(1, rounds - kDrawnTailLog + 1);
+    DrawnTailArgs t{};
+    uint64_t np = 0;
+    for (int i = 0; i < i0; i++) np += (uint64_t)(t.blocks[i] = round_blocks(n >> (i + 1))) * nc;
+    fe *partial = alloc<fe>(np);
     fe *buf[2][6] = {};
     for (int b = 0; b < 2; b++)
       for (int k = 0; k < nv; k++) buf[b][k] = alloc<fe>(std::max<uint64_t>(n / 2, 1));
-    RoundArgs a{};
-    for (int k = 0; k < nv; k++) a.in[k] = v[k];
-    a.pairs = n / 2;
-    a.partial = partial;
-    form_step_launch(form, a, 0, round_blocks(a.pairs), s);
-    k_sc_finish<<<1, kT, 0, s>>>(partial, round_blocks(a.pairs), nc, y, draw + first, ch, 0, flags, bit, tr, op);
-    check();
-    // rounds with at most 2^14 entries entering them, and the final fold,
-    // in one CTA (form_tail_drawn_kernel)
-    const int i0 = std::max(1, rounds - 13);
-    for (int i = 1; i < i0; i++) {
-      RoundArgs b{};
+    for (int i = 0; i < i0; i++) {
+      RoundArgs a{};
       for (int k = 0; k < nv; k++) {
-        b.in[k] = i == 1 ? v[k] : buf[(i - 2) & 1][k];
-        b.out[k] = buf[(i - 1) & 1][k];
+        a.in[k] = i <= 1 ? v[k] : buf[(i - 2) & 1][k];
+        a.out[k] = i ? buf[(i - 1) & 1][k] : nullptr;
       }
-      b.pairs = n >> (i + 1);
-      b.r = ch + (i - 1);
-      b.partial = partial;
-      form_step_launch(form, b, 1, round_blocks(b.pairs), s);
-      k_sc_finish<<<1, kT, 0, s>>>(partial, round_blocks(b.pairs), nc, y, draw + first + (uint64_t)stride * i, ch, i,
-                                   flags, bit, tr, op);
-      check();
+      a.pairs = n >> (i + 1);
+      a.r = i ? draw + first + (uint64_t)stride * (i - 1) : nullptr;
+      a.partial = partial;
+      t.partial[i] = partial;
+      partial += (uint64_t)t.blocks[i] * nc;
+      form_step_launch(form, a, i ? 1 : 0, t.blocks[i], s);
     }
-    DrawnTailArgs t{};
-    for (int k = 0; k < nv; k++) {
-      t.in[k] = i0 == 1 ? v[k] : buf[(i0 - 2) & 1][k];
-      t.buf[0][k] = buf[(i0 - 1) & 1][k];
-      t.buf[1][k] = buf[i0 & 1][k];
-    }
+    for (int k = 0; k < nv; k++) t.in[k] = i0 == 1 ? v[k] : buf[(i0 - 2) & 1][k];
     t.n = n;
     t.i0 = i0;
     t.rounds = rounds;

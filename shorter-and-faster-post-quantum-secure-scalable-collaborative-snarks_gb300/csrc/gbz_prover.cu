@@ -316,16 +316,6 @@ struct SchedArgs {
 constexpr int kFieldDraws = 40;     // random() outputs behind one F::_random() (two 20-digit numbers)
 constexpr int kMaxDraws = kMaxWhirIter * (3 * kFieldDraws + kMaxQueries) + 8 * kFieldDraws;
 
-// randomNumber (fieldElement.cpp:363-368) from 20 consecutive outputs.
-__device__ uint64_t number_from(const int32_t *d) {
-  uint64_t ret = (uint64_t)(d[0] % 10);
-  for (int i = 1; i < 20; i++) {
-    ret = ret * 10ull + (uint64_t)(d[i] % 10);
-    ret = ret >= P ? ret % P : ret;
-  }
-  return ret;
-}
-
 // The first warp runs the generator and stores the N outputs in shared
 // memory; then all threads derive the field elements (40 outputs each, a
 // thread an element) and the query positions from them.  With one thread
@@ -358,7 +348,7 @@ __global__ void __launch_bounds__(256) k_whir_schedule(ProofState *st, SchedArgs
     const int k = (int)threadIdx.x - 3 * t;
     if (k >= 0 && k < 3) {
       const int o = k < 2 ? off + kFieldDraws * k : off + 2 * kFieldDraws + l;
-      const fe v = fe_make(number_from(draws + o) % P, number_from(draws + o + 20) % P);
+      const fe v = fe_make(prng_number_from(draws + o) % P, prng_number_from(draws + o + 20) % P);
       if (k < 2) st->wr[t][k] = v;
       else st->wrb[t] = v;
     }
@@ -366,7 +356,7 @@ __global__ void __launch_bounds__(256) k_whir_schedule(ProofState *st, SchedArgs
   }
   for (int i = (int)blockDim.x - 1 - (int)threadIdx.x; i < a.lg_final; i += blockDim.x) {
     const int o = off + kFieldDraws * i;
-    st->fin_r[i] = fe_make(number_from(draws + o) % P, number_from(draws + o + 20) % P);
+    st->fin_r[i] = fe_make(prng_number_from(draws + o) % P, prng_number_from(draws + o + 20) % P);
   }
 }
 

@@ -278,26 +278,39 @@ __device__ fe finish_round(const fe *H, int nc, fe &fs, fe &y, uint32_t &error, 
   return ch;
 }
 
-// Sums the partials into the round polynomial H (nc coefficients) and
-// finishes the round.
-__global__ void form_finalize_kernel(const fe *partial, int blocks, int nc, RoundState *st, int round,
-                                     const fe *drawn, fe *polys, fe *chal) {
-  __shared__ fe red[4][kThreads];
-  fe acc[4] = {fe_zero(), fe_zero(), fe_zero(), fe_zero()};
-  for (int i = threadIdx.x; i < blocks; i += kThreads)
-    for (int k = 0; k < nc; k++) acc[k] = fadd(acc[k], partial[(uint64_t)i * nc + k]);
-  for (int k = 0; k < 4; k++) red[k][threadIdx.x] = acc[k];
-  __syncthreads();
-  for (int w = kThreads / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w)
-      for (int k = 0; k < 4; k++) red[k][threadIdx.x] = fadd(red[k][threadIdx.x], red[k][threadIdx.x + w]);
-    __syncthreads();
-  }
-  if (threadIdx.x) return;
-  fe H[4];
-  for (int k = 0; k < nc; k++) H[k] = red[k][0];
+__device__ __forceinline__ fe shfl_xor_fe(fe x, int d) {
+  return fe_make(__shfl_xor_sync(0xffffffffu, x.re, d), __shfl_xor_sync(0xffffffffu, x.im, d));
+}
+
+// Sum of coefficient k of `blocks` partials over a warp's lanes.
+__device__ __forceinline__ fe warp_partial_sum(const fe *partial, int blocks, int nc, int k, int first, int step) {
+  fe x = fe_zero();
+#pragma unroll 4
+  for (int i = first; i < blocks; i += step) x = fadd(x, partial[(uint64_t)i * nc + k]);
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) x = fadd(x, shfl_xor_fe(x, d));
+  return x;
+}
+
+// Sums the partials into the round polynomial H (nc coefficients, two warps
+// each) and finishes the round.
+__global__ void __launch_bounds__(256)
+form_finalize_kernel(const fe *partial, int blocks, int nc, RoundState *st, int round, const fe *drawn, fe *polys,
+                     fe *chal) {
+  __shared__ fe red[4][2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k = warp >> 1;
   fe fs = st->fs, y = st->y;
   uint32_t error = st->error;
+  if (k < nc) {
+    const fe x = warp_partial_sum(partial, blocks, nc, k, lane + 32 * (warp & 1), 64);
+    if (lane == 0) red[k][warp & 1] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x) return;
+  fe H[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    if (q < nc) H[q] = fadd(red[q][0], red[q][1]);
   finish_round(H, nc, fs, y, error, round, drawn, polys, chal);
   st->fs = fs;
   st->y = y;
@@ -305,73 +318,60 @@ __global__ void form_finalize_kernel(const fe *partial, int blocks, int nc, Roun
 }
 
 // The leader's rounds take the fourth of every four F::_random() draws
-// (Distributed_Sumcheck.cpp); the glibc stream depends on nothing the rounds
-// compute, so its n challenges are drawn in one thread while the first,
-// largest rounds run, and the stream's final state goes back to st->prng.
-__global__ void prng_draw_kernel(RoundState *st, int n, fe *out) {
-  __shared__ glibc_prng g;  // dynamically indexed table: work on a shared copy
-  if (threadIdx.x) return;
-  g = st->prng;
+// (Distributed_Sumcheck.cpp), 160 outputs of the generator; the glibc stream
+// depends on nothing the rounds compute, so a warp draws its n challenges
+// while the first, largest rounds run, and the stream's final state goes back
+// to st->prng.  Of a challenge's outputs the last 40 are its digits.  (One
+// thread took 22 us a challenge.)
+__global__ void __launch_bounds__(32) prng_draw_kernel(RoundState *st, int n, fe *out) {
+  constexpr int kDraws = 160, kFull = kDraws / 31, kRest = kDraws % 31;
+  __shared__ int32_t d[kDraws + 31];
+  const int lane = threadIdx.x, f0 = st->prng.f;
+  uint32_t x = prng_warp_load(st->prng, lane);
+#pragma unroll 1
   for (int j = 0; j < n; j++) {
-    fe ch;
-    for (int k = 0; k < 4; k++) ch = prng_field(g);
-    out[j] = ch;
+#pragma unroll 1
+    for (int b = 0; b < kFull; b++) {
+      x = prng_warp_next(x, lane);
+      if (lane < 31) d[31 * b + lane] = (int32_t)(x >> 1);
+    }
+    const uint32_t y = prng_warp_next(x, lane);
+    if (lane < kRest) d[31 * kFull + lane] = (int32_t)(y >> 1);
+    x = prng_warp_shift(x, y, kRest, lane);
+    __syncwarp();
+    uint64_t v = 0;
+    if (lane < 2) v = prng_number_from(d + kDraws - 40 + 20 * lane) % P;
+    const uint64_t im = __shfl_sync(0xffffffffu, v, 1);
+    if (lane == 0) out[j] = fe_make(v, im);
+    __syncwarp();
   }
-  st->prng = g;
+  __syncwarp();
+  prng_warp_store(st->prng, x, f0, (uint64_t)kDraws * n, lane);
 }
 
-constexpr int kTailThreads = 512;
+constexpr int kTailThreads = 512, kTailWarps = kTailThreads / 32;
 
-struct TailArgs {
-  const fe *in[3];  // entries entering round i0, before its fold
-  fe *buf[2][3];    // ping-pong outputs (buf[0] differs from in)
-  uint64_t cur;     // entries of every vector entering round i0
-  int i0, total, fs_rounds;
-  RoundState *st;
-  const fe *drawn;  // glibc challenges of rounds fs_rounds.. (or null)
-  fe *polys, *chal, *fin;
-};
-
-// Rounds i0..total-1 of the party sumcheck and the final fold in one CTA,
-// once the vectors are small: every round is the fused fold + message of
-// form_step_kernel<FORM, 1>, a block reduction and finish_round, with no
-// launch between rounds.
+// One round of a one-CTA tail: folds the form's vectors (cur entries) by r
+// into out and leaves the message's sums, a warp each, in red[k][warp].
+// Returns the number of warps that had work.
 template <int FORM>
-__global__ void __launch_bounds__(kTailThreads) form_tail_kernel(TailArgs t) {
+__device__ __forceinline__ int tail_round(const fe *const *in, fe *const *out, uint64_t cur, fe r,
+                                          fe (*red)[kTailWarps]) {
   constexpr int NV = Form<FORM>::NV, NC = Form<FORM>::NC;
-  __shared__ fe red[NC][kTailThreads / 32];
-  __shared__ fe sh_r;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const fe *in[NV];
-#pragma unroll
-  for (int k = 0; k < NV; k++) in[k] = t.in[k];
-  fe r = t.chal[t.i0 - 1];
-  fe fs = fe_zero(), y = fe_zero();  // the running state, in thread 0's registers
-  uint32_t error = 0;
-  if (threadIdx.x == 0) {
-    fs = t.st->fs;
-    y = t.st->y;
-    error = t.st->error;
-  }
-  uint64_t cur = t.cur;
-  int pp = 0;
-  for (int i = t.i0; i < t.total; i++) {
+  const int pairs = (int)(cur / 4), active = min(kTailWarps, (pairs + 31) / 32);
+  if (wid < active) {
     typename Sums<FORM>::type sums[NC];
 #pragma unroll
     for (int k = 0; k < NC; k++) sum_zero(sums[k]);
-    const uint64_t pairs = cur / 4;
-    for (uint64_t g = threadIdx.x; g < pairs; g += kTailThreads) {
-      fe xs[NV][4];
-#pragma unroll
-      for (int k = 0; k < NV; k++)
-#pragma unroll
-        for (int q = 0; q < 4; q++) xs[k][q] = in[k][4 * g + q];
+    for (int g = threadIdx.x; g < pairs; g += kTailThreads) {
       Line l[NV];
 #pragma unroll
       for (int k = 0; k < NV; k++) {
-        const fe f0 = ffold(xs[k][0], xs[k][1], r), f1 = ffold(xs[k][2], xs[k][3], r);
-        t.buf[pp][k][2 * g] = f0;
-        t.buf[pp][k][2 * g + 1] = f1;
+        const fe *p = in[k] + 4 * g;
+        const fe f0 = ffold(p[0], p[1], r), f1 = ffold(p[2], p[3], r);
+        out[k][2 * g] = f0;
+        out[k][2 * g + 1] = f1;
         l[k] = line(f0, f1);
       }
       accumulate<FORM>(l, fe_zero(), sums);
@@ -387,25 +387,86 @@ __global__ void __launch_bounds__(kTailThreads) form_tail_kernel(TailArgs t) {
     if (lane == 0)
 #pragma unroll
       for (int k = 0; k < NC; k++) red[k][wid] = acc[k];
-    __syncthreads();  // also orders this round's stores before the next round's loads
-    if (wid == 0) {
+  }
+  return active;
+}
+
+// Shared memory of a tail entered with `cur` entries: the vectors' folds,
+// cur/2 entries and cur/4 in turn.
+template <int FORM>
+constexpr size_t tail_shared(uint64_t cur) {
+  return sizeof(fe) * Form<FORM>::NV * (cur / 2 + cur / 4);
+}
+template <int FORM>
+__device__ __forceinline__ void tail_buffers(fe *sm, uint64_t cur, fe *(*buf)[Form<FORM>::NV]) {
+  constexpr int NV = Form<FORM>::NV;
+  for (int k = 0; k < NV; k++) {
+    buf[0][k] = sm + k * (cur / 2);
+    buf[1][k] = sm + NV * (cur / 2) + k * (cur / 4);
+  }
+}
+
+struct TailArgs {
+  const fe *in[3];  // entries entering round i0, before its fold
+  uint64_t cur;     // entries of every vector entering round i0
+  int i0, total, fs_rounds;
+  RoundState *st;
+  const fe *drawn;  // glibc challenges of rounds fs_rounds.. (or null)
+  fe *polys, *chal, *fin;
+};
+
+// Rounds i0..total-1 of the party sumcheck and the final fold in one CTA,
+// once the vectors are small: every round is the fused fold + message of
+// form_step_kernel<FORM, 1> in shared memory, a reduction and finish_round.
+// A round costs its four hashes (2.2 us) and about as much again, where a
+// launch of a step and one of the finish take 9; from 2^13 entries on the
+// folds of one SM take longer than that.  (From 2^14 entries and through L2
+// the last 14 rounds took 116 us; these last 12 take 51.)
+template <int FORM>
+__global__ void __launch_bounds__(kTailThreads) form_tail_kernel(TailArgs t) {
+  constexpr int NV = Form<FORM>::NV, NC = Form<FORM>::NC;
+  extern __shared__ fe tail_sm[];
+  __shared__ fe red[NC][kTailWarps];
+  __shared__ fe sh_r;
+  const fe *in[NV];
+  fe *buf[2][NV];
+  tail_buffers<FORM>(tail_sm, t.cur, buf);
 #pragma unroll
-      for (int k = 0; k < NC; k++) acc[k] = red[k][lane % (kTailThreads / 32)];
-      if (lane >= kTailThreads / 32)
+  for (int k = 0; k < NV; k++) in[k] = t.in[k];
+  fe r = t.chal[t.i0 - 1];
+  fe fs = fe_zero(), y = fe_zero();  // the running state, in thread 0's registers
+  uint32_t error = 0;
+  if (threadIdx.x == 0) {
+    fs = t.st->fs;
+    y = t.st->y;
+    error = t.st->error;
+  }
+  uint64_t cur = t.cur;
+  int pp = 0;
+#pragma unroll 1
+  for (int i = t.i0; i < t.total; i++) {
+    const int active = tail_round<FORM>(in, buf[pp], cur, r, red);
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      // lane 8 k + w takes warps w and w + 8 of coefficient k
+      const int k = threadIdx.x >> 3, w = threadIdx.x & 7;
+      fe x = fe_zero();
+      if (k < NC && w < active) x = red[k][w];
+      if (k < NC && w + 8 < active) x = fadd(x, red[k][w + 8]);
 #pragma unroll
-        for (int k = 0; k < NC; k++) acc[k] = fe_zero();
+      for (int d = 4; d > 0; d >>= 1) x = fadd(x, shfl_xor_fe(x, d));
+      fe H[4];
 #pragma unroll
-      for (int d = 16; d > 0; d >>= 1)
-#pragma unroll
-        for (int k = 0; k < NC; k++) acc[k] = fadd(acc[k], shfl_down_fe(acc[k], d));
-      if (lane == 0)
-        sh_r = finish_round(acc, NC, fs, y, error, i,
+      for (int q = 0; q < 4; q++)
+        H[q] = fe_make(__shfl_sync(0xffffffffu, x.re, 8 * q), __shfl_sync(0xffffffffu, x.im, 8 * q));
+      if (threadIdx.x == 0)
+        sh_r = finish_round(H, NC, fs, y, error, i,
                             i >= t.fs_rounds && t.drawn ? t.drawn + (i - t.fs_rounds) : nullptr, t.polys, t.chal);
     }
     __syncthreads();
     r = sh_r;
 #pragma unroll
-    for (int k = 0; k < NV; k++) in[k] = t.buf[pp][k];
+    for (int k = 0; k < NV; k++) in[k] = buf[pp][k];
     pp ^= 1;
     cur /= 2;
   }
@@ -422,84 +483,86 @@ __global__ void __launch_bounds__(kTailThreads) form_tail_kernel(TailArgs t) {
 
 // Rounds i0..rounds-1 of a sumcheck whose challenges were drawn ahead
 // (the leader's glibc sumchecks of delegate_protocol.cpp) and its final
-// fold, in one CTA: every round the fused fold + message, a block
-// reduction, then thread 0 checks H(0) + H(1) against the running claim
-// (flag `bit` when it differs, none when bit is 0), stores H, takes the
-// round's challenge and updates the claim.
+// fold, in one CTA, and the messages of all its rounds.  No fold waits for a
+// message, so they are finished together at the end, a warp a round: the sum
+// of its partials, H(0) + H(1) against the claim that the round before leaves
+// (flag `bit` when it differs, none when bit is 0), H and the challenge.  A
+// round takes a fold and a barrier (finished one by one, and through L2 from
+// 2^14 entries on, the quadruple form took 111 us and the cubic 105, now 46 and 31).
 template <int FORM>
 __global__ void __launch_bounds__(kTailThreads) form_tail_drawn_kernel(DrawnTailArgs t) {
   constexpr int NV = Form<FORM>::NV, NC = Form<FORM>::NC;
-  __shared__ fe red[NC][kTailThreads / 32];
-  __shared__ fe sh_r;
+  extern __shared__ fe tail_sm[];
+  __shared__ fe red[kDrawnTailLog][NC][kTailWarps];
+  __shared__ fe claim[kMaxLogN + 2];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  auto challenge = [&](int i) { return t.draw[t.first + (uint64_t)t.stride * i]; };
   const fe *in[NV];
+  fe *buf[2][NV];
+  uint64_t cur = t.n >> (t.i0 - 1);
+  tail_buffers<FORM>(tail_sm, cur, buf);
 #pragma unroll
   for (int k = 0; k < NV; k++) in[k] = t.in[k];
-  fe r = t.ch[t.i0 - 1];
-  fe y = fe_zero();
-  if (threadIdx.x == 0) y = *t.y;
   int pp = 0;
+#pragma unroll 1
   for (int i = t.i0; i < t.rounds; i++) {
-    typename Sums<FORM>::type sums[NC];
-#pragma unroll
-    for (int k = 0; k < NC; k++) sum_zero(sums[k]);
-    const uint64_t pairs = t.n >> (i + 1);
-    for (uint64_t g = threadIdx.x; g < pairs; g += kTailThreads) {
-      Line l[NV];
-#pragma unroll
-      for (int k = 0; k < NV; k++) {
-        const fe *p = in[k] + 4 * g;
-        const fe f0 = ffold(p[0], p[1], r), f1 = ffold(p[2], p[3], r);
-        t.buf[pp][k][2 * g] = f0;
-        t.buf[pp][k][2 * g + 1] = f1;
-        l[k] = line(f0, f1);
-      }
-      accumulate<FORM>(l, fe_zero(), sums);
-    }
-    fe acc[NC];
-#pragma unroll
-    for (int k = 0; k < NC; k++) acc[k] = sum_value(sums[k]);
-    acc_to_coeffs<FORM>(acc);
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1)
-#pragma unroll
-      for (int k = 0; k < NC; k++) acc[k] = fadd(acc[k], shfl_down_fe(acc[k], d));
-    if (lane == 0)
-#pragma unroll
-      for (int k = 0; k < NC; k++) red[k][wid] = acc[k];
-    __syncthreads();  // also orders this round's stores before the next round's loads
-    if (wid == 0) {
-#pragma unroll
-      for (int k = 0; k < NC; k++) acc[k] = lane < kTailThreads / 32 ? red[k][lane] : fe_zero();
-#pragma unroll
-      for (int d = 16; d > 0; d >>= 1)
-#pragma unroll
-        for (int k = 0; k < NC; k++) acc[k] = fadd(acc[k], shfl_down_fe(acc[k], d));
-      if (lane == 0) {
-        fe s = acc[NC - 1];
-        for (int k = 0; k < NC; k++) s = fadd(s, acc[k]);
-        if (t.bit && !fe_eq(s, y)) atomicOr(t.flags, t.bit);
-        for (int k = 0; k < NC; k++) put_fe(t.tr, t.off_polys + 16ull * ((uint64_t)i * NC + k), acc[k]);
-        const fe c = t.draw[t.first + (uint64_t)t.stride * i];
-        t.ch[i] = c;
-        y = eval_poly(acc, NC, c);
-        sh_r = c;
-      }
-    }
+    tail_round<FORM>(in, buf[pp], cur, challenge(i - 1), red[i - t.i0]);
     __syncthreads();
-    r = sh_r;
 #pragma unroll
-    for (int k = 0; k < NV; k++) in[k] = t.buf[pp][k];
+    for (int k = 0; k < NV; k++) in[k] = buf[pp][k];
     pp ^= 1;
+    cur /= 2;
   }
-  if (threadIdx.x == 0) *t.y = y;
   // the final fold of the length-2 vectors: their v[0]
   if ((int)threadIdx.x < NV) {
     const fe *p = in[threadIdx.x];
-    const fe v = fadd(p[0], fmul(r, fsub(p[1], p[0])));
+    const fe v = fadd(p[0], fmul(challenge(t.rounds - 1), fsub(p[1], p[0])));
     t.fin[threadIdx.x] = v;
     put_fe(t.tr, t.off_fin + 16ull * threadIdx.x, v);
   }
+  if (threadIdx.x == 0) claim[0] = *t.y;
+  // a warp a round; claim[i + 1] is what round i leaves
+  fe at01[(kMaxLogN + 2 + kTailWarps - 1) / kTailWarps];
+  int q = 0;
+#pragma unroll
+  for (int base = 0; base < kMaxLogN + 2; base += kTailWarps, q++) {
+    const int i = base + wid;
+    if (i >= t.rounds) continue;
+    fe H[NC];
+    if (i < t.i0) {
+#pragma unroll
+      for (int k = 0; k < NC; k++) H[k] = warp_partial_sum(t.partial[i], t.blocks[i], NC, k, lane, 32);
+    } else {
+      const int active = min(kTailWarps, (int)(((t.n >> (i + 1)) + 31) / 32));
+#pragma unroll
+      for (int k = 0; k < NC; k++) {
+        fe x = lane < active ? red[i - t.i0][k][lane] : fe_zero();
+#pragma unroll
+        for (int d = kTailWarps / 2; d > 0; d >>= 1) x = fadd(x, shfl_xor_fe(x, d));
+        H[k] = x;
+      }
+    }
+    if (lane == 0) {
+      const fe c = challenge(i);
+      fe e = H[NC - 1];
+#pragma unroll
+      for (int k = 0; k < NC; k++) {
+        e = fadd(e, H[k]);
+        put_fe(t.tr, t.off_polys + 16ull * ((uint64_t)i * NC + k), H[k]);
+      }
+      at01[q] = e;
+      t.ch[i] = c;
+      claim[i + 1] = eval_poly(H, NC, c);
+    }
+  }
+  __syncthreads();
+  q = 0;
+#pragma unroll
+  for (int base = 0; base < kMaxLogN + 2; base += kTailWarps, q++) {
+    const int i = base + wid;
+    if (i < t.rounds && lane == 0 && t.bit && !fe_eq(at01[q], claim[i])) atomicOr(t.flags, t.bit);
+  }
+  if (threadIdx.x == 0) *t.y = claim[t.rounds];
 }
 
 __global__ void form_sum_kernel(const fe *partial, int blocks, int nc, fe *out) {
@@ -572,11 +635,29 @@ void form_step_launch(int form, const RoundArgs &a, int mode, int blocks, cudaSt
   }
 }
 
+namespace {
+template <int FORM>
+void launch_tail_drawn(const DrawnTailArgs &a, cudaStream_t s) {
+  const size_t sh = tail_shared<FORM>(a.n >> (a.i0 - 1));
+  GBZ_CUDA(cudaFuncSetAttribute(form_tail_drawn_kernel<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)tail_shared<FORM>(1ull << kDrawnTailLog)));
+  form_tail_drawn_kernel<FORM><<<1, kTailThreads, sh, s>>>(a);
+}
+template <int FORM>
+void launch_tail(const TailArgs &a, cudaStream_t s) {
+  GBZ_CUDA(cudaFuncSetAttribute(form_tail_kernel<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)tail_shared<FORM>(kTailEntries)));
+  form_tail_kernel<FORM><<<1, kTailThreads, tail_shared<FORM>(a.cur), s>>>(a);
+}
+}  // namespace
+
 void form_tail_drawn_launch(int form, const DrawnTailArgs &a, cudaStream_t s) {
+  if (a.rounds > kMaxLogN || (a.n >> (a.i0 - 1)) > (1ull << kDrawnTailLog))
+    throw ArgError("sumcheck tail: too many rounds or entries");
   switch (form) {
-    case SC_QUADRATIC: form_tail_drawn_kernel<SC_QUADRATIC><<<1, kTailThreads, 0, s>>>(a); break;
-    case SC_CUBIC: form_tail_drawn_kernel<SC_CUBIC><<<1, kTailThreads, 0, s>>>(a); break;
-    case SC_QUADRUPLE: form_tail_drawn_kernel<SC_QUADRUPLE><<<1, kTailThreads, 0, s>>>(a); break;
+    case SC_QUADRATIC: launch_tail_drawn<SC_QUADRATIC>(a, s); break;
+    case SC_CUBIC: launch_tail_drawn<SC_CUBIC>(a, s); break;
+    case SC_QUADRUPLE: launch_tail_drawn<SC_QUADRUPLE>(a, s); break;
     default: throw ArgError("sumcheck tail: quadratic, cubic or quadruple form");
   }
   GBZ_CUDA(cudaGetLastError());
@@ -666,11 +747,7 @@ void party_sumcheck_enqueue(int form, const fe *const *v, uint64_t M, int N, con
       if (i >= 2 && cur <= kTailEntries) {
         // the remaining rounds and the final fold in one CTA
         TailArgs t{};
-        for (int k = 0; k < nv; k++) {
-          t.in[k] = a.in[k];
-          t.buf[0][k] = scratch[pp * 6 + k];
-          t.buf[1][k] = scratch[(pp ^ 1) * 6 + k];
-        }
+        for (int k = 0; k < nv; k++) t.in[k] = a.in[k];
         t.cur = cur;
         t.i0 = i;
         t.total = total;
@@ -681,8 +758,8 @@ void party_sumcheck_enqueue(int form, const fe *const *v, uint64_t M, int N, con
         t.chal = chal;
         t.fin = fin;
         join(total - 1);
-        if (form == SC_QUADRATIC) form_tail_kernel<SC_QUADRATIC><<<1, kTailThreads, 0, s>>>(t);
-        else form_tail_kernel<SC_CUBIC><<<1, kTailThreads, 0, s>>>(t);
+        if (form == SC_QUADRATIC) launch_tail<SC_QUADRATIC>(t, s);
+        else launch_tail<SC_CUBIC>(t, s);
         GBZ_CUDA(cudaGetLastError());
         return;
       }

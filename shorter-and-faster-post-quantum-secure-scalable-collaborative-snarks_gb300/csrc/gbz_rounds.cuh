@@ -34,15 +34,19 @@ int round_blocks(uint64_t pairs);
 // 2: fold only.
 void form_step_launch(int form, const RoundArgs &a, int mode, int blocks, cudaStream_t s);
 // The rounds i0 (>= 1) .. rounds-1 and the final fold of a sumcheck of
-// n-entry vectors whose challenges are drawn ahead, in one CTA (for n >> i0
-// up to a few thousand entries): in holds the vectors entering round i0
-// (n >> (i0 - 1) entries), buf two sets of n >> i0 entries; round i's
-// challenge is draw[first + stride i] (ch[i0 - 1] the previous one); round
-// messages go to the transcript at off_polys (coefficients of round i at
-// i nc), the final values to fin and to off_fin; *y is the running claim.
+// n-entry vectors whose challenges are drawn ahead, in one CTA: in holds the
+// vectors entering round i0 (n >> (i0 - 1) entries, 2^kDrawnTailLog at most);
+// round i's challenge is draw[first + stride i], stored to ch[i]; the messages
+// of all rounds, those before i0 from their partials (partial[i], blocks[i]),
+// go to the transcript at off_polys (coefficients of round i at i nc), the
+// final values to fin and to off_fin; *y is the running claim.
+// Up to 2^11 entries: a round of the quadruple form on one SM takes 4.4 us
+// there, a launch 4 to 5.
+constexpr int kDrawnTailLog = 11;
 struct DrawnTailArgs {
   const fe *in[4];
-  fe *buf[2][4];
+  const fe *partial[kMaxLogN + 1];
+  int blocks[kMaxLogN + 1];
   uint64_t n;
   int i0, rounds;
   const fe *draw;
@@ -75,7 +79,7 @@ struct SideStream {
 };
 // Entries per vector from which the party sumcheck runs its remaining
 // rounds in one CTA.
-constexpr uint64_t kTailEntries = 1u << 14;
+constexpr uint64_t kTailEntries = 1u << 12;
 // drawn: room for one challenge per glibc round (rounds minus FS rounds).
 void party_sumcheck_enqueue(int form, const fe *const *v, uint64_t M, int N, const fe *w, int offset, RoundState *st,
                             fe *const *scratch, fe *partial, fe *polys, fe *chal, fe *fin, fe *drawn,
