@@ -69,11 +69,11 @@ __global__ void powers_kernel(fe r, uint64_t n, fe *out) {
   if (i < n) out[i] = fpow(r, i);
 }
 
-// x[j] *= omega^{-j} for j < n (omega^{-e} from the inverse tables).
-__global__ void coset_kernel(fe *x, uint64_t n, const fe *inv_lo, const fe *inv_hi, uint64_t row_stride) {
+// f[j] = scale * w^-j, w = root_of_unity(t.logn): the factors of Encode's coset
+// shift (coPCS.cpp:139) with the inverse transform's scale.
+__global__ void coset_factors_kernel(fe *f, uint64_t n, const fe *inv_lo, const fe *inv_hi, fe scale) {
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  x += blockIdx.y * row_stride;
-  if (j < n) x[j] = fmul(x[j], pow_tab(inv_lo, inv_hi, j));
+  if (j < n) f[j] = fmul(scale, pow_tab(inv_lo, inv_hi, j));
 }
 
 // Column roots of distributed_MT (coPCS.cpp:168-176): the root of
@@ -387,9 +387,8 @@ void strided_copy_launch(const fe *x, uint64_t n, fe *out, uint64_t L, int rate,
   GBZ_CUDA(cudaGetLastError());
 }
 
-void coset_launch(fe *x, uint64_t n, const NttTables &t, cudaStream_t s, int rows, uint64_t row_stride) {
-  if (rows < 1) return;
-  coset_kernel<<<dim3(grid(n), (unsigned)rows), 256, 0, s>>>(x, n, t.lo_inv, t.hi_inv, row_stride);
+void coset_factors_launch(fe *f, uint64_t n, const NttTables &t, fe scale, cudaStream_t s) {
+  coset_factors_kernel<<<grid(n), 256, 0, s>>>(f, n, t.lo_inv, t.hi_inv, scale);
   GBZ_CUDA(cudaGetLastError());
 }
 

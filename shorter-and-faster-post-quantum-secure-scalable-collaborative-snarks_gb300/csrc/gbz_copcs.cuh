@@ -14,9 +14,8 @@ void multifold5_launch(const fe *cw, uint64_t n, const fe *a, int logd, fe *out,
                        cudaStream_t s);
 // out[i] = r^i for i < n.
 void powers_launch(fe r, uint64_t n, fe *out, cudaStream_t s);
-// x[j] *= omega_T^{-j} for j < n, T = 2^t.logn.
-// rows vectors of n entries, row_stride apart
-void coset_launch(fe *x, uint64_t n, const NttTables &t, cudaStream_t s, int rows = 1, uint64_t row_stride = 0);
+// f[j] = scale omega_T^{-j} for j < n, T = 2^t.logn.
+void coset_factors_launch(fe *f, uint64_t n, const NttTables &t, fe scale, cudaStream_t s);
 // out[r L + rate t + off] = x[r n + t] for t < n, r < rows.
 void strided_copy_launch(const fe *x, uint64_t n, fe *out, uint64_t L, int rate, int off, int rows, cudaStream_t s);
 // distributed_MT (coPCS.cpp:152-202) of `parties` parties in the same

@@ -60,7 +60,8 @@ struct PassArgs {
   // The outer twiddle of output k is omega_L^{l k 2^tw_shift}.
   const fe *tw_lo;   // omega_L^t, t < 2^12 (nullptr: no outer twiddle)
   const fe *tw_hi;   // omega_L^{2^12 t}
-  const fe *tw_full; // the twiddle at l out_gstride + k out_kstride (optional)
+  const fe *tw_full; // the twiddle at l out_gstride + k out_kstride + h tw_hstride (optional)
+  uint64_t tw_hstride;
   int tw_shift;
   fe scale;
   int logS, logB, has_scale, inverse;
@@ -313,20 +314,21 @@ __device__ __forceinline__ fe load_once(const fe *p) {
 // Writes one output group: values v[q] at positions k + q dk of column l,
 // times the outer twiddle and the scale where the pass has them.
 template <int N>
-__device__ __forceinline__ void emit(const PassArgs &a, fe *out, uint64_t l, uint32_t k, uint32_t dk, const fe *v) {
+__device__ __forceinline__ void emit(const PassArgs &a, fe *out, const fe *tw_full, uint64_t l, uint32_t k,
+                                     uint32_t dk, const fe *v) {
   const uint64_t base = l * a.out_gstride + (uint64_t)k * a.out_kstride, step = (uint64_t)dk * a.out_kstride;
 #pragma unroll
   for (int q = 0; q < N; q++) {
     fe x = v[q];
     const uint64_t addr = base + q * step;
-    if (a.tw_full) {
-      x = fmul(x, a.tw_full[addr]);
+    if (tw_full) {
+      x = fmul(x, tw_full[addr]);
     } else if (a.tw_lo) {
       const uint64_t ex = l * (k + q * dk) << a.tw_shift;
       x = fmul(x, fmul(a.tw_lo[ex & ((1u << kTwLoBits) - 1)], a.tw_hi[ex >> kTwLoBits]));
     }
     if (a.has_scale) x = fmul(x, a.scale);
-    else if (!a.tw_lo && !a.tw_full) x = canon_fe(x);
+    else if (!a.tw_lo && !tw_full) x = canon_fe(x);
     if (!a.acc) out[addr] = x;
     else if (addr < a.acc_n) out[addr] = fadd(out[addr], x);
   }
@@ -358,6 +360,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs
   const uint64_t l0 = g0 & ((1ull << a.logG) - 1), h = g0 >> a.logG;
   const fe *in = a.in + blockIdx.y * a.row_in + h * a.in_hstride;
   fe *out = a.out + blockIdx.y * a.row_out + h * a.out_hstride;
+  const fe *tw_full = a.tw_full ? a.tw_full + h * a.tw_hstride : nullptr;
   fe v[PER][R];
   // first stage: v[r] = x[j + r S/R]
   if (a.sp_l > 0) {
@@ -446,7 +449,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs
     for (int i = 0; i < PER; i++) {
       const uint32_t u = tid + i * blockDim.x;
       const uint32_t b = in_order ? u >> LOGJ : u & ((1u << logB) - 1);
-      if (u < (total >> LOGR)) emit<R>(a, out, l0 + b, 0, 1, v[i]);
+      if (u < (total >> LOGR)) emit<R>(a, out, tw_full, l0 + b, 0, 1, v[i]);
     }
   } else {
 #pragma unroll
@@ -479,16 +482,16 @@ __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs
       for (int r = 0; r < 8; r++) w[r] = sm[slot_step<LOGS - 3>(s0, r)];
       const uint64_t base = (l0 + b) * a.out_gstride + (uint64_t)j * a.out_kstride;
       const uint64_t step = a.out_kstride * (S / 8);
-      const bool staged_tw = a.tw_full && !a.has_scale && !a.acc;
+      const bool staged_tw = tw_full && !a.has_scale && !a.acc;
       twiddle_inputs<LOGS - 3>(w, a.stages, j);
       if (staged_tw) {
         // The outer twiddles arrive during the butterfly, in the slots that
         // this thread alone has read.  Those reads have returned: w[1..7]
         // went through the products, and the first address waits for w[0]
         // (below 2^62, so its top bit adds nothing).
-        copy_async(sm + s0, a.tw_full + base + (w[0].re >> 63));
+        copy_async(sm + s0, tw_full + base + (w[0].re >> 63));
 #pragma unroll
-        for (int r = 1; r < 8; r++) copy_async(sm + slot_step<LOGS - 3>(s0, r), a.tw_full + base + r * step);
+        for (int r = 1; r < 8; r++) copy_async(sm + slot_step<LOGS - 3>(s0, r), tw_full + base + r * step);
       }
       dft8<INV, true>(w);
       if (staged_tw) {
@@ -496,7 +499,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs
 #pragma unroll
         for (int r = 0; r < 8; r++) out[base + r * step] = fmul(w[r], sm[slot_step<LOGS - 3>(s0, r)]);
       } else {
-        emit<8>(a, out, l0 + b, j, S / 8, w);
+        emit<8>(a, out, tw_full, l0 + b, j, S / 8, w);
       }
     }
   }
@@ -661,7 +664,8 @@ void ensure_stages() {
 constexpr int kSmallTotal = 16, kCosetTotal = 18;
 
 bool small_launch(const PassArgs &a, uint64_t groups, int rows) {
-  return a.in_lo || (a.logS >= 1 && a.logS <= kSmallLog && a.logG == 0 && !a.tw_lo && !a.sp_l && !a.acc &&
+  return a.in_lo || (a.logS >= 1 && a.logS <= kSmallLog && a.logG == 0 && !a.tw_lo && !a.tw_full && !a.sp_l &&
+                     !a.acc &&
                      ((groups * (uint64_t)rows) << a.logS) <= (1ull << kSmallTotal));
 }
 
@@ -954,6 +958,7 @@ struct PassGate {
   int pack_real = 0;
   uint32_t *nonreal = nullptr;
   const uint32_t *run_if = nullptr;
+  const fe *out_tab = nullptr;  // output k is multiplied by out_tab[k] (the inverse transform's scale included)
 };
 
 void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe *tmp, bool inverse,
@@ -977,7 +982,8 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
   const int logv = n_valid ? ilog2(2 * n_valid - 1) : 0;  // 2^logv >= n_valid
   const fe *in_end = in + (uint64_t)(rows - 1) * row_in + n_valid;
   const fe *out_end = out + (uint64_t)(rows - 1) * row_out + ((L - 1) * out_elem_stride + 1);
-  if (!gate.pack_real && coset_form(logn, n_valid, rows) && (in_end <= out || out_end <= in)) {
+  if (gate.out_tab && out_elem_stride != 1) throw ArgError("transform: output factors need unit stride");
+  if (!gate.pack_real && !gate.out_tab && coset_form(logn, n_valid, rows) && (in_end <= out || out_end <= in)) {
     a.in = in;
     a.out = out;
     a.n_valid = n_valid;
@@ -1002,9 +1008,10 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
     a.out_kstride = out_elem_stride;
     a.logS = logn;
     a.logB = 0;
-    a.has_scale = inverse;
+    a.has_scale = inverse && !gate.out_tab;
     a.tw_lo = nullptr;
     a.tw_hi = nullptr;
+    a.tw_full = gate.out_tab;
     launch_pass(a, 1, s, rows);
     return;
   }
@@ -1064,7 +1071,9 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
   b.out_kstride = out_elem_stride << done;
   b.logS = rest;
   b.logB = sc.logB[sc.passes - 1];
-  b.has_scale = inverse;
+  b.has_scale = inverse && !gate.out_tab;
+  b.tw_full = gate.out_tab;
+  b.tw_hstride = gate.out_tab ? b.out_hstride : 0;
   launch_pass(b, L >> rest, s, rows);
 }
 
@@ -1131,10 +1140,13 @@ int ntt_launch_real_count(int logn, uint64_t n_valid) {
 }
 
 void ntt_launch_rows(const NttTables &t, const fe *in, uint64_t n_valid, uint64_t in_stride, fe *out,
-                     uint64_t out_stride, int rows, fe *tmp, bool inverse, cudaStream_t s, uint64_t out_elem_stride) {
+                     uint64_t out_stride, int rows, fe *tmp, bool inverse, cudaStream_t s, uint64_t out_elem_stride,
+                     const fe *out_tab) {
   if (rows < 1) return;
   if (out_elem_stride < 1) throw ArgError("transform: output element stride >= 1");
-  ntt_passes(t, in, n_valid, out, tmp, inverse, s, rows, in_stride, out_stride, PassGate(), out_elem_stride);
+  PassGate g;
+  g.out_tab = out_tab;
+  ntt_passes(t, in, n_valid, out, tmp, inverse, s, rows, in_stride, out_stride, g, out_elem_stride);
 }
 
 void ntt_batched(const NttTables &t, const fe *in, uint64_t in_stride, uint32_t j_valid, fe *out, uint64_t count,
