@@ -35,15 +35,6 @@ __global__ void k_dpcs_gather(const fe *arr, uint64_t A, uint64_t S, int N, fe *
   G[(uint64_t)k * S * N + i] = arr[p * A + (uint64_t)k * S + t];
 }
 
-// Party r's row k: out[r][k][m L/N + j] = X_k[r L/N + j + m L], j < L/N.
-__global__ void k_dpcs_scatter(const fe *X, uint64_t L, int N, int rows, fe *out) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;  // position in the party's row
-  if (i >= L) return;
-  const int k = blockIdx.y, r = blockIdx.z;
-  const uint64_t blk = L / N, m = i / blk, j = i % blk;
-  out[((uint64_t)r * rows + k) * L + i] = X[(uint64_t)k * N * L + r * blk + j + m * L];
-}
-
 // Column hashes of every party: column j of a party's nrows x len rows is
 // MT_commit_Blake over its nrows entries (merkle_tree.cpp:201-221): the
 // leaf of its first four entries, then log2(nrows / 4) self-hashes (an
@@ -92,20 +83,22 @@ T *out_view(OpenBufs &ob, T *p, uint64_t count, int mem) {
   return mem == GBZ_MEM_DEVICE ? p : ob.alloc<T>(count);
 }
 
-// The codewords of `rows` batch rows of every party: gather, one transform
-// of length N L per row, scatter into [party][row][L].
+// The codewords of `rows` batch rows of every party: gather, then one
+// transform of length N L per row whose last pass stores into
+// [party][row][L]: party r's row k is out[r][k][m L/N + j] =
+// X_k[r L/N + j + m L], j < L/N.  (A scatter of its own took 351 of the
+// 2360 us at 16 rows of 2^18 and 16 parties.)
 void dpcs_codewords(gbz_ctx *ctx, OpenBufs &ob, const fe *darr, uint64_t A, int N, int rows, int rate, fe *cw) {
   const cudaStream_t s = ctx->stream;
   const uint64_t S = A / rows, L = S * rate, len = L * N;
   const int lg = ilog2(len);
   if (lg > kMaxNttLogN) throw ArgError("dpcs: the distributed transform is longer than 2^26");
-  fe *G = ob.alloc<fe>((uint64_t)rows * S * N), *X = ob.alloc<fe>((uint64_t)rows * len);
+  if (L < (uint64_t)N) throw ArgError("dpcs: codewords shorter than the number of parties");
+  fe *G = ob.alloc<fe>((uint64_t)rows * S * N);
   fe *tmp = lg > 13 ? ob.alloc<fe>((uint64_t)rows * len) : nullptr;
   k_dpcs_gather<<<dim3(nblk2(S * N), rows), 256, 0, s>>>(darr, A, S, N, G);
   GBZ_CUDA(cudaGetLastError());
-  ntt_launch_rows(ctx->tables(lg), G, S * N, S * N, X, len, rows, tmp, false, s);
-  k_dpcs_scatter<<<dim3(nblk2(L), rows, N), 256, 0, s>>>(X, L, N, rows, cw);
-  GBZ_CUDA(cudaGetLastError());
+  ntt_launch_rows_scatter(ctx->tables(lg), G, S * N, S * N, cw, L, rows, tmp, ilog2((uint64_t)N), rows * L, s);
 }
 
 }  // namespace
@@ -240,23 +233,35 @@ __global__ void k_rowsum_global(const fe *cw, int nrows, uint64_t L, int N, cons
   X[r * blk + j + m * L] = facc_value(acc);
 }
 
-// One CTA per (i, j != i, party): sum_k b2_j[k] cdb_i[p][k] (the local
-// part of the eval claims, :1223-1231).
-__global__ void k_cross_dots(const fe *cdb, const fe *b2, uint64_t S, int P, int N, fe *out) {
-  __shared__ fe red[256];
-  const int p = blockIdx.x % N, pair = blockIdx.x / N;
+// One row of CTAs per (i, j != i, party): sum_k b2_j[k] cdb_i[p][k] (the local
+// part of the eval claims, :1223-1231), each CTA a part of k; then a warp per
+// sum over the parts.  (One CTA a sum kept 32 SMs busy at 16 parties: 138 us
+// for 2^16 entries, now 15.)
+constexpr int kDotParts = 16;
+__global__ void __launch_bounds__(256) k_cross_dots(const fe *cdb, const fe *b2, uint64_t S, int P, int N, fe *part) {
+  __shared__ fe red[8];
+  const int p = blockIdx.y % N, pair = blockIdx.y / N;
   const int i = pair / (P - 1), jj = pair % (P - 1), j = jj < i ? jj : jj + 1;
   const fe *a = cdb + ((uint64_t)i * N + p) * S, *b = b2 + (uint64_t)j * S;
   facc acc = facc_zero();
 #pragma unroll 4
-  for (uint64_t k = threadIdx.x; k < S; k += blockDim.x) facc_mul(acc, a[k], b[k]);
-  red[threadIdx.x] = facc_value(acc);
+  for (uint64_t k = blockIdx.x * 256 + threadIdx.x; k < S; k += 256 * kDotParts) facc_mul(acc, a[k], b[k]);
+  fe x = facc_value(acc);
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1)
+    x = fadd(x, fe_make(__shfl_xor_sync(0xffffffffu, x.re, d), __shfl_xor_sync(0xffffffffu, x.im, d)));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
   __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] = fadd(red[threadIdx.x], red[threadIdx.x + s]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[blockIdx.x] = red[0];
+  if (threadIdx.x) return;
+  for (int w = 1; w < 8; w++) x = fadd(x, red[w]);
+  part[blockIdx.y * kDotParts + blockIdx.x] = x;
+}
+__global__ void __launch_bounds__(32) k_cross_sum(const fe *part, fe *out) {
+  fe x = threadIdx.x < kDotParts ? part[blockIdx.x * kDotParts + threadIdx.x] : fe_zero();
+#pragma unroll
+  for (int d = kDotParts / 2; d > 0; d >>= 1)
+    x = fadd(x, fe_make(__shfl_xor_sync(0xffffffffu, x.re, d), __shfl_xor_sync(0xffffffffu, x.im, d)));
+  if (threadIdx.x == 0) out[blockIdx.x] = x;
 }
 
 // arr[p] = sum_l w[l] cdb[l][p]; betas[p] = sum_l v[l][p] b2_l (v: the
@@ -469,8 +474,10 @@ gbz_status gbz_dpcs_open(gbz_ctx *ctx, int N, int P, int rows, uint64_t S, int r
   }
   GBZ_CUDA(cudaGetLastError());
   // the eval claims: every party's cross evaluations, summed with b1_j[p]
-  fe *dx = ob.alloc<fe>((uint64_t)P * (P - 1) * N);
-  k_cross_dots<<<P * (P - 1) * N, 256, 0, s>>>(cdb, db2, S, P, N, dx);
+  const unsigned dots = (unsigned)(P * (P - 1) * N);
+  fe *dx = ob.alloc<fe>(dots), *dxp = ob.alloc<fe>((uint64_t)dots * kDotParts);
+  k_cross_dots<<<dim3(kDotParts, dots), 256, 0, s>>>(cdb, db2, S, P, N, dxp);
+  k_cross_sum<<<dots, 32, 0, s>>>(dxp, dx);
   GBZ_CUDA(cudaGetLastError());
   std::vector<fe> hx((size_t)P * (P - 1) * N);
   GBZ_CUDA(cudaMemcpyAsync(hx.data(), dx, 16 * hx.size(), cudaMemcpyDeviceToHost, s));

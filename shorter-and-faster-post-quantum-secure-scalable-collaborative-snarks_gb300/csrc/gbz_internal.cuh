@@ -158,6 +158,12 @@ int ntt_launch_real_count(int logn, uint64_t n_valid);
 void ntt_launch_rows(const NttTables &t, const fe *in, uint64_t n_valid, uint64_t in_stride, fe *out,
                      uint64_t out_stride, int rows, fe *tmp, bool inverse, cudaStream_t s,
                      uint64_t out_elem_stride = 1, const fe *out_tab = nullptr);
+// `rows` forward transforms whose outputs are dealt to 2^log_parts parts: output
+// i = m len / P + r len / P^2 + j of row y (P parts, j < len / P^2, len =
+// 2^t.logn >= P^2) goes to out + y out_stride + r part_stride + m len / P^2 + j.
+void ntt_launch_rows_scatter(const NttTables &t, const fe *in, uint64_t n_valid, uint64_t in_stride, fe *out,
+                             uint64_t out_stride, int rows, fe *tmp, int log_parts, uint64_t part_stride,
+                             cudaStream_t s);
 // acc[j] += sum_i c[i] * omega_L^{q[i] j} for j < nacc (L = 2^t.logn > 2^13,
 // 1 <= l <= kMaxQueries): the forward transform of the sparse vector
 // sum_i c_i e_{q_i} as one second-pass launch whose rows are formed directly

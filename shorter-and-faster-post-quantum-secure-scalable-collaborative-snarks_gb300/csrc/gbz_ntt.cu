@@ -97,6 +97,10 @@ struct PassArgs {
   // among them sets *nonreal.
   int pack_real;
   uint32_t *nonreal;
+  // Scattered output: output i of the row, with the fields (m, r, j) of
+  // sc_n, sc_n and sc_lo bits from the top, goes to r sc_stride + m 2^sc_lo + j.
+  int sc_lo, sc_n;
+  uint64_t sc_stride;
   // When set, the pass does nothing unless *run_if is non-zero.
   const uint32_t *run_if;
 };
@@ -312,10 +316,11 @@ __device__ __forceinline__ fe load_once(const fe *p) {
 }
 
 // Writes one output group: values v[q] at positions k + q dk of column l,
-// times the outer twiddle and the scale where the pass has them.
-template <int N>
-__device__ __forceinline__ void emit(const PassArgs &a, fe *out, const fe *tw_full, uint64_t l, uint32_t k,
-                                     uint32_t dk, const fe *v) {
+// times the outer twiddle and the scale where the pass has them (SCATTER: at
+// the places of a scattered output, hoff the block's offset in the row).
+template <int N, bool SCATTER>
+__device__ __forceinline__ void emit(const PassArgs &a, fe *out, uint64_t hoff, const fe *tw_full, uint64_t l,
+                                     uint32_t k, uint32_t dk, const fe *v) {
   const uint64_t base = l * a.out_gstride + (uint64_t)k * a.out_kstride, step = (uint64_t)dk * a.out_kstride;
 #pragma unroll
   for (int q = 0; q < N; q++) {
@@ -329,7 +334,11 @@ __device__ __forceinline__ void emit(const PassArgs &a, fe *out, const fe *tw_fu
     }
     if (a.has_scale) x = fmul(x, a.scale);
     else if (!a.tw_lo && !tw_full) x = canon_fe(x);
-    if (!a.acc) out[addr] = x;
+    if (SCATTER) {
+      const uint64_t i = addr + hoff;
+      out[((i >> a.sc_lo) & ((1u << a.sc_n) - 1)) * a.sc_stride + ((i >> (a.sc_lo + a.sc_n)) << a.sc_lo) +
+          (i & ((1ull << a.sc_lo) - 1))] = x;
+    } else if (!a.acc) out[addr] = x;
     else if (addr < a.acc_n) out[addr] = fadd(out[addr], x);
   }
 }
@@ -344,11 +353,14 @@ __device__ __forceinline__ void emit(const PassArgs &a, fe *out, const fe *tw_fu
 // threads an SM at 64 registers) keep other tiles computing while one waits
 // for memory or a barrier.  A pass of 2^8 over 2^24 elements takes 183 us,
 // 0.8 of the sum of its stages alone.
-// PACK: the first pass of a packed real transform.
-template <int LOGS, bool INV, bool PACK>
+// MODE: a plain pass, the first pass of a packed real transform, or the last
+// pass of one with a scattered output.
+enum { PASS_PLAIN, PASS_PACKED, PASS_SCATTER };
+template <int LOGS, bool INV, int MODE>
 __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs a) {
   if (a.run_if && *a.run_if == 0) return;  // uniform over the grid
   extern __shared__ fe smem[];
+  constexpr bool PACK = MODE == PASS_PACKED, SCATTER = MODE == PASS_SCATTER;
   constexpr int LOGR = first_log(LOGS), R = 1 << LOGR, PER = kPerThread / R, LOGJ = LOGS - LOGR;
   constexpr uint32_t S = 1u << LOGS;
   const int logB = a.logB;
@@ -359,7 +371,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs
   const uint64_t g0 = (uint64_t)blockIdx.x << logB;
   const uint64_t l0 = g0 & ((1ull << a.logG) - 1), h = g0 >> a.logG;
   const fe *in = a.in + blockIdx.y * a.row_in + h * a.in_hstride;
-  fe *out = a.out + blockIdx.y * a.row_out + h * a.out_hstride;
+  const uint64_t hoff = h * a.out_hstride;
+  fe *out = a.out + blockIdx.y * a.row_out + (SCATTER ? 0 : hoff);
   const fe *tw_full = a.tw_full ? a.tw_full + h * a.tw_hstride : nullptr;
   fe v[PER][R];
   // first stage: v[r] = x[j + r S/R]
@@ -449,7 +462,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs
     for (int i = 0; i < PER; i++) {
       const uint32_t u = tid + i * blockDim.x;
       const uint32_t b = in_order ? u >> LOGJ : u & ((1u << logB) - 1);
-      if (u < (total >> LOGR)) emit<R>(a, out, tw_full, l0 + b, 0, 1, v[i]);
+      if (u < (total >> LOGR)) emit<R, SCATTER>(a, out, hoff, tw_full, l0 + b, 0, 1, v[i]);
     }
   } else {
 #pragma unroll
@@ -482,7 +495,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs
       for (int r = 0; r < 8; r++) w[r] = sm[slot_step<LOGS - 3>(s0, r)];
       const uint64_t base = (l0 + b) * a.out_gstride + (uint64_t)j * a.out_kstride;
       const uint64_t step = a.out_kstride * (S / 8);
-      const bool staged_tw = tw_full && !a.has_scale && !a.acc;
+      const bool staged_tw = !SCATTER && tw_full && !a.has_scale && !a.acc;
       twiddle_inputs<LOGS - 3>(w, a.stages, j);
       if (staged_tw) {
         // The outer twiddles arrive during the butterfly, in the slots that
@@ -499,7 +512,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs
 #pragma unroll
         for (int r = 0; r < 8; r++) out[base + r * step] = fmul(w[r], sm[slot_step<LOGS - 3>(s0, r)]);
       } else {
-        emit<8>(a, out, tw_full, l0 + b, j, S / 8, w);
+        emit<8, SCATTER>(a, out, hoff, tw_full, l0 + b, j, S / 8, w);
       }
     }
   }
@@ -594,26 +607,27 @@ __global__ void sparse_chain_kernel(const int32_t *q, int l, int shift, uint32_t
 
 typedef void (*PassKernel)(const PassArgs);
 template <int LOGS>
-PassKernel pass_kernel(bool inverse, bool pack) {
-  if (pack) return ntt_pass_kernel<LOGS, false, true>;
-  return inverse ? ntt_pass_kernel<LOGS, true, false> : ntt_pass_kernel<LOGS, false, false>;
+PassKernel pass_kernel(bool inverse, int mode) {
+  if (mode == PASS_PACKED) return ntt_pass_kernel<LOGS, false, PASS_PACKED>;
+  if (mode == PASS_SCATTER) return ntt_pass_kernel<LOGS, false, PASS_SCATTER>;
+  return inverse ? ntt_pass_kernel<LOGS, true, PASS_PLAIN> : ntt_pass_kernel<LOGS, false, PASS_PLAIN>;
 }
-PassKernel pass_kernel(int logS, bool inverse, bool pack) {
+PassKernel pass_kernel(int logS, bool inverse, int mode) {
   switch (logS) {
-    case 0: return pass_kernel<0>(inverse, pack);
-    case 1: return pass_kernel<1>(inverse, pack);
-    case 2: return pass_kernel<2>(inverse, pack);
-    case 3: return pass_kernel<3>(inverse, pack);
-    case 4: return pass_kernel<4>(inverse, pack);
-    case 5: return pass_kernel<5>(inverse, pack);
-    case 6: return pass_kernel<6>(inverse, pack);
-    case 7: return pass_kernel<7>(inverse, pack);
-    case 8: return pass_kernel<8>(inverse, pack);
-    case 9: return pass_kernel<9>(inverse, pack);
-    case 10: return pass_kernel<10>(inverse, pack);
-    case 11: return pass_kernel<11>(inverse, pack);
-    case 12: return pass_kernel<12>(inverse, pack);
-    default: return pass_kernel<13>(inverse, pack);
+    case 0: return pass_kernel<0>(inverse, mode);
+    case 1: return pass_kernel<1>(inverse, mode);
+    case 2: return pass_kernel<2>(inverse, mode);
+    case 3: return pass_kernel<3>(inverse, mode);
+    case 4: return pass_kernel<4>(inverse, mode);
+    case 5: return pass_kernel<5>(inverse, mode);
+    case 6: return pass_kernel<6>(inverse, mode);
+    case 7: return pass_kernel<7>(inverse, mode);
+    case 8: return pass_kernel<8>(inverse, mode);
+    case 9: return pass_kernel<9>(inverse, mode);
+    case 10: return pass_kernel<10>(inverse, mode);
+    case 11: return pass_kernel<11>(inverse, mode);
+    case 12: return pass_kernel<12>(inverse, mode);
+    default: return pass_kernel<13>(inverse, mode);
   }
 }
 
@@ -652,9 +666,9 @@ void ensure_stages() {
                                 (int)(sizeof(fe) * (5u << (kSmallLog - 1)))));
   g_stages_device = dev;
   for (int logS = 0; logS <= kSubLog; logS++)
-    for (int kind = 0; kind < 3; kind++)
-      GBZ_CUDA(cudaFuncSetAttribute(pass_kernel(logS, kind == 1, kind == 2), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(sizeof(fe) * kCtaElems)));
+    for (PassKernel k : {pass_kernel(logS, false, PASS_PLAIN), pass_kernel(logS, true, PASS_PLAIN),
+                         pass_kernel(logS, false, PASS_PACKED), pass_kernel(logS, false, PASS_SCATTER)})
+      GBZ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(fe) * kCtaElems)));
 }
 
 // Launches of up to 2^kSmallTotal elements in sub-transforms of up to
@@ -665,7 +679,7 @@ constexpr int kSmallTotal = 16, kCosetTotal = 18;
 
 bool small_launch(const PassArgs &a, uint64_t groups, int rows) {
   return a.in_lo || (a.logS >= 1 && a.logS <= kSmallLog && a.logG == 0 && !a.tw_lo && !a.tw_full && !a.sp_l &&
-                     !a.acc &&
+                     !a.acc && !a.sc_n &&
                      ((groups * (uint64_t)rows) << a.logS) <= (1ull << kSmallTotal));
 }
 
@@ -687,7 +701,8 @@ void launch_pass(PassArgs a, uint64_t groups, cudaStream_t s, int rows = 1) {
   if (a.logG == 0) a.logG = 40;  // every g is a column of its own
   const uint64_t last = (groups - 1) * a.in_gstride + ((1ull << a.logS) - 1) * a.in_jstride;
   a.dense = a.j_valid >= (1u << a.logS) && (a.n_valid == ~0ull || last < a.n_valid);
-  pass_kernel(a.logS, a.inverse != 0, a.pack_real != 0)<<<dim3((unsigned)tiles, (unsigned)rows), threads, smem, s>>>(a);
+  const int mode = a.pack_real ? PASS_PACKED : a.sc_n ? PASS_SCATTER : PASS_PLAIN;
+  pass_kernel(a.logS, a.inverse != 0, mode)<<<dim3((unsigned)tiles, (unsigned)rows), threads, smem, s>>>(a);
   GBZ_CUDA(cudaGetLastError());
 }
 
@@ -959,6 +974,8 @@ struct PassGate {
   uint32_t *nonreal = nullptr;
   const uint32_t *run_if = nullptr;
   const fe *out_tab = nullptr;  // output k is multiplied by out_tab[k] (the inverse transform's scale included)
+  int sc_lo = 0, sc_n = 0;      // scattered output (PassArgs)
+  uint64_t sc_stride = 0;
 };
 
 void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe *tmp, bool inverse,
@@ -983,7 +1000,9 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
   const fe *in_end = in + (uint64_t)(rows - 1) * row_in + n_valid;
   const fe *out_end = out + (uint64_t)(rows - 1) * row_out + ((L - 1) * out_elem_stride + 1);
   if (gate.out_tab && out_elem_stride != 1) throw ArgError("transform: output factors need unit stride");
-  if (!gate.pack_real && !gate.out_tab && coset_form(logn, n_valid, rows) && (in_end <= out || out_end <= in)) {
+  if (gate.sc_n && (inverse || out_elem_stride != 1 || gate.sc_lo + 2 * gate.sc_n != logn))
+    throw ArgError("transform: scattered output");
+  if (!gate.pack_real && !gate.out_tab && !gate.sc_n && coset_form(logn, n_valid, rows) && (in_end <= out || out_end <= in)) {
     a.in = in;
     a.out = out;
     a.n_valid = n_valid;
@@ -1012,6 +1031,9 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
     a.tw_lo = nullptr;
     a.tw_hi = nullptr;
     a.tw_full = gate.out_tab;
+    a.sc_lo = gate.sc_lo;
+    a.sc_n = gate.sc_n;
+    a.sc_stride = gate.sc_stride;
     launch_pass(a, 1, s, rows);
     return;
   }
@@ -1074,6 +1096,9 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
   b.has_scale = inverse && !gate.out_tab;
   b.tw_full = gate.out_tab;
   b.tw_hstride = gate.out_tab ? b.out_hstride : 0;
+  b.sc_lo = gate.sc_lo;
+  b.sc_n = gate.sc_n;
+  b.sc_stride = gate.sc_stride;
   launch_pass(b, L >> rest, s, rows);
 }
 
@@ -1147,6 +1172,17 @@ void ntt_launch_rows(const NttTables &t, const fe *in, uint64_t n_valid, uint64_
   PassGate g;
   g.out_tab = out_tab;
   ntt_passes(t, in, n_valid, out, tmp, inverse, s, rows, in_stride, out_stride, g, out_elem_stride);
+}
+
+void ntt_launch_rows_scatter(const NttTables &t, const fe *in, uint64_t n_valid, uint64_t in_stride, fe *out,
+                             uint64_t out_stride, int rows, fe *tmp, int log_parts, uint64_t part_stride,
+                             cudaStream_t s) {
+  if (rows < 1) return;
+  PassGate g;
+  g.sc_n = log_parts;
+  g.sc_lo = t.logn - 2 * log_parts;
+  g.sc_stride = part_stride;
+  ntt_passes(t, in, n_valid, out, tmp, false, s, rows, in_stride, out_stride, g);
 }
 
 void ntt_batched(const NttTables &t, const fe *in, uint64_t in_stride, uint32_t j_valid, fe *out, uint64_t count,
