@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(kCalThreads) blake3_peak_kernel(uint32_t *out,
       m[k] = h[k];
       m[8 + k] = h[k];
     }
-    blake3_block64(m, h);
+    blake3_block64<true>(m, h);
   }
   uint32_t s = 0;
 #pragma unroll

@@ -91,10 +91,10 @@ __global__ void column_root_kernel(const fe *rows, int nrows, uint64_t L, uint8_
   for (int k = 0; k < 4; k++) e[k] = k < nrows ? rows[(uint64_t)k * L + j] : fe_zero();
   uint32_t m[16], h[8];
   fe4_words(e[0], e[1], e[2], e[3], m);
-  blake3_block64(m, h);
+  blake3_block64<true>(m, h);
   for (int lv = 0; lv < 3; lv++) {  // 8 leaves -> 4 -> 2 -> 1
     for (int k = 0; k < 8; k++) { m[k] = h[k]; m[8 + k] = h[k]; }
-    blake3_block64(m, h);
+    blake3_block64<true>(m, h);
   }
   uint4 *o = reinterpret_cast<uint4 *>(roots + 32 * j);
   o[0] = make_uint4(h[0], h[1], h[2], h[3]);

@@ -46,10 +46,10 @@ __global__ void k_dpcs_columns(const fe *rows, int nrows, uint64_t len, uint64_t
   const fe *c = rows + blockIdx.y * pstride + j;
   uint32_t m[16], h[8];
   fe4_words(c[0], c[len], c[2 * len], c[3 * len], m);
-  blake3_block64(m, h);
+  blake3_block64<true>(m, h);
   for (int lv = 0; lv < col_levels; lv++) {
     for (int k = 0; k < 8; k++) m[k] = m[8 + k] = h[k];
-    blake3_block64(m, h);
+    blake3_block64<true>(m, h);
   }
   uint4 *o = reinterpret_cast<uint4 *>(levels + blockIdx.y * lstride + 32 * j);
   o[0] = make_uint4(h[0], h[1], h[2], h[3]);

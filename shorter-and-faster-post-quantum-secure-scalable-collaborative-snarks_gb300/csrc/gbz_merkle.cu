@@ -86,7 +86,7 @@ merkle_levels_kernel(const fe *elems, const uint8_t *child, uint64_t cnt0, uint8
 #pragma unroll
       for (int k = 0; k < 8; k++) m[8 + k] = m[k];
     }
-    blake3_block64(m, h);
+    blake3_block64<true>(m, h);
     store_hash(out + 32 * gi, h);
     if (!(i & 1)) {
 #pragma unroll
@@ -107,7 +107,7 @@ merkle_levels_kernel(const fe *elems, const uint8_t *child, uint64_t cnt0, uint8
       uint32_t m[16], h[8];
 #pragma unroll
       for (int k = 0; k < 8; k++) { m[k] = rd[i].w[k]; m[8 + k] = m[k]; }
-      blake3_block64(m, h);
+      blake3_block64<true>(m, h);
       store_hash(o + 32 * (cta_base + i), h);
       if (!(i & 1)) {
 #pragma unroll
@@ -129,7 +129,7 @@ __global__ void blake3_batch_kernel(const uint8_t *in, uint8_t *out, uint64_t co
   for (int k = 0; k < 16; k++)
     m[k] = (uint32_t)p[4 * k] | ((uint32_t)p[4 * k + 1] << 8) | ((uint32_t)p[4 * k + 2] << 16) |
            ((uint32_t)p[4 * k + 3] << 24);
-  blake3_block64(m, h);
+  blake3_block64<true>(m, h);
   for (int k = 0; k < 8; k++)
     for (int b = 0; b < 4; b++) out[32 * i + 4 * k + b] = (uint8_t)(h[k] >> (8 * b));
 }
