@@ -27,6 +27,7 @@ __device__ __forceinline__ fe pow_tab(const fe *lo, const fe *hi, uint64_t e) {
 }
 
 __global__ void bo_init_kernel(ProofState *st, glibc_prng g, fe K0) {
+  pdl_wait();
   if (threadIdx.x) return;
   st->prng = g;
   st->K = K0;
@@ -52,6 +53,7 @@ struct BoQueryArgs {
 // kappa NL / L = 2) and update_betas' weights c_i = r^(i+1) with
 // K += sum_i c_i y_i (:325-342, :383-384).  Thread i handles query i.
 __global__ void __launch_bounds__(kMaxQueries) bo_query_kernel(BoQueryArgs a) {
+  pdl_wait();
   __shared__ int32_t q[kMaxQueries];
   __shared__ fe rb_s;
   __shared__ fe red[kMaxQueries / 32];
@@ -118,6 +120,7 @@ __global__ void __launch_bounds__(kMaxQueries) bo_query_kernel(BoQueryArgs a) {
 // The aggregation challenges (Whir.cpp:809-814): g draws for ch1, g for
 // ch2, then ch1[0] = ch2[0] = 1.  coef = (ch1, ch2).
 __global__ void bo_aggr_draw_kernel(ProofState *st, int g, fe *coef, uint8_t *tr, uint64_t off) {
+  pdl_wait();
   __shared__ glibc_prng gs;
   if (threadIdx.x) return;
   gs = st->prng;
@@ -134,6 +137,7 @@ __global__ void bo_aggr_draw_kernel(ProofState *st, int g, fe *coef, uint8_t *tr
 // K = sum_{i,j} ch2[i] ch1[j] <A_i, B_j>.
 __global__ void bo_aggr_k_kernel(ProofState *st, const fe *evals, const fe *coef, int g, uint8_t *tr,
                                  uint64_t off) {
+  pdl_wait();
   if (threadIdx.x) return;
   fe K = fe_zero();
   for (int i = 0; i < g; i++)
@@ -144,6 +148,7 @@ __global__ void bo_aggr_k_kernel(ProofState *st, const fe *evals, const fe *coef
 
 // The openings aggregate_commitments draws (Whir.cpp:574-576).
 __global__ void bo_aggr_queries_kernel(ProofState *st, int la, int32_t qmod, uint8_t *tr, uint64_t off) {
+  pdl_wait();
   __shared__ glibc_prng gs;
   if (threadIdx.x) return;
   gs = st->prng;
@@ -316,9 +321,10 @@ void batch_open_walk(BatchResources &R, const BatchPlan &P, const fe *const *arr
     if (!hashes) return;
     if (depth != ilog2(lv)) throw ArgError("batch open: path length does not match the tree");
     const unsigned blocks = (unsigned)((hashes + 127) / 128);
-    if (kind == TREE_LEVELS) k_whir_paths<<<blocks, 128, 0, s>>>(levels, lv, l, tr, off_q, off_path);
-    else if (kind == TREE_CODEWORD) k_whir_paths_chain<<<blocks, 128, 0, s>>>(codeword, lv, l, tr, off_q, off_path, 0, 0);
-    else k_zero_tree_paths<<<(unsigned)((depth + 31) / 32), 32, 0, s>>>(depth, l, tr, off_path);
+    if (kind == TREE_LEVELS) launch_kernel(k_whir_paths, blocks, 128, 0, s, levels, lv, l, tr, off_q, off_path);
+    else if (kind == TREE_CODEWORD) launch_kernel(k_whir_paths_chain, blocks, 128, 0, s, codeword, lv, l, tr, off_q,
+                                                  off_path, 0, 0);
+    else launch_kernel(k_zero_tree_paths, (unsigned)((depth + 31) / 32), 32, 0, s, depth, l, tr, off_path);
     GBZ_CUDA(cudaGetLastError());
   };
   uint64_t m = n0, L = L0, leaves = P.zero_tree0 && !P.steps.empty() ? (1ull << P.steps[0].depth) : L0 / 4;
@@ -336,7 +342,7 @@ void batch_open_walk(BatchResources &R, const BatchPlan &P, const fe *const *arr
             sc_step_launch(A[ai], B[ai], m, nullptr, nullptr, nullptr, true, partial, blocks, s);
           else
             sc_step_launch(A[ai], B[ai], m, &st->rw[i - 1], A[ai ^ 1], B[ai ^ 1], true, partial, blocks, s);
-          k_whir_round<<<1, 256, 0, s>>>(partial, blocks, st, i, tr, op, oc);
+          launch_kernel(k_whir_round, 1, 256, 0, s, partial, blocks, st, i, tr, op, oc);
           GBZ_CUDA(cudaGetLastError());
         }
         if (i > 0) {
@@ -355,7 +361,7 @@ void batch_open_walk(BatchResources &R, const BatchPlan &P, const fe *const *arr
       const uint64_t off_root = lay.rec(T_WHIR_ROOT, 1, 32);
       if (!dry) {
         ntt_launch(R.tables(ilog2(NL)), A[ai], m, C[nci], tmp, false, s);
-        k_merkle_root<<<1, 32, 0, s>>>(C[nci], ilog2(NL / 4), tr, off_root);
+        launch_kernel(k_merkle_root, 1, 32, 0, s, C[nci], ilog2(NL / 4), tr, off_root);
         GBZ_CUDA(cudaGetLastError());
       }
       // whir_query on the current codeword and tree
@@ -387,7 +393,7 @@ void batch_open_walk(BatchResources &R, const BatchPlan &P, const fe *const *arr
         qa.new_lo = tnew.lo_fwd;
         qa.new_hi = tnew.hi_fwd;
         qa.len_inv = finv(fe_make((uint64_t)e.kappa, 0));
-        bo_query_kernel<<<1, kMaxQueries, 0, s>>>(qa);
+        launch_kernel(bo_query_kernel, 1, kMaxQueries, 0, s, qa);
         GBZ_CUDA(cudaGetLastError());
         launch_paths(tree_kind, tree, cw, leaves, e.l, e.depth, off_path, qa.off_q);
         // update_betas on the new codeword length: exponents 2 q_i of
@@ -412,7 +418,7 @@ void batch_open_walk(BatchResources &R, const BatchPlan &P, const fe *const *arr
       const uint64_t off_root = lay.rec(T_AGGR_ROOT, 1, 32);
       const int nci = ci == 0 ? 1 : 0;
       if (!dry) {
-        bo_aggr_draw_kernel<<<1, 32, 0, s>>>(st, g, coef, tr, off_ch);
+        launch_kernel(bo_aggr_draw_kernel, 1, 32, 0, s, st, g, coef, tr, off_ch);
         GBZ_CUDA(cudaGetLastError());
         VecList va{}, vb{}, vc{};
         va.p[0] = A[ai];
@@ -426,7 +432,7 @@ void batch_open_walk(BatchResources &R, const BatchPlan &P, const fe *const *arr
         // aggregate_arrays: the inner products first (they read arr and b
         // as they were), then arr += sum_{i>=1} ch2_i A_i, b += sum ch1_i B_i
         multidot_launch(va, g, vb, g, m, mdp, evals, s);
-        bo_aggr_k_kernel<<<1, 32, 0, s>>>(st, evals, coef, g, tr, off_K);
+        launch_kernel(bo_aggr_k_kernel, 1, 32, 0, s, st, evals, coef, g, tr, off_K);
         GBZ_CUDA(cudaGetLastError());
         if (g > 1) {
           VecList oa{}, ob{};
@@ -440,10 +446,10 @@ void batch_open_walk(BatchResources &R, const BatchPlan &P, const fe *const *arr
         // aggregate_commitments: codeword = sum ch2_i C_i, openings in the
         // current tree, then the tree over zero leaves
         lincomb_launch(vc, coef + g, g, L, C[nci], false, s);
-        bo_aggr_queries_kernel<<<1, 32, 0, s>>>(st, e.la, (int32_t)(L / 4), tr, off_q);
+        launch_kernel(bo_aggr_queries_kernel, 1, 32, 0, s, st, e.la, (int32_t)(L / 4), tr, off_q);
         GBZ_CUDA(cudaGetLastError());
         launch_paths(tree_kind, tree, cw, leaves, e.la, e.depth_a, off_p, off_q);
-        k_zero_tree_root<<<1, 32, 0, s>>>(ilog2(e.leaves_after), tr, off_root);
+        launch_kernel(k_zero_tree_root, 1, 32, 0, s, ilog2(e.leaves_after), tr, off_root);
         GBZ_CUDA(cudaGetLastError());
         cw = C[nci];
       }
@@ -465,7 +471,7 @@ void batch_open_walk(BatchResources &R, const BatchPlan &P, const fe *const *arr
     trace->final_arr = A[ai];
   }
   if (!dry) {
-    k_final<<<1, 32, 0, s>>>(st, A[ai], B[ai], (int)m, tr, off_poly, off_point, off_eval, 1, nullptr);
+    launch_kernel(k_final, 1, 32, 0, s, st, A[ai], B[ai], (int)m, tr, off_poly, off_point, off_eval, 1, nullptr);
     GBZ_CUDA(cudaGetLastError());
   }
 }
@@ -485,7 +491,7 @@ void batch_open_enqueue(BatchResources &R, const BatchPlan &P, const fe *const *
   }
   GBZ_CUDA(cudaMemcpyAsync(dtr, img.data(), lay.len, cudaMemcpyHostToDevice, R.s));
   GBZ_CUDA(cudaStreamSynchronize(R.s));  // img is host memory
-  bo_init_kernel<<<1, 32, 0, R.s>>>(R.st, g0, K0);
+  launch_kernel(bo_init_kernel, 1, 32, 0, R.s, R.st, g0, K0);
   GBZ_CUDA(cudaGetLastError());
   Layout lay2;
   batch_open_walk(R, P, arrays, betas, codewords, levels0, dtr, lay2, false);

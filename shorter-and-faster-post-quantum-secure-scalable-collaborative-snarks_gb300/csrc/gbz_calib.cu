@@ -15,6 +15,7 @@ constexpr int kChains = 4;
 // kChains independent multiply chains per thread (enough independent work
 // to keep the pipes busy); the result is stored so nothing is removed.
 __global__ void __launch_bounds__(kCalThreads) fmul_peak_kernel(fe *out, int iters, fe seed) {
+  pdl_wait();
   const uint32_t t = blockIdx.x * kCalThreads + threadIdx.x;
   fe a[kChains];
   const fe w = fe_make((seed.re + t) & P, (seed.im ^ (t * 0x9E37u)) & P);
@@ -31,6 +32,7 @@ __global__ void __launch_bounds__(kCalThreads) fmul_peak_kernel(fe *out, int ite
 
 // One chain of compressions per thread: h <- blake3(h || h).
 __global__ void __launch_bounds__(kCalThreads) blake3_peak_kernel(uint32_t *out, int iters, uint32_t seed) {
+  pdl_wait();
   const uint32_t t = blockIdx.x * kCalThreads + threadIdx.x;
   uint32_t m[16], h[8];
 #pragma unroll
@@ -77,7 +79,7 @@ void calibrate_int_pipes(cudaStream_t s, void *scratch, double *fmul_per_s, doub
   if (fmul_per_s) {
     const int iters = 2048;
     const double ms = time_ms(s, [&] {
-      fmul_peak_kernel<<<blocks, kCalThreads, 0, s>>>((fe *)scratch, iters, fe_make(12345, 678910));
+      launch_kernel(fmul_peak_kernel, blocks, kCalThreads, 0, s, (fe *)scratch, iters, fe_make(12345, 678910));
       GBZ_CUDA(cudaGetLastError());
     });
     *fmul_per_s = (double)threads * kChains * iters / (ms * 1e-3);
@@ -85,7 +87,7 @@ void calibrate_int_pipes(cudaStream_t s, void *scratch, double *fmul_per_s, doub
   if (blake3_per_s) {
     const int iters = 512;
     const double ms = time_ms(s, [&] {
-      blake3_peak_kernel<<<blocks, kCalThreads, 0, s>>>((uint32_t *)scratch, iters, 0x5EEDu);
+      launch_kernel(blake3_peak_kernel, blocks, kCalThreads, 0, s, (uint32_t *)scratch, iters, 0x5EEDu);
       GBZ_CUDA(cudaGetLastError());
     });
     *blake3_per_s = (double)threads * iters / (ms * 1e-3);

@@ -23,6 +23,7 @@ using namespace gbz_api;
 namespace {
 
 __global__ void field_ops_kernel(const fe *a, const fe *b, uint64_t n, fe *s, fe *d, fe *p) {
+  pdl_wait();
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   fe x = a[i], y = b[i];
@@ -33,6 +34,7 @@ __global__ void field_ops_kernel(const fe *a, const fe *b, uint64_t n, fe *s, fe
 
 // comb_i = r^(i+1), omega_q[i] = omega_N^{q_i}.
 __global__ void ub_prep_kernel(ProofState *st, const int32_t *q, int l, int logN, fe r) {
+  pdl_wait();
   if (threadIdx.x == 0) {
     fe c = r;
     for (int i = 0; i < l; i++) {
@@ -53,6 +55,7 @@ __global__ void ub_prep_kernel(ProofState *st, const int32_t *q, int l, int logN
 
 // Loads arbitrary weights: comb_i = c_i, q_i = q_i mod N, omega_q_i = omega_N^{q_i}.
 __global__ void geo_prep_kernel(ProofState *st, const int32_t *q, const fe *c, int l, int logN) {
+  pdl_wait();
   const fe om = root_of_unity(logN);
   const uint32_t mask = (1u << logN) - 1;
   for (int i = threadIdx.x; i < l; i += blockDim.x) {
@@ -76,7 +79,7 @@ static void geometric_update(gbz_ctx *ctx, fe *db, uint64_t nb, const int32_t *h
     fe *dc = (fe *)ctx->buf(99, 16ull * kMaxQueries);
     GBZ_CUDA(cudaMemcpyAsync(dq, hq + i0, 4ull * cnt, cudaMemcpyHostToDevice, ctx->stream));
     GBZ_CUDA(cudaMemcpyAsync(dc, hc + i0, 16ull * cnt, cudaMemcpyHostToDevice, ctx->stream));
-    geo_prep_kernel<<<1, 256, 0, ctx->stream>>>(ctx->st, dq, dc, cnt, logN);
+    launch_kernel(geo_prep_kernel, 1, 256, 0, ctx->stream, ctx->st, dq, dc, cnt, logN);
     GBZ_CUDA(cudaGetLastError());
     const uint64_t N = 1ull << logN;
     if (nb <= N && update_betas_by_transform(cnt, nb, N)) {
@@ -310,7 +313,7 @@ gbz_status gbz_field_ops(gbz_ctx *ctx, const uint64_t *a, const uint64_t *b, uin
   fe *ds = sum ? dev_view(ctx, 2, (fe *)sum, bytes, mem, false) : nullptr;
   fe *dd = diff ? dev_view(ctx, 3, (fe *)diff, bytes, mem, false) : nullptr;
   fe *dp = prod ? dev_view(ctx, 4, (fe *)prod, bytes, mem, false) : nullptr;
-  field_ops_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(da, db, n, ds, dd, dp);
+  launch_kernel(field_ops_kernel, (unsigned)((n + 255) / 256), 256, 0, ctx->stream, da, db, n, ds, dd, dp);
   GBZ_CUDA(cudaGetLastError());
   if (sum) copy_out(ctx, (fe *)sum, ds, bytes, mem);
   if (diff) copy_out(ctx, (fe *)diff, dd, bytes, mem);
@@ -520,7 +523,7 @@ gbz_status gbz_whir_update_betas(gbz_ctx *ctx, uint64_t *b, uint64_t nb, const i
   if (!ctx->ub_scratch) GBZ_CUDA(device_malloc((void **)&ctx->ub_scratch, sizeof(fe) * kUpdateBetasScratch));
   fe *db = dev_view(ctx, 0, (fe *)b, 16 * nb, mem, true);
   const int32_t *dq = dev_view(ctx, 1, queries, 4ull * (l ? l : 1), mem, true);
-  ub_prep_kernel<<<1, 256, 0, ctx->stream>>>(ctx->st, dq, l, ilog2(N), fe_make(r[0], r[1]));
+  launch_kernel(ub_prep_kernel, 1, 256, 0, ctx->stream, ctx->st, dq, l, ilog2(N), fe_make(r[0], r[1]));
   GBZ_CUDA(cudaGetLastError());
   if (nb == 0 || l == 0) {
     // nothing to update; the combination weights are still written

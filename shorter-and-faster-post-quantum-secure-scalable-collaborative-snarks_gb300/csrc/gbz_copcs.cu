@@ -27,6 +27,7 @@ template <int LOGD>
 __global__ void __launch_bounds__(256)
 multifold5_kernel(const fe *cw, uint64_t n, const fe *a, fe *out, const fe *inv_lo, const fe *inv_hi, fe len_inv,
                   FoldConsts k) {
+  pdl_wait();
   constexpr int D = 1 << LOGD;
   const uint64_t nout = n >> LOGD;
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -65,6 +66,7 @@ multifold5_kernel(const fe *cw, uint64_t n, const fe *a, fe *out, const fe *inv_
 }
 
 __global__ void powers_kernel(fe r, uint64_t n, fe *out) {
+  pdl_wait();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = fpow(r, i);
 }
@@ -72,6 +74,7 @@ __global__ void powers_kernel(fe r, uint64_t n, fe *out) {
 // f[j] = scale * w^-j, w = root_of_unity(t.logn): the factors of Encode's coset
 // shift (coPCS.cpp:139) with the inverse transform's scale.
 __global__ void coset_factors_kernel(fe *f, uint64_t n, const fe *inv_lo, const fe *inv_hi, fe scale) {
+  pdl_wait();
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j < n) f[j] = fmul(scale, pow_tab(inv_lo, inv_hi, j));
 }
@@ -83,6 +86,7 @@ __global__ void coset_factors_kernel(fe *f, uint64_t n, const fe *inv_lo, const 
 // computed here.
 __global__ void column_root_kernel(const fe *rows, int nrows, uint64_t L, uint8_t *roots, uint64_t rows_stride,
                                    uint64_t roots_stride) {
+  pdl_wait();
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= L) return;
   rows += rows_stride * blockIdx.y;  // grid.y: parties
@@ -104,6 +108,7 @@ __global__ void column_root_kernel(const fe *rows, int nrows, uint64_t L, uint8_
 // The leader's root tree over {root, 0, ..., 0} of N parties: its root is
 // log2(N) self-hashes of the party root (coPCS.cpp:193-201).
 __global__ void party_root_kernel(const uint8_t *root, int logN, uint8_t *out, uint64_t root_stride) {
+  pdl_wait();
   if (threadIdx.x) return;
   root += root_stride * blockIdx.x;  // one CTA per party
   out += 32 * blockIdx.x;
@@ -120,6 +125,7 @@ __global__ void party_root_kernel(const uint8_t *root, int logN, uint8_t *out, u
 // maps to party j's share by a fixed linear form mu[j][t].
 __global__ void __launch_bounds__(256)
 shares_kernel(const fe *v, const fe *fill, uint64_t groups, int N, int k, int kk, const fe *mu, fe *shares) {
+  pdl_wait();
   __shared__ fe smu[64 * 32];
   for (int t = threadIdx.x; t < N * kk; t += blockDim.x) smu[t] = mu[t];
   __syncthreads();
@@ -142,6 +148,7 @@ shares_kernel(const fe *v, const fe *fill, uint64_t groups, int N, int k, int kk
 constexpr int kAggrCols = 32, kAggrRows = 8;
 __global__ void __launch_bounds__(kAggrCols * kAggrRows)
 aggregate_kernel(const fe *msgs, int N, uint64_t len, const fe *lambda, fe *out) {
+  pdl_wait();
   __shared__ fe red[kAggrRows][kAggrCols];
   const uint64_t i = (uint64_t)blockIdx.x * kAggrCols + threadIdx.x;
   facc acc = facc_zero();
@@ -162,6 +169,7 @@ aggregate_kernel(const fe *msgs, int N, uint64_t len, const fe *lambda, fe *out)
 // g[2j] = b_j (both transform matrices are symmetric).
 constexpr int kLambdaMax = 1024;
 __global__ void __launch_bounds__(1024) lambda_kernel(const fe *b, int N, int logN, fe *lambda) {
+  pdl_wait();
   __shared__ fe g[kLambdaMax], h[kLambdaMax], W[kLambdaMax];
   const int k = threadIdx.x;
   const fe w = root_of_unity(logN);
@@ -185,6 +193,7 @@ __global__ void __launch_bounds__(1024) lambda_kernel(const fe *b, int N, int lo
 
 // flags[blk] = 1 when block blk of v has a non-zero entry.
 __global__ void nonzero_blocks_kernel(const fe *v, uint64_t nblocks, int logd, uint8_t *flags) {
+  pdl_wait();
   const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nblocks) return;
   const fe *p = v + (b << logd);
@@ -200,6 +209,7 @@ __global__ void nonzero_blocks_kernel(const fe *v, uint64_t nblocks, int logd, u
 __global__ void __launch_bounds__(256)
 cophase1_partial_kernel(const fe *e1, const fe *e2, const fe *e3, const fe *e4, const uint8_t *flags,
                         uint64_t nblocks, int logD, int blocks_per_cta, fe *partial) {
+  pdl_wait();
   __shared__ fe red[256];
   // grid.z: the party; its blocks and partials follow the previous party's
   const uint64_t pe = (uint64_t)blockIdx.z * (nblocks << logD);
@@ -233,6 +243,7 @@ cophase1_partial_kernel(const fe *e1, const fe *e2, const fe *e3, const fe *e4, 
 // H[z D + k] = sum_c partial[z][c][k]: one warp per coefficient k, its
 // lanes over the partials (grid.y: the party).
 __global__ void sum_partials_kernel(const fe *partial, uint64_t nparts, uint32_t D, fe *H) {
+  pdl_wait();
   const uint32_t k = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (k >= D) return;
   partial += (uint64_t)blockIdx.y * nparts * D;
@@ -254,6 +265,7 @@ __global__ void sum_partials_kernel(const fe *partial, uint64_t nparts, uint32_t
 // us, then 3.
 template <int LOGW>
 __global__ void __launch_bounds__(256) cophase2_kernel(const fe *v, uint64_t nout, const fe *L, int logd, fe *out) {
+  pdl_wait();
   __shared__ fe sl[1024];
   const uint32_t d = 1u << logd, lane = threadIdx.x & ((1u << LOGW) - 1);
   for (uint32_t k = threadIdx.x; k < d; k += blockDim.x) sl[k] = L[k];
@@ -357,16 +369,20 @@ void multifold5_launch(const fe *cw, uint64_t n, const fe *a, int logd, fe *out,
     for (int g = 0; g < (1 << (logd - 1 - lv)); g++) k.c[lv][g] = fpow(om_inv, ((uint64_t)g * step << lv) & (n - 1));
   const unsigned blocks = grid(n >> logd);
   switch (logd) {
-    case 1: multifold5_kernel<1><<<blocks, 256, 0, s>>>(cw, n, a, out, tn.lo_inv, tn.hi_inv, len_inv, k); break;
-    case 2: multifold5_kernel<2><<<blocks, 256, 0, s>>>(cw, n, a, out, tn.lo_inv, tn.hi_inv, len_inv, k); break;
-    case 3: multifold5_kernel<3><<<blocks, 256, 0, s>>>(cw, n, a, out, tn.lo_inv, tn.hi_inv, len_inv, k); break;
-    default: multifold5_kernel<4><<<blocks, 256, 0, s>>>(cw, n, a, out, tn.lo_inv, tn.hi_inv, len_inv, k); break;
+    case 1: launch_kernel(multifold5_kernel<1>, blocks, 256, 0, s, cw, n, a, out, tn.lo_inv, tn.hi_inv, len_inv,
+                          k); break;
+    case 2: launch_kernel(multifold5_kernel<2>, blocks, 256, 0, s, cw, n, a, out, tn.lo_inv, tn.hi_inv, len_inv,
+                          k); break;
+    case 3: launch_kernel(multifold5_kernel<3>, blocks, 256, 0, s, cw, n, a, out, tn.lo_inv, tn.hi_inv, len_inv,
+                          k); break;
+    default: launch_kernel(multifold5_kernel<4>, blocks, 256, 0, s, cw, n, a, out, tn.lo_inv, tn.hi_inv, len_inv,
+                           k); break;
   }
   GBZ_CUDA(cudaGetLastError());
 }
 
 void powers_launch(fe r, uint64_t n, fe *out, cudaStream_t s) {
-  powers_kernel<<<grid(n), 256, 0, s>>>(r, n, out);
+  launch_kernel(powers_kernel, grid(n), 256, 0, s, r, n, out);
   GBZ_CUDA(cudaGetLastError());
 }
 
@@ -374,6 +390,7 @@ namespace {
 // out[r L + rate t + off] = x[r n + t]: a row's values at one residue of a
 // codeword's positions.
 __global__ void strided_copy_kernel(const fe *x, uint64_t n, fe *out, uint64_t L, int rate, int off) {
+  pdl_wait();
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   out[blockIdx.y * L + (uint64_t)rate * t + off] = x[blockIdx.y * n + t];
@@ -383,12 +400,12 @@ __global__ void strided_copy_kernel(const fe *x, uint64_t n, fe *out, uint64_t L
 void strided_copy_launch(const fe *x, uint64_t n, fe *out, uint64_t L, int rate, int off, int rows, cudaStream_t s) {
   if (rows < 1) return;
   if (rows > 65535) throw ArgError("strided copy: at most 65535 rows per launch");
-  strided_copy_kernel<<<dim3(grid(n), (unsigned)rows), 256, 0, s>>>(x, n, out, L, rate, off);
+  launch_kernel(strided_copy_kernel, dim3(grid(n), (unsigned)rows), 256, 0, s, x, n, out, L, rate, off);
   GBZ_CUDA(cudaGetLastError());
 }
 
 void coset_factors_launch(fe *f, uint64_t n, const NttTables &t, fe scale, cudaStream_t s) {
-  coset_factors_kernel<<<grid(n), 256, 0, s>>>(f, n, t.lo_inv, t.hi_inv, scale);
+  launch_kernel(coset_factors_kernel, grid(n), 256, 0, s, f, n, t.lo_inv, t.hi_inv, scale);
   GBZ_CUDA(cudaGetLastError());
 }
 
@@ -396,32 +413,34 @@ void column_merkle_launch(const fe *rows, int nrows, uint64_t L, uint8_t *levels
                           cudaStream_t s, int parties, uint64_t rows_stride) {
   if (parties < 1 || parties > 65535) throw ArgError("column trees: 1..65535 parties per launch");
   const uint64_t tree = 32 * (2 * L - 1);
-  column_root_kernel<<<dim3(grid(L), (unsigned)parties), 256, 0, s>>>(rows, nrows, L, levels, rows_stride, tree);
+  launch_kernel(column_root_kernel, dim3(grid(L), (unsigned)parties), 256, 0, s, rows, nrows, L, levels, rows_stride,
+                tree);
   GBZ_CUDA(cudaGetLastError());
   merkle_from_leaves_launch(levels, L, s, parties);
-  party_root_kernel<<<parties, 32, 0, s>>>(levels + 32 * (2 * L - 2), logN, root, tree);
+  launch_kernel(party_root_kernel, parties, 32, 0, s, levels + 32 * (2 * L - 2), logN, root, tree);
   GBZ_CUDA(cudaGetLastError());
 }
 
 void shares_launch(const fe *v, const fe *fill, uint64_t groups, int N, const fe *mu, fe *shares, cudaStream_t s) {
-  shares_kernel<<<grid(groups), 256, 0, s>>>(v, fill, groups, N, N / 4, N / 2, mu, shares);
+  launch_kernel(shares_kernel, grid(groups), 256, 0, s, v, fill, groups, N, N / 4, N / 2, mu, shares);
   GBZ_CUDA(cudaGetLastError());
 }
 
 void aggregate_weights_launch(const fe *b, int N, fe *lambda, cudaStream_t s) {
   if (N < 4 || N > kLambdaMax || (N & (N - 1))) throw ArgError("aggregate: N must be a power of two in [4, 1024]");
-  lambda_kernel<<<1, N, 0, s>>>(b, N, ilog2((uint64_t)N), lambda);
+  launch_kernel(lambda_kernel, 1, N, 0, s, b, N, ilog2((uint64_t)N), lambda);
   GBZ_CUDA(cudaGetLastError());
 }
 
 void aggregate_launch(const fe *msgs, int N, uint64_t len, const fe *lambda, fe *out, cudaStream_t s) {
-  aggregate_kernel<<<(unsigned)((len + kAggrCols - 1) / kAggrCols), dim3(kAggrCols, kAggrRows), 0, s>>>(msgs, N, len,
+  launch_kernel(aggregate_kernel, (unsigned)((len + kAggrCols - 1) / kAggrCols), dim3(kAggrCols, kAggrRows), 0, s,
+                msgs, N, len,
                                                                                                  lambda, out);
   GBZ_CUDA(cudaGetLastError());
 }
 
 void nonzero_blocks_launch(const fe *v, uint64_t nblocks, int logd, uint8_t *flags, cudaStream_t s) {
-  nonzero_blocks_kernel<<<grid(nblocks), 256, 0, s>>>(v, nblocks, logd, flags);
+  launch_kernel(nonzero_blocks_kernel, grid(nblocks), 256, 0, s, v, nblocks, logd, flags);
   GBZ_CUDA(cudaGetLastError());
 }
 
@@ -436,10 +455,11 @@ void cophase1_reduce_launch(const fe *e1, const fe *e2, const fe *e3, const fe *
   if (parties < 1 || parties > 65535) throw ArgError("coSumcheck: 1..65535 parties per launch");
   const uint64_t parts = cophase1_parts(nblocks, blocks_per_cta);
   const unsigned chunks = logD > 8 ? 1u << (logD - 8) : 1u;
-  cophase1_partial_kernel<<<dim3((unsigned)parts, chunks, (unsigned)parties), 256, 0, s>>>(
-      e1, e2, e3, e4, flags, nblocks, logD, blocks_per_cta, partial);
+  launch_kernel(cophase1_partial_kernel, dim3((unsigned)parts, chunks, (unsigned)parties), 256, 0, s, e1, e2, e3, e4,
+                flags, nblocks, logD, blocks_per_cta, partial);
   GBZ_CUDA(cudaGetLastError());
-  sum_partials_kernel<<<dim3(grid(1ull << logD, 8), (unsigned)parties), 256, 0, s>>>(partial, parts, 1u << logD, H);
+  launch_kernel(sum_partials_kernel, dim3(grid(1ull << logD, 8), (unsigned)parties), 256, 0, s, partial, parts,
+                1u << logD, H);
   GBZ_CUDA(cudaGetLastError());
 }
 
@@ -449,9 +469,10 @@ void cophase2_launch(const fe *v, uint64_t n, const fe *L, int logd, fe *out, cu
   // eight lanes an output; a warp where that leaves SMs without work (1024
   // outputs of 1024 entries: 38 us with one lane, 3 with 32); blocks below
   // eight entries have no work for more lanes
-  if (logd < 3) cophase2_kernel<0><<<grid(nout), 256, 0, s>>>(v, nout, L, logd, out);
-  else if (logd < 5 || nout >= (1u << 14)) cophase2_kernel<3><<<grid(nout << 3), 256, 0, s>>>(v, nout, L, logd, out);
-  else cophase2_kernel<5><<<grid(nout << 5), 256, 0, s>>>(v, nout, L, logd, out);
+  if (logd < 3) launch_kernel(cophase2_kernel<0>, grid(nout), 256, 0, s, v, nout, L, logd, out);
+  else if (logd < 5 || nout >= (1u << 14)) launch_kernel(cophase2_kernel<3>, grid(nout << 3), 256, 0, s, v, nout, L,
+                                                         logd, out);
+  else launch_kernel(cophase2_kernel<5>, grid(nout << 5), 256, 0, s, v, nout, L, logd, out);
   GBZ_CUDA(cudaGetLastError());
 }
 

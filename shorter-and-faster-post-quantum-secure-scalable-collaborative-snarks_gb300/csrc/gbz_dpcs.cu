@@ -28,6 +28,7 @@ unsigned nblk2(uint64_t n, unsigned t = 256) { return (unsigned)((n + t - 1) / t
 
 // G_k[t N + p] = arr_p[k S + t] for t < S: row k of the interleaved message.
 __global__ void k_dpcs_gather(const fe *arr, uint64_t A, uint64_t S, int N, fe *G) {
+  pdl_wait();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;  // index in the row, t N + p
   if (i >= S * N) return;
   const int k = blockIdx.y;
@@ -41,6 +42,7 @@ __global__ void k_dpcs_gather(const fe *arr, uint64_t A, uint64_t S, int N, fe *
 // inner node hashes its left child twice, merkle_tree.cpp:267-299).
 __global__ void k_dpcs_columns(const fe *rows, int nrows, uint64_t len, uint64_t pstride, int col_levels,
                                uint8_t *levels, uint64_t lstride) {
+  pdl_wait();
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= len) return;
   const fe *c = rows + blockIdx.y * pstride + j;
@@ -96,7 +98,7 @@ void dpcs_codewords(gbz_ctx *ctx, OpenBufs &ob, const fe *darr, uint64_t A, int 
   if (L < (uint64_t)N) throw ArgError("dpcs: codewords shorter than the number of parties");
   fe *G = ob.alloc<fe>((uint64_t)rows * S * N);
   fe *tmp = lg > 13 ? ob.alloc<fe>((uint64_t)rows * len) : nullptr;
-  k_dpcs_gather<<<dim3(nblk2(S * N), rows), 256, 0, s>>>(darr, A, S, N, G);
+  launch_kernel(k_dpcs_gather, dim3(nblk2(S * N), rows), 256, 0, s, darr, A, S, N, G);
   GBZ_CUDA(cudaGetLastError());
   ntt_launch_rows_scatter(ctx->tables(lg), G, S * N, S * N, cw, L, rows, tmp, ilog2((uint64_t)N), rows * L, s);
 }
@@ -142,7 +144,8 @@ gbz_status gbz_dpcs_batch_commit(gbz_ctx *ctx, int N, uint64_t A, const uint64_t
     GBZ_CUDA(cudaMemcpyAsync(commit_data, arr2, 16ull * N * A, k, s));
   }
   // column hashes over the batch rows (distributed_PCS.cpp:76-88), every party's tree
-  k_dpcs_columns<<<dim3(nblk2(L), N), 256, 0, s>>>(cw, batch, L, (uint64_t)batch * L, ilog2((uint64_t)batch / 4), lv,
+  launch_kernel(k_dpcs_columns, dim3(nblk2(L), N), 256, 0, s, cw, batch, L, (uint64_t)batch * L,
+                ilog2((uint64_t)batch / 4), lv,
                                                    32 * nh);
   GBZ_CUDA(cudaGetLastError());
   trees(ctx, lv, L, N, roots, leader_root);
@@ -183,7 +186,7 @@ gbz_status gbz_dpcs_commit(gbz_ctx *ctx, int N, uint64_t A, const uint64_t *arr,
   if (!lv) lv = ob.alloc<uint8_t>(32ull * N * nh);
   dpcs_codewords(ctx, ob, darr, A, N, 1, rate, cw);
   // column i gathers codeword[j L/d1 + i], j < d1 (distributed_PCS.cpp:160-167)
-  k_dpcs_columns<<<dim3(nblk2(leaves), N), 256, 0, s>>>(cw, (int)d1, leaves, L, ilog2(d1 / 4), lv, 32 * nh);
+  launch_kernel(k_dpcs_columns, dim3(nblk2(leaves), N), 256, 0, s, cw, (int)d1, leaves, L, ilog2(d1 / 4), lv, 32 * nh);
   GBZ_CUDA(cudaGetLastError());
   trees(ctx, lv, leaves, N, roots, leader_root);
   if (mem == GBZ_MEM_HOST) {
@@ -209,6 +212,7 @@ enum : uint32_t {
 // out[p][k] = sum_h w[h] rows[p][h][k] (the row batching of commit data,
 // distributed_PCS.cpp:1207-1213).
 __global__ void k_rowsum(const fe *rows, int nrows, uint64_t len, const fe *w, fe *out) {
+  pdl_wait();
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= len) return;
   const fe *r = rows + (uint64_t)blockIdx.y * nrows * len + k;
@@ -222,6 +226,7 @@ __global__ void k_rowsum(const fe *rows, int nrows, uint64_t len, const fe *w, f
 // layout): X[r L/N + j + m L] = sum_h w[h] cw[r][h][m L/N + j]
 // (distributed_PCS.cpp:1214-1219 on the reference's distributed layout).
 __global__ void k_rowsum_global(const fe *cw, int nrows, uint64_t L, int N, const fe *w, fe *X) {
+  pdl_wait();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;  // position in party r's row
   if (i >= L) return;
   const int r = blockIdx.y;
@@ -239,6 +244,7 @@ __global__ void k_rowsum_global(const fe *cw, int nrows, uint64_t L, int N, cons
 // for 2^16 entries, now 15.)
 constexpr int kDotParts = 16;
 __global__ void __launch_bounds__(256) k_cross_dots(const fe *cdb, const fe *b2, uint64_t S, int P, int N, fe *part) {
+  pdl_wait();
   __shared__ fe red[8];
   const int p = blockIdx.y % N, pair = blockIdx.y / N;
   const int i = pair / (P - 1), jj = pair % (P - 1), j = jj < i ? jj : jj + 1;
@@ -257,6 +263,7 @@ __global__ void __launch_bounds__(256) k_cross_dots(const fe *cdb, const fe *b2,
   part[blockIdx.y * kDotParts + blockIdx.x] = x;
 }
 __global__ void __launch_bounds__(32) k_cross_sum(const fe *part, fe *out) {
+  pdl_wait();
   fe x = threadIdx.x < kDotParts ? part[blockIdx.x * kDotParts + threadIdx.x] : fe_zero();
 #pragma unroll
   for (int d = kDotParts / 2; d > 0; d >>= 1)
@@ -268,6 +275,7 @@ __global__ void __launch_bounds__(32) k_cross_sum(const fe *part, fe *out) {
 // parties' weights b1_l[p] times a_l, :1290-1301).
 __global__ void k_batch_vectors(const fe *cdb, const fe *b2, uint64_t S, int P, int N, fe w1, fe w2, const fe *v,
                                 fe *arr, fe *betas) {
+  pdl_wait();
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= S) return;
   const int p = blockIdx.y;
@@ -283,6 +291,7 @@ __global__ void k_batch_vectors(const fe *cdb, const fe *b2, uint64_t S, int P, 
 
 // X = sum_l w[l] Xl[l] over n entries.
 __global__ void k_combine3(const fe *Xl, uint64_t n, int P, fe w1, fe w2, fe *X) {
+  pdl_wait();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   fe acc = Xl[i];
@@ -293,6 +302,7 @@ __global__ void k_combine3(const fe *Xl, uint64_t n, int P, fe w1, fe w2, fe *X)
 // Party r's slice of the global codeword in the distributed layout: for
 // m < nb, the L/N entries from r L/N + m L.
 __global__ void k_party_slices(const fe *X, uint64_t L, int N, uint64_t len, fe *out) {
+  pdl_wait();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= len) return;
   const int r = blockIdx.y;
@@ -366,8 +376,9 @@ void commit_round(gbz_ctx *ctx, OpenBufs &ob, const fe *X, uint64_t L, int N, ui
   const uint64_t len = L / D, leaves = len / d, nh = 2 * leaves - 1;
   fe *sl = ob.alloc<fe>((uint64_t)N * len);
   uint8_t *lv = ob.alloc<uint8_t>(32ull * N * nh);
-  k_party_slices<<<dim3(nblk2(len), N), 256, 0, s>>>(X, L, N, len, sl);
-  k_dpcs_columns<<<dim3(nblk2(leaves), N), 256, 0, s>>>(sl, d, leaves, len, ilog2((uint64_t)d / 4), lv, 32 * nh);
+  launch_kernel(k_party_slices, dim3(nblk2(len), N), 256, 0, s, X, L, N, len, sl);
+  launch_kernel(k_dpcs_columns, dim3(nblk2(leaves), N), 256, 0, s, sl, d, leaves, len, ilog2((uint64_t)d / 4), lv,
+                32 * nh);
   GBZ_CUDA(cudaGetLastError());
   std::vector<uint8_t> roots(32ull * (N + 1));
   trees(ctx, lv, leaves, N, roots.data(), nullptr);
@@ -467,17 +478,18 @@ gbz_status gbz_dpcs_open(gbz_ctx *ctx, int N, int P, int rows, uint64_t S, int r
   // row batching of the data and of the codewords (global order)
   fe *cdb = ob.alloc<fe>((uint64_t)P * N * S), *cwb = ob.alloc<fe>((uint64_t)P * N * L);
   for (int q = 0; q < P; q++) {
-    k_rowsum<<<dim3(nblk2(S), N), 256, 0, s>>>(dcd + (uint64_t)q * N * rows * S, rows, S, db3 + (uint64_t)q * rows,
+    launch_kernel(k_rowsum, dim3(nblk2(S), N), 256, 0, s, dcd + (uint64_t)q * N * rows * S, rows, S,
+                  db3 + (uint64_t)q * rows,
                                               cdb + (uint64_t)q * N * S);
-    k_rowsum_global<<<dim3(nblk2(L), N), 256, 0, s>>>(dcw + (uint64_t)q * N * rows * L, rows, L, N,
+    launch_kernel(k_rowsum_global, dim3(nblk2(L), N), 256, 0, s, dcw + (uint64_t)q * N * rows * L, rows, L, N,
                                                      db3 + (uint64_t)q * rows, cwb + (uint64_t)q * N * L);
   }
   GBZ_CUDA(cudaGetLastError());
   // the eval claims: every party's cross evaluations, summed with b1_j[p]
   const unsigned dots = (unsigned)(P * (P - 1) * N);
   fe *dx = ob.alloc<fe>(dots), *dxp = ob.alloc<fe>((uint64_t)dots * kDotParts);
-  k_cross_dots<<<dim3(kDotParts, dots), 256, 0, s>>>(cdb, db2, S, P, N, dxp);
-  k_cross_sum<<<dots, 32, 0, s>>>(dxp, dx);
+  launch_kernel(k_cross_dots, dim3(kDotParts, dots), 256, 0, s, cdb, db2, S, P, N, dxp);
+  launch_kernel(k_cross_sum, dots, 32, 0, s, dxp, dx);
   GBZ_CUDA(cudaGetLastError());
   std::vector<fe> hx((size_t)P * (P - 1) * N);
   GBZ_CUDA(cudaMemcpyAsync(hx.data(), dx, 16 * hx.size(), cudaMemcpyDeviceToHost, s));
@@ -516,8 +528,8 @@ gbz_status gbz_dpcs_open(gbz_ctx *ctx, int N, int P, int rows, uint64_t S, int r
   fe *dvw = ob.alloc<fe>((uint64_t)P * N), *arr = ob.alloc<fe>((uint64_t)N * S), *bet = ob.alloc<fe>((uint64_t)N * S);
   fe *tmpv = ob.alloc<fe>((uint64_t)N * S), *X = ob.alloc<fe>((uint64_t)N * L), *Xt = ob.alloc<fe>((uint64_t)N * L);
   GBZ_CUDA(cudaMemcpyAsync(dvw, vw.data(), 16 * vw.size(), cudaMemcpyHostToDevice, s));
-  k_batch_vectors<<<dim3(nblk2(S), N), 256, 0, s>>>(cdb, db2, S, P, N, fe_zero(), b1, dvw, arr, bet);
-  k_combine3<<<nblk2((uint64_t)N * L), 256, 0, s>>>(cwb, (uint64_t)N * L, P, fe_zero(), b1, X);
+  launch_kernel(k_batch_vectors, dim3(nblk2(S), N), 256, 0, s, cdb, db2, S, P, N, fe_zero(), b1, dvw, arr, bet);
+  launch_kernel(k_combine3, nblk2((uint64_t)N * L), 256, 0, s, cwb, (uint64_t)N * L, P, fe_zero(), b1, X);
   GBZ_CUDA(cudaGetLastError());
   commit_round(ctx, ob, X, L, N, 1, degs[0], l, L, hfs, rec);
   // the rounds (:1365-1421)

@@ -59,6 +59,7 @@ template <int LOGN>
 __global__ void __launch_bounds__(kThreads)
 merkle_levels_kernel(const fe *elems, const uint8_t *child, uint64_t cnt0, uint8_t *levels,
                      uint64_t level_off0, int nlevels, uint64_t tree_hashes) {
+  pdl_wait();
   // grid.y: independent trees of the same shape, tree_hashes apart (the
   // child levels live in the same tree)
   levels += 32 * tree_hashes * blockIdx.y;
@@ -122,6 +123,7 @@ merkle_levels_kernel(const fe *elems, const uint8_t *child, uint64_t cnt0, uint8
 }
 
 __global__ void blake3_batch_kernel(const uint8_t *in, uint8_t *out, uint64_t count) {
+  pdl_wait();
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   uint32_t m[16], h[8];
@@ -138,10 +140,14 @@ void launch_levels(int logn_cta, const fe *elems, const uint8_t *child, uint64_t
                    uint64_t off, int nlev, cudaStream_t s, int trees = 1, uint64_t tree_hashes = 0) {
   const dim3 g((unsigned)((cnt + (1ull << logn_cta) - 1) >> logn_cta), (unsigned)trees);
   switch (logn_cta) {
-    case 11: merkle_levels_kernel<11><<<g, kThreads, 0, s>>>(elems, child, cnt, levels, off, nlev, tree_hashes); break;
-    case 10: merkle_levels_kernel<10><<<g, kThreads, 0, s>>>(elems, child, cnt, levels, off, nlev, tree_hashes); break;
-    case 9: merkle_levels_kernel<9><<<g, kThreads, 0, s>>>(elems, child, cnt, levels, off, nlev, tree_hashes); break;
-    default: merkle_levels_kernel<8><<<g, kThreads, 0, s>>>(elems, child, cnt, levels, off, nlev, tree_hashes); break;
+    case 11: launch_kernel(merkle_levels_kernel<11>, g, kThreads, 0, s, elems, child, cnt, levels, off, nlev,
+                           tree_hashes); break;
+    case 10: launch_kernel(merkle_levels_kernel<10>, g, kThreads, 0, s, elems, child, cnt, levels, off, nlev,
+                           tree_hashes); break;
+    case 9: launch_kernel(merkle_levels_kernel<9>, g, kThreads, 0, s, elems, child, cnt, levels, off, nlev,
+                          tree_hashes); break;
+    default: launch_kernel(merkle_levels_kernel<8>, g, kThreads, 0, s, elems, child, cnt, levels, off, nlev,
+                           tree_hashes); break;
   }
   GBZ_CUDA(cudaGetLastError());
 }
@@ -207,7 +213,7 @@ int merkle_launch_count(uint64_t N) {
 
 void blake3_batch_launch(const uint8_t *in, uint8_t *out, uint64_t count, cudaStream_t s) {
   if (!count) return;
-  blake3_batch_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(in, out, count);
+  launch_kernel(blake3_batch_kernel, (unsigned)((count + 255) / 256), 256, 0, s, in, out, count);
   GBZ_CUDA(cudaGetLastError());
 }
 

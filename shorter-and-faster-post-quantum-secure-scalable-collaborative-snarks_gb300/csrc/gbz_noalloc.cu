@@ -62,6 +62,7 @@ cudaError_t scratch_on_current_device(cudaStream_t s, NoAllocScratch **out) {
 // comb_i = r^(i+1) (also written to `challenges` when given), the query
 // reduced mod N, and omega_N^{q_i}.
 __global__ void noalloc_prep_kernel(ProofState *st, const int32_t *q, int l, int logN, fe r, fe *challenges) {
+  pdl_wait();
   if (threadIdx.x == 0) {
     fe c = r;
     for (int i = 0; i < l; i++) {
@@ -93,7 +94,7 @@ extern "C" gbz_status gbz_whir_update_betas_noalloc(uint64_t *b, uint64_t nb, co
   cudaStream_t s = (cudaStream_t)cuda_stream;
   NoAllocScratch *scratch = nullptr;
   if (scratch_on_current_device(s, &scratch) != cudaSuccess) return GBZ_ECUDA;
-  noalloc_prep_kernel<<<1, 256, 0, s>>>(&scratch->st, queries, l, ilog2(N), fe_make(r[0], r[1]),
+  launch_kernel(noalloc_prep_kernel, 1, 256, 0, s, &scratch->st, queries, l, ilog2(N), fe_make(r[0], r[1]),
                                         reinterpret_cast<fe *>(challenges));
   if (cudaGetLastError() != cudaSuccess) return GBZ_ECUDA;
   if (nb == 0) return GBZ_OK;  // the weights are written; there is nothing to update

@@ -358,6 +358,7 @@ __device__ __forceinline__ void emit(const PassArgs &a, fe *out, uint64_t hoff, 
 enum { PASS_PLAIN, PASS_PACKED, PASS_SCATTER };
 template <int LOGS, bool INV, int MODE>
 __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs a) {
+  pdl_wait();
   if (a.run_if && *a.run_if == 0) return;  // uniform over the grid
   extern __shared__ fe smem[];
   constexpr bool PACK = MODE == PASS_PACKED, SCATTER = MODE == PASS_SCATTER;
@@ -528,6 +529,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs
 // transform of 2^11 gains nothing).
 // half_tw: omega_{2^kSmallLog}^k of the direction, k < 2^(kSmallLog - 1).
 __global__ void __launch_bounds__(1 << (kSmallLog - 1)) ntt_small_kernel(const PassArgs a, const fe *half_tw) {
+  pdl_wait();
   if (a.run_if && *a.run_if == 0) return;
   extern __shared__ fe smem[];
   const int logS = a.logS, logB = a.logB;
@@ -589,6 +591,7 @@ __global__ void __launch_bounds__(1 << (kSmallLog - 1)) ntt_small_kernel(const P
 // entry of each column.  One thread per entry (l <= kMaxQueries).
 __global__ void sparse_chain_kernel(const int32_t *q, int l, int shift, uint32_t colmask, int16_t *next,
                                     uint8_t *lead) {
+  pdl_wait();
   __shared__ uint32_t col[kMaxQueries];
   const int t = threadIdx.x;
   if (t < l) col[t] = ((uint32_t)q[t] >> shift) & colmask;
@@ -689,8 +692,8 @@ void launch_pass(PassArgs a, uint64_t groups, cudaStream_t s, int rows = 1) {
     // a warp of butterflies a CTA at least
     a.logB = std::min(std::max(0, 6 - a.logS), ilog2(groups & (~groups + 1)));
     const uint32_t threads = 1u << (a.logS - 1 + a.logB);
-    ntt_small_kernel<<<dim3((unsigned)(groups >> a.logB), (unsigned)rows), threads, sizeof(fe) * 5 * threads, s>>>(
-        a, g_half_tw[a.inverse ? 1 : 0]);
+    launch_kernel(ntt_small_kernel, dim3((unsigned)(groups >> a.logB), (unsigned)rows), threads,
+                  sizeof(fe) * 5 * threads, s, a, g_half_tw[a.inverse ? 1 : 0]);
     GBZ_CUDA(cudaGetLastError());
     return;
   }
@@ -702,7 +705,7 @@ void launch_pass(PassArgs a, uint64_t groups, cudaStream_t s, int rows = 1) {
   const uint64_t last = (groups - 1) * a.in_gstride + ((1ull << a.logS) - 1) * a.in_jstride;
   a.dense = a.j_valid >= (1u << a.logS) && (a.n_valid == ~0ull || last < a.n_valid);
   const int mode = a.pack_real ? PASS_PACKED : a.sc_n ? PASS_SCATTER : PASS_PLAIN;
-  pass_kernel(a.logS, a.inverse != 0, mode)<<<dim3((unsigned)tiles, (unsigned)rows), threads, smem, s>>>(a);
+  launch_kernel(pass_kernel(a.logS, a.inverse != 0, mode), dim3((unsigned)tiles, (unsigned)rows), threads, smem, s, a);
   GBZ_CUDA(cudaGetLastError());
 }
 
@@ -720,6 +723,7 @@ bool g_use_outer = true;  // gbz_ntt_full_twiddles
 // T[n1 + N1 k] = w^(n1 k) for n1 < N1, k < N2: thread (n1, chunk) walks 64
 // consecutive k from w^(n1 k0) by products with w^n1.
 __global__ void outer_table_kernel(fe w, int logL, int k1, fe *T) {
+  pdl_wait();
   const uint64_t N1 = 1ull << k1, N2 = 1ull << (logL - k1);
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t chunks = (N2 + 63) / 64;
@@ -765,7 +769,7 @@ void outer_table_build(int logn, int key_k1) {
     fe w = root_of_unity(logn);
     if (dir) w = finv(w);
     const uint64_t threads = (1ull << k1) * (((L >> k1) + 63) / 64);
-    outer_table_kernel<<<(unsigned)((threads + 255) / 256), 256>>>(w, logn, k1, T);
+    launch_kernel(outer_table_kernel, (unsigned)((threads + 255) / 256), 256, 0, 0, w, logn, k1, T);
     GBZ_CUDA(cudaGetLastError());
     GBZ_CUDA(cudaDeviceSynchronize());
     std::lock_guard<std::mutex> lk(g_outer_mu);
@@ -1002,7 +1006,8 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
   if (gate.out_tab && out_elem_stride != 1) throw ArgError("transform: output factors need unit stride");
   if (gate.sc_n && (inverse || out_elem_stride != 1 || gate.sc_lo + 2 * gate.sc_n != logn))
     throw ArgError("transform: scattered output");
-  if (!gate.pack_real && !gate.out_tab && !gate.sc_n && coset_form(logn, n_valid, rows) && (in_end <= out || out_end <= in)) {
+  if (!gate.pack_real && !gate.out_tab && !gate.sc_n && coset_form(logn, n_valid, rows) &&
+      (in_end <= out || out_end <= in)) {
     a.in = in;
     a.out = out;
     a.n_valid = n_valid;
@@ -1123,6 +1128,7 @@ __device__ __forceinline__ fe conj_fe(fe x) { return fe_make(x.re, x.im ? P - x.
 // k = t and M - t (t = 0 and t = M/2 alone): 2 reads, 4 writes, 2 multiplies.
 __global__ void real_unpack_kernel(const fe *__restrict__ Z, uint64_t M, const fe *lo, const fe *hi,
                                    fe *__restrict__ X) {
+  pdl_wait();
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t > M / 2) return;
   const fe a = Z[t], b = Z[t == 0 ? 0 : M - t];
@@ -1152,7 +1158,8 @@ void ntt_launch_real(const NttTables &t_half, const NttTables &t_full, const fe 
   g.nonreal = nonreal;
   ntt_passes(t_half, in, n_valid / 2, Z, tmp, false, s, 1, 0, 0, g);
   const uint64_t threads = M / 2 + 1;
-  real_unpack_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(Z, M, t_full.lo_fwd, t_full.hi_fwd, out);
+  launch_kernel(real_unpack_kernel, (unsigned)((threads + 255) / 256), 256, 0, s, Z, M, t_full.lo_fwd, t_full.hi_fwd,
+                out);
   GBZ_CUDA(cudaGetLastError());
   // any imaginary word: the general transform replaces the result
   PassGate f;
@@ -1268,7 +1275,7 @@ void ntt_sparse_accumulate(const NttTables &t, const int32_t *q, const fe *c, in
   // column chains in the (otherwise unused) scratch
   int16_t *next = reinterpret_cast<int16_t *>(tmp);
   uint8_t *lead = reinterpret_cast<uint8_t *>(next + kMaxQueries);
-  sparse_chain_kernel<<<1, kMaxQueries, 0, s>>>(q, l, q_shift, (uint32_t)(N1 - 1), next, lead);
+  launch_kernel(sparse_chain_kernel, 1, kMaxQueries, 0, s, q, l, q_shift, (uint32_t)(N1 - 1), next, lead);
   GBZ_CUDA(cudaGetLastError());
   PassArgs b{};
   b.stages = t.sub_fwd;

@@ -73,6 +73,7 @@ struct Hdr {
   uint32_t tag, count;
 };
 __global__ void k_headers(const Hdr *h, int n, uint8_t *tr) {
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint32_t *p = reinterpret_cast<uint32_t *>(tr + h[i].off);
@@ -81,6 +82,7 @@ __global__ void k_headers(const Hdr *h, int n, uint8_t *tr) {
 }
 
 __global__ void k_init(PcsDev *st, fe fs, fe K) {
+  pdl_wait();
   st->fs = fs;
   st->K = K;
   st->r_first = st->c = st->s = fe_zero();
@@ -90,6 +92,7 @@ __global__ void k_init(PcsDev *st, fe fs, fe K) {
 // b3' = the packed-Shamir share map applied to b3 (coPCS.cpp:1370-1376):
 // party j's scale of the beta vector.
 __global__ void k_b3p(const fe *b3, int nb3, const fe *mu, int N, fe *b3p) {
+  pdl_wait();
   const int j = threadIdx.x;
   if (j >= N) return;
   fe acc = fe_zero();
@@ -100,6 +103,7 @@ __global__ void k_b3p(const fe *b3, int nb3, const fe *mu, int N, fe *b3p) {
 // out[p][j] = sum_{i < nrows} coef[i] rows[p][i][j] (coPCS.cpp:1352-1356).
 __global__ void k_lincomb(const fe *rows, uint64_t pstride, uint64_t rstride, int nrows, uint64_t len, const fe *coef,
                           fe *out, uint64_t ostride) {
+  pdl_wait();
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= len) return;
   const fe *r = rows + blockIdx.y * pstride + j;
@@ -113,6 +117,7 @@ __global__ void k_lincomb(const fe *rows, uint64_t pstride, uint64_t rstride, in
 // (coPCS.cpp:1385-1397), omega = w_{2 rate_offset Bs}.
 __global__ void k_open_prep(fe *bcd, fe *cdl, fe *B, const fe *b2, const fe *b3p, uint64_t Bs, const fe *lo,
                             const fe *hi, const fe *ilo, const fe *ihi) {
+  pdl_wait();
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= Bs) return;
   const uint64_t at = blockIdx.y * Bs + j;
@@ -127,6 +132,7 @@ __global__ void k_open_prep(fe *bcd, fe *cdl, fe *B, const fe *b2, const fe *b3p
 constexpr int kRedThreads = 256;
 __global__ void __launch_bounds__(kRedThreads)
 k_first_partial(const fe *bcd, const fe *cdl, const fe *B, uint64_t Bs, fe *partial) {
+  pdl_wait();
   __shared__ fe ra[kRedThreads], rb[kRedThreads];
   const uint64_t base = blockIdx.y * Bs;
   facc a = facc_zero(), b = facc_zero();
@@ -154,6 +160,7 @@ k_first_partial(const fe *bcd, const fe *cdl, const fe *B, uint64_t Bs, fe *part
 
 // Party messages H[p] = (a, b, 0) from the partials; also their record.
 __global__ void k_first_reduce(const fe *partial, int nblk, int N, fe *H, uint8_t *tr, uint64_t off_pp) {
+  pdl_wait();
   const int p = threadIdx.x;
   if (p >= N) return;
   fe a = fe_zero(), b = fe_zero();
@@ -172,6 +179,7 @@ __global__ void k_first_reduce(const fe *partial, int nblk, int N, fe *H, uint8_
 // The leader's check and challenge of the batching round (coPCS.cpp:1428-1435).
 __global__ void k_first_verify(PcsDev *st, const fe *poly, uint8_t *tr, uint64_t off_poly, uint64_t off_chal,
                                uint64_t off_K) {
+  pdl_wait();
   if (threadIdx.x) return;
   const fe p0 = poly[0], p1 = poly[1], p2 = poly[2];
   if (!fe_eq(fadd(p0, p1), st->K)) st->error |= 1;
@@ -193,6 +201,7 @@ __global__ void k_first_verify(PcsDev *st, const fe *poly, uint8_t *tr, uint64_t
 // bcd = r bcd + (1 - r) cdl, C' = r C' + (1 - r) codeword[batches - 1].
 __global__ void k_first_fold(fe *bcd, const fe *cdl, fe *B, fe *Cp, const fe *cw_last, uint64_t cw_pstride,
                              uint64_t Bs, uint64_t L, const PcsDev *st) {
+  pdl_wait();
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= L) return;
   const fe r = st->r_first;
@@ -214,6 +223,7 @@ __global__ void k_first_fold(fe *bcd, const fe *cdl, fe *B, fe *Cp, const fe *cw
 // roots is party 0's root hashed log2(N) times.
 __global__ void k_roots(const fe *data, uint64_t pstride, uint64_t estride, int levels, int N, int logN,
                         const uint8_t *stale, uint8_t *roots, uint8_t *tr, uint64_t off_roots, uint64_t off_leader) {
+  pdl_wait();
   __shared__ uint32_t r0[8];
   const int p = threadIdx.x;
   if (p < N) {
@@ -247,6 +257,7 @@ __global__ void k_roots(const fe *data, uint64_t pstride, uint64_t estride, int 
 // 1's, ..., each in draw order.
 __global__ void k_indexes(PcsDev *st, int l, int N, uint32_t Mq, int32_t *qp, int32_t *qpos, uint8_t *tr,
                           uint64_t off) {
+  pdl_wait();
   __shared__ int32_t sp[kPcsMaxQueries], sq[kPcsMaxQueries];
   __shared__ int32_t start[kPcsMaxParties + 1];
   if (threadIdx.x == 0) {
@@ -358,6 +369,7 @@ __device__ fe hash_chain(fe fs, const fe *x, int n) {
 __global__ void __launch_bounds__(256)
 k_round_verify(PcsDev *st, const fe *poly, int logd, fe wi, fe invD, fe invd, fe *L, fe *scratch, uint8_t *tr,
                uint64_t off_poly, uint64_t off_chal) {
+  pdl_wait();
   __shared__ fe chal;
   const int d = 1 << logd, D = 2 * d;
   // (wi = omega_D^-1, invD, invd: constants of the shape, formed on the host)
@@ -388,6 +400,7 @@ k_round_verify(PcsDev *st, const fe *poly, int logd, fe wi, fe invD, fe invd, fe
 __global__ void k_gather(const fe *Cp, uint64_t pstride, uint64_t seg_n, int d, const fe *fold, uint64_t fstride,
                          const int32_t *qp, const int32_t *qpos, int l, fe *y, uint8_t *tr, uint64_t off_y,
                          uint64_t off_seg, fe *seg_out) {
+  pdl_wait();
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (uint64_t)l * d) return;
   const int j = (int)(t / d), k = (int)(t % d);
@@ -406,6 +419,7 @@ __global__ void k_gather(const fe *Cp, uint64_t pstride, uint64_t seg_n, int d, 
 // query's position scaled by rate_{i+2} / rate_{i+1}.
 __global__ void k_check_y(const fe *Cpn, uint64_t pstride, uint32_t mul, uint32_t div, const int32_t *qp,
                           const int32_t *qpos, const fe *y, int l, PcsDev *st) {
+  pdl_wait();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= l) return;
   const uint64_t pos = (uint64_t)mul * (uint32_t)qpos[j] / div;
@@ -418,6 +432,7 @@ __global__ void k_check_y(const fe *Cpn, uint64_t pstride, uint32_t mul, uint32_
 // squarings), the block's sum on thread 0.  Launched with 256 threads.
 __global__ void __launch_bounds__(256)
 k_s_update(PcsDev *st, const fe *y, int l, int addK, uint8_t *tr, uint64_t off_s, uint64_t off_K) {
+  pdl_wait();
   __shared__ fe sh_s;
   __shared__ fe red[256];
   if (threadIdx.x == 0) {
@@ -450,6 +465,7 @@ k_s_update(PcsDev *st, const fe *y, int l, int addK, uint8_t *tr, uint64_t off_s
 // position writes it), one batched transform over the N rows follows.
 __global__ void k_phase3_prep(const PcsDev *st, const int32_t *qp, const int32_t *qpos, int l, uint32_t mul,
                               uint32_t div, int logw, const fe *scale, int N, uint32_t *q, fe *w) {
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= l) return;
   q[i] = (uint32_t)(((uint64_t)mul * (uint32_t)qpos[i] / div) & ((1ull << logw) - 1));
@@ -459,6 +475,7 @@ __global__ void k_phase3_prep(const PcsDev *st, const int32_t *qp, const int32_t
 
 // V (N x W, zero) gets V[p][q_i] = sum of w[p][j] over the queries j at q_i.
 __global__ void k_phase3_scatter(const uint32_t *q, const fe *w, int l, uint64_t W, fe *V) {
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= l) return;
   const uint64_t p = blockIdx.y;
@@ -474,6 +491,7 @@ __global__ void k_phase3_scatter(const uint32_t *q, const fe *w, int l, uint64_t
 
 // B[p][j] += T[p][j] for j < rows (T: N rows of W entries).
 __global__ void k_phase3_add(fe *B, uint64_t rows, const fe *T, uint64_t W) {
+  pdl_wait();
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= rows) return;
   const uint64_t p = blockIdx.y;
@@ -488,6 +506,7 @@ __global__ void k_phase3_add(fe *B, uint64_t rows, const fe *T, uint64_t W) {
 // Q[e] = P_L(w_n^{-e}) = n IDFT_n(L, zero-padded)[e].  So
 // out[p][i] = (n/d) sum_t cw[p][i + t m] iQ[i + t m],  iQ = IDFT_n(L padded).
 __global__ void k_fold_q(const fe *cw, uint64_t n, int logd, const fe *iQ, fe scale, fe *out, uint64_t ostride) {
+  pdl_wait();
   const uint64_t m = n >> logd;
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
@@ -507,6 +526,7 @@ __global__ void k_fold_q(const fe *cw, uint64_t n, int logd, const fe *iQ, fe sc
 __global__ void __launch_bounds__(kRedThreads)
 k_fip_partial(const fe *rows, uint64_t pstride, int nrows, uint64_t len, const fe *brow, const fe *bcol,
               fe *partial) {
+  pdl_wait();
   __shared__ fe red[kRedThreads];
   __shared__ fe sr[32];
   if (threadIdx.x < 32) sr[threadIdx.x] = brow[threadIdx.x];
@@ -531,6 +551,7 @@ k_fip_partial(const fe *rows, uint64_t pstride, int nrows, uint64_t len, const f
 // The leader's combination (MPI_utils.cpp:514-527): K = sum_p lambda_p y_p,
 // thread p forming y_p (launched with at least N <= 64 threads).
 __global__ void k_fip_combine(const fe *partial, int nblk, int N, const fe *lambda, fe *K) {
+  pdl_wait();
   __shared__ fe t[kPcsMaxParties];
   const int p = threadIdx.x;
   if (p < N) {
@@ -547,6 +568,7 @@ __global__ void k_fip_combine(const fe *partial, int nblk, int N, const fe *lamb
 
 // A record payload copied from party-major vectors: out[p][0..len) -> tr.
 __global__ void k_put_party(const fe *v, uint64_t len, int N, uint8_t *tr, uint64_t off, uint64_t rec_stride) {
+  pdl_wait();
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= len) return;
   put_fe(tr, off + blockIdx.y * rec_stride + 16 * j, v[blockIdx.y * len + j]);
@@ -574,6 +596,7 @@ struct CoscDev {
 
 // c = hash_to_field({K, K_r}), K += c K_r (coSumcheck.cpp:234-235).
 __global__ void k_cosc_init(CoscDev *st, fe fs, fe K, fe Kr, uint8_t *tr, uint64_t off_c) {
+  pdl_wait();
   fs = hash_F(fs, K);
   fs = hash_F(fs, Kr);
   st->fs = fs;
@@ -593,6 +616,7 @@ struct ROffs {
 // (coSumcheck.cpp:47-60, 181-193).  One CTA per party.
 __global__ void __launch_bounds__(256)
 k_cosc_add_hr(fe *H, int D, const fe *R, uint64_t rstride, ROffs ro, int iter, int step, const CoscDev *st) {
+  pdl_wait();
   const uint64_t p = blockIdx.x;
   const fe *Rp = R + p * rstride;
   __shared__ fe red[8];
@@ -622,6 +646,7 @@ k_cosc_add_hr(fe *H, int D, const fe *R, uint64_t rstride, ROffs ro, int iter, i
 __global__ void __launch_bounds__(256)
 k_cosc_verify(CoscDev *st, const fe *poly, int logd, int ext, int round, fe wi, fe invD, fe invd, fe *LD, fe *Ld,
               fe *scratch, uint8_t *tr, uint64_t off_poly, uint64_t off_chal) {
+  pdl_wait();
   __shared__ fe chal;
   const int d = 1 << logd, D = d << ext;
   // (wi = omega_D^-1, invD, invd: constants of the shape, formed on the host)
@@ -652,6 +677,7 @@ k_cosc_verify(CoscDev *st, const fe *poly, int logd, int ext, int round, fe wi, 
 constexpr int kCoscThreads = 256;
 __global__ void __launch_bounds__(kCoscThreads)
 k_cosc_sparse(fe *R, uint64_t rstride, ROffs ro, int iter, const fe *LD, int D, int N, CoscDev *st) {
+  pdl_wait();
   const int p = blockIdx.x;
   if (p >= N) return;
   fe *Rp = R + (uint64_t)p * rstride;
@@ -675,6 +701,7 @@ k_cosc_sparse(fe *R, uint64_t rstride, ROffs ro, int iter, const fe *LD, int D, 
 // other round's LD (each round scales all other rounds' entries by its
 // LD[0]).  One CTA per round.
 __global__ void k_cosc_ip(const fe *LD, ROffs ro, fe *ip) {
+  pdl_wait();
   const int i = blockIdx.x;
   fe others = fe_one();
   for (int t = 0; t < ro.n; t++)
@@ -694,6 +721,7 @@ __global__ void k_cosc_final(CoscDev *st, int cubic, int N, const fe *p1, const 
                              uint64_t mstride, const fe *U, const fe *b2, const fe *Ld_hist, const int *logd_hist,
                              int nrounds, const fe *r1, fe wi, fe iq, fe *claims, uint8_t *tr, uint64_t off_shares,
                              uint64_t off_unpacked, uint64_t off_r, uint64_t off_claims) {
+  pdl_wait();
   const int rows = cubic ? 4 : 5, half = N / 2, quarter = N / 4;
   __shared__ fe H[kCoscMaxRows][kPcsMaxParties / 2];
   __shared__ fe L[kPcsMaxParties / 4], r;
@@ -808,6 +836,7 @@ struct PrepareArgs {
 __global__ void __launch_bounds__(256)
 k_prepare(const fe *sh, const fe *rn, uint64_t S, uint64_t R, uint64_t Bs, PrepareArgs a,
           fe *cd) {
+  pdl_wait();
   const RowPart p = a.part[blockIdx.y][0], q = a.part[blockIdx.y][1];
   sh += S * blockIdx.z + p.off - p.col;
   rn += R * blockIdx.z + q.off - q.col;
@@ -1236,9 +1265,9 @@ CoscOut cosumcheck_run(gbz_ctx *ctx, int form, int N, uint64_t n, const fe *p1, 
   uint8_t *tr = ob.alloc<uint8_t>(lay.bytes);
   Hdr *dh = ob.alloc<Hdr>(lay.hdr.size());
   GBZ_CUDA(cudaMemcpyAsync(dh, lay.hdr.data(), sizeof(Hdr) * lay.hdr.size(), cudaMemcpyHostToDevice, s));
-  k_headers<<<grid(lay.hdr.size()), 256, 0, s>>>(dh, (int)lay.hdr.size(), tr);
+  launch_kernel(k_headers, grid(lay.hdr.size()), 256, 0, s, dh, (int)lay.hdr.size(), tr);
   CoscDev *st = ob.alloc<CoscDev>(1);
-  k_cosc_init<<<1, 1, 0, s>>>(st, hfs, hK, hKr, tr, off_c);
+  launch_kernel(k_cosc_init, 1, 1, 0, s, st, hfs, hK, hKr, tr, off_c);
   GBZ_CUDA(cudaGetLastError());
   const int maxD = 1024 << ext;
   // every round's Lagrange vector over its extended block, kept for ip_vec
@@ -1273,14 +1302,14 @@ CoscOut cosumcheck_run(gbz_ctx *ctx, int form, int N, uint64_t n, const fe *p1, 
     const int per_cta = (int)std::max<uint64_t>((uint64_t)lanes, (pblocks + 607) / 608);
     fe *cpart = ob.alloc<fe>((uint64_t)N * D * cophase1_parts(pblocks, per_cta));
     cophase1_reduce_launch(ex[0], ex[1], ex[2], ex[3], zf, pblocks, logd[i] + ext, per_cta, cpart, H, s, N);
-    k_cosc_add_hr<<<N, 256, 0, s>>>(H, D, dR, Rst, ro, i, step, st);
-    k_put_party<<<dim3(grid(D), N), 256, 0, s>>>(H, D, N, tr, off_pp[i], 16ull * D);
+    launch_kernel(k_cosc_add_hr, N, 256, 0, s, H, D, dR, Rst, ro, i, step, st);
+    launch_kernel(k_put_party, dim3(grid(D), N), 256, 0, s, H, D, N, tr, off_pp[i], 16ull * D);
     aggregate_launch(H, N, D, dl, poly, s);
     fe *LD = LDall + ro.off[i];
-    k_cosc_verify<<<1, 256, 0, s>>>(st, poly, logd[i], ext, i, finv(root_of_unity(logd[i] + ext)),
+    launch_kernel(k_cosc_verify, 1, 256, 0, s, st, poly, logd[i], ext, i, finv(root_of_unity(logd[i] + ext)),
                                     finv(fe_make((uint64_t)D, 0)), finv(fe_make(1ull << logd[i], 0)), LD, Ldh + at,
                                     scr, tr, off_poly[i], off_chal[i]);
-    k_cosc_sparse<<<N, kCoscThreads, 0, s>>>(dR, Rst, ro, i, LD, D, N, st);
+    launch_kernel(k_cosc_sparse, N, kCoscThreads, 0, s, dR, Rst, ro, i, LD, D, N, st);
     GBZ_CUDA(cudaGetLastError());
     // phase 2 (coSumcheck.cpp:66-148, 201-213): every vector folded by Ld
     for (fe *v : {v1, v2, v3, vb}) {
@@ -1293,11 +1322,12 @@ CoscOut cosumcheck_run(gbz_ctx *ctx, int form, int N, uint64_t n, const fe *p1, 
   }
   fe *dcl = ob.alloc<fe>(rows);
   const fe wq = N > 4 ? finv(root_of_unity(ilog2(N / 4))) : fe_one();
-  k_cosc_final<<<1, kCoscThreads, 0, s>>>(st, cubic ? 1 : 0, N, v1, v2, v3, vb, m, dU, db2, Ldh, dlog, ndeg, dr1, wq,
+  launch_kernel(k_cosc_final, 1, kCoscThreads, 0, s, st, cubic ? 1 : 0, N, v1, v2, v3, vb, m, dU, db2, Ldh, dlog,
+                ndeg, dr1, wq,
                                           finv(fe_make((uint64_t)(N / 4), 0)), dcl, tr, off_sh, off_un, off_r, off_cl);
   GBZ_CUDA(cudaGetLastError());
   if (ip) {
-    k_cosc_ip<<<ndeg, 256, 0, s>>>(LDall, ro, ip);
+    launch_kernel(k_cosc_ip, ndeg, 256, 0, s, LDall, ro, ip);
     GBZ_CUDA(cudaGetLastError());
   }
   CoscDev hst;
@@ -1395,7 +1425,7 @@ gbz_status gbz_pcs_commit(gbz_ctx *ctx, int N, uint64_t M, int rounds, const int
     if (q.count) throw ArgError("pcs: row layout");
     q = {r.src_off, r.col, r.count};
   }
-  k_prepare<<<dim3((unsigned)((Bs + 1023) / 1024), nb, N), 256, 0, s>>>(dsh, drn, S, R, Bs, pa, pc->cd);
+  launch_kernel(k_prepare, dim3((unsigned)((Bs + 1023) / 1024), nb, N), 256, 0, s, dsh, drn, S, R, Bs, pa, pc->cd);
   GBZ_CUDA(cudaGetLastError());
   // Encode (coPCS.cpp:131-147): every party's rows in the same launches
   encode_rows_device(ctx, pc->cd, N * nb, ilog2(Bs), sc.rate0[0], sc.log_rate_offset, pc->cw);
@@ -1493,9 +1523,10 @@ gbz_status gbz_pcs_claim(gbz_ctx *ctx, const gbz_pcs *pcs, const uint64_t *r, in
   const int nblk = (int)std::min<uint64_t>(64, (pcs->Bs + kRedThreads - 1) / kRedThreads);
   fe *partial = ob.alloc<fe>((uint64_t)N * nblk);
   if (nb - 1 > 32) throw ArgError("pcs: F_ip over more than 32 rows");
-  k_fip_partial<<<dim3(nblk, N), kRedThreads, 0, s>>>(pcs->cd, (uint64_t)nb * pcs->Bs, nb - 1, pcs->Bs, brow, bcol,
+  launch_kernel(k_fip_partial, dim3(nblk, N), kRedThreads, 0, s, pcs->cd, (uint64_t)nb * pcs->Bs, nb - 1, pcs->Bs,
+                brow, bcol,
                                                        partial);
-  k_fip_combine<<<1, kPcsMaxParties, 0, s>>>(partial, nblk, N, dl, dK);
+  launch_kernel(k_fip_combine, 1, kPcsMaxParties, 0, s, partial, nblk, N, dl, dK);
   GBZ_CUDA(cudaGetLastError());
   if (mem == GBZ_MEM_DEVICE) GBZ_CUDA(cudaMemcpyAsync(K, dK, 16, cudaMemcpyDeviceToDevice, s));
   else GBZ_CUDA(cudaMemcpyAsync(K, dK, 16, cudaMemcpyDeviceToHost, s));
@@ -1541,8 +1572,9 @@ gbz_status gbz_pcs_claim_piop(gbz_ctx *ctx, const gbz_pcs *pcs, const uint64_t *
   const int nblk = (int)std::min<uint64_t>(64, (Bs + kRedThreads - 1) / kRedThreads);
   fe *partial = ob.alloc<fe>((uint64_t)N * nblk);
   if (nb - 1 > 32) throw ArgError("pcs: F_ip over more than 32 rows");
-  k_fip_partial<<<dim3(nblk, N), kRedThreads, 0, s>>>(pcs->cd, (uint64_t)nb * Bs, nb - 1, Bs, d1, d2, partial);
-  k_fip_combine<<<1, kPcsMaxParties, 0, s>>>(partial, nblk, N, dl, dK);
+  launch_kernel(k_fip_partial, dim3(nblk, N), kRedThreads, 0, s, pcs->cd, (uint64_t)nb * Bs, nb - 1, Bs, d1, d2,
+                partial);
+  launch_kernel(k_fip_combine, 1, kPcsMaxParties, 0, s, partial, nblk, N, dl, dK);
   GBZ_CUDA(cudaGetLastError());
   if (mem == GBZ_MEM_DEVICE) GBZ_CUDA(cudaMemcpyAsync(K, dK, 16, cudaMemcpyDeviceToDevice, s));
   else GBZ_CUDA(cudaMemcpyAsync(K, dK, 16, cudaMemcpyDeviceToHost, s));
@@ -1606,7 +1638,7 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
   // headers
   Hdr *dh = ob.alloc<Hdr>(lay.hdr.size());
   GBZ_CUDA(cudaMemcpyAsync(dh, lay.hdr.data(), sizeof(Hdr) * lay.hdr.size(), cudaMemcpyHostToDevice, s));
-  k_headers<<<grid(lay.hdr.size()), 256, 0, s>>>(dh, (int)lay.hdr.size(), tr);
+  launch_kernel(k_headers, grid(lay.hdr.size()), 256, 0, s, dh, (int)lay.hdr.size(), tr);
   GBZ_CUDA(cudaGetLastError());
   // The leader's draws depend on the generator alone: the script draws them
   // on the side stream while the parties' rounds run.
@@ -1655,7 +1687,7 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
     hfs = fe_make(fs[0], fs[1]);
   }
   PcsDev *st = ob.alloc<PcsDev>(1);
-  k_init<<<1, 1, 0, s>>>(st, hfs, hK);
+  launch_kernel(k_init, 1, 1, 0, s, st, hfs, hK);
   GBZ_CUDA(cudaGetLastError());
   std::vector<fe> mu = shamir_share_matrix(N), scale((size_t)N * N);
   for (int a = 0; a < N; a++)
@@ -1697,12 +1729,12 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
       GBZ_CUDA(cudaMemcpyAsync(b3, &one, 16, cudaMemcpyHostToDevice, s));
     }
   }
-  k_b3p<<<1, 64, 0, s>>>(b3, N / 4, dmu, N, b3p);
+  launch_kernel(k_b3p, 1, 64, 0, s, b3, N / 4, dmu, N, b3p);
   GBZ_CUDA(cudaGetLastError());
   // row batching (coPCS.cpp:1352-1356) and the transforms of :1359-1366
   fe *Cp = ob.alloc<fe>((uint64_t)N * L), *bcd = ob.alloc<fe>((uint64_t)N * Bs), *cdl = ob.alloc<fe>((uint64_t)N * Bs);
   fe *B = ob.alloc<fe>((uint64_t)N * Bs), *tmp = ob.alloc<fe>(std::max<uint64_t>((uint64_t)N * L, 1ull << 13));
-  k_lincomb<<<dim3(grid(Bs), N), 256, 0, s>>>(pcs->cd, (uint64_t)nb * Bs, Bs, nb - 1, Bs, b1, bcd, Bs);
+  launch_kernel(k_lincomb, dim3(grid(Bs), N), 256, 0, s, pcs->cd, (uint64_t)nb * Bs, Bs, nb - 1, Bs, b1, bcd, Bs);
   GBZ_CUDA(cudaGetLastError());
   // C' = sum_i b1[i] Codeword[i] is Encode of the batched data: every
   // codeword row is Encode(Commit_data row) and Encode is linear, so one
@@ -1715,18 +1747,19 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
   ntt_launch_rows(tB, bcd, Bs, Bs, bcd, Bs, N, tmp, true, s);
   ntt_launch_rows(tB, cdl, Bs, Bs, cdl, Bs, N, tmp, true, s);
   const NttTables &tw = ctx->tables(1 + sc.log_rate_offset + logBs);
-  k_open_prep<<<dim3(grid(Bs), N), 256, 0, s>>>(bcd, cdl, B, b2, b3p, Bs, tw.lo_fwd, tw.hi_fwd, tw.lo_inv,
+  launch_kernel(k_open_prep, dim3(grid(Bs), N), 256, 0, s, bcd, cdl, B, b2, b3p, Bs, tw.lo_fwd, tw.hi_fwd, tw.lo_inv,
                                                  tw.hi_inv);
   GBZ_CUDA(cudaGetLastError());
   // the batching round
   const int nblk = (int)std::min<uint64_t>(64, (Bs + kRedThreads - 1) / kRedThreads);
   fe *partial = ob.alloc<fe>(2ull * N * nblk), *H = ob.alloc<fe>((uint64_t)N * (2 << kPcsMaxLogDeg));
   fe *poly = ob.alloc<fe>(2 << kPcsMaxLogDeg);
-  k_first_partial<<<dim3(nblk, N), kRedThreads, 0, s>>>(bcd, cdl, B, Bs, partial);
-  k_first_reduce<<<1, 64, 0, s>>>(partial, nblk, N, H, tr, off.pp0);
+  launch_kernel(k_first_partial, dim3(nblk, N), kRedThreads, 0, s, bcd, cdl, B, Bs, partial);
+  launch_kernel(k_first_reduce, 1, 64, 0, s, partial, nblk, N, H, tr, off.pp0);
   aggregate_launch(H, N, 3, dlam, poly, s);
-  k_first_verify<<<1, 1, 0, s>>>(st, poly, tr, off.poly0, off.chal0, off.K0);
-  k_first_fold<<<dim3(grid(L), N), 256, 0, s>>>(bcd, cdl, B, Cp, pcs->cw + (uint64_t)(nb - 1) * L, (uint64_t)nb * L,
+  launch_kernel(k_first_verify, 1, 1, 0, s, st, poly, tr, off.poly0, off.chal0, off.K0);
+  launch_kernel(k_first_fold, dim3(grid(L), N), 256, 0, s, bcd, cdl, B, Cp, pcs->cw + (uint64_t)(nb - 1) * L,
+                (uint64_t)nb * L,
                                                 Bs, L, st);
   GBZ_CUDA(cudaGetLastError());
   // batch_commitments_new (coPCS.cpp:1242-1308): the root over C' in columns
@@ -1737,7 +1770,8 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
   int batch_depth = 0;
   {
     const uint64_t c = L / sc.degrees[1];
-    k_roots<<<1, 64, 0, s>>>(Cp, L, c, ilog2(sc.degrees[1] / 4) + ilog2(c), N, logN, nullptr, rts, tr, off.broots,
+    launch_kernel(k_roots, 1, 64, 0, s, Cp, L, c, ilog2(sc.degrees[1] / 4) + ilog2(c), N, logN, nullptr, rts, tr,
+                  off.broots,
                              off.bleader);
     GBZ_CUDA(cudaGetLastError());
     // the batch tree is the commitment a tensor code would inherit when no
@@ -1747,7 +1781,7 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
   }
   int32_t *qp = ob.alloc<int32_t>(kPcsMaxQueries), *qpos = ob.alloc<int32_t>(kPcsMaxQueries);
   if (!is_pow2(L) || L > 0xFFFFFFFFull) throw ArgError("pcs: codeword length must be a power of two below 2^32");
-  k_indexes<<<1, 256, 0, s>>>(st, sc.queries[0], N, (uint32_t)L, qp, qpos, tr, off.bqueries);
+  launch_kernel(k_indexes, 1, 256, 0, s, st, sc.queries[0], N, (uint32_t)L, qp, qpos, tr, off.bqueries);
   GBZ_CUDA(cudaGetLastError());
 
   // the rounds (coPCS.cpp:1452-1600)
@@ -1764,7 +1798,7 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
     GBZ_CUDA(cudaMemcpyAsync(iQ, Ld, 16ull << logd, cudaMemcpyDeviceToDevice, s));
     ntt_launch(ctx->tables(ilog2(len)), iQ, len, iQ, t2, true, s);
     const fe scale = fe_make(len >> logd, 0);
-    k_fold_q<<<dim3(grid(len >> logd), N), 256, 0, s>>>(cw, len, logd, iQ, scale, out, ostride);
+    launch_kernel(k_fold_q, dim3(grid(len >> logd), N), 256, 0, s, cw, len, logd, iQ, scale, out, ostride);
     GBZ_CUDA(cudaGetLastError());
   };
   const int nrounds = sc.rounds - 1;
@@ -1785,9 +1819,10 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
     const int per_cta = (int)std::max<uint64_t>((uint64_t)lanes, (pblocks + 607) / 608);
     fe *cpart = ob.alloc<fe>((uint64_t)N * D * cophase1_parts(pblocks, per_cta));
     cophase1_reduce_launch(e1, e2, nullptr, nullptr, nullptr, pblocks, logd + 1, per_cta, cpart, H, s, N);
-    k_put_party<<<dim3(grid(D), N), 256, 0, s>>>(H, D, N, tr, ro.pp, 16ull * D);
+    launch_kernel(k_put_party, dim3(grid(D), N), 256, 0, s, H, D, N, tr, ro.pp, 16ull * D);
     aggregate_launch(H, N, D, dlam, poly, s);
-    k_round_verify<<<1, 256, 0, s>>>(st, poly, logd, finv(root_of_unity(logd + 1)), finv(fe_make(2ull << logd, 0)),
+    launch_kernel(k_round_verify, 1, 256, 0, s, st, poly, logd, finv(root_of_unity(logd + 1)),
+                  finv(fe_make(2ull << logd, 0)),
                                      finv(fe_make(1ull << logd, 0)), Ld, vscr, tr, ro.poly, ro.chal);
     GBZ_CUDA(cudaGetLastError());
     // pcs_sumcheck_phase2 (coPCS.cpp:571-587)
@@ -1816,7 +1851,7 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
         ntt_batched_strided(tc, Cpn + (uint64_t)p * cpl_new, rows, (uint32_t)d2, Cn + (uint64_t)p * rows * Dc, rows,
                             false, s);
       const uint64_t clen = rows * Dc;
-      k_roots<<<1, 64, 0, s>>>(Cn, clen, 1, ilog2(clen / 4), N, logN, nullptr, rts, tr, ro.roots, ro.leader);
+      launch_kernel(k_roots, 1, 64, 0, s, Cn, clen, 1, ilog2(clen / 4), N, logN, nullptr, rts, tr, ro.roots, ro.leader);
       GBZ_CUDA(cudaGetLastError());
       GBZ_CUDA(cudaMemcpyAsync(prev_rts, rts, 32ull * N, cudaMemcpyDeviceToDevice, s));
       prev_depth = ilog2(clen / 4);
@@ -1838,14 +1873,15 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
       // behaviour in the reference (create_tree_blake writes past its end)
       if (depth > prev_depth) throw ArgError("pcs: tensor code deeper than the previous commitment");
       const bool stale = prev_depth > depth;
-      k_roots<<<1, 64, 0, s>>>(Cpn, cpl_new, 1, depth, N, logN, stale ? prev_rts : nullptr, rts, tr, ro.roots,
+      launch_kernel(k_roots, 1, 64, 0, s, Cpn, cpl_new, 1, depth, N, logN, stale ? prev_rts : nullptr, rts, tr,
+                    ro.roots,
                                ro.leader);
       GBZ_CUDA(cudaGetLastError());
     }
     // delegate_checks (coPCS.cpp:740-891)
     const int l = sc.queries[i + 1];
     if (!is_pow2(seg_n)) throw ArgError("pcs: segment count must be a power of two");
-    k_indexes<<<1, 256, 0, s>>>(st, l, N, (uint32_t)seg_n, qp, qpos, tr, ro.queries);
+    launch_kernel(k_indexes, 1, 256, 0, s, st, l, N, (uint32_t)seg_n, qp, qpos, tr, ro.queries);
     LeaderRound &lr = lead.rounds[i];
     lr.d = d;
     lr.l = l;
@@ -1864,7 +1900,8 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
       lr.qpos = qposc;
       lr.seg = seg_copy;
     }
-    k_gather<<<grid((uint64_t)l * d), 256, 0, s>>>(Cp, cpl, seg_n, d, fold, seg_n, qp, qpos, l, y, tr, ro.y, ro.seg,
+    launch_kernel(k_gather, grid((uint64_t)l * d), 256, 0, s, Cp, cpl, seg_n, d, fold, seg_n, qp, qpos, l, y, tr,
+                  ro.y, ro.seg,
                                                    seg_copy);
     GBZ_CUDA(cudaGetLastError());
     if (full) {
@@ -1874,11 +1911,12 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
       GBZ_CUDA(cudaMemcpyAsync((void *)lr.qpos, qpos, 4ull * l, cudaMemcpyDeviceToDevice, s));
     }
     if (!last) {
-      k_check_y<<<grid(l), 256, 0, s>>>(Cpn, cpl_new, (uint32_t)sc.rate0[i + 2], (uint32_t)sc.rate0[i + 1], qp, qpos,
+      launch_kernel(k_check_y, grid(l), 256, 0, s, Cpn, cpl_new, (uint32_t)sc.rate0[i + 2], (uint32_t)sc.rate0[i + 1],
+                    qp, qpos,
                                         y, l, st);
       GBZ_CUDA(cudaGetLastError());
     }
-    k_s_update<<<1, 256, 0, s>>>(st, y, l, last ? 0 : 1, tr, ro.s, ro.K);
+    launch_kernel(k_s_update, 1, 256, 0, s, st, y, l, last ? 0 : 1, tr, ro.s, ro.K);
     GBZ_CUDA(cudaGetLastError());
     if (full) {
       fe *sc_ = ob.alloc<fe>(1);
@@ -1893,12 +1931,13 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
       fe *V = ob.alloc<fe>((uint64_t)N * W), *T = ob.alloc<fe>((uint64_t)N * W);
       fe *tmp3 = logw > 13 ? ob.alloc<fe>((uint64_t)N * W) : nullptr;
       GBZ_CUDA(cudaMemsetAsync(V, 0, 16ull * N * W, s));
-      k_phase3_prep<<<grid(l), 256, 0, s>>>(st, qp, qpos, l, (uint32_t)sc.rate0[i + 2], (uint32_t)sc.rate0[i + 1],
+      launch_kernel(k_phase3_prep, grid(l), 256, 0, s, st, qp, qpos, l, (uint32_t)sc.rate0[i + 2],
+                    (uint32_t)sc.rate0[i + 1],
                                              logw, dscale, N, q3, wts);
-      k_phase3_scatter<<<dim3(grid(l), N), 256, 0, s>>>(q3, wts, l, W, V);
+      launch_kernel(k_phase3_scatter, dim3(grid(l), N), 256, 0, s, q3, wts, l, W, V);
       GBZ_CUDA(cudaGetLastError());
       ntt_launch_rows(ctx->tables(logw), V, W, W, T, W, N, tmp3, false, s);
-      k_phase3_add<<<dim3(grid(n), N), 256, 0, s>>>(B, n, T, W);
+      launch_kernel(k_phase3_add, dim3(grid(n), N), 256, 0, s, B, n, T, W);
       GBZ_CUDA(cudaGetLastError());
     }
     Cp = Cpn;
@@ -1907,9 +1946,9 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
   // send_pcs_data: every party's data, B and C'
   {
     const uint64_t per = 2 * n + cpl;
-    k_put_party<<<dim3(grid(n), N), 256, 0, s>>>(bcd, n, N, tr, off.final_, 16 * per);
-    k_put_party<<<dim3(grid(n), N), 256, 0, s>>>(B, n, N, tr, off.final_ + 16 * n, 16 * per);
-    k_put_party<<<dim3(grid(cpl), N), 256, 0, s>>>(Cp, cpl, N, tr, off.final_ + 32 * n, 16 * per);
+    launch_kernel(k_put_party, dim3(grid(n), N), 256, 0, s, bcd, n, N, tr, off.final_, 16 * per);
+    launch_kernel(k_put_party, dim3(grid(n), N), 256, 0, s, B, n, N, tr, off.final_ + 16 * n, 16 * per);
+    launch_kernel(k_put_party, dim3(grid(cpl), N), 256, 0, s, Cp, cpl, N, tr, off.final_ + 32 * n, 16 * per);
     GBZ_CUDA(cudaGetLastError());
   }
   // the leader's delegation proofs, final checks and WHIR opening

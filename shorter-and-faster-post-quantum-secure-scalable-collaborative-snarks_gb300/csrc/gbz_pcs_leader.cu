@@ -79,6 +79,7 @@ __device__ fe block_sum_fe(fe v) {
 // end state into after_walk), and the final state.
 __global__ void k_draw_script(glibc_prng g0, const DrawOp *ops, int nops, fe *arena, uint8_t *tr, ProofState *st,
                               glibc_prng *after_walk, glibc_prng *final_state) {
+  pdl_wait();
   __shared__ glibc_prng g;  // dynamically indexed table: work on a shared copy
   if (threadIdx.x) return;
   g = g0;
@@ -101,6 +102,7 @@ __global__ void k_draw_script(glibc_prng g0, const DrawOp *ops, int nops, fe *ar
 
 // The WHIR opening drew as many values as the script skipped for it.
 __global__ void k_prng_check(const ProofState *st, const glibc_prng *expect, uint32_t *flags) {
+  pdl_wait();
   if (threadIdx.x) return;
   bool same = st->prng.f == expect->f && st->prng.r == expect->r;
   for (int i = 0; i < 31; i++) same = same && st->prng.tbl[i] == expect->tbl[i];
@@ -108,6 +110,7 @@ __global__ void k_prng_check(const ProofState *st, const glibc_prng *expect, uin
 }
 
 __global__ void k_tail_init(ProofState *st, glibc_prng g, uint32_t *flags) {
+  pdl_wait();
   if (threadIdx.x) return;
   st->prng = g;
   st->K = fe_zero();
@@ -119,6 +122,7 @@ __global__ void k_tail_init(ProofState *st, glibc_prng g, uint32_t *flags) {
 
 // ---- the delegation sumchecks ------------------------------------------------
 __global__ void k_set(fe *dst, const fe *src) {
+  pdl_wait();
   if (threadIdx.x == 0) *dst = *src;
 }
 
@@ -130,6 +134,7 @@ __global__ void k_set(fe *dst, const fe *src) {
 // (pad_vector) are zero in V1 and V2.  twd[k] = omega_d^-k.
 __global__ void k_pmf_vectors(const fe *seg, const int32_t *qpos, int l, int d, int logd, const fe *twd, fe wn_inv,
                               const fe *L, const fe *b1, fe *V1, fe *V2, fe *V3, fe *V4) {
+  pdl_wait();
   extern __shared__ fe sh[];
   fe *X = sh, *Y = sh + d;
   __shared__ fe wt;
@@ -173,6 +178,7 @@ __global__ void k_pmf_vectors(const fe *seg, const int32_t *qpos, int l, int d, 
 
 // out = scale * sum_{t < n} a[t] b[t] (one CTA), also into *y2 when given.
 __global__ void k_dot(const fe *a, const fe *b, uint64_t n, fe scale, fe *out) {
+  pdl_wait();
   fe acc = fe_zero();
   for (uint64_t t = threadIdx.x; t < n; t += kT) acc = fadd(acc, fmul(a[t], b[t]));
   acc = block_sum_fe(acc);
@@ -185,6 +191,7 @@ __global__ void k_dot(const fe *a, const fe *b, uint64_t n, fe scale, fe *out) {
 __global__ void k_pmf_checks(const fe *fin, const fe *ch, int logd, int logS, const fe *r1, const fe *b12,
                              const fe *b11, const fe *L, const int32_t *qpos, int l, int d, fe wn_inv,
                              uint32_t *flags) {
+  pdl_wait();
   fe acc = fe_zero();
   for (int t = threadIdx.x; t < l; t += kT) {
     fe w = fpow(wn_inv, (uint64_t)(uint32_t)qpos[t]), c = fe_one();
@@ -213,6 +220,7 @@ __global__ void k_pmf_checks(const fe *fin, const fe *ch, int logd, int logS, co
 
 // out[j] = sum_{t < l} w[t] seg[t d + j] for j < d (one CTA per j).
 __global__ void k_seg_comb(const fe *seg, const fe *w, int l, int d, fe *out) {
+  pdl_wait();
   const int j = blockIdx.x;
   fe acc = fe_zero();
   for (int t = threadIdx.x; t < l; t += kT) acc = fadd(acc, fmul(w[t], seg[(uint64_t)t * d + j]));
@@ -224,6 +232,7 @@ __global__ void k_seg_comb(const fe *seg, const fe *w, int l, int d, fe *out) {
 // rm[j] = (1 - r_0 +- omega_d^-j' r_0) prod_{i >= 1} (1 - r_i + omega_d^-(2^i j') r_i), j' = j mod d/2,
 // the sign negative in the upper half.
 __global__ void k_reduced_matrix(const fe *r, int logd, int d, const fe *twd, fe *out) {
+  pdl_wait();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= d) return;
   const int h = j & (d / 2 - 1);
@@ -238,6 +247,7 @@ __global__ void k_reduced_matrix(const fe *r, int logd, int d, const fe *twd, fe
 // evaluate_vector (utils.cpp:1201-1214) of n <= 2^13 entries in one CTA:
 // folds by r[0], r[1], ... through two scratch halves.
 __global__ void k_eval(const fe *v, int logn, const fe *r, fe *s0, fe *s1, fe *out) {
+  pdl_wait();
   const int n = 1 << logn;
   const fe *src = v;
   fe *dst = s0;
@@ -253,6 +263,7 @@ __global__ void k_eval(const fe *v, int logn, const fe *r, fe *s0, fe *s1, fe *o
 }
 
 __global__ void k_check_eq(const fe *a, const fe *b, uint32_t *flags, uint32_t bit) {
+  pdl_wait();
   if (threadIdx.x == 0 && !fe_eq(*a, *b)) atomicOr(flags, bit);
 }
 
@@ -260,6 +271,7 @@ __global__ void k_check_eq(const fe *a, const fe *b, uint32_t *flags, uint32_t b
 // pad) (delegate_protocol.cpp:246-249, coPCS.cpp:843-853).
 __global__ void k_claim(const fe *value, const fe *ra, int na, const fe *rb, int nb, int pad, fe *claim, uint8_t *tr,
                         uint64_t off) {
+  pdl_wait();
   const int k = threadIdx.x;
   if (k > pad) return;
   fe v;
@@ -275,6 +287,7 @@ __global__ void k_claim(const fe *value, const fe *ra, int na, const fe *rb, int
 // o_t = E[t][q_t], the one-hot rows V2 and the weights V3[t][j] = b[t].
 __global__ void k_pe_vectors(const fe *E, const int32_t *q2, int l, uint64_t C0, const fe *b, fe *o, fe *V2, fe *V3,
                              uint64_t total, uint8_t *tr, uint64_t off_o) {
+  pdl_wait();
   const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= total) return;
   const uint64_t t = g / C0, j = g % C0;
@@ -292,6 +305,7 @@ __global__ void k_pe_vectors(const fe *E, const int32_t *q2, int l, uint64_t C0,
 // fin[2] = prod_i eq(r2_i, r_i).
 __global__ void k_pe_checks(const fe *fin, const fe *b1e, const fe *b2e, const int32_t *q2, int l, const fe *r2e,
                             const fe *r, int logS, uint32_t *flags) {
+  pdl_wait();
   fe acc = fe_zero();
   for (int t = threadIdx.x; t < l; t += kT) acc = fadd(acc, fmul(b1e[(uint32_t)q2[t]], b2e[t]));
   acc = block_sum_fe(acc);
@@ -309,6 +323,7 @@ __global__ void k_pe_checks(const fe *fin, const fe *b1e, const fe *b2e, const i
 // b < 2^(n-1), zero above; omega = omega_{2^n} from the tables (lo, hi).
 // With nr < n the missing r_m are zero (their factor is 1).
 __global__ void k_phi(const fe *r, int nr, int n, const fe *lo, const fe *hi, fe scale, fe *out) {
+  pdl_wait();
   const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, N = 1ull << n;
   if (b >= N) return;
   if (b >= N / 2) {
@@ -325,6 +340,7 @@ __global__ void k_phi(const fe *r, int nr, int n, const fe *lo, const fe *hi, fe
 // point without its last log2(rate) entries.
 __global__ void k_ext_claim(const fe *fin, const fe *rpf, int npf, int lograte, const fe *r2e, int logS, uint8_t *tr,
                             uint64_t off) {
+  pdl_wait();
   if (threadIdx.x) return;
   fe c = fin[1];
   const fe inv = finv(fsub(fe_one(), rpf[npf - 1]));
@@ -338,6 +354,7 @@ __global__ void k_ext_claim(const fe *fin, const fe *rpf, int npf, int lograte, 
 // ---- the final steps (coPCS.cpp:1697-1752) ---------------------------------------
 // Decoding: the first n entries of every party's inverse-transformed C' are its data.
 __global__ void k_decode_check(const fe *dec, uint64_t cpl, const fe *data, uint64_t n, int N, uint32_t *flags) {
+  pdl_wait();
   const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (uint64_t)N * n) return;
   const uint64_t p = g / n, j = g % n;
@@ -348,6 +365,7 @@ __global__ void k_decode_check(const fe *dec, uint64_t cpl, const fe *data, uint
 // then K - sum final_poly final_B = 0 (final verification step 1).
 __global__ void k_unpack_final(const fe *U, const fe *bcd, const fe *B, int N, const fe *K, fe *fp, fe *fB,
                                uint32_t *flags, uint8_t *tr, uint64_t off) {
+  pdl_wait();
   const int j = threadIdx.x;
   __shared__ fe prod[32];
   if (j < N / 2) {
@@ -373,6 +391,7 @@ __global__ void k_unpack_final(const fe *U, const fe *bcd, const fe *B, int N, c
 // (Sums row-major, R x R), into the opening's running claim.
 __global__ void k_aggr_K(const fe *sums, const fe *ch, int R, ProofState *st, uint8_t *tr, uint64_t off_ch,
                          uint64_t off_K) {
+  pdl_wait();
   if (threadIdx.x) return;
   fe K = fe_zero();
   for (int a = 0; a < R; a++)
@@ -390,6 +409,7 @@ struct ChalOffs {
 // total_r of _Whir_Open (Whir.cpp:506-509): every round challenge, then the
 // final point.
 __global__ void k_gather_r(const uint8_t *tr, ChalOffs c, uint64_t off_point, int npoint, fe *out) {
+  pdl_wait();
   const int k = threadIdx.x;
   if (k < c.n) out[k] = get_fe(tr, c.off[k]);
   else if (k < c.n + npoint) out[k] = get_fe(tr, off_point + 16ull * (k - c.n));
@@ -399,6 +419,7 @@ __global__ void k_gather_r(const uint8_t *tr, ChalOffs c, uint64_t off_point, in
 // re-encoded at the final rate equals the last codeword.
 __global__ void k_reencode_check(const fe *arr, int m, const fe *cw, uint64_t L, const fe *lo, const fe *hi,
                                  ProofState *st) {
+  pdl_wait();
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= L) return;
   fe v = fe_zero();
@@ -420,6 +441,7 @@ struct Step3Args {
 // omega identities of every iteration's scaled queries (weights c_i).
 __global__ void k_whir_step3(const uint8_t *tr, Step3Args a, const fe *claims, const fe *bac, const fe *total_r,
                              uint32_t *flags) {
+  pdl_wait();
   fe acc = fe_zero();
   for (int it = 0; it < a.iters; it++) {
     const fe om = root_of_unity(ilog2_dev(a.NL[it]));
@@ -447,6 +469,7 @@ __global__ void k_whir_step3(const uint8_t *tr, Step3Args a, const fe *claims, c
 }
 
 __global__ void k_put_claim_value(const fe *v, const fe *r, int nr, uint8_t *tr, uint64_t off) {
+  pdl_wait();
   const int k = threadIdx.x;
   if (k == 0) put_fe(tr, off, *v);
   else if (k <= nr) put_fe(tr, off + 16ull * k, r[k - 1]);
@@ -473,6 +496,7 @@ struct FinalArgs {
 // inverse transform of length N/2 of the powers of omega_{2N}^(2p+1),
 // evaluated as a polynomial in r_c.
 __global__ void k_powers_y(int N, const fe *rcp, fe *py) {
+  pdl_wait();
   const int p = threadIdx.x;
   if (p >= N) return;
   const fe rc = *rcp;
@@ -501,6 +525,7 @@ __global__ void k_powers_y(int N, const fe *rcp, fe *py) {
 // times fast_eval_powers_y of its party.  One warp per query, its lanes over
 // the Lagrange weights; terms[g] for the g-th query over all rounds.
 __global__ void k_final_terms(FinalArgs a, const fe *py, fe *terms) {
+  pdl_wait();
   const int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   int r = 0, t = g;
   while (r < a.nq && t >= a.q[r].l) t -= a.q[r++].l;
@@ -531,6 +556,7 @@ __global__ void k_final_terms(FinalArgs a, const fe *py, fe *terms) {
 // r_first b2[0] b3(r_c) + sum of the terms = B_eval_claim ("final
 // verification step", coPCS.cpp:1711-1752).
 __global__ void k_final_eval(FinalArgs a, const fe *terms, int nterms, uint32_t *flags, uint8_t *tr) {
+  pdl_wait();
   fe acc = fe_zero();
   for (int g = threadIdx.x; g < nterms; g += kT) acc = fadd(acc, terms[g]);
   acc = block_sum_fe(acc);
@@ -563,6 +589,7 @@ struct TensorArgs {
   int logd[8];
 };
 __global__ void k_tensor(TensorArgs a, uint64_t total, fe *out) {
+  pdl_wait();
   const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= total) return;
   uint64_t x = g;
@@ -575,6 +602,7 @@ __global__ void k_tensor(TensorArgs a, uint64_t total, fe *out) {
 }
 
 __global__ void k_mul(const fe *a, const fe *b, uint64_t n, fe *out) {
+  pdl_wait();
   const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g < n) out[g] = fmul(a[g], b[g]);
 }
@@ -585,6 +613,7 @@ __global__ void k_mul(const fe *a, const fe *b, uint64_t n, fe *out) {
 // evaluations go to the transcript.  scratch: 3/4 of the longest factor.
 __global__ void k_beta_evals(TensorArgs a, const fe *r, const fe *fin, uint32_t bit, fe *scratch, uint32_t *flags,
                              uint8_t *tr, uint64_t off) {
+  pdl_wait();
   __shared__ fe ev[8];
   int base = 0;
   for (int k = 0; k < a.n; k++) {
@@ -618,6 +647,7 @@ __global__ void k_beta_evals(TensorArgs a, const fe *r, const fe *fin, uint32_t 
 // the point, prod_i (1 - r_i + r_i omega^(2^i)), against the sumcheck's
 // value of the omega vector.
 __global__ void k_lag_omega(const fe *r, int n, fe omega, const fe *fin, uint32_t *flags) {
+  pdl_wait();
   if (threadIdx.x) return;
   fe p = fe_one();
   for (int i = 0; i < n; i++) {
@@ -631,6 +661,7 @@ __global__ void k_lag_omega(const fe *r, int n, fe omega, const fe *fin, uint32_
 // vector's value plus the equality weights of its q zeroed entries
 // Bs - q .. Bs - 1 at the point is one.
 __global__ void k_lag_ones(const fe *fin, const fe *r, int n, uint64_t Bs, uint64_t q, uint32_t *flags) {
+  pdl_wait();
   __shared__ fe part[kT];
   fe acc = fe_zero();
   for (uint64_t i = Bs - q + threadIdx.x; i < Bs; i += blockDim.x) {
@@ -648,15 +679,18 @@ __global__ void k_lag_ones(const fe *fin, const fe *r, int n, uint64_t Bs, uint6
 
 // v[i] = 1 for i < m, 0 for m <= i < n.
 __global__ void k_fill_prefix(fe *v, uint64_t n, uint64_t m) {
+  pdl_wait();
   const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g < n) v[g] = g < m ? fe_one() : fe_zero();
 }
 
 __global__ void k_put1(const fe *v, uint8_t *tr, uint64_t off) {
+  pdl_wait();
   if (threadIdx.x == 0) put_fe(tr, off, *v);
 }
 
 __global__ void k_whir_flags(const ProofState *st, uint32_t *flags) {
+  pdl_wait();
   if (threadIdx.x == 0 && st->error) atomicOr(flags, LF_WHIR);
 }
 
@@ -788,7 +822,7 @@ struct Tail {
       GBZ_CUDA(cudaMemcpyAsync(out.A, rd.seg, 16ull * l * d, cudaMemcpyDeviceToDevice, s));
       fe *tmp = alloc<fe>(Lw);
       ntt_launch(R.tables(ilog2(Lw)), out.A, (uint64_t)l * d, out.W, tmp, false, s);
-      k_merkle_root<<<1, 32, 0, s>>>(out.W, ilog2(Lw / 4), tr, off_root);
+      launch_kernel(k_merkle_root, 1, 32, 0, s, out.W, ilog2(Lw / 4), tr, off_root);
       check();
     }
     // queries2[i] = rand() % C[0].size() (coPCS.cpp:789)
@@ -805,10 +839,11 @@ struct Tail {
     if (!dry) {
       beta_launch(D, logS, b1, s);
       powers_launch(finv(root_of_unity(logd)), (uint64_t)d, twd, s);
-      k_pmf_vectors<<<(unsigned)S, 256, 32ull * d, s>>>(rd.seg, rd.qpos, l, d, logd, twd, wn_inv, rd.L, b1, V[0],
+      launch_kernel(k_pmf_vectors, (unsigned)S, 256, 32ull * d, s, rd.seg, rd.qpos, l, d, logd, twd, wn_inv, rd.L, b1,
+                    V[0],
                                                          V[1], V[2], V[3]);
       // K = d sum_t b1[t] y[t] (pad_vector(y): zeros beyond l)
-      k_dot<<<1, kT, 0, s>>>(b1, rd.y, (uint64_t)l, fe_make((uint64_t)d, 0), y);
+      launch_kernel(k_dot, 1, kT, 0, s, b1, rd.y, (uint64_t)l, fe_make((uint64_t)d, 0), y);
       check();
     }
     fe *ch4 = alloc<fe>(R4), *fin4 = alloc<fe>(4);
@@ -820,15 +855,15 @@ struct Tail {
     if (!dry) {
       beta_launch(ch4 + logd, logS, b12, s);
       beta_launch(ch4, logd, b11, s);
-      k_pmf_checks<<<1, kT, 0, s>>>(fin4, ch4, logd, logS, D, b12, b11, rd.L, rd.qpos, l, d, wn_inv, flags);
+      launch_kernel(k_pmf_checks, 1, kT, 0, s, fin4, ch4, logd, logS, D, b12, b11, rd.L, rd.qpos, l, d, wn_inv, flags);
       check();
     }
     // the second sumcheck: sum_t b12[t] segment_t against the reduced matrix at r11
     fe *U1 = alloc<fe>(d), *U2 = alloc<fe>(d), *chq = alloc<fe>(logd), *finq = alloc<fe>(2);
     if (!dry) {
-      k_seg_comb<<<d, kT, 0, s>>>(rd.seg, b12, l, d, U1);
-      k_reduced_matrix<<<nblk(d), kT, 0, s>>>(ch4, logd, d, twd, U2);
-      k_set<<<1, 32, 0, s>>>(y, fin4);
+      launch_kernel(k_seg_comb, d, kT, 0, s, rd.seg, b12, l, d, U1);
+      launch_kernel(k_reduced_matrix, nblk(d), kT, 0, s, ch4, logd, d, twd, U2);
+      launch_kernel(k_set, 1, 32, 0, s, y, fin4);
       check();
     }
     {
@@ -838,15 +873,15 @@ struct Tail {
     // evaluate_vector scratch: halves of up to 2^13 entries
     fe *ev = alloc<fe>(1), *es = alloc<fe>(8192);
     if (!dry) {
-      k_eval<<<1, kT, 0, s>>>(U2, logd, chq, es, es + 4096, ev);
-      k_check_eq<<<1, 32, 0, s>>>(ev, finq + 1, flags, LF_DELEGATION);
+      launch_kernel(k_eval, 1, kT, 0, s, U2, logd, chq, es, es + 4096, ev);
+      launch_kernel(k_check_eq, 1, 32, 0, s, ev, finq + 1, flags, LF_DELEGATION);
       check();
     }
     // the claim (finq[0], r_q ++ r12) padded with zeros to log2 max_delegation
     const uint64_t off_claim = lay.rec(T_D_CLAIM, (uint32_t)(1 + logmd), 16);
     out.claim = alloc<fe>(1 + logmd);
     if (!dry) {
-      k_claim<<<1, 64, 0, s>>>(finq, chq, logd, ch4 + logd, logS, logmd, out.claim, tr, off_claim);
+      launch_kernel(k_claim, 1, 64, 0, s, finq, chq, logd, ch4 + logd, logS, logmd, out.claim, tr, off_claim);
       check();
     }
     // ---- extended segments and prove_extension
@@ -858,8 +893,8 @@ struct Tail {
     if (!dry) {
       ntt_batched(R.tables(logC0), rd.seg, (uint64_t)d, (uint32_t)d, E, (uint64_t)l, false, s);
       beta_launch(De, logS, bb, s);
-      k_pe_vectors<<<nblk(S * C0), kT, 0, s>>>(E, q2, l, C0, bb, o, W2, W3, S * C0, tr, off_o);
-      k_dot<<<1, kT, 0, s>>>(o, bb, (uint64_t)l, fe_one(), y);
+      launch_kernel(k_pe_vectors, nblk(S * C0), kT, 0, s, E, q2, l, C0, bb, o, W2, W3, S * C0, tr, off_o);
+      launch_kernel(k_dot, 1, kT, 0, s, o, bb, (uint64_t)l, fe_one(), y);
       check();
     }
     fe *ch3 = alloc<fe>(R3), *fin3 = alloc<fe>(3);
@@ -872,12 +907,12 @@ struct Tail {
     if (!dry) {
       beta_launch(ch3, logC0, b1e, s);
       beta_launch(ch3 + logC0, logS, b2e, s);
-      k_pe_checks<<<1, kT, 0, s>>>(fin3, b1e, b2e, q2, l, ch3 + logC0, De, logS, flags);
+      launch_kernel(k_pe_checks, 1, kT, 0, s, fin3, b1e, b2e, q2, l, ch3 + logC0, De, logS, flags);
       // prove_fft (delegate_protocol.cpp:119-145) of sum_t b2[t] segment_t at r1
-      k_seg_comb<<<d, kT, 0, s>>>(rd.seg, b2e, l, d, v);
+      launch_kernel(k_seg_comb, d, kT, 0, s, rd.seg, b2e, l, d, v);
       const NttTables &tc = R.tables(logC0);
-      k_phi<<<nblk(C0), kT, 0, s>>>(ch3, logC0, logC0, tc.lo_fwd, tc.hi_fwd, fe_one(), Wp);
-      k_set<<<1, 32, 0, s>>>(y, fin3);
+      launch_kernel(k_phi, nblk(C0), kT, 0, s, ch3, logC0, logC0, tc.lo_fwd, tc.hi_fwd, fe_one(), Wp);
+      launch_kernel(k_set, 1, 32, 0, s, y, fin3);
       check();
     }
     {
@@ -886,9 +921,9 @@ struct Tail {
     }
     const uint64_t off_ext = lay.rec(T_D_EXT_CLAIM, (uint32_t)(1 + logd + logS), 16);
     if (!dry) {
-      k_eval<<<1, kT, 0, s>>>(Wp, logC0, chp, es, es + 4096, ev);
-      k_check_eq<<<1, 32, 0, s>>>(ev, finp, flags, LF_DELEGATION);
-      k_ext_claim<<<1, 32, 0, s>>>(finp, chp, logC0, lograte, ch3 + logC0, logS, tr, off_ext);
+      launch_kernel(k_eval, 1, kT, 0, s, Wp, logC0, chp, es, es + 4096, ev);
+      launch_kernel(k_check_eq, 1, 32, 0, s, ev, finp, flags, LF_DELEGATION);
+      launch_kernel(k_ext_claim, 1, 32, 0, s, finp, chp, logC0, lograte, ch3 + logC0, logS, tr, off_ext);
       check();
     }
     return out;
@@ -951,15 +986,15 @@ struct Tail {
     }
     fe *L2v = alloc<fe>(Bs), *L1v = alloc<fe>(Bs), *L1f = alloc<fe>(Bs), *ones = alloc<fe>(Bs), *y = alloc<fe>(1);
     if (!dry) {
-      k_tensor<<<nblk(Bs), kT, 0, s>>>(ta, Bs, L2v);
-      k_tensor<<<nblk(Bs), kT, 0, s>>>(t1, Bs, L1v);
+      launch_kernel(k_tensor, nblk(Bs), kT, 0, s, ta, Bs, L2v);
+      launch_kernel(k_tensor, nblk(Bs), kT, 0, s, t1, Bs, L1v);
       GBZ_CUDA(cudaMemcpyAsync(L1f, L1v, 16 * Bs, cudaMemcpyDeviceToDevice, s));
       if (q) GBZ_CUDA(cudaMemsetAsync(L1f + (Bs - q), 0, 16 * q, s));
       fe *tmp = alloc<fe>(Bs);
       ntt_launch(R.tables(logBs), L1f, Bs, L1f, tmp, false, s);
-      k_fill_prefix<<<nblk(Bs), kT, 0, s>>>(ones, Bs, Bs - q);
-      k_set<<<1, 32, 0, s>>>(y, b2f);
-      k_put1<<<1, 32, 0, s>>>(b2f, tr, off_y);
+      launch_kernel(k_fill_prefix, nblk(Bs), kT, 0, s, ones, Bs, Bs - q);
+      launch_kernel(k_set, 1, 32, 0, s, y, b2f);
+      launch_kernel(k_put1, 1, 32, 0, s, b2f, tr, off_y);
       check();
     }
     fe *ch = alloc<fe>(logBs), *fin = alloc<fe>(3);
@@ -973,11 +1008,11 @@ struct Tail {
       int dmax = 0;
       for (int i = 0; i < nr; i++) dmax = std::max(dmax, in.rounds[i].d);
       fe *es = alloc<fe>((uint64_t)std::max(dmax, 1 << lmax));
-      k_beta_evals<<<1, kT, 0, s>>>(ta, ch, fin, LF_BETAS, es, flags, tr, off_le);
-      k_lag_omega<<<1, 32, 0, s>>>(ch, logBs, root_of_unity(1 + in.log_rate_offset + logBs), fin, flags);
+      launch_kernel(k_beta_evals, 1, kT, 0, s, ta, ch, fin, LF_BETAS, es, flags, tr, off_le);
+      launch_kernel(k_lag_omega, 1, 32, 0, s, ch, logBs, root_of_unity(1 + in.log_rate_offset + logBs), fin, flags);
       const NttTables &tb = R.tables(logBs);
-      k_phi<<<nblk(Bs), kT, 0, s>>>(ch, logBs, logBs, tb.lo_fwd, tb.hi_fwd, finv(fe_make(Bs, 0)), W);
-      k_set<<<1, 32, 0, s>>>(y, fin + 1);
+      launch_kernel(k_phi, nblk(Bs), kT, 0, s, ch, logBs, logBs, tb.lo_fwd, tb.hi_fwd, finv(fe_make(Bs, 0)), W);
+      launch_kernel(k_set, 1, 32, 0, s, y, fin + 1);
       check();
     }
     {
@@ -987,8 +1022,8 @@ struct Tail {
     const uint64_t off_l1 = lay.rec(T_L_LAG_EVALS, (uint32_t)in.nlag, 16);
     if (!dry) {
       fe *es = alloc<fe>(1ull << lmax);
-      k_beta_evals<<<1, kT, 0, s>>>(t1, ch2, fin2 + 1, LF_LAG2, es, flags, tr, off_l1);
-      k_lag_ones<<<1, kT, 0, s>>>(fin2, ch2, logBs, Bs, q, flags);
+      launch_kernel(k_beta_evals, 1, kT, 0, s, t1, ch2, fin2 + 1, LF_LAG2, es, flags, tr, off_l1);
+      launch_kernel(k_lag_ones, 1, kT, 0, s, fin2, ch2, logBs, Bs, q, flags);
       check();
     }
   }
@@ -1014,8 +1049,8 @@ struct Tail {
       } else {
         GBZ_CUDA(cudaMemcpyAsync(dec, in.Cp, 16ull * N * cpl, cudaMemcpyDeviceToDevice, s));
       }
-      k_decode_check<<<nblk((uint64_t)N * in.n_final), kT, 0, s>>>(dec, cpl, in.bcd, in.n_final, N, flags);
-      k_unpack_final<<<1, 32, 0, s>>>(in.unpack, in.bcd, in.B, N, in.K, fp, fB, flags, tr, off_unp);
+      launch_kernel(k_decode_check, nblk((uint64_t)N * in.n_final), kT, 0, s, dec, cpl, in.bcd, in.n_final, N, flags);
+      launch_kernel(k_unpack_final, 1, 32, 0, s, in.unpack, in.bcd, in.B, N, in.K, fp, fB, flags, tr, off_unp);
       check();
     }
     if (in.piop) {
@@ -1038,7 +1073,7 @@ struct Tail {
       }
       const fe *ch = draws(2 * nR);
       if (!dry) {
-        k_aggr_K<<<1, 32, 0, s>>>(sums, ch, nR, st, tr, off_ch, off_K);
+        launch_kernel(k_aggr_K, 1, 32, 0, s, sums, ch, nR, st, tr, off_ch, off_K);
         check();
         VecList va{}, vb{}, vc{};
         for (int i = 0; i < nR; i++) {
@@ -1058,9 +1093,10 @@ struct Tail {
       const uint64_t off_ar = lay.rec(T_AGGR_ROOT, 1, 32);
       draw_mod(la, (uint32_t)(Lw / 4), off_aq);
       if (!dry) {
-        k_whir_paths_chain<<<nblk((uint64_t)la * depth_a, 128), 128, 0, s>>>(ro[0].W, Lw / 4, la, tr, off_aq, off_ap,
+        launch_kernel(k_whir_paths_chain, nblk((uint64_t)la * depth_a, 128), 128, 0, s, ro[0].W, Lw / 4, la, tr,
+                      off_aq, off_ap,
                                                                              0, 0);
-        k_zero_tree_root<<<1, 32, 0, s>>>(ilog2(Lw / 8), tr, off_ar);
+        launch_kernel(k_zero_tree_root, 1, 32, 0, s, ilog2(Lw / 8), tr, off_ar);
         check();
       }
       // _Whir_Open (Whir.cpp:469-545) with whir_k = 8 from the zero-leaf tree
@@ -1095,7 +1131,7 @@ struct Tail {
         calls += 40ull * ilog2(P.m_final);
         if (script) script->push_back({DRAW_SKIP, (int)calls, 0u, 0});
         if (!dry) {
-          k_prng_check<<<1, 32, 0, s>>>(st, after_walk, flags);
+          launch_kernel(k_prng_check, 1, 32, 0, s, st, after_walk, flags);
           check();
         }
       }
@@ -1105,21 +1141,22 @@ struct Tail {
       const uint64_t off_wc = lay.rec(T_L_WHIR_CLAIM, (uint32_t)(1 + logmd), 16);
       if (!dry) {
         const NttTables &tf = R.tables(ilog2(wt.L_final));
-        k_reencode_check<<<nblk(wt.L_final), kT, 0, s>>>(wt.final_arr, (int)wt.m_final, wt.last_codeword, wt.L_final,
+        launch_kernel(k_reencode_check, nblk(wt.L_final), kT, 0, s, wt.final_arr, (int)wt.m_final, wt.last_codeword,
+                      wt.L_final,
                                                         tf.lo_fwd, tf.hi_fwd, st);
-        k_whir_flags<<<1, 32, 0, s>>>(st, flags);
+        launch_kernel(k_whir_flags, 1, 32, 0, s, st, flags);
         // the final claim (evaluate_vector(_initial_b, total_r), total_r)
         ChalOffs co{};
         co.n = (int)wt.chal.size();
         for (int i = 0; i < co.n; i++) co.off[i] = wt.chal[i];
         fe *total_r = alloc<fe>(logmd), *eb = alloc<fe>(md), *val = alloc<fe>(1), *mdp = alloc<fe>(multidot_scratch(md));
-        k_gather_r<<<1, 64, 0, s>>>(tr, co, wt.final_point, ilog2(wt.m_final), total_r);
+        launch_kernel(k_gather_r, 1, 64, 0, s, tr, co, wt.final_point, ilog2(wt.m_final), total_r);
         beta_launch(total_r, logmd, eb, s);
         VecList a1{}, a2{};
         a1.p[0] = eb;
         a2.p[0] = baggr;
         multidot_launch(a1, 1, a2, 1, md, mdp, val, s);
-        k_put_claim_value<<<1, 64, 0, s>>>(val, total_r, logmd, tr, off_wc);
+        launch_kernel(k_put_claim_value, 1, 64, 0, s, val, total_r, logmd, tr, off_wc);
         check();
         // verification step 3
         Step3Args a3{};
@@ -1142,7 +1179,7 @@ struct Tail {
         for (int c = 0; c < nR; c++)
           GBZ_CUDA(cudaMemcpyAsync(claims + (uint64_t)c * (1 + logmd), ro[c].claim, 16ull * (1 + logmd),
                                    cudaMemcpyDeviceToDevice, s));
-        k_whir_step3<<<1, kT, 0, s>>>(tr, a3, claims, ch, total_r, flags);
+        launch_kernel(k_whir_step3, 1, kT, 0, s, tr, a3, claims, ch, total_r, flags);
         check();
       }
     }
@@ -1154,7 +1191,7 @@ struct Tail {
     fe *om = alloc<fe>(in.Bs), *b2c = alloc<fe>(in.Bs), *b2t = alloc<fe>(in.Bs), *b2f = nullptr;
     if (!dry) {
       powers_launch(om_off, in.Bs, om, s);
-      k_mul<<<nblk(in.Bs), kT, 0, s>>>(in.b2, om, in.Bs, b2c);
+      launch_kernel(k_mul, nblk(in.Bs), kT, 0, s, in.b2, om, in.Bs, b2c);
       check();
       fe *cur = b2c, *nxt = b2t;
       uint64_t len = in.Bs;
@@ -1197,9 +1234,9 @@ struct Tail {
       int nterms = 0;
       for (int j = 0; j < fa.nq; j++) nterms += fa.q[j].l;
       fe *py = alloc<fe>(64), *terms = alloc<fe>(std::max(nterms, 1));
-      k_powers_y<<<1, 64, 0, s>>>(N, rc, py);
-      if (nterms) k_final_terms<<<nblk((uint64_t)nterms * 32), kT, 0, s>>>(fa, py, terms);
-      k_final_eval<<<1, kT, 0, s>>>(fa, terms, nterms, flags, tr);
+      launch_kernel(k_powers_y, 1, 64, 0, s, N, rc, py);
+      if (nterms) launch_kernel(k_final_terms, nblk((uint64_t)nterms * 32), kT, 0, s, fa, py, terms);
+      launch_kernel(k_final_eval, 1, kT, 0, s, fa, terms, nterms, flags, tr);
       check();
     }
     if (in.piop) {
@@ -1218,9 +1255,9 @@ struct Tail {
     }
     fe *Lv = alloc<fe>(in.Bs), *y = alloc<fe>(1);
     if (!dry) {
-      k_tensor<<<nblk(in.Bs), kT, 0, s>>>(ta, in.Bs, Lv);
-      k_set<<<1, 32, 0, s>>>(y, b2f);
-      k_put1<<<1, 32, 0, s>>>(b2f, tr, off_by);
+      launch_kernel(k_tensor, nblk(in.Bs), kT, 0, s, ta, in.Bs, Lv);
+      launch_kernel(k_set, 1, 32, 0, s, y, b2f);
+      launch_kernel(k_put1, 1, 32, 0, s, b2f, tr, off_by);
       check();
     }
     fe *chb = alloc<fe>(logBs), *finb = alloc<fe>(3);
@@ -1232,13 +1269,13 @@ struct Tail {
     fe *Wr = alloc<fe>(2 * in.Bs), *bx = zeros(2 * in.Bs), *chw = alloc<fe>(logBs + 1), *finw = alloc<fe>(2);
     if (!dry) {
       fe *es = alloc<fe>(1024);
-      k_beta_evals<<<1, kT, 0, s>>>(ta, chb, finb, LF_BETAS, es, flags, tr, off_le);
+      launch_kernel(k_beta_evals, 1, kT, 0, s, ta, chb, finb, LF_BETAS, es, flags, tr, off_le);
       const NttTables &t2 = R.tables(logBs + 1);
-      k_phi<<<nblk(2 * in.Bs), kT, 0, s>>>(chb, logBs, logBs + 1, t2.lo_fwd, t2.hi_fwd, fe_one(), Wr);
+      launch_kernel(k_phi, nblk(2 * in.Bs), kT, 0, s, chb, logBs, logBs + 1, t2.lo_fwd, t2.hi_fwd, fe_one(), Wr);
       // b = precompute_beta(r2), zero beyond its length (the reference reads
       // past the end of b there: the value is never used)
       beta_launch(in.r2, logBs, bx, s);
-      k_set<<<1, 32, 0, s>>>(y, finb + 1);
+      launch_kernel(k_set, 1, 32, 0, s, y, finb + 1);
       check();
     }
     {
@@ -1259,13 +1296,13 @@ void leader_tail(LeaderResources &R, const LeaderInputs &in, ProofState *st, uin
 }
 
 void leader_tail_init(ProofState *st, const glibc_prng &g, uint32_t *flags, cudaStream_t s) {
-  k_tail_init<<<1, 32, 0, s>>>(st, g, flags);
+  launch_kernel(k_tail_init, 1, 32, 0, s, st, g, flags);
   GBZ_CUDA(cudaGetLastError());
 }
 
 void leader_draws_launch(const glibc_prng &g0, const DrawOp *ops, int nops, const LeaderDraws &d, uint8_t *tr,
                          ProofState *st, cudaStream_t s) {
-  k_draw_script<<<1, 32, 0, s>>>(g0, ops, nops, d.arena, tr, st, d.after_walk, d.final_state);
+  launch_kernel(k_draw_script, 1, 32, 0, s, g0, ops, nops, d.arena, tr, st, d.after_walk, d.final_state);
   GBZ_CUDA(cudaGetLastError());
 }
 

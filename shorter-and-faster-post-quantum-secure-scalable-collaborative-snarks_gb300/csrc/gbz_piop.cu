@@ -122,12 +122,14 @@ struct Segs {
   uint32_t off[kPiopMaxRounds + 1];
 };
 
-__global__ void k_one(fe *out) { out[0] = fe_one(); }
+__global__ void k_one(fe *out) {
+  pdl_wait(); out[0] = fe_one(); }
 
 // out[j + k na] = b[k] a[j] (the products of _reduce_R1CS_matrixes_multivariate
 // and compute_beta_shares_multivariate, Distributed_Sumcheck.cpp:2304-2313,
 // coPIOP.cpp:352-363).
 __global__ void k_tensor(const fe *a, uint64_t na, const fe *b, uint64_t nb, fe *out) {
+  pdl_wait();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= na * nb) return;
   out[i] = fmul(b[i / na], a[i % na]);
@@ -141,6 +143,7 @@ __global__ void k_tensor(const fe *a, uint64_t na, const fe *b, uint64_t nb, fe 
 // One CTA, a thread per party.
 __global__ void k_piop_y(const fe *masks, const fe *R1, uint64_t rlen, Segs sg, int N, fe b0, fe b1, fe b2, fe b3,
                          const fe *lambda, fe rlast, fe *out, uint8_t *tr, uint64_t off_y) {
+  pdl_wait();
   __shared__ fe ys[kPiopMaxParties], ks[kPiopMaxParties];
   const int p = threadIdx.x;
   if (p < N) {
@@ -175,6 +178,7 @@ __global__ void k_piop_y(const fe *masks, const fe *R1, uint64_t rlen, Segs sg, 
 // vO of every party doubled in length, the party's four masks rL, rR, rO at
 // the start of the new half, zeros after (coPIOP.cpp:289-298).
 __global__ void k_piop_extend(const fe *vL, const fe *vR, const fe *vO, const fe *masks, uint64_t n, int N, fe *out) {
+  pdl_wait();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 2 * n) return;
   const int p = blockIdx.y, v = blockIdx.z;
@@ -198,6 +202,7 @@ struct R1csView {
 };
 __global__ void k_r1cs_rows(R1csView m, uint64_t nrows, const fe *beta1, const fe *beta2, int logS, fe scale,
                             fe *out) {
+  pdl_wait();
   const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= nrows) return;
   const uint32_t S1 = (1u << logS) - 1;
@@ -222,6 +227,7 @@ __global__ void k_r1cs_rows(R1csView m, uint64_t nrows, const fe *beta1, const f
 // to segment s div fill at offset s mod fill (fill = seg - mask_l).
 __global__ void k_reshare_segments(const fe *v, uint64_t rows, int N, const fe *mu, uint64_t seg, uint64_t fill,
                                    fe *out, uint64_t pstride) {
+  pdl_wait();
   const int k = N / 4, kk = N / 2;
   const uint64_t per = rows / k, len = per * N;
   const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -236,6 +242,7 @@ __global__ void k_reshare_segments(const fe *v, uint64_t rows, int N, const fe *
 
 // out[p ostride + off + j] = v[j] scal[p] for j < n.
 __global__ void k_scale_parties(const fe *v, uint64_t n, const fe *scal, fe *out, uint64_t ostride, uint64_t off) {
+  pdl_wait();
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const int p = blockIdx.y;
@@ -246,6 +253,7 @@ __global__ void k_scale_parties(const fe *v, uint64_t n, const fe *scal, fe *out
 // party's witness w, then rL resized to |w| with its first four entries
 // a rL + b rR + c rO.
 __global__ void k_piop_p1(const fe *w, uint64_t nw, const fe *masks, fe a, fe b, fe c, fe *out) {
+  pdl_wait();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 2 * nw) return;
   const int p = blockIdx.y;
@@ -264,7 +272,7 @@ __global__ void k_piop_p1(const fe *w, uint64_t nw, const fe *masks, fe a, fe b,
 // powers of r, inverse transform.
 void lagrange_dev(gbz_ctx *ctx, fe r, int logd, fe *out, cudaStream_t s) {
   if (logd == 0) {
-    k_one<<<1, 1, 0, s>>>(out);
+    launch_kernel(k_one, 1, 1, 0, s, out);
     GBZ_CUDA(cudaGetLastError());
     return;
   }
@@ -280,13 +288,13 @@ uint64_t lagrange_tensor(gbz_ctx *ctx, const std::vector<int> &degs, const std::
                          fe *t1, cudaStream_t s) {
   uint64_t len = 1;
   fe *cur = t0;
-  k_one<<<1, 1, 0, s>>>(cur);
+  launch_kernel(k_one, 1, 1, 0, s, cur);
   for (size_t i = 0; i < degs.size(); i++) {
     const int lg = ilog2((uint64_t)degs[i]);
     fe *L = out;  // staged through out, then folded into the other buffer
     lagrange_dev(ctx, pts[i], lg, L, s);
     fe *nxt = cur == t0 ? t1 : t0;
-    k_tensor<<<nblk(len * degs[i]), 256, 0, s>>>(cur, len, L, (uint64_t)degs[i], nxt);
+    launch_kernel(k_tensor, nblk(len * degs[i]), 256, 0, s, cur, len, L, (uint64_t)degs[i], nxt);
     GBZ_CUDA(cudaGetLastError());
     cur = nxt;
     len *= (uint64_t)degs[i];
@@ -391,7 +399,7 @@ int reduce_tables(gbz_ctx *ctx, OpenBufs &ob, int N, int logm, const std::vector
   std::vector<int> d1(d.begin(), d.end() - 1);
   std::vector<fe> r1(r.begin(), r.end() - 1);
   if (d1.empty()) {
-    k_one<<<1, 1, 0, s>>>(beta1);
+    launch_kernel(k_one, 1, 1, 0, s, beta1);
   } else {
     lagrange_tensor(ctx, d1, r1, beta1, t0, t1, s);
   }
@@ -487,7 +495,7 @@ gbz_status gbz_r1cs_reduce(gbz_ctx *ctx, const gbz_r1cs *m, const uint64_t *r, i
     v.cols[0] = m->cols[t];
     v.w[0] = fe_one();
     fe *o = mem == GBZ_MEM_DEVICE ? (fe *)outs[t] : ob.alloc<fe>(total);
-    k_r1cs_rows<<<nblk(total), 256, 0, s>>>(v, total, beta1, beta2, logS, fe_one(), o);
+    launch_kernel(k_r1cs_rows, nblk(total), 256, 0, s, v, total, beta1, beta2, logS, fe_one(), o);
     GBZ_CUDA(cudaGetLastError());
     if (mem == GBZ_MEM_HOST) GBZ_CUDA(cudaMemcpyAsync(outs[t], o, 16 * total, cudaMemcpyDeviceToHost, s));
   }
@@ -577,14 +585,15 @@ gbz_status gbz_piop_phase1(gbz_ctx *ctx, int N, uint64_t n, const uint64_t *vL, 
   const fe *dR1 = in_view(ctx, ob, (const fe *)R1, (uint64_t)N * rlen, mem);
   fe *dl = ob.alloc<fe>(N), *dy = ob.alloc<fe>(3);
   GBZ_CUDA(cudaMemcpyAsync(dl, lambda.data(), 16ull * N, cudaMemcpyHostToDevice, s));
-  k_piop_y<<<1, kPiopMaxParties, 0, s>>>(dm, dR1, rlen, sg, N, bt[0], bt[1], bt[2], bt[3], dl, r1.back(), dy, tr,
+  launch_kernel(k_piop_y, 1, kPiopMaxParties, 0, s, dm, dR1, rlen, sg, N, bt[0], bt[1], bt[2], bt[3], dl, r1.back(),
+                dy, tr,
                                          off_y);
   GBZ_CUDA(cudaGetLastError());
   fe hy[3];
   GBZ_CUDA(cudaMemcpyAsync(hy, dy, sizeof hy, cudaMemcpyDeviceToHost, s));
   // the masked, doubled vectors
   fe *P = ob.alloc<fe>(3ull * N * 2 * n);
-  k_piop_extend<<<dim3(nblk(2 * n), N, 3), 256, 0, s>>>(dvL, dvR, dvO, dm, n, N, P);
+  launch_kernel(k_piop_extend, dim3(nblk(2 * n), N, 3), 256, 0, s, dvL, dvR, dvO, dm, n, N, P);
   GBZ_CUDA(cudaGetLastError());
   GBZ_CUDA(cudaStreamSynchronize(s));
   // cubic_coSumcheck(vL, vR, vO, r1, r2, R1, y, K_r, degrees) (coPIOP.cpp:311-312)
@@ -599,7 +608,7 @@ gbz_status gbz_piop_phase1(gbz_ctx *ctx, int N, uint64_t n, const uint64_t *vL, 
   const std::vector<fe> sc = share_scalars(b1, N);
   fe *dsc = ob.alloc<fe>(N), *dip = ob.alloc<fe>((uint64_t)N * rlen);
   GBZ_CUDA(cudaMemcpyAsync(dsc, sc.data(), 16ull * N, cudaMemcpyHostToDevice, s));
-  k_scale_parties<<<dim3(nblk(rlen), N), 256, 0, s>>>(ipb, rlen, dsc, dip, rlen, 0);
+  launch_kernel(k_scale_parties, dim3(nblk(rlen), N), 256, 0, s, ipb, rlen, dsc, dip, rlen, 0);
   GBZ_CUDA(cudaGetLastError());
   put_out(ctx, claims, res.claims.data(), 16 * res.claims.size(), mem, false);
   put_out(ctx, fs, &res.fs, 16, mem, false);
@@ -691,18 +700,19 @@ gbz_status gbz_piop_phase2(gbz_ctx *ctx, int N, uint64_t nw, const uint64_t *w, 
   v.w[0] = a;
   v.w[1] = b;
   v.w[2] = c;
-  k_r1cs_rows<<<nblk(total), 256, 0, s>>>(v, total, beta1, beta2, logS, Ll[0], aggr);
+  launch_kernel(k_r1cs_rows, nblk(total), 256, 0, s, v, total, beta1, beta2, logS, Ll[0], aggr);
   GBZ_CUDA(cudaGetLastError());
   // the second coSumcheck's vectors: P1 = (w, rL'), P2 = (segments of the
   // reshared R_aggr, beta shares L_last[1], zeros)
   fe *P = ob.alloc<fe>(2ull * N * 2 * nw);
   fe *P1 = P, *P2 = P + (uint64_t)N * 2 * nw;
-  k_piop_p1<<<dim3(nblk(2 * nw), N), 256, 0, s>>>(dw, nw, dm, a, b, c, P1);
+  launch_kernel(k_piop_p1, dim3(nblk(2 * nw), N), 256, 0, s, dw, nw, dm, a, b, c, P1);
   GBZ_CUDA(cudaMemsetAsync(P2, 0, 16ull * N * 2 * nw, s));
   const std::vector<fe> mu = shamir_share_matrix(N);
   fe *dmu = ob.alloc<fe>(mu.size());
   GBZ_CUDA(cudaMemcpyAsync(dmu, mu.data(), 16 * mu.size(), cudaMemcpyHostToDevice, s));
-  k_reshare_segments<<<dim3(nblk(len), N), 256, 0, s>>>(aggr, m->rows, N, dmu, seg, seg - mask_l, P2, 2 * nw);
+  launch_kernel(k_reshare_segments, dim3(nblk(len), N), 256, 0, s, aggr, m->rows, N, dmu, seg, seg - mask_l, P2,
+                2 * nw);
   GBZ_CUDA(cudaGetLastError());
   // compute_beta_shares_multivariate (coPIOP.cpp:348-379) times L_last[1]
   std::vector<int> bd(degrees1, degrees1 + ndeg1 - 1);
@@ -713,7 +723,7 @@ gbz_status gbz_piop_phase2(gbz_ctx *ctx, int N, uint64_t nw, const uint64_t *w, 
   for (auto &x : bs) x = fmul(x, Ll[1]);
   fe *dbs = ob.alloc<fe>(N);
   GBZ_CUDA(cudaMemcpyAsync(dbs, bs.data(), 16ull * N, cudaMemcpyHostToDevice, s));
-  k_scale_parties<<<dim3(nblk(nvl), N), 256, 0, s>>>(bsh, nvl, dbs, P2, 2 * nw, 2 * len);
+  launch_kernel(k_scale_parties, dim3(nblk(nvl), N), 256, 0, s, bsh, nvl, dbs, P2, 2 * nw, 2 * len);
   GBZ_CUDA(cudaGetLastError());
   // quadratic_coSumcheck(w, R_aggr, R2, a yL + b yR + c yO, K_r, degrees2) (coPIOP.cpp:495-496)
   const fe K2 = fadd(fadd(fmul(a, y[0]), fmul(b, y[1])), fmul(c, y[2]));
@@ -727,7 +737,7 @@ gbz_status gbz_piop_phase2(gbz_ctx *ctx, int N, uint64_t nw, const uint64_t *w, 
   const std::vector<fe> sc = share_scalars(b1, N);
   fe *dsc = ob.alloc<fe>(N), *dip = ob.alloc<fe>((uint64_t)N * rlen);
   GBZ_CUDA(cudaMemcpyAsync(dsc, sc.data(), 16ull * N, cudaMemcpyHostToDevice, s));
-  k_scale_parties<<<dim3(nblk(rlen), N), 256, 0, s>>>(ipb, rlen, dsc, dip, rlen, 0);
+  launch_kernel(k_scale_parties, dim3(nblk(rlen), N), 256, 0, s, ipb, rlen, dsc, dip, rlen, 0);
   GBZ_CUDA(cudaGetLastError());
   std::vector<fe> L = host_lagrange_head(res.claims[2], ilog2((uint64_t)degrees2[0]), 4);
   for (int i = 1; i < ndeg2; i++) {

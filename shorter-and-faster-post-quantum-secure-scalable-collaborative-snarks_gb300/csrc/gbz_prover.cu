@@ -29,10 +29,12 @@ namespace {
 
 // The generator of a proof (a batch: one CTA per proof).
 __global__ void __launch_bounds__(32) k_init(ProofState *st, uint32_t seed, int seed_in_state) {
+  pdl_wait();
   st += blockIdx.x;
   prng_warp_seed(st->prng, seed_in_state ? st->seed_in : seed, threadIdx.x);
 }
 __global__ void k_init_open(ProofState *st, glibc_prng g, const fe *point, int logn, fe K) {
+  pdl_wait();
   if (threadIdx.x == 0) {
     st->fs = fe_zero();
     st->prng = g;
@@ -46,6 +48,7 @@ __global__ void k_init_open(ProofState *st, glibc_prng g, const fe *point, int l
 // z_i = hash_to_field({0}) for i < logn.
 // The start of a proof's protocol state and its evaluation point.
 __global__ void k_point(ProofState *st, int logn, uint8_t *tr, uint64_t off, uint64_t trs) {
+  pdl_wait();
   st += blockIdx.x;
   tr += trs * blockIdx.x;
   if (threadIdx.x) return;
@@ -142,6 +145,7 @@ __device__ __forceinline__ fe shfl_xor_fe(fe x, int d) {
 __global__ void __launch_bounds__(256)
 k_sc_rounds_eq(const fe *partial, int blocks, ProofState *st, int round, uint8_t *tr, int64_t off_claim,
                uint64_t off_poly, uint64_t ps, uint64_t trs) {
+  pdl_wait();
   __shared__ fe red[8][4];
   partial = badv(partial, ps, blockIdx.x);
   st += blockIdx.x;
@@ -186,6 +190,7 @@ constexpr size_t kScTailShared = sizeof(fe) * (kScTailMax / 2 + kScTailMax / 4 +
 __global__ void __launch_bounds__(kScTailThreads)
 k_sc_tail(ProofState *st, const fe *a, const fe *E, int m, int round0, int logn, uint8_t *tr, int64_t off_claim,
           uint64_t off_poly0, uint64_t off_final, BStr bs) {
+  pdl_wait();
   extern __shared__ fe tail_sm[];
   __shared__ fe red[kScTailWorkers / 32][4], T[2][4], zs[64], chal[2];
   // a batch: one CTA per proof; bs = strides of (a, E, tr)
@@ -321,6 +326,7 @@ constexpr int kMaxDraws = kMaxWhirIter * (3 * kFieldDraws + kMaxQueries) + 8 * k
 // thread an element) and the query positions from them.  With one thread
 // drawing and three deriving a launch took 17.5 us at 2^10, now 12.
 __global__ void __launch_bounds__(256) k_whir_schedule(ProofState *st, SchedArgs a) {
+  pdl_wait();
   __shared__ int32_t draws[kMaxDraws + 31];
   st += blockIdx.x;
   int N = kFieldDraws * a.lg_final;
@@ -379,6 +385,7 @@ struct UbPrepArgs {
   const fe *lo[kMaxWhirIter], *hi[kMaxWhirIter];  // omega_NL^e
 };
 __global__ void __launch_bounds__(128) k_ub_prep(const ProofState *st, UbSlots *u, uint64_t us, UbPrepArgs a) {
+  pdl_wait();
   st += blockIdx.y;
   u = badv(u, us, blockIdx.y);
   const int i = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;  // a warp per query
@@ -404,6 +411,7 @@ __global__ void __launch_bounds__(128) k_ub_prep(const ProofState *st, UbSlots *
 // consistency check K == h(0) + h(1), challenge F::_random(), K = h(r).
 __global__ void k_whir_round(const fe *partial, int blocks, ProofState *st, int i, uint8_t *tr,
                              uint64_t off_poly, uint64_t off_chal) {
+  pdl_wait();
   fe H[3];
   sum_partials(partial, blocks, H);
   if (threadIdx.x) return;
@@ -461,11 +469,13 @@ __device__ void merkle_root_dev(const fe *cw, int depth, uint8_t *tr, uint64_t o
   put_hash(tr + off, h);
 }
 __global__ void k_merkle_root(const fe *cw, int depth, uint8_t *tr, uint64_t off) {
+  pdl_wait();
   if (threadIdx.x) return;
   merkle_root_dev(cw, depth, tr, off);
 }
 // The same for a batch: proof p (grid.x) reads cw + p cws, writes tr + p trs.
 __global__ void k_merkle_root_b(const fe *cw, uint64_t cws, int depth, uint8_t *tr, uint64_t trs, uint64_t off) {
+  pdl_wait();
   if (threadIdx.x) return;
   merkle_root_dev(badv(cw, cws, blockIdx.x), depth, tr + trs * blockIdx.x, off);
 }
@@ -485,6 +495,7 @@ __device__ __forceinline__ void path_entry(const fe *cw, int depth, int l, uint6
 }
 __global__ void k_whir_paths_chain(const fe *cw, uint64_t leaves, int l, uint8_t *tr, uint64_t off_q,
                                    uint64_t off_path, uint64_t cws, uint64_t trs) {
+  pdl_wait();
   cw = badv(cw, cws, blockIdx.y);  // a batch: grid.y = proof
   tr += trs * blockIdx.y;
   path_entry(cw, 63 - __clzll((long long)leaves), l, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, tr,
@@ -565,6 +576,7 @@ __device__ void whir_query_dev(const QueryArgs &a, int t) {
 // and bound the opening.  Four warps a block: a compression fills the integer
 // issue slots of an SM's quarter.
 __global__ void __launch_bounds__(kOpenThreads) k_whir_open(QueryArgs a, int t) {
+  pdl_wait();
   a.st += blockIdx.y;
   a.cw = badv(a.cw, a.cws, blockIdx.y);
   a.tr += a.trs * blockIdx.y;
@@ -588,12 +600,14 @@ __global__ void __launch_bounds__(kOpenThreads) k_whir_open(QueryArgs a, int t) 
 // leaf hashes, so its level-d nodes all equal G^d(0): the root of a tree of
 // 2^depth leaves, and every query's path entry d.
 __global__ void k_zero_tree_root(int depth, uint8_t *tr, uint64_t off) {
+  pdl_wait();
   if (threadIdx.x) return;
   uint32_t h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   for (int d = 0; d < depth; d++) node_hash(h);
   put_hash(tr + off, h);
 }
 __global__ void k_zero_tree_paths(int depth, int l, uint8_t *tr, uint64_t off_path) {
+  pdl_wait();
   const int d = blockIdx.x * blockDim.x + threadIdx.x;  // one thread per level
   if (d >= depth) return;
   uint32_t h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -607,6 +621,7 @@ __global__ void k_zero_tree_paths(int depth, int l, uint8_t *tr, uint64_t off_pa
 // thread so that all the scattered tree reads are in flight together.
 __global__ void k_whir_paths(const uint8_t *tree, uint64_t leaves, int l, uint8_t *tr, uint64_t off_q,
                              uint64_t off_path) {
+  pdl_wait();
   const int depth = 63 - __clzll((long long)leaves);
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (uint64_t)l * depth) return;
@@ -656,6 +671,7 @@ __device__ void final_dev(ProofState *st, const fe *arr, const fe *b, int m, uin
 }
 __global__ void k_final(ProofState *st, const fe *arr, const fe *b, int m, uint8_t *tr, uint64_t off_poly,
                         uint64_t off_point, uint64_t off_eval, int check_K, const fe *point) {
+  pdl_wait();
   __shared__ glibc_prng g;
   if (threadIdx.x) return;
   final_dev(st, arr, b, m, tr, off_poly, off_point, off_eval, check_K, point, g);
@@ -664,6 +680,7 @@ __global__ void k_final(ProofState *st, const fe *arr, const fe *b, int m, uint8
 // (st->fin_r): proof p = grid.x, bs = strides of (arr, b, tr).
 __global__ void k_final_b(ProofState *st, const fe *arr, const fe *b, int m, uint8_t *tr, uint64_t off_poly,
                           uint64_t off_point, uint64_t off_eval, BStr bs) {
+  pdl_wait();
   __shared__ glibc_prng g;
   if (threadIdx.x) return;
   st += blockIdx.x;
@@ -886,10 +903,10 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
   };
   if (fork_first) fork();
   if (open) {
-    RUN(PC_PROTOCOL, 1, k_init_open<<<1, 32, 0, s>>>(st, open->prng, open->point, logn, open->K));
+    RUN(PC_PROTOCOL, 1, launch_kernel(k_init_open, 1, 32, 0, s, st, open->prng, open->point, logn, open->K));
   } else {
     const cudaStream_t is = fork_first ? q : s;
-    RUN_ON(is, PC_PROTOCOL, 1, k_init<<<B, 32, 0, is>>>(st, prng_seed, seed_in_state ? 1 : 0));
+    RUN_ON(is, PC_PROTOCOL, 1, launch_kernel(k_init, B, 32, 0, is, st, prng_seed, seed_in_state ? 1 : 0));
   }
   if (!fork_first) fork();
   // The records before the opening; the root's payload is written by its
@@ -903,7 +920,7 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
   auto sumcheck = [&]() {
   // 1. evaluation point and its eq table.
   off = lay.rec(T_EVAL_POINT, logn, 16);
-  RUN(PC_PROTOCOL, 1, k_point<<<B, 32, 0, s>>>(st, logn, tr, off, trs));
+  RUN(PC_PROTOCOL, 1, launch_kernel(k_point, B, 32, 0, s, st, logn, tr, off, trs));
   // 2. sumcheck of sum w(x) eq(z, x), two rounds a pass: w is folded by both
   //    challenges, the eq vector is represented by the shrinking tables
   //    E_{i+1} (vb ping-pong) and the prefix product epre; the last rounds
@@ -927,7 +944,7 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
     RUN(PC_SUMCHECK, 1, sc_eq_reduce_launch(a, p.vb[0], m, p.partial, blocks, s, B, rs));
     for (; m > (uint64_t)kScTailMax; i += 2, m /= 4, pp ^= 1) {
       RUN(PC_PROTOCOL, 1,
-          k_sc_rounds_eq<<<B, 256, 0, s>>>(p.partial, blocks, st, i, tr, i == 0 ? (int64_t)off_claim : -1,
+          launch_kernel(k_sc_rounds_eq, B, 256, 0, s, p.partial, blocks, st, i, tr, i == 0 ? (int64_t)off_claim : -1,
                                            off_poly0 + 80ull * (uint64_t)i, p.bs_part, trs));
       blocks = sc_blocks(m / 4);
       BStr fs;  // (a, chal, a4, E, E4, partial)
@@ -949,7 +966,7 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
   tb.s[1] = p.bs_v;
   tb.s[2] = trs;
   RUN(PC_SUMCHECK, 1,
-      (k_sc_tail<<<B, kScTailThreads, kScTailShared, s>>>(st, a, p.vb[pp], (int)m, i, logn, tr,
+      (launch_kernel(k_sc_tail, B, kScTailThreads, kScTailShared, s, st, a, p.vb[pp], (int)m, i, logn, tr,
                                                          i == 0 ? (int64_t)off_claim : -1,
                                                          off_poly0 + 80ull * (uint64_t)i, off, tb)));
   };
@@ -973,7 +990,7 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
       if (mm <= (uint64_t)kWhirK) break;
     }
     sa.lg_final = ilog2(mm);
-    RUN_ON(q, PC_PROTOCOL, 1, k_whir_schedule<<<B, 256, 0, q>>>(st, sa));
+    RUN_ON(q, PC_PROTOCOL, 1, launch_kernel(k_whir_schedule, B, 256, 0, q, st, sa));
     ua.T = sa.T;
     LL = p.L;
     mm = p.n;
@@ -989,7 +1006,7 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
     }
     if (ua.base[sa.T] > kUbSlots) throw ArgError("prover: too many queries");
     RUN_ON(q, PC_UPDATE_BETAS, 1,
-           k_ub_prep<<<dim3((unsigned)(ua.base[sa.T] + 3) / 4, B), 128, 0, q>>>(st, slots, p.bs_ub, ua));
+           launch_kernel(k_ub_prep, dim3((unsigned)(ua.base[sa.T] + 3) / 4, B), 128, 0, q, st, slots, p.bs_ub, ua));
     if (go) GBZ_CUDA(cudaEventRecord(p.ev_sched, q));
   };
 
@@ -1132,7 +1149,8 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
              ntt_launch_rows(p.tables(ilog2(NL)), a, m, p.bs_arr / sizeof(fe), p.cw[nci], cw_s[nci] / sizeof(fe), B,
                              p.tmp, false, c));
     } else {
-      RUN_ON(c, PC_NTT, ntt_launch_count(ilog2(NL), m), ntt_launch(p.tables(ilog2(NL)), a, m, p.cw[nci], p.tmp, false, c));
+      RUN_ON(c, PC_NTT, ntt_launch_count(ilog2(NL), m),
+             ntt_launch(p.tables(ilog2(NL)), a, m, p.cw[nci], p.tmp, false, c));
     }
     off_root[iter + 1] = off;
     if (go) GBZ_CUDA(cudaEventRecord(p.ev_commit[iter + 1], c));
@@ -1181,8 +1199,8 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
     const uint64_t hashes = (uint64_t)l * depth;
     if (hashes == 0) throw ArgError("prover: empty authentication paths");
     RUN_ON(q, PC_QUERY, 1,
-           k_whir_open<<<dim3((unsigned)(2 + (hashes + kOpenThreads - 1) / kOpenThreads), B), kOpenThreads, 0, q>>>(
-               qa, iter));
+           launch_kernel(k_whir_open, dim3((unsigned)(2 + (hashes + kOpenThreads - 1) / kOpenThreads), B),
+                         kOpenThreads, 0, q, qa, iter));
     if (go) GBZ_CUDA(cudaEventRecord(p.ev_query[iter], q));
     // update_betas on s: b[j] += sum_i c_i omega_NL^{q_i j} is the forward
     // transform of a vector with l nonzeros.  When l * |b| exceeds a few
@@ -1218,12 +1236,12 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
     fb.s[0] = ast;
     fb.s[1] = bst;
     fb.s[2] = trs;
-    RUN(PC_PROTOCOL, 1, k_final_b<<<B, 32, 0, s>>>(st, a, b, (int)m, tr, off_poly, off_point, off_eval, fb));
+    RUN(PC_PROTOCOL, 1, launch_kernel(k_final_b, B, 32, 0, s, st, a, b, (int)m, tr, off_poly, off_point, off_eval, fb));
   }
   // root of the last commitment (never opened) on the query stream
   if (go) GBZ_CUDA(cudaStreamWaitEvent(q, p.ev_commit[iter], 0));
   RUN_ON(q, PC_MERKLE, 1,
-         k_merkle_root_b<<<B, 32, 0, q>>>(p.cw[cwi], cw_s[cwi], ilog2(L / 4), tr, trs, off_root[iter]));
+         launch_kernel(k_merkle_root_b, B, 32, 0, q, p.cw[cwi], cw_s[cwi], ilog2(L / 4), tr, trs, off_root[iter]));
   if (go) {  // join the commit and query chains
     GBZ_CUDA(cudaEventRecord(p.ev_root_tail, q));
     GBZ_CUDA(cudaStreamWaitEvent(s, p.ev_commit[iter], 0));
@@ -1276,18 +1294,20 @@ Profiler::~Profiler() {
 
 namespace {
 __global__ void k_set_seed(ProofState *st, uint32_t seed) {
+  pdl_wait();
   if (threadIdx.x == 0) st->seed_in = seed;
 }
 struct SeedChunk {
   uint32_t v[64];
 };
 __global__ void k_set_seeds(ProofState *st, SeedChunk c, int count) {
+  pdl_wait();
   if ((int)threadIdx.x < count) st[threadIdx.x].seed_in = c.v[threadIdx.x];
 }
 }  // namespace
 
 void set_seed_launch(ProofPlan &p, uint32_t seed, cudaStream_t s) {
-  k_set_seed<<<1, 32, 0, s>>>(p.st, seed);
+  launch_kernel(k_set_seed, 1, 32, 0, s, p.st, seed);
   GBZ_CUDA(cudaGetLastError());
 }
 
@@ -1296,7 +1316,7 @@ void set_seeds_launch(ProofPlan &p, const uint32_t *seeds, int count, cudaStream
     SeedChunk c{};
     const int k = std::min(64, count - o);
     for (int i = 0; i < k; i++) c.v[i] = seeds[o + i];
-    k_set_seeds<<<1, 64, 0, s>>>(p.st + o, c, k);
+    launch_kernel(k_set_seeds, 1, 64, 0, s, p.st + o, c, k);
     GBZ_CUDA(cudaGetLastError());
   }
 }

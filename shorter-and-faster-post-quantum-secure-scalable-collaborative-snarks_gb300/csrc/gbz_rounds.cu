@@ -169,6 +169,7 @@ __device__ void block_sum(fe *x) {
 // as it is read (the parties' weights of the cubic form).
 template <int FORM, int MODE>
 __global__ void __launch_bounds__(kThreads) form_step_kernel(RoundArgs a) {
+  pdl_wait();
   constexpr int NV = Form<FORM>::NV, NC = Form<FORM>::NC;
   typename Sums<FORM>::type sums[NC];
 #pragma unroll
@@ -241,6 +242,7 @@ __global__ void __launch_bounds__(kThreads) form_step_kernel(RoundArgs a) {
 // Copies the first entry of every vector (with the weight scale of vector
 // 2) to fin: the final values when no round is left.
 __global__ void form_first_kernel(RoundArgs a, int nv, fe *fin) {
+  pdl_wait();
   const int k = threadIdx.x;
   if (k >= nv) return;
   fe x = a.in[k][0];
@@ -297,6 +299,7 @@ __device__ __forceinline__ fe warp_partial_sum(const fe *partial, int blocks, in
 __global__ void __launch_bounds__(256)
 form_finalize_kernel(const fe *partial, int blocks, int nc, RoundState *st, int round, const fe *drawn, fe *polys,
                      fe *chal) {
+  pdl_wait();
   __shared__ fe red[4][2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k = warp >> 1;
   fe fs = st->fs, y = st->y;
@@ -324,6 +327,7 @@ form_finalize_kernel(const fe *partial, int blocks, int nc, RoundState *st, int 
 // to st->prng.  Of a challenge's outputs the last 40 are its digits.  (One
 // thread took 22 us a challenge.)
 __global__ void __launch_bounds__(32) prng_draw_kernel(RoundState *st, int n, fe *out) {
+  pdl_wait();
   constexpr int kDraws = 160, kFull = kDraws / 31, kRest = kDraws % 31;
   __shared__ int32_t d[kDraws + 31];
   const int lane = threadIdx.x, f0 = st->prng.f;
@@ -424,6 +428,7 @@ struct TailArgs {
 // the last 14 rounds took 116 us; these last 12 take 51.)
 template <int FORM>
 __global__ void __launch_bounds__(kTailThreads) form_tail_kernel(TailArgs t) {
+  pdl_wait();
   constexpr int NV = Form<FORM>::NV, NC = Form<FORM>::NC;
   extern __shared__ fe tail_sm[];
   __shared__ fe red[NC][kTailWarps];
@@ -491,6 +496,7 @@ __global__ void __launch_bounds__(kTailThreads) form_tail_kernel(TailArgs t) {
 // 2^14 entries on, the quadruple form took 111 us and the cubic 105, now 46 and 31).
 template <int FORM>
 __global__ void __launch_bounds__(kTailThreads) form_tail_drawn_kernel(DrawnTailArgs t) {
+  pdl_wait();
   constexpr int NV = Form<FORM>::NV, NC = Form<FORM>::NC;
   extern __shared__ fe tail_sm[];
   __shared__ fe red[kDrawnTailLog][NC][kTailWarps];
@@ -566,6 +572,7 @@ __global__ void __launch_bounds__(kTailThreads) form_tail_drawn_kernel(DrawnTail
 }
 
 __global__ void form_sum_kernel(const fe *partial, int blocks, int nc, fe *out) {
+  pdl_wait();
   __shared__ fe red[kMaxFormCoeffs][kThreads];
   fe acc[kMaxFormCoeffs];
   for (int k = 0; k < kMaxFormCoeffs; k++) acc[k] = fe_zero();
@@ -583,7 +590,7 @@ __global__ void form_sum_kernel(const fe *partial, int blocks, int nc, fe *out) 
 
 template <int FORM, int MODE>
 void launch_step(const RoundArgs &a, int blocks, cudaStream_t s) {
-  form_step_kernel<FORM, MODE><<<blocks, kThreads, 0, s>>>(a);
+  launch_kernel(form_step_kernel<FORM, MODE>, blocks, kThreads, 0, s, a);
   GBZ_CUDA(cudaGetLastError());
 }
 
@@ -641,13 +648,13 @@ void launch_tail_drawn(const DrawnTailArgs &a, cudaStream_t s) {
   const size_t sh = tail_shared<FORM>(a.n >> (a.i0 - 1));
   GBZ_CUDA(cudaFuncSetAttribute(form_tail_drawn_kernel<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)tail_shared<FORM>(1ull << kDrawnTailLog)));
-  form_tail_drawn_kernel<FORM><<<1, kTailThreads, sh, s>>>(a);
+  launch_kernel(form_tail_drawn_kernel<FORM>, 1, kTailThreads, sh, s, a);
 }
 template <int FORM>
 void launch_tail(const TailArgs &a, cudaStream_t s) {
   GBZ_CUDA(cudaFuncSetAttribute(form_tail_kernel<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)tail_shared<FORM>(kTailEntries)));
-  form_tail_kernel<FORM><<<1, kTailThreads, tail_shared<FORM>(a.cur), s>>>(a);
+  launch_kernel(form_tail_kernel<FORM>, 1, kTailThreads, tail_shared<FORM>(a.cur), s, a);
 }
 }  // namespace
 
@@ -664,18 +671,18 @@ void form_tail_drawn_launch(int form, const DrawnTailArgs &a, cudaStream_t s) {
 }
 
 void form_sum_launch(const fe *partial, int blocks, int nc, fe *out, cudaStream_t s) {
-  form_sum_kernel<<<1, kThreads, 0, s>>>(partial, blocks, nc, out);
+  launch_kernel(form_sum_kernel, 1, kThreads, 0, s, partial, blocks, nc, out);
   GBZ_CUDA(cudaGetLastError());
 }
 
 void form_finalize_launch(const fe *partial, int blocks, int nc, RoundState *st, int round, const fe *drawn, fe *polys,
                           fe *chal, cudaStream_t s) {
-  form_finalize_kernel<<<1, kThreads, 0, s>>>(partial, blocks, nc, st, round, drawn, polys, chal);
+  launch_kernel(form_finalize_kernel, 1, kThreads, 0, s, partial, blocks, nc, st, round, drawn, polys, chal);
   GBZ_CUDA(cudaGetLastError());
 }
 
 void form_first_launch(const RoundArgs &a, int nv, fe *fin, cudaStream_t s) {
-  form_first_kernel<<<1, 32, 0, s>>>(a, nv, fin);
+  launch_kernel(form_first_kernel, 1, 32, 0, s, a, nv, fin);
   GBZ_CUDA(cudaGetLastError());
 }
 
@@ -725,7 +732,7 @@ void party_sumcheck_enqueue(int form, const fe *const *v, uint64_t M, int N, con
       GBZ_CUDA(cudaEventRecord(side.fork, s));
       GBZ_CUDA(cudaStreamWaitEvent(side.stream, side.fork, 0));
     }
-    prng_draw_kernel<<<1, 32, 0, ds>>>(st, total - fs_rounds, drawn);
+    launch_kernel(prng_draw_kernel, 1, 32, 0, ds, st, total - fs_rounds, drawn);
     GBZ_CUDA(cudaGetLastError());
     if (side.stream) GBZ_CUDA(cudaEventRecord(side.join, side.stream));
   }

@@ -63,6 +63,7 @@ __device__ __forceinline__ void acc_pair(fe a0, fe a1, fe b0, fe b1, facc &A, fa
 // partial[3*blk + {0,1,2}] = (sum A, sum C, sum D) of the block.
 __global__ void __launch_bounds__(kScThreads)
 sc_reduce_kernel(const fe *__restrict__ a, const fe *__restrict__ b, uint64_t pairs, fe *partial) {
+  pdl_wait();
   facc sA = facc_zero(), sC = facc_zero(), sD = facc_zero();
   const uint64_t stride = (uint64_t)gridDim.x * kScThreads;
   for (uint64_t j = (uint64_t)blockIdx.x * kScThreads + threadIdx.x; j < pairs; j += stride) {
@@ -83,6 +84,7 @@ sc_reduce_kernel(const fe *__restrict__ a, const fe *__restrict__ b, uint64_t pa
 __global__ void __launch_bounds__(kScThreads)
 sc_fold_kernel(const fe *__restrict__ a, const fe *__restrict__ b, uint64_t m, const fe *chal,
                fe *__restrict__ a2, fe *__restrict__ b2, int reduce, fe *partial) {
+  pdl_wait();
   const fe r = *chal;
   facc sA = facc_zero(), sC = facc_zero(), sD = facc_zero();
   const uint64_t stride = (uint64_t)gridDim.x * kScThreads;
@@ -118,6 +120,7 @@ sc_fold_kernel(const fe *__restrict__ a, const fe *__restrict__ b, uint64_t m, c
 __global__ void __launch_bounds__(kScThreads, 2)
 sc_fold2_kernel(const fe *__restrict__ a, const fe *__restrict__ b, uint64_t m, const fe *chal0, const fe *chal1,
                 fe *__restrict__ a4, fe *__restrict__ b4, fe *partial0, fe *partial1, BStr bs) {
+  pdl_wait();
   const uint32_t pb = blockIdx.y;
   a = badv(a, bs.s[0], pb);
   b = badv(b, bs.s[1], pb);
@@ -170,6 +173,7 @@ sc_fold2_kernel(const fe *__restrict__ a, const fe *__restrict__ b, uint64_t m, 
 __global__ void __launch_bounds__(kScThreads, 2)
 sc_fold2_eq_kernel(const fe *__restrict__ a, const fe *__restrict__ E2, uint64_t m, const fe *c, const fe *chal0,
                    const fe *chal1, fe *__restrict__ a4, fe *__restrict__ b4, fe *partial0, fe *partial1, BStr bs) {
+  pdl_wait();
   const uint32_t pb = blockIdx.y;
   a = badv(a, bs.s[0], pb);
   E2 = badv(E2, bs.s[1], pb);
@@ -263,6 +267,7 @@ __device__ void block_sum_classes(const facc &acc, fe *partial) {
 
 __global__ void __launch_bounds__(kScThreads)
 sc_eq_reduce_kernel(const fe *__restrict__ a, const fe *__restrict__ E, uint64_t m, fe *partial, BStr bs) {
+  pdl_wait();
   a = badv(a, bs.s[0], blockIdx.y);
   E = badv(E, bs.s[1], blockIdx.y);
   partial = badv(partial, bs.s[2], blockIdx.y);
@@ -282,6 +287,7 @@ sc_eq_reduce_kernel(const fe *__restrict__ a, const fe *__restrict__ E, uint64_t
 __global__ void __launch_bounds__(kScThreads)
 sc_eq_fold_kernel(const fe *__restrict__ a, uint64_t m, const fe *chal, fe *__restrict__ a4,
                   const fe *__restrict__ E, fe *__restrict__ E4, int reduce, fe *partial, BStr bs) {
+  pdl_wait();
   a = badv(a, bs.s[0], blockIdx.y);
   chal = badv(chal, bs.s[1], blockIdx.y);
   a4 = badv(a4, bs.s[2], blockIdx.y);
@@ -315,6 +321,7 @@ sc_eq_fold_kernel(const fe *__restrict__ a, uint64_t m, const fe *chal, fe *__re
 
 // out = (a, b, c) of the round message from (A, C, D) partials.
 __global__ void __launch_bounds__(kScThreads) sc_sum_kernel(const fe *partial, int blocks, fe *out) {
+  pdl_wait();
   fe A = fe_zero(), C = fe_zero(), D = fe_zero();
   for (int i = threadIdx.x; i < blocks; i += kScThreads) {
     A = fadd(A, partial[3 * i]);
@@ -336,6 +343,7 @@ __global__ void __launch_bounds__(kScThreads) sc_sum_kernel(const fe *partial, i
 // coalesced 16-byte stores.
 constexpr int kBetaBlockLog = 11;
 __global__ void __launch_bounds__(256) beta_block_kernel(const fe *r, int nr, fe *B, BStr bs) {
+  pdl_wait();
   __shared__ fe T[1 << kBetaBlockLog];
   __shared__ fe rs[64];
   r = badv(r, bs.s[0], blockIdx.y);
@@ -378,6 +386,7 @@ __global__ void __launch_bounds__(256) beta_block_kernel(const fe *r, int nr, fe
 // CTA is amortised over 2^15 entries.
 constexpr int kBetaChunksLog = 4;  // at most 16 blocks of 2^11 entries per CTA
 __global__ void __launch_bounds__(256) beta_tensor_kernel(const fe *r, int nr, int chunks_log, fe *B, BStr bs) {
+  pdl_wait();
   __shared__ fe T[1 << kBetaBlockLog];
   __shared__ fe hi_pre[1 << kBetaChunksLog];
   __shared__ fe rs[64];
@@ -434,6 +443,7 @@ constexpr int kUbWarps = kUbThreads / 32;
 
 // pw[i*32 + L] = w_i^(L * per)
 __global__ void __launch_bounds__(32) ub_table_kernel(const fe *w, int per, fe *pw) {
+  pdl_wait();
   const int i = blockIdx.x, t = threadIdx.x;
   pw[i * 32 + t] = fpow(w[i], (uint64_t)t * per);
 }
@@ -441,6 +451,7 @@ __global__ void __launch_bounds__(32) ub_table_kernel(const fe *w, int per, fe *
 template <int PER>
 __global__ void __launch_bounds__(kUbThreads)
 ub_kernel(fe *b, uint64_t nb, const fe *w, const fe *c, int l, const fe *pw, uint64_t b_stride, uint64_t u_stride) {
+  pdl_wait();
   constexpr int SPAN = 32 * PER;
   __shared__ fe s_start[kMaxQueries], s_w[kMaxQueries];
   __shared__ fe part[kUbWarps][SPAN];
@@ -493,9 +504,9 @@ int sc_blocks(uint64_t pairs) {
 void sc_step_launch(const fe *a, const fe *b, uint64_t m, const fe *chal, fe *a2, fe *b2, bool reduce,
                     fe *partial, int blocks, cudaStream_t s) {
   if (!chal) {
-    sc_reduce_kernel<<<blocks, kScThreads, 0, s>>>(a, b, m / 2, partial);
+    launch_kernel(sc_reduce_kernel, blocks, kScThreads, 0, s, a, b, m / 2, partial);
   } else {
-    sc_fold_kernel<<<blocks, kScThreads, 0, s>>>(a, b, m, chal, a2, b2, reduce ? 1 : 0, partial);
+    launch_kernel(sc_fold_kernel, blocks, kScThreads, 0, s, a, b, m, chal, a2, b2, reduce ? 1 : 0, partial);
   }
   GBZ_CUDA(cudaGetLastError());
 }
@@ -503,33 +514,35 @@ void sc_step_launch(const fe *a, const fe *b, uint64_t m, const fe *chal, fe *a2
 void sc_fold2_launch(const fe *a, const fe *b, uint64_t m, const fe *chal0, const fe *chal1, fe *a4, fe *b4,
                      fe *partial0, fe *partial1, int blocks, cudaStream_t s, int batch, const BStr &bs) {
   if (m < 4) throw ArgError("two-round fold needs at least 4 entries");
-  sc_fold2_kernel<<<dim3(blocks, batch), kScThreads, 0, s>>>(a, b, m, chal0, chal1, a4, b4, partial0, partial1, bs);
+  launch_kernel(sc_fold2_kernel, dim3(blocks, batch), kScThreads, 0, s, a, b, m, chal0, chal1, a4, b4, partial0,
+                partial1, bs);
   GBZ_CUDA(cudaGetLastError());
 }
 
 void sc_fold2_eq_launch(const fe *a, const fe *E2, uint64_t m, const fe *c, const fe *chal0, const fe *chal1, fe *a4,
                         fe *b4, fe *partial0, fe *partial1, int blocks, cudaStream_t s, int batch, const BStr &bs) {
   if (m < 4) throw ArgError("two-round fold needs at least 4 entries");
-  sc_fold2_eq_kernel<<<dim3(blocks, batch), kScThreads, 0, s>>>(a, E2, m, c, chal0, chal1, a4, b4, partial0,
+  launch_kernel(sc_fold2_eq_kernel, dim3(blocks, batch), kScThreads, 0, s, a, E2, m, c, chal0, chal1, a4, b4, partial0,
                                                                 partial1, bs);
   GBZ_CUDA(cudaGetLastError());
 }
 
 void sc_eq_reduce_launch(const fe *a, const fe *E, uint64_t m, fe *partial, int blocks, cudaStream_t s, int batch,
                          const BStr &bs) {
-  sc_eq_reduce_kernel<<<dim3(blocks, batch), kScThreads, 0, s>>>(a, E, m, partial, bs);
+  launch_kernel(sc_eq_reduce_kernel, dim3(blocks, batch), kScThreads, 0, s, a, E, m, partial, bs);
   GBZ_CUDA(cudaGetLastError());
 }
 
 void sc_eq_fold_launch(const fe *a, const fe *E, uint64_t m, const fe *chal, fe *a4, fe *E4, bool reduce, fe *partial,
                        int blocks, cudaStream_t s, int batch, const BStr &bs) {
   if (m < 128 || m % 128) throw ArgError("two-round fold of w needs a multiple of 128 entries");
-  sc_eq_fold_kernel<<<dim3(blocks, batch), kScThreads, 0, s>>>(a, m, chal, a4, E, E4, reduce ? 1 : 0, partial, bs);
+  launch_kernel(sc_eq_fold_kernel, dim3(blocks, batch), kScThreads, 0, s, a, m, chal, a4, E, E4, reduce ? 1 : 0,
+                partial, bs);
   GBZ_CUDA(cudaGetLastError());
 }
 
 void sc_sum_launch(const fe *partial, int blocks, fe *out3, cudaStream_t s) {
-  sc_sum_kernel<<<1, kScThreads, 0, s>>>(partial, blocks, out3);
+  launch_kernel(sc_sum_kernel, 1, kScThreads, 0, s, partial, blocks, out3);
   GBZ_CUDA(cudaGetLastError());
 }
 
@@ -541,13 +554,13 @@ void beta_launch(const fe *r, int nr, fe *B, cudaStream_t s, int batch, uint64_t
   if (nr >= kBetaBlockLog + 4) {
     // enough CTAs to cover the SMs (at least 2^9), up to 16 blocks each
     const int chunks_log = std::max(0, std::min(kBetaChunksLog, nr - kBetaBlockLog - 9));
-    beta_tensor_kernel<<<dim3((unsigned)(1ull << (nr - kBetaBlockLog - chunks_log)), batch), 256, 0, s>>>(
-        r, nr, chunks_log, B, bs);
+    launch_kernel(beta_tensor_kernel, dim3((unsigned)(1ull << (nr - kBetaBlockLog - chunks_log)), batch), 256, 0, s,
+                  r, nr, chunks_log, B, bs);
     GBZ_CUDA(cudaGetLastError());
     return;
   }
   const int low = nr < kBetaBlockLog ? nr : kBetaBlockLog;
-  beta_block_kernel<<<dim3((unsigned)(1ull << (nr - low)), batch), 256, 0, s>>>(r, nr, B, bs);
+  launch_kernel(beta_block_kernel, dim3((unsigned)(1ull << (nr - low)), batch), 256, 0, s, r, nr, B, bs);
   GBZ_CUDA(cudaGetLastError());
 }
 
@@ -563,16 +576,16 @@ void update_betas_powers_launch(fe *b, uint64_t nb, const fe *w, const fe *c, in
   const int per = update_betas_per(nb, batch), span = 32 * per;
   const dim3 grid((unsigned)((nb + span - 1) / span), batch);
   if (!grid.x) return;
-  if (per == 8) ub_kernel<8><<<grid, kUbThreads, 0, s>>>(b, nb, w, c, l, pw, b_stride, u_stride);
-  else if (per == 2) ub_kernel<2><<<grid, kUbThreads, 0, s>>>(b, nb, w, c, l, pw, b_stride, u_stride);
-  else ub_kernel<1><<<grid, kUbThreads, 0, s>>>(b, nb, w, c, l, pw, b_stride, u_stride);
+  if (per == 8) launch_kernel(ub_kernel<8>, grid, kUbThreads, 0, s, b, nb, w, c, l, pw, b_stride, u_stride);
+  else if (per == 2) launch_kernel(ub_kernel<2>, grid, kUbThreads, 0, s, b, nb, w, c, l, pw, b_stride, u_stride);
+  else launch_kernel(ub_kernel<1>, grid, kUbThreads, 0, s, b, nb, w, c, l, pw, b_stride, u_stride);
   GBZ_CUDA(cudaGetLastError());
 }
 
 void update_betas_launch(fe *b, uint64_t nb, const ProofState *st, int l, fe *pw_scratch, cudaStream_t s) {
   if (l <= 0) return;
   if (l > kMaxQueries) throw ArgError("update_betas: too many queries");
-  ub_table_kernel<<<l, 32, 0, s>>>(st->omega_q, update_betas_per(nb, 1), pw_scratch);
+  launch_kernel(ub_table_kernel, l, 32, 0, s, st->omega_q, update_betas_per(nb, 1), pw_scratch);
   GBZ_CUDA(cudaGetLastError());
   update_betas_powers_launch(b, nb, st->omega_q, st->comb, l, pw_scratch, s, 1, 0, 0);
 }

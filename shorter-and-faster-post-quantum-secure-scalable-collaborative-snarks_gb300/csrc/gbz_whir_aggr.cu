@@ -21,6 +21,7 @@ __device__ __forceinline__ fe shfl_down_fe(fe v, int d) {
 // out[t] = (acc ? out[t] : 0) + sum_i coef[i] * v.p[i][t]
 __global__ void __launch_bounds__(kThreads) lincomb_kernel(VecList v, const fe *coef, int k, uint64_t n, fe *out,
                                                            int acc) {
+  pdl_wait();
   __shared__ fe c[kMaxVecs];
   for (int i = threadIdx.x; i < k; i += kThreads) c[i] = coef[i];
   __syncthreads();
@@ -36,6 +37,7 @@ __global__ void __launch_bounds__(kThreads) lincomb_kernel(VecList v, const fe *
 // Per-CTA partial sums of the TA x TB inner products <a_i, b_j>.
 template <int TA, int TB>
 __global__ void __launch_bounds__(kThreads, 2) multidot_kernel(VecList a, VecList b, uint64_t n, fe *partial) {
+  pdl_wait();
   // more than nine 96-bit accumulators would leave one CTA an SM
   typename std::conditional<(TA * TB > 9), facc64, facc>::type acc[TA * TB] = {};
   const uint64_t stride = (uint64_t)gridDim.x * kThreads;
@@ -70,6 +72,7 @@ __global__ void __launch_bounds__(kThreads, 2) multidot_kernel(VecList a, VecLis
 // out[q] = sum over blocks of partial[block * nq + q]: one CTA per q
 // (launched with nq CTAs of kThreads), the blocks spread over its threads.
 __global__ void __launch_bounds__(kThreads) sum_cols_kernel(const fe *partial, int blocks, int nq, fe *out) {
+  pdl_wait();
   const int q = blockIdx.x;
   fe s = fe_zero();
   for (int b = threadIdx.x; b < blocks; b += kThreads) s = fadd(s, partial[(uint64_t)b * nq + q]);
@@ -94,7 +97,7 @@ int grid_for(uint64_t n) {
 
 template <int TA, int TB>
 void md_launch(const VecList &a, const VecList &b, uint64_t n, fe *partial, int blocks, cudaStream_t s) {
-  multidot_kernel<TA, TB><<<blocks, kThreads, 0, s>>>(a, b, n, partial);
+  launch_kernel(multidot_kernel<TA, TB>, blocks, kThreads, 0, s, a, b, n, partial);
   GBZ_CUDA(cudaGetLastError());
 }
 
@@ -115,7 +118,7 @@ void md_dispatch(int ta, int tb, const VecList &a, const VecList &b, uint64_t n,
 void lincomb_launch(const VecList &v, const fe *coef, int k, uint64_t n, fe *out, bool accumulate, cudaStream_t s) {
   if (k < 0 || k > kMaxVecs) throw ArgError("linear combination of more than 64 vectors");
   if (!n) return;
-  lincomb_kernel<<<grid_for(n), kThreads, 0, s>>>(v, coef, k, n, out, accumulate ? 1 : 0);
+  launch_kernel(lincomb_kernel, grid_for(n), kThreads, 0, s, v, coef, k, n, out, accumulate ? 1 : 0);
   GBZ_CUDA(cudaGetLastError());
 }
 
@@ -135,7 +138,7 @@ void multidot_launch(const VecList &a, int ka, const VecList &b, int kb, uint64_
       md_dispatch(ta, tb, at, bt, n, partial, blocks, s);
       // tile results go to a staging row, then into out[i][j] (row-major ka x kb)
       fe *tile = partial + (uint64_t)blocks * 16;
-      sum_cols_kernel<<<ta * tb, kThreads, 0, s>>>(partial, blocks, ta * tb, tile);
+      launch_kernel(sum_cols_kernel, ta * tb, kThreads, 0, s, partial, blocks, ta * tb, tile);
       GBZ_CUDA(cudaGetLastError());
       for (int i = 0; i < ta; i++)
         GBZ_CUDA(cudaMemcpyAsync(out + (uint64_t)(i0 + i) * kb + j0, tile + i * tb, sizeof(fe) * tb,
@@ -157,6 +160,7 @@ template <int TA, int TC>
 __global__ void __launch_bounds__(kThreads, 2)
 aggr_claims_pass_kernel(VecList a, const fe *elo, const fe *ehi, int h, uint64_t lo_len, uint64_t hi_len,
                         uint64_t n, const fe *bw, const fe *aw, int first, fe *arr, fe *baggr, fe *partial) {
+  pdl_wait();
   __shared__ fe sw[TA + TC];
   if (threadIdx.x < TC) sw[threadIdx.x] = bw[threadIdx.x];
   if (aw && threadIdx.x < TA) sw[TC + threadIdx.x] = aw[threadIdx.x];
@@ -206,7 +210,8 @@ aggr_claims_pass_kernel(VecList a, const fe *elo, const fe *ehi, int h, uint64_t
 template <int TA, int TC>
 void pass_launch(const VecList &a, const fe *elo, const fe *ehi, int h, int lg, uint64_t n, const fe *bw,
                  const fe *aw, int first, fe *arr, fe *baggr, fe *partial, int blocks, cudaStream_t s) {
-  aggr_claims_pass_kernel<TA, TC><<<blocks, kThreads, 0, s>>>(a, elo, ehi, h, 1ull << h, 1ull << (lg - h), n, bw,
+  launch_kernel(aggr_claims_pass_kernel<TA, TC>, blocks, kThreads, 0, s, a, elo, ehi, h, 1ull << h, 1ull << (lg - h),
+                n, bw,
                                                               aw, first, arr, baggr, partial);
   GBZ_CUDA(cudaGetLastError());
 }
@@ -227,7 +232,7 @@ bool aggr_claims_fused(const VecList &a, int k, int c, const fe *elo, const fe *
     if (k == A && tc == C) pass_launch<A, C>(a, el, eh, h, lg, n, w + j0, aw, j0 == 0, arr, baggr, partial, blocks, s);
     GBZ_AP(1, 1) GBZ_AP(1, 2) GBZ_AP(2, 1) GBZ_AP(2, 2) GBZ_AP(3, 1) GBZ_AP(3, 2) GBZ_AP(4, 1) GBZ_AP(4, 2)
 #undef GBZ_AP
-    sum_cols_kernel<<<k * tc, kThreads, 0, s>>>(partial, blocks, k * tc, tile);
+    launch_kernel(sum_cols_kernel, k * tc, kThreads, 0, s, partial, blocks, k * tc, tile);
     GBZ_CUDA(cudaGetLastError());
     // the pass's k x tc sums into columns j0.. of the row-major k x c sums
     GBZ_CUDA(cudaMemcpy2DAsync(sums + j0, sizeof(fe) * c, tile, sizeof(fe) * tc, sizeof(fe) * tc, k,
