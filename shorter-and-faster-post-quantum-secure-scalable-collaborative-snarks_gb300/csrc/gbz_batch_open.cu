@@ -54,16 +54,18 @@ struct BoQueryArgs {
 // K += sum_i c_i y_i (:325-342, :383-384).  Thread i handles query i.
 __global__ void __launch_bounds__(kMaxQueries) bo_query_kernel(BoQueryArgs a) {
   pdl_wait();
-  __shared__ int32_t q[kMaxQueries];
+  __shared__ int32_t q[kMaxQueries + kFieldDraws];
   __shared__ fe rb_s;
   __shared__ fe red[kMaxQueries / 32];
-  __shared__ glibc_prng g;
   ProofState *st = a.st;
-  if (threadIdx.x == 0) {
-    g = st->prng;
-    for (int i = 0; i < a.l; i++) q[i] = prng_next(g) % (int32_t)a.qmod;
-    rb_s = prng_field(g);  // update_betas' F::_random(), drawn after the queries
-    st->prng = g;
+  if (threadIdx.x < 32) {  // (one thread drew for 12 of 23 us at 100 queries)
+    const int lane = threadIdx.x, n = a.l + kFieldDraws, f0 = st->prng.f;
+    const uint32_t x = prng_warp_draw(prng_warp_load(st->prng, lane), q, n, lane);
+    const fe c = prng_warp_field(q + a.l, lane);  // update_betas' F::_random(), drawn after the queries
+    for (int i = lane; i < a.l; i += 32) q[i] %= (int32_t)a.qmod;
+    __syncwarp();
+    prng_warp_store(st->prng, x, f0, n, lane);
+    if (lane == 0) rb_s = c;
   }
   __syncthreads();
   const int i = threadIdx.x;
@@ -121,16 +123,21 @@ __global__ void __launch_bounds__(kMaxQueries) bo_query_kernel(BoQueryArgs a) {
 // ch2, then ch1[0] = ch2[0] = 1.  coef = (ch1, ch2).
 __global__ void bo_aggr_draw_kernel(ProofState *st, int g, fe *coef, uint8_t *tr, uint64_t off) {
   pdl_wait();
-  __shared__ glibc_prng gs;
-  if (threadIdx.x) return;
-  gs = st->prng;
+  __shared__ int32_t d[kFieldDraws];
+  const int lane = threadIdx.x, f0 = st->prng.f;
+  uint32_t x = prng_warp_load(st->prng, lane);
   for (int i = 0; i < 2 * g; i++) {
-    fe c = prng_field(gs);
+    x = prng_warp_draw(x, d, kFieldDraws, lane);
+    fe c = prng_warp_field(d, lane);
     if (i == 0 || i == g) c = fe_one();
-    coef[i] = c;
-    put_fe(tr, off + 16 * (uint64_t)i, c);
+    if (lane == 0) {
+      coef[i] = c;
+      put_fe(tr, off + 16 * (uint64_t)i, c);
+    }
+    __syncwarp();
   }
-  st->prng = gs;
+  __syncwarp();
+  prng_warp_store(st->prng, x, f0, (uint64_t)kFieldDraws * 2 * g, lane);
 }
 
 // aggregate_arrays' claim (Whir.cpp:695-702) with r1 = ch2, r2 = ch1:
@@ -149,12 +156,13 @@ __global__ void bo_aggr_k_kernel(ProofState *st, const fe *evals, const fe *coef
 // The openings aggregate_commitments draws (Whir.cpp:574-576).
 __global__ void bo_aggr_queries_kernel(ProofState *st, int la, int32_t qmod, uint8_t *tr, uint64_t off) {
   pdl_wait();
-  __shared__ glibc_prng gs;
-  if (threadIdx.x) return;
-  gs = st->prng;
+  __shared__ int32_t d[kMaxQueries];
+  const int lane = threadIdx.x, f0 = st->prng.f;
+  const uint32_t x = prng_warp_draw(prng_warp_load(st->prng, lane), d, la, lane);
   int32_t *q = reinterpret_cast<int32_t *>(tr + off);
-  for (int i = 0; i < la; i++) q[i] = prng_next(gs) % qmod;
-  st->prng = gs;
+  for (int i = lane; i < la; i += 32) q[i] = d[i] % qmod;
+  __syncwarp();
+  prng_warp_store(st->prng, x, f0, la, lane);
 }
 
 int ilog2i(uint64_t x) { return ilog2(x); }

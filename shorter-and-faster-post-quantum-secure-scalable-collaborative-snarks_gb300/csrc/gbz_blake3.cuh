@@ -198,6 +198,30 @@ __device__ __forceinline__ void prng_warp_store(glibc_prng &g, uint32_t x, int f
     g.r = (f + 28) % 31;
   }
 }
+// The next n outputs into d (shared memory), by a warp from its state x; the
+// state after them.
+__device__ __forceinline__ uint32_t prng_warp_draw(uint32_t x, int32_t *d, int n, int lane) {
+  int i = 0;
+#pragma unroll 1
+  for (; i + 31 <= n; i += 31) {
+    x = prng_warp_next(x, lane);
+    if (lane < 31) d[i + lane] = (int32_t)(x >> 1);
+  }
+  if (i < n) {
+    const uint32_t y = prng_warp_next(x, lane);
+    if (lane < n - i) d[i + lane] = (int32_t)(y >> 1);
+    x = prng_warp_shift(x, y, n - i, lane);
+  }
+  __syncwarp();
+  return x;
+}
+constexpr int kFieldDraws = 40;  // outputs behind one F::_random() (two 20-digit numbers)
+// F::_random (fieldElement.cpp:119-125) from 40 outputs, by a warp.
+__device__ __forceinline__ fe prng_warp_field(const int32_t *d, int lane) {
+  uint64_t v = 0;
+  if (lane < 2) v = prng_number_from(d + 20 * lane) % P;
+  return fe_make(__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, 1));
+}
 // srandom(seed): entry i of the fill is 16807^i seed mod 2^31 - 1 (the first
 // is the seed itself), then 310 = 10 * 31 outputs are discarded.
 __device__ __forceinline__ void prng_warp_seed(glibc_prng &g, uint32_t seed, int lane) {

@@ -298,15 +298,32 @@ GBZ_HD fe fpow(fe x, uint64_t e) {
   return r;
 }
 
-// inv (fieldElement.cpp:207-210): x^(p^2 - 2).  The exponent needs 122
-// bits, so it is split as e = hi * 2^64 + lo and x^e = (x^(2^64))^hi * x^lo.
+// inv (fieldElement.cpp:207-210), 0 for 0: 1 / x = conj(x) / (re^2 + im^2), the
+// norm (zero for x = 0 only, p = 3 mod 4) inverted as N^(p - 2), p - 2 =
+// 2^61 - 3: N^(2^k - 1) up to k = 59, then N^(4 (2^59 - 1) + 1).  70 products
+// in the base field where x^(p^2 - 2) took 300 in the extension (2 us instead
+// of 20 on one thread).
+GBZ_HD uint64_t mulp_red(uint64_t a, uint64_t b) { return redp(mulp_lazy(a, b)); }
 GBZ_HD fe finv(fe x) {
-  // p^2 - 2 = 2^122 - 2^62 - 1 ; hi = 2^58 - 1, lo = 2^64 - 2^62 - 1
-  const uint64_t lo = 0xBFFFFFFFFFFFFFFFull;
-  const uint64_t hi = 0x03FFFFFFFFFFFFFFull;
-  fe x64 = x;
-  for (int i = 0; i < 64; i++) x64 = fmul(x64, x64);  // x^(2^64)
-  return fmul(fpow(x64, hi), fpow(x, lo));
+  const uint64_t n = addp(mulp_red(x.re, x.re), mulp_red(x.im, x.im));
+  uint64_t r = n;  // n^(2^k - 1)
+  int k = 1;
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+  for (int bit = 4; bit >= 0; bit--) {  // 59 = 111011 in binary
+    uint64_t t = r;
+    for (int q = 0; q < k; q++) t = mulp_red(t, t);
+    r = mulp_red(t, r);
+    k *= 2;
+    if ((59 >> bit) & 1) {
+      r = mulp_red(mulp_red(r, r), n);
+      k++;
+    }
+  }
+  r = mulp_red(r, r);
+  r = mulp_red(mulp_red(r, r), n);
+  return fe_make(mulp_red(x.re, r), mulp_red(x.im ? P - x.im : 0, r));
 }
 
 // getRootOfUnity (utils.cpp:706-717): generator of order 2^61 squared

@@ -286,30 +286,6 @@ __global__ void k_indexes(PcsDev *st, int l, int N, uint32_t Mq, int32_t *qp, in
   }
 }
 
-// 1 / x = conj(x) / (re^2 + im^2) for x != 0 (the norm vanishes for x = 0
-// only, p = 3 mod 4), the norm inverted as N^(p - 2), p - 2 = 2^61 - 3:
-// x_k = N^(2^k - 1) up to k = 59, then N^(4 (2^59 - 1) + 1).
-__device__ __forceinline__ uint64_t mulp1(uint64_t a, uint64_t b) { return redp(mulp_lazy(a, b)); }
-__device__ fe inverse_dev(fe x) {
-  const uint64_t n = addp(mulp1(x.re, x.re), mulp1(x.im, x.im));
-  uint64_t r = n;  // n^(2^k - 1)
-  int k = 1;
-#pragma unroll 1
-  for (int bit = 4; bit >= 0; bit--) {  // 59 = 111011 in binary
-    uint64_t t = r;
-    for (int q = 0; q < k; q++) t = mulp1(t, t);
-    r = mulp1(t, r);
-    k *= 2;
-    if ((59 >> bit) & 1) {
-      r = mulp1(mulp1(r, r), n);
-      k++;
-    }
-  }
-  r = mulp1(r, r);
-  r = mulp1(mulp1(r, r), n);
-  return fe_make(mulp1(x.re, r), mulp1(x.im ? P - x.im : 0, r));
-}
-
 // The Lagrange weights at c over the D = 2^logD points w^k and over the d =
 // D >> ext points w^(k << ext) (compute_lagrange_coeff, utils.cpp:169-197: the
 // inverse transform of the powers of c), and the value of the polynomial with
@@ -330,7 +306,7 @@ __device__ fe lagrange_dev(fe c, int logD, int ext, const fe *wp, const fe *poly
   for (int k = threadIdx.x; k < D; k += 256) {
     const fe den = fsub(fmul(c, wp[k]), fe_one());
     const bool hit = !(den.re | den.im);
-    const fe inv = inverse_dev(den);
+    const fe inv = finv(den);
     const fe l = hit ? fe_one() : fmul(cD, inv);
     if (LD) LD[k] = l;
     facc_mul(acc, poly[k], l);
@@ -434,7 +410,7 @@ __global__ void __launch_bounds__(256)
 k_s_update(PcsDev *st, const fe *y, int l, int addK, uint8_t *tr, uint64_t off_s, uint64_t off_K) {
   pdl_wait();
   __shared__ fe sh_s;
-  __shared__ fe red[256];
+  __shared__ fe red[8];
   if (threadIdx.x == 0) {
     sh_s = hash_F(st->fs, fe_zero());
     st->fs = sh_s;
@@ -445,11 +421,14 @@ k_s_update(PcsDev *st, const fe *y, int l, int addK, uint8_t *tr, uint64_t off_s
   fe acc = fe_zero();
   if (addK)
     for (int j = threadIdx.x; j < l; j += blockDim.x) acc = fadd(acc, fmul(fpow(s, (uint64_t)j + 1), y[j]));
-  red[threadIdx.x] = acc;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1)
+    acc = fadd(acc, fe_make(__shfl_xor_sync(0xffffffffu, acc.re, d), __shfl_xor_sync(0xffffffffu, acc.im, d)));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();
   if (threadIdx.x) return;
   fe K = st->K;
-  for (int t = 0; t < (int)blockDim.x; t++) K = fadd(K, red[t]);
+  for (int t = 0; t < (int)blockDim.x / 32; t++) K = fadd(K, red[t]);
   st->K = K;
   put_fe(tr, off_s, s);
   put_fe(tr, off_K, K);
@@ -476,16 +455,22 @@ __global__ void k_phase3_prep(const PcsDev *st, const int32_t *qp, const int32_t
 // V (N x W, zero) gets V[p][q_i] = sum of w[p][j] over the queries j at q_i.
 __global__ void k_phase3_scatter(const uint32_t *q, const fe *w, int l, uint64_t W, fe *V) {
   pdl_wait();
+  __shared__ uint32_t sq[kPcsMaxQueries];
+  for (int j = threadIdx.x; j < l; j += blockDim.x) sq[j] = q[j];
+  __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= l) return;
   const uint64_t p = blockIdx.y;
-  const uint32_t qi = q[i];
-  for (int j = 0; j < i; j++)
-    if (q[j] == qi) return;
+  const uint32_t qi = sq[i];
+  bool first = true;
+#pragma unroll 8
+  for (int j = 0; j < i; j++) first = first && sq[j] != qi;
+  if (!first) return;
   const fe *wp = w + p * l;
   fe acc = wp[i];
+#pragma unroll 8
   for (int j = i + 1; j < l; j++)
-    if (q[j] == qi) acc = fadd(acc, wp[j]);
+    if (sq[j] == qi) acc = fadd(acc, wp[j]);
   V[p * W + qi] = acc;
 }
 

@@ -72,32 +72,51 @@ __device__ fe block_sum_fe(fe v) {
 }
 
 // ---- the generator ---------------------------------------------------------
-// The tail's draws in the reference's order, one thread: F::_random()
+// The tail's draws in the reference's order, one warp: F::_random()
 // (fieldElement.cpp:119-125) into the arena, rand() % mod (coPCS.cpp:789,
 // Whir.cpp:574-576) into the transcript, the state the WHIR opening starts
 // from into st->prng, the calls the opening makes itself skipped (their
-// end state into after_walk), and the final state.
-__global__ void k_draw_script(glibc_prng g0, const DrawOp *ops, int nops, fe *arena, uint8_t *tr, ProofState *st,
-                              glibc_prng *after_walk, glibc_prng *final_state) {
+// end state into after_walk), and the final state.  31 elements of 40 outputs
+// at a time, a lane an element: one thread took 1650 us for an opening of 8 x
+// 2^16, this 90.
+__global__ void __launch_bounds__(32)
+k_draw_script(glibc_prng g0, const DrawOp *ops, int nops, fe *arena, uint8_t *tr, ProofState *st,
+              glibc_prng *after_walk, glibc_prng *final_state) {
   pdl_wait();
-  __shared__ glibc_prng g;  // dynamically indexed table: work on a shared copy
-  if (threadIdx.x) return;
-  g = g0;
+  constexpr int kChunk = 31 * kFieldDraws;
+  __shared__ int32_t d[kChunk];
+  const int lane = threadIdx.x, f0 = g0.f;
+  uint32_t x = lane < 31 ? (uint32_t)g0.tbl[(f0 + lane) % 31] : 0u;
+  uint64_t n = 0;
   for (int k = 0; k < nops; k++) {
     const DrawOp o = ops[k];
     if (o.kind == DRAW_FIELDS) {
-      for (int i = 0; i < o.count; i++) arena[o.off + i] = prng_field(g);
+      for (int i = 0; i < o.count; i += 31) {
+        const int c = min(31, o.count - i);
+        x = prng_warp_draw(x, d, c * kFieldDraws, lane);
+        const int32_t *e = d + kFieldDraws * lane;
+        if (lane < c) arena[o.off + i + lane] = fe_make(prng_number_from(e) % P, prng_number_from(e + 20) % P);
+        __syncwarp();
+      }
+      n += (uint64_t)kFieldDraws * o.count;
     } else if (o.kind == DRAW_INTS) {
       uint32_t *q = reinterpret_cast<uint32_t *>(tr + o.off);
-      for (int i = 0; i < o.count; i++) q[i] = (uint32_t)(prng_next(g) % (int32_t)o.mod);
+      for (int i = 0; i < o.count; i += kChunk) {
+        const int c = min(kChunk, o.count - i);
+        x = prng_warp_draw(x, d, c, lane);
+        for (int j = lane; j < c; j += 32) q[i + j] = (uint32_t)(d[j] % (int32_t)o.mod);
+        __syncwarp();
+      }
+      n += o.count;
     } else if (o.kind == DRAW_STATE) {
-      st->prng = g;
+      prng_warp_store(st->prng, x, f0, n, lane);
     } else {
-      for (int i = 0; i < o.count; i++) (void)prng_next(g);
-      *after_walk = g;
+      for (int i = 0; i < o.count; i += kChunk) x = prng_warp_draw(x, d, min(kChunk, o.count - i), lane);
+      n += o.count;
+      prng_warp_store(*after_walk, x, f0, n, lane);
     }
   }
-  *final_state = g;
+  prng_warp_store(*final_state, x, f0, n, lane);
 }
 
 // The WHIR opening drew as many values as the script skipped for it.
@@ -429,7 +448,8 @@ __global__ void k_reencode_check(const fe *arr, int m, const fe *cw, uint64_t L,
 
 struct Step3Args {
   int iters, nr;                       // iterations; entries of total_r
-  uint64_t off_q[kMaxTailIter], off_c[kMaxTailIter], NL[kMaxTailIter];
+  uint64_t off_q[kMaxTailIter], off_c[kMaxTailIter];
+  fe om[kMaxTailIter];                 // omega_NL of the iterations
   int l[kMaxTailIter], skip[kMaxTailIter];  // queries; total_r entries erased before iteration i's identities
   int R, npt;                          // claims and their point length
   uint64_t off_eval, off_claim;
@@ -444,7 +464,7 @@ __global__ void k_whir_step3(const uint8_t *tr, Step3Args a, const fe *claims, c
   pdl_wait();
   fe acc = fe_zero();
   for (int it = 0; it < a.iters; it++) {
-    const fe om = root_of_unity(ilog2_dev(a.NL[it]));
+    const fe om = a.om[it];
     for (int j = threadIdx.x; j < a.l[it]; j += kT) {
       const uint32_t q = reinterpret_cast<const uint32_t *>(tr + a.off_q[it])[j];
       fe w = fpow(om, 2ull * q), e = fe_one();
@@ -482,8 +502,7 @@ struct FinalRound {
   int nL;                       // Lagrange vectors of the later rounds
   const fe *L[8];
   int d[8];
-  uint64_t rows;                // instance_size[i]
-  int rate;                     // _rates[i][0]
+  fe om;                        // omega of _rates[i][0] instance_size[i]
 };
 struct FinalArgs {
   int nq, N;
@@ -493,30 +512,21 @@ struct FinalArgs {
 };
 
 // fast_eval_powers_y (New_PCS.cpp:582-605) per party p < N, at r_c: the
-// inverse transform of length N/2 of the powers of omega_{2N}^(2p+1),
-// evaluated as a polynomial in r_c.
-__global__ void k_powers_y(int N, const fe *rcp, fe *py) {
+// inverse transform of length h = N/2 of the powers of w1 = omega_{2N}^(2p+1),
+// evaluated as a polynomial in r_c.  Coefficient k is a geometric sum,
+// (w1^h - 1) / (h (w1 omega_h^-k - 1)) (w1 is no h-th root of unity); one warp
+// a party, a lane a coefficient.  (As sums in one thread a party, with the
+// roots and their inverses: 50 us at 8 parties, now 6.7.)
+__global__ void __launch_bounds__(32) k_powers_y(int h, const fe *rcp, fe w2n, fe winv, fe hinv, fe *py) {
   pdl_wait();
-  const int p = threadIdx.x;
-  if (p >= N) return;
-  const fe rc = *rcp;
-  const int h = N / 2, lh = ilog2_dev((uint64_t)h);
-  const fe w1 = fpow(root_of_unity(1 + ilog2_dev((uint64_t)N)), 2ull * p + 1);
-  const fe winv = finv(root_of_unity(lh)), hinv = finv(fe_make((uint64_t)h, 0));
-  fe acc = fe_zero(), rk = fe_one();
-  for (int k = 0; k < h; k++) {
-    fe c = fe_zero();
-    const fe wk = fpow(winv, (uint64_t)k);
-    fe x = fe_one(), wi = fe_one();
-    for (int i = 0; i < h; i++) {
-      c = fadd(c, fmul(x, wi));
-      x = fmul(x, w1);
-      wi = fmul(wi, wk);
-    }
-    acc = fadd(acc, fmul(rk, fmul(c, hinv)));
-    rk = fmul(rk, rc);
-  }
-  py[p] = acc;
+  const int k = threadIdx.x;
+  const fe w1 = fpow(w2n, 2ull * blockIdx.x + 1), num = fmul(fsub(fpow(w1, (uint64_t)h), fe_one()), hinv);
+  const fe den = fsub(fmul(w1, fpow(winv, (uint64_t)k)), fe_one());
+  fe x = k < h ? fmul(fmul(num, finv(den)), fpow(*rcp, (uint64_t)k)) : fe_zero();
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1)
+    x = fadd(x, fe_make(__shfl_xor_sync(0xffffffffu, x.re, d), __shfl_xor_sync(0xffffffffu, x.im, d)));
+  if (k == 0) py[blockIdx.x] = x;
 }
 
 // The partial evaluations of the queries of the rounds before the last
@@ -532,7 +542,7 @@ __global__ void k_final_terms(FinalArgs a, const fe *py, fe *terms) {
   if (r >= a.nq) return;
   const FinalRound &q = a.q[r];
   const uint64_t pos = (uint64_t)(uint32_t)q.qpos[t] * (uint64_t)q.mul / (uint64_t)q.div;
-  fe om = fpow(root_of_unity(ilog2_dev((uint64_t)q.rate * q.rows)), pos), fx = fe_one();
+  fe om = fpow(q.om, pos), fx = fe_one();
   for (int k = 0; k < q.nL; k++) {
     if (k) om = fpow(om, (uint64_t)q.d[k - 1]);
     fe sum = fe_zero(), x = fpow(om, (uint64_t)lane);
@@ -1167,7 +1177,7 @@ struct Tail {
           skip += ilog2((uint64_t)wt.kappa[i]);
           a3.off_q[i] = wt.queries[i];
           a3.off_c[i] = wt.comb[i];
-          a3.NL[i] = wt.NL[i];
+          a3.om[i] = root_of_unity(ilog2(wt.NL[i]));
           a3.l[i] = wt.l[i];
           a3.skip[i] = skip;
         }
@@ -1222,8 +1232,7 @@ struct Tail {
           f.L[k] = in.rounds[j + 1 + k].L;
           f.d[k] = in.rounds[j + 1 + k].d;
         }
-        f.rows = rows;
-        f.rate = in.rate0[j + 2];
+        f.om = root_of_unity(ilog2((uint64_t)in.rate0[j + 2] * rows));
       }
       fa.fB = fB;
       fa.b3 = in.b3;
@@ -1234,7 +1243,9 @@ struct Tail {
       int nterms = 0;
       for (int j = 0; j < fa.nq; j++) nterms += fa.q[j].l;
       fe *py = alloc<fe>(64), *terms = alloc<fe>(std::max(nterms, 1));
-      launch_kernel(k_powers_y, 1, 64, 0, s, N, rc, py);
+      const int h = N / 2;
+      launch_kernel(k_powers_y, N, 32, 0, s, h, rc, root_of_unity(ilog2(2ull * N)),
+                    finv(root_of_unity(ilog2((uint64_t)h))), finv(fe_make((uint64_t)h, 0)), py);
       if (nterms) launch_kernel(k_final_terms, nblk((uint64_t)nterms * 32), kT, 0, s, fa, py, terms);
       launch_kernel(k_final_eval, 1, kT, 0, s, fa, terms, nterms, flags, tr);
       check();

@@ -318,7 +318,6 @@ struct SchedArgs {
   int32_t qmod[kMaxWhirIter];       // codeword length / 4 per iteration
   int lg_final;                     // log2 of the final polynomial's length
 };
-constexpr int kFieldDraws = 40;     // random() outputs behind one F::_random() (two 20-digit numbers)
 constexpr int kMaxDraws = kMaxWhirIter * (3 * kFieldDraws + kMaxQueries) + 8 * kFieldDraws;
 
 // The first warp runs the generator and stores the N outputs in shared
@@ -327,22 +326,13 @@ constexpr int kMaxDraws = kMaxWhirIter * (3 * kFieldDraws + kMaxQueries) + 8 * k
 // drawing and three deriving a launch took 17.5 us at 2^10, now 12.
 __global__ void __launch_bounds__(256) k_whir_schedule(ProofState *st, SchedArgs a) {
   pdl_wait();
-  __shared__ int32_t draws[kMaxDraws + 31];
+  __shared__ int32_t draws[kMaxDraws];
   st += blockIdx.x;
   int N = kFieldDraws * a.lg_final;
   for (int t = 0; t < a.T; t++) N += 3 * kFieldDraws + a.l[t];
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x, f0 = st->prng.f;
-    uint32_t x = prng_warp_load(st->prng, lane);
-    int n = 0;
-    for (; n + 31 <= N; n += 31) {
-      x = prng_warp_next(x, lane);
-      if (lane < 31) draws[n + lane] = (int32_t)(x >> 1);
-    }
-    const uint32_t y = prng_warp_next(x, lane);
-    if (lane < N - n) draws[n + lane] = (int32_t)(y >> 1);
-    x = prng_warp_shift(x, y, N - n, lane);
-    __syncwarp();
+    const uint32_t x = prng_warp_draw(prng_warp_load(st->prng, lane), draws, N, lane);
     prng_warp_store(st->prng, x, f0, N, lane);
   }
   __syncthreads();
@@ -412,6 +402,17 @@ __global__ void __launch_bounds__(128) k_ub_prep(const ProofState *st, UbSlots *
 __global__ void k_whir_round(const fe *partial, int blocks, ProofState *st, int i, uint8_t *tr,
                              uint64_t off_poly, uint64_t off_chal) {
   pdl_wait();
+  __shared__ int32_t draws[kFieldDraws];
+  __shared__ fe drawn;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x / 32 == 1) {  // the challenge, beside the sums (one thread drew for 5 of 9 us)
+    const int f0 = st->prng.f;
+    const uint32_t x = prng_warp_draw(prng_warp_load(st->prng, lane), draws, kFieldDraws, lane);
+    const fe c = prng_warp_field(draws, lane);
+    __syncwarp();
+    prng_warp_store(st->prng, x, f0, kFieldDraws, lane);
+    if (lane == 0) drawn = c;
+  }
   fe H[3];
   sum_partials(partial, blocks, H);
   if (threadIdx.x) return;
@@ -421,10 +422,7 @@ __global__ void k_whir_round(const fe *partial, int blocks, ProofState *st, int 
     put_fe(tr, off_poly + 16 * k, H[k]);
     st->hw[i][k] = H[k];
   }
-  __shared__ glibc_prng g;
-  g = st->prng;
-  fe r = prng_field(g);
-  st->prng = g;
+  const fe r = drawn;
   st->rw[i] = r;
   put_fe(tr, off_chal, r);
   st->K = quad_eval(H[0], H[1], H[2], r);
