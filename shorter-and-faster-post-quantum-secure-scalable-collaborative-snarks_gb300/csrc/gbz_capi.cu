@@ -807,19 +807,18 @@ gbz_status gbz_cosumcheck_phase1(gbz_ctx *ctx, const uint64_t *p1, const uint64_
   for (int v = 0; v < nv; v++) {  // ext(v) per block: inverse of length d, forward of length D
     dsrc[v] = dev_view(ctx, 11 + v, src[v], 16 * n, mem, true);
     ex[v] = (fe *)ctx->buf(20 + v, 16 * nblocks * D);
-    ntt_batched(td, dsrc[v], d, (uint32_t)d, coef, nblocks, true, ctx->stream);
-    ntt_batched(tD, coef, d, (uint32_t)d, ex[v], nblocks, false, ctx->stream);
   }
   uint8_t *flags = nullptr;
   if (cubic) {  // blocks whose p1 part is all zero are skipped (coSumcheck.cpp:21-27)
     flags = (uint8_t *)ctx->buf(30, nblocks);
     nonzero_blocks_launch(dsrc[0], nblocks, logd, flags, ctx->stream);
   }
-  const int lanes = D >= 256 ? 1 : (int)(256 / D);
-  const int per_cta = (int)std::max<uint64_t>((uint64_t)lanes, (nblocks + 607) / 608);
-  fe *partial = (fe *)ctx->buf(31, 16 * D * cophase1_parts(nblocks, per_cta));
+  fe *partial = (fe *)ctx->buf(31, 16 * cophase1_partials(nblocks, logD));
   fe *dH = (fe *)ctx->buf(32, 16 * D);
-  cophase1_reduce_launch(ex[0], ex[1], ex[2], ex[3], flags, nblocks, logD, per_cta, partial, dH, ctx->stream);
+  CoVectors cv;
+  cv.nv = nv;
+  for (int v = 0; v < nv; v++) cv.v[v] = dsrc[v];
+  cophase1_launch(td, tD, cv, n, logd, ext, flags, 1, ex, coef, partial, dH, ctx->stream);
   GBZ_CUDA(cudaMemcpyAsync(H, dH, 16 * D, cudaMemcpyDeviceToHost, ctx->stream));
   GBZ_CUDA(cudaStreamSynchronize(ctx->stream));
   API_END(ctx)

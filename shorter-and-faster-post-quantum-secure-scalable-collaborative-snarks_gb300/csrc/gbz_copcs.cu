@@ -192,51 +192,61 @@ __global__ void __launch_bounds__(1024) lambda_kernel(const fe *b, int N, int lo
 }
 
 // flags[blk] = 1 when block blk of v has a non-zero entry.
-__global__ void nonzero_blocks_kernel(const fe *v, uint64_t nblocks, int logd, uint8_t *flags) {
+__global__ void __launch_bounds__(256)
+nonzero_blocks_kernel(const fe *v, uint64_t nblocks, int logd, uint8_t *flags) {
   pdl_wait();
-  const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nblocks) return;
-  const fe *p = v + (b << logd);
-  uint8_t nz = 0;
-  for (uint32_t k = 0; k < (1u << logd); k++) nz |= (p[k].re | p[k].im) ? 1 : 0;
-  flags[b] = nz;
+  // a warp's lanes read neighbouring entries: 2^min(logd, 5) of them a block
+  const int logg = logd < 5 ? logd : 5;
+  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, b = t >> logg;
+  uint64_t any = 0;
+  if (b < nblocks)
+    for (uint32_t k = (uint32_t)t & ((1u << logg) - 1); k < (1u << logd); k += 1u << logg) {
+      const fe x = v[(b << logd) + k];
+      any |= x.re | x.im;
+    }
+  const uint32_t votes = __ballot_sync(0xffffffffu, any != 0);
+  const uint32_t lane = threadIdx.x & 31, group = logg == 5 ? ~0u : ((1u << (1 << logg)) - 1) << (lane >> logg << logg);
+  if (b < nblocks && (lane & ((1u << logg) - 1)) == 0) flags[b] = (votes & group) ? 1 : 0;
 }
 
 // Per-CTA partial sums of the extended-block products:
 // quadratic: e1 * e2; cubic: (e1 * e2 - e4) * e3 over blocks with flags set.
-// blockIdx.y selects a chunk of Dc = min(D, 256) positions k; within the
-// CTA k = chunk * Dc + tid % Dc and lane = tid / Dc walks the blocks.
+// blockIdx.y selects a chunk of Dc = min(D, 256) positions; within the CTA
+// lane = tid / Dc walks the blocks.  Position s d + k stands for point
+// k 2^ext + s where the blocks come in cosets (split), else for its own.
 __global__ void __launch_bounds__(256)
-cophase1_partial_kernel(const fe *e1, const fe *e2, const fe *e3, const fe *e4, const uint8_t *flags,
-                        uint64_t nblocks, int logD, int blocks_per_cta, fe *partial) {
+cophase1_partial_kernel(CoVectors a, const uint8_t *flags, uint64_t nblocks, int logd, int ext, int split,
+                        int blocks_per_cta, fe *partial) {
   pdl_wait();
   __shared__ fe red[256];
   // grid.z: the party; its blocks and partials follow the previous party's
-  const uint64_t pe = (uint64_t)blockIdx.z * (nblocks << logD);
-  e1 += pe;
-  e2 += pe;
-  if (e3) e3 += pe;
-  if (e4) e4 += pe;
   if (flags) flags += (uint64_t)blockIdx.z * nblocks;
+  const int logD = logd + ext, logDc = logD < 8 ? logD : 8, sh = split ? logd : logD;
   partial += (uint64_t)blockIdx.z * ((uint64_t)gridDim.x << logD);
-  const int logDc = logD < 8 ? logD : 8;
   const uint32_t Dc = 1u << logDc, lane = threadIdx.x >> logDc, lanes = 256u >> logDc;
-  const uint32_t k = blockIdx.y * Dc + (threadIdx.x & (Dc - 1));
+  const uint32_t at = blockIdx.y * Dc + (threadIdx.x & (Dc - 1)), cs = at >> logd, k = at & ((1u << logd) - 1);
+  const fe *e[4];
+#pragma unroll
+  for (int v = 0; v < 4; v++) {
+    const uint64_t party = a.shared[v] ? 0 : blockIdx.z, total = (nblocks << logd) * (a.shared[v] ? 1 : gridDim.z);
+    if (!split) e[v] = a.o[v] + party * (nblocks << logD) + at;
+    else e[v] = (cs ? a.o[v] + (cs - 1) * total : a.v[v]) + party * (nblocks << logd) + k;
+  }
   const uint64_t b0 = (uint64_t)blockIdx.x * blocks_per_cta;
   const uint64_t b1 = min(b0 + blocks_per_cta, nblocks);
   facc sum = facc_zero();
   for (uint64_t b = b0 + lane; b < b1; b += lanes) {
     if (flags && !flags[b]) continue;
-    const uint64_t at = (b << logD) + k;
-    if (e3) facc_mul(sum, fsub(fmul(e1[at], e2[at]), e4[at]), e3[at]);
-    else facc_mul(sum, e1[at], e2[at]);
+    const uint64_t i = b << sh;
+    if (a.nv == 4) facc_mul(sum, fsub(fmul(e[0][i], e[1][i]), e[3][i]), e[2][i]);
+    else facc_mul(sum, e[0][i], e[1][i]);
   }
   fe acc = facc_value(sum);
   red[threadIdx.x] = acc;
   __syncthreads();
   if (lane == 0) {
     for (uint32_t l = 1; l < lanes; l++) acc = fadd(acc, red[threadIdx.x + (l << logDc)]);
-    partial[((uint64_t)blockIdx.x << logD) + k] = acc;
+    partial[((uint64_t)blockIdx.x << logD) + (split ? (k << ext) + cs : at)] = acc;
   }
 }
 
@@ -440,23 +450,50 @@ void aggregate_launch(const fe *msgs, int N, uint64_t len, const fe *lambda, fe 
 }
 
 void nonzero_blocks_launch(const fe *v, uint64_t nblocks, int logd, uint8_t *flags, cudaStream_t s) {
-  launch_kernel(nonzero_blocks_kernel, grid(nblocks), 256, 0, s, v, nblocks, logd, flags);
+  launch_kernel(nonzero_blocks_kernel, grid(nblocks << (logd < 5 ? logd : 5)), 256, 0, s, v, nblocks, logd, flags);
   GBZ_CUDA(cudaGetLastError());
 }
 
-uint64_t cophase1_parts(uint64_t nblocks, int blocks_per_cta) {
-  return (nblocks + blocks_per_cta - 1) / blocks_per_cta;
+static int cophase1_per_cta(uint64_t nblocks, int logD) {
+  const uint64_t lanes = logD >= 8 ? 1 : 1ull << (8 - logD);
+  return (int)std::max<uint64_t>(lanes, (nblocks + 607) / 608);
+}
+uint64_t cophase1_partials(uint64_t nblocks, int logD) {
+  const int per = cophase1_per_cta(nblocks, logD);
+  return ((nblocks + per - 1) / per) << logD;
 }
 
-void cophase1_reduce_launch(const fe *e1, const fe *e2, const fe *e3, const fe *e4, const uint8_t *flags,
-                            uint64_t nblocks, int logD, int blocks_per_cta, fe *partial, fe *H, cudaStream_t s,
-                            int parties) {
+void cophase1_launch(const NttTables &td, const NttTables &tD, CoVectors a, uint64_t n, int logd, int ext,
+                     const uint8_t *flags, int parties, fe *const *ex, fe *coef, fe *partial, fe *H, cudaStream_t s) {
+  const int logD = logd + ext;
   if (logD > kMaxCoLogD) throw ArgError("coSumcheck: extended block longer than 2^13");
   if (parties < 1 || parties > 65535) throw ArgError("coSumcheck: 1..65535 parties per launch");
-  const uint64_t parts = cophase1_parts(nblocks, blocks_per_cta);
+  const uint64_t nblocks = n >> logd;
+  // the new points alone where every vector's length allows it; a vector all
+  // parties share is extended once
+  bool split = true;
+  for (int v = 0; v < a.nv; v++) split = split && coset_extend_fits(a.shared[v] ? n : n * parties, logd, ext);
+  if (split) coset_extend_factors_launch(td, tD, ext, partial, s);
+  for (int v = 0; v < 4; v++) {
+    a.o[v] = ex[v < a.nv ? v : 0];
+    if (v >= a.nv) {
+      a.v[v] = a.v[0];
+      a.shared[v] = a.shared[0];
+      continue;
+    }
+    const uint64_t total = a.shared[v] ? n : n * parties;
+    if (split) {
+      coset_extend_launch(td, a.v[v], total, ext, partial, ex[v], s);
+    } else {
+      ntt_batched(td, a.v[v], 1ull << logd, 1u << logd, coef, total >> logd, true, s);
+      ntt_batched(tD, coef, 1ull << logd, 1u << logd, ex[v], total >> logd, false, s);
+    }
+  }
+  const int per = cophase1_per_cta(nblocks, logD);
+  const uint64_t parts = (nblocks + per - 1) / per;
   const unsigned chunks = logD > 8 ? 1u << (logD - 8) : 1u;
-  launch_kernel(cophase1_partial_kernel, dim3((unsigned)parts, chunks, (unsigned)parties), 256, 0, s, e1, e2, e3, e4,
-                flags, nblocks, logD, blocks_per_cta, partial);
+  launch_kernel(cophase1_partial_kernel, dim3((unsigned)parts, chunks, (unsigned)parties), 256, 0, s, a, flags,
+                nblocks, logd, ext, split ? 1 : 0, per, partial);
   GBZ_CUDA(cudaGetLastError());
   launch_kernel(sum_partials_kernel, dim3(grid(1ull << logD, 8), (unsigned)parties), 256, 0, s, partial, parts,
                 1u << logD, H);

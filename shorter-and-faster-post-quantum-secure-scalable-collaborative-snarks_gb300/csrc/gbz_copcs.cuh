@@ -39,13 +39,23 @@ void aggregate_weights_launch(const fe *b, int N, fe *lambda, cudaStream_t s);
 // batched transform per block).
 constexpr int kMaxCoLogD = 13;
 void nonzero_blocks_launch(const fe *v, uint64_t nblocks, int logd, uint8_t *flags, cudaStream_t s);
-uint64_t cophase1_parts(uint64_t nblocks, int blocks_per_cta);
-// parties > 1: that many parties one after the other in every array (e*:
-// nblocks << logD entries each, flags: nblocks, partial:
-// cophase1_parts(nblocks, blocks_per_cta) << logD, H: 1 << logD).
-void cophase1_reduce_launch(const fe *e1, const fe *e2, const fe *e3, const fe *e4, const uint8_t *flags,
-                            uint64_t nblocks, int logD, int blocks_per_cta, fe *partial, fe *H, cudaStream_t s,
-                            int parties = 1);
+// The vectors of phase 1: two (their product), or four ((v0 v1 - v3) v2), of n
+// entries a party, party-major, or of one copy that all parties share.  o is
+// set by cophase1_launch.
+struct CoVectors {
+  int nv = 0;
+  const fe *v[4] = {nullptr, nullptr, nullptr, nullptr};
+  bool shared[4] = {false, false, false, false};
+  const fe *o[4] = {nullptr, nullptr, nullptr, nullptr};
+};
+// Phase 1 (coSumcheck.cpp:9-46, 150-179): every block of 2^logd entries
+// extended to 2^(logd + ext) points, and the sums of the products over a
+// party's blocks (those with flags set) into H, 2^(logd + ext) a party.  ex[v]:
+// the vector's entries << ext; coef: parties n; partial: parties
+// cophase1_partials(n >> logd, logd + ext).
+uint64_t cophase1_partials(uint64_t nblocks, int logD);
+void cophase1_launch(const NttTables &td, const NttTables &tD, CoVectors a, uint64_t n, int logd, int ext,
+                     const uint8_t *flags, int parties, fe *const *ex, fe *coef, fe *partial, fe *H, cudaStream_t s);
 // coSumcheck phase 2 (coSumcheck.cpp:66-148, 201-213).
 void cophase2_launch(const fe *v, uint64_t n, const fe *L, int logd, fe *out, cudaStream_t s);
 

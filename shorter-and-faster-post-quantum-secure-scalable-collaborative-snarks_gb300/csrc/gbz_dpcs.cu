@@ -548,14 +548,12 @@ gbz_status gbz_dpcs_open(gbz_ctx *ctx, int N, int P, int rows, uint64_t S, int r
     const uint64_t blocks = (uint64_t)N * n / d, pblocks = n / d;
     const NttTables &td = ctx->tables(logd), &tD = ctx->tables(logd + 1);
     fe *e1 = ob.alloc<fe>(blocks * Dd), *e2 = ob.alloc<fe>(blocks * Dd);
-    ntt_batched(td, arr, d, (uint32_t)d, tmpv, blocks, true, s);
-    ntt_batched(tD, tmpv, d, (uint32_t)d, e1, blocks, false, s);
-    ntt_batched(td, bet, d, (uint32_t)d, tmpv, blocks, true, s);
-    ntt_batched(tD, tmpv, d, (uint32_t)d, e2, blocks, false, s);
-    const int lanes = Dd >= 256 ? 1 : 256 / Dd;
-    const int per_cta = (int)std::max<uint64_t>((uint64_t)lanes, (pblocks + 607) / 608);
-    fe *cpart = ob.alloc<fe>((uint64_t)N * Dd * cophase1_parts(pblocks, per_cta));
-    cophase1_reduce_launch(e1, e2, nullptr, nullptr, nullptr, pblocks, logd + 1, per_cta, cpart, H, s, N);
+    fe *cpart = ob.alloc<fe>((uint64_t)N * cophase1_partials(pblocks, logd + 1)), *ex[4] = {e1, e2, nullptr, nullptr};
+    CoVectors cv;
+    cv.nv = 2;
+    cv.v[0] = arr;
+    cv.v[1] = bet;
+    cophase1_launch(td, tD, cv, n, logd, 1, nullptr, N, ex, tmpv, cpart, H, s);
     aggregate_launch(H, N, Dd, ones, poly, s);  // aggregate_plaintext_poly_batch: the plain sum
     std::vector<fe> hp(Dd);
     GBZ_CUDA(cudaMemcpyAsync(hp.data(), poly, 16ull * Dd, cudaMemcpyDeviceToHost, s));

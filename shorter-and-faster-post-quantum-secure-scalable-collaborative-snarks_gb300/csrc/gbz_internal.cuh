@@ -185,6 +185,15 @@ void ntt_launch_rows(const NttTables &t, const fe *in, uint64_t n_valid, uint64_
 void ntt_launch_rows_scatter(const NttTables &t, const fe *in, uint64_t n_valid, uint64_t in_stride, fe *out,
                              uint64_t out_stride, int rows, fe *tmp, int log_parts, uint64_t part_stride,
                              cudaStream_t s);
+// Blocks of 2^tS.logn evaluations over their subgroup, extended to the one
+// 2^ext times as large (tL's): the evaluations at its points w^(s + k 2^ext),
+// 0 < s < 2^ext, of block b at out + (s - 1) total + (b << tS.logn) + k; total
+// entries of all blocks, a power of two.  factors: (2^ext - 1) << tS.logn
+// entries, formed by coset_extend_factors_launch.
+bool coset_extend_fits(uint64_t total, int logS, int ext);
+void coset_extend_factors_launch(const NttTables &tS, const NttTables &tL, int ext, fe *factors, cudaStream_t s);
+void coset_extend_launch(const NttTables &tS, const fe *in, uint64_t total, int ext, const fe *factors, fe *out,
+                         cudaStream_t s);
 // acc[j] += sum_i c[i] * omega_L^{q[i] j} for j < nacc (L = 2^t.logn > 2^13,
 // 1 <= l <= kMaxQueries): the forward transform of the sparse vector
 // sum_i c_i e_{q_i} as one second-pass launch whose rows are formed directly

@@ -1204,21 +1204,25 @@ CoscOut cosumcheck_run(gbz_ctx *ctx, int form, int N, uint64_t n, const fe *p1, 
     for (int i = 0; i < ndeg; i++) key += ":" + std::to_string(degrees[i]);
     ob.pool = &ctx->pools[key];
   }
-  // party-major inputs, copied: the call folds them in place as the reference does
+  // party-major inputs, read where they are when they are device memory: a
+  // round folds into buffers of its own.  b1's table is one for all parties.
   const uint64_t Rst = ro.off[ndeg];
-  fe *v1 = ob.alloc<fe>((uint64_t)N * n), *v2 = ob.alloc<fe>((uint64_t)N * n), *v3 = nullptr, *vb = nullptr;
-  fe *dR = ob.alloc<fe>((uint64_t)N * Rst);
-  GBZ_CUDA(cudaMemcpyAsync(v1, p1, 16ull * N * n, kin, s));
-  GBZ_CUDA(cudaMemcpyAsync(v2, p2, 16ull * N * n, kin, s));
+  const fe *cur[4] = {nullptr, nullptr, nullptr, nullptr};  // p1, p2, b1's table, p3
+  auto input = [&](const fe *p) -> const fe * {
+    if (kin == cudaMemcpyDeviceToDevice) return p;
+    fe *v = ob.alloc<fe>((uint64_t)N * n);
+    GBZ_CUDA(cudaMemcpyAsync(v, p, 16ull * N * n, kin, s));
+    return v;
+  };
+  fe *dR = ob.alloc<fe>((uint64_t)N * Rst), *vb = cubic ? ob.alloc<fe>(n) : nullptr;
+  cur[0] = input(p1);
+  cur[1] = input(p2);
+  cur[2] = vb;
+  if (cubic) cur[3] = input(p3);
   GBZ_CUDA(cudaMemcpyAsync(dR, R, 16ull * N * Rst, kin, s));
   // the quadratic form takes no points (r1, r2 may be null there)
   std::vector<fe> hr1(cubic ? r1 : nullptr, cubic ? r1 + nr1 : nullptr), hr2(lq, fe_zero());
   if (cubic && lq) hr2.assign(r2, r2 + lq);
-  if (cubic) {
-    v3 = ob.alloc<fe>((uint64_t)N * n);
-    vb = ob.alloc<fe>((uint64_t)N * n);
-    GBZ_CUDA(cudaMemcpyAsync(v3, p3, 16ull * N * n, kin, s));
-  }
   // b1 = precompute_beta(r1) for every party (the same vector), b2 = precompute_beta(r2)
   std::vector<fe> b2(N / 4, fe_one());
   for (int i = 0; i < N / 4; i++) {
@@ -1231,7 +1235,6 @@ CoscOut cosumcheck_run(gbz_ctx *ctx, int form, int N, uint64_t n, const fe *p1, 
   if (cubic) {
     GBZ_CUDA(cudaMemcpyAsync(dr1, hr1.data(), 16ull * nr1, cudaMemcpyHostToDevice, s));
     beta_launch(dr1, nr1, vb, s);
-    for (int p = 1; p < N; p++) GBZ_CUDA(cudaMemcpyAsync(vb + (uint64_t)p * n, vb, 16 * n, cudaMemcpyDeviceToDevice, s));
   }
   // sumcheck_aggr's weights: ones (quadratic, coSumcheck.cpp:194) or b2 (cubic)
   std::vector<fe> ones(N / 4, fe_one());
@@ -1263,6 +1266,9 @@ CoscOut cosumcheck_run(gbz_ctx *ctx, int form, int N, uint64_t n, const fe *p1, 
   fe *Ldh = ob.alloc<fe>(dsum);
   int *dlog = ob.alloc<int>(ndeg);
   GBZ_CUDA(cudaMemcpyAsync(dlog, logd.data(), 4ull * ndeg, cudaMemcpyHostToDevice, s));
+  fe *alt[2][4] = {};
+  for (int b = 0; b < 2; b++)
+    for (int v = 0; v < (cubic ? 4 : 2); v++) alt[b][v] = ob.alloc<fe>((v == 2 ? n : (uint64_t)N * n) / degrees[0]);
   m = n;
   uint64_t at = 0;
   for (int i = 0; i < ndeg; i++) {
@@ -1271,22 +1277,21 @@ CoscOut cosumcheck_run(gbz_ctx *ctx, int form, int N, uint64_t n, const fe *p1, 
     // phase 1 (coSumcheck.cpp:9-46, 150-179): extended blocks of every vector
     const NttTables &td = ctx->tables(logd[i]), &tD = ctx->tables(logd[i] + ext);
     if (logd[i] + ext > kMaxCoLogD) throw ArgError("coSumcheck: extended block longer than 2^13");
-    fe *src[4] = {v1, v2, cubic ? vb : nullptr, cubic ? v3 : nullptr};
+    CoVectors cv;
+    cv.nv = cubic ? 4 : 2;
     fe *ex[4] = {nullptr, nullptr, nullptr, nullptr};
-    for (int v = 0; v < (cubic ? 4 : 2); v++) {
-      ex[v] = ob.alloc<fe>(blocks * D);
-      ntt_batched(td, src[v], d, (uint32_t)d, coef, blocks, true, s);
-      ntt_batched(tD, coef, d, (uint32_t)d, ex[v], blocks, false, s);
+    for (int v = 0; v < cv.nv; v++) {
+      cv.v[v] = cur[v];
+      cv.shared[v] = v == 2;  // b1's table is every party's
+      ex[v] = ob.alloc<fe>((cv.shared[v] ? m : (uint64_t)N * m) << ext);
     }
     uint8_t *zf = nullptr;
     if (cubic) {  // blocks whose p1 part is all zero are skipped (coSumcheck.cpp:21-27)
       zf = ob.alloc<uint8_t>(blocks);
-      nonzero_blocks_launch(v1, blocks, logd[i], zf, s);
+      nonzero_blocks_launch(cur[0], blocks, logd[i], zf, s);
     }
-    const int lanes = D >= 256 ? 1 : 256 / D;
-    const int per_cta = (int)std::max<uint64_t>((uint64_t)lanes, (pblocks + 607) / 608);
-    fe *cpart = ob.alloc<fe>((uint64_t)N * D * cophase1_parts(pblocks, per_cta));
-    cophase1_reduce_launch(ex[0], ex[1], ex[2], ex[3], zf, pblocks, logd[i] + ext, per_cta, cpart, H, s, N);
+    fe *cpart = ob.alloc<fe>((uint64_t)N * cophase1_partials(pblocks, logd[i] + ext));
+    cophase1_launch(td, tD, cv, m, logd[i], ext, zf, N, ex, coef, cpart, H, s);
     launch_kernel(k_cosc_add_hr, N, 256, 0, s, H, D, dR, Rst, ro, i, step, st);
     launch_kernel(k_put_party, dim3(grid(D), N), 256, 0, s, H, D, N, tr, off_pp[i], 16ull * D);
     aggregate_launch(H, N, D, dl, poly, s);
@@ -1297,19 +1302,17 @@ CoscOut cosumcheck_run(gbz_ctx *ctx, int form, int N, uint64_t n, const fe *p1, 
     launch_kernel(k_cosc_sparse, N, kCoscThreads, 0, s, dR, Rst, ro, i, LD, D, N, st);
     GBZ_CUDA(cudaGetLastError());
     // phase 2 (coSumcheck.cpp:66-148, 201-213): every vector folded by Ld
-    for (fe *v : {v1, v2, v3, vb}) {
-      if (!v) continue;
-      cophase2_launch(v, (uint64_t)N * m, Ldh + at, logd[i], coef, s);
-      GBZ_CUDA(cudaMemcpyAsync(v, coef, 16ull * N * m / d, cudaMemcpyDeviceToDevice, s));
+    for (int v = 0; v < cv.nv; v++) {
+      cophase2_launch(cur[v], cv.shared[v] ? m : (uint64_t)N * m, Ldh + at, logd[i], alt[i & 1][v], s);
+      cur[v] = alt[i & 1][v];
     }
     m /= d;
     at += d;
   }
   fe *dcl = ob.alloc<fe>(rows);
   const fe wq = N > 4 ? finv(root_of_unity(ilog2(N / 4))) : fe_one();
-  launch_kernel(k_cosc_final, 1, kCoscThreads, 0, s, st, cubic ? 1 : 0, N, v1, v2, v3, vb, m, dU, db2, Ldh, dlog,
-                ndeg, dr1, wq,
-                                          finv(fe_make((uint64_t)(N / 4), 0)), dcl, tr, off_sh, off_un, off_r, off_cl);
+  launch_kernel(k_cosc_final, 1, kCoscThreads, 0, s, st, cubic ? 1 : 0, N, cur[0], cur[1], cur[3], cur[2], m, dU, db2,
+                Ldh, dlog, ndeg, dr1, wq, finv(fe_make((uint64_t)(N / 4), 0)), dcl, tr, off_sh, off_un, off_r, off_cl);
   GBZ_CUDA(cudaGetLastError());
   if (ip) {
     launch_kernel(k_cosc_ip, ndeg, 256, 0, s, LDall, ro, ip);
@@ -1787,6 +1790,9 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
     GBZ_CUDA(cudaGetLastError());
   };
   const int nrounds = sc.rounds - 1;
+  // the folds' other buffers
+  const uint64_t folded = nrounds > 0 ? (uint64_t)N * n / sc.degrees[1] : 0;
+  fe *bcd2 = ob.alloc<fe>(folded), *B2 = ob.alloc<fe>(folded);
   for (int i = 0; i < nrounds; i++) {
     const RoundOffs &ro = off.r[i];
     const int d = sc.degrees[i + 1], logd = ilog2((uint64_t)d), D = 2 * d;
@@ -1794,27 +1800,24 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
     // pcs_sumcheck_phase1 (coPCS.cpp:547-566): every party's blocks in one
     // batched transform, the products summed per party
     const NttTables &td = ctx->tables(logd), &tD = ctx->tables(logd + 1);
-    fe *e1 = ob.alloc<fe>(blocks * D), *e2 = ob.alloc<fe>(blocks * D), *coef = ob.alloc<fe>((uint64_t)N * n);
-    ntt_batched(td, bcd, d, (uint32_t)d, coef, blocks, true, s);
-    ntt_batched(tD, coef, d, (uint32_t)d, e1, blocks, false, s);
-    ntt_batched(td, B, d, (uint32_t)d, coef, blocks, true, s);
-    ntt_batched(tD, coef, d, (uint32_t)d, e2, blocks, false, s);
-    const uint64_t pblocks = n / d;
-    const int lanes = D >= 256 ? 1 : 256 / D;
-    const int per_cta = (int)std::max<uint64_t>((uint64_t)lanes, (pblocks + 607) / 608);
-    fe *cpart = ob.alloc<fe>((uint64_t)N * D * cophase1_parts(pblocks, per_cta));
-    cophase1_reduce_launch(e1, e2, nullptr, nullptr, nullptr, pblocks, logd + 1, per_cta, cpart, H, s, N);
+    fe *ex[4] = {ob.alloc<fe>(blocks * D), ob.alloc<fe>(blocks * D), nullptr, nullptr};
+    fe *coef = ob.alloc<fe>((uint64_t)N * n);
+    fe *cpart = ob.alloc<fe>((uint64_t)N * cophase1_partials(n / d, logd + 1));
+    CoVectors cv;
+    cv.nv = 2;
+    cv.v[0] = bcd;
+    cv.v[1] = B;
+    cophase1_launch(td, tD, cv, n, logd, 1, nullptr, N, ex, coef, cpart, H, s);
     launch_kernel(k_put_party, dim3(grid(D), N), 256, 0, s, H, D, N, tr, ro.pp, 16ull * D);
     aggregate_launch(H, N, D, dlam, poly, s);
     launch_kernel(k_round_verify, 1, 256, 0, s, st, poly, logd, finv(root_of_unity(logd + 1)),
-                  finv(fe_make(2ull << logd, 0)),
-                                     finv(fe_make(1ull << logd, 0)), Ld, vscr, tr, ro.poly, ro.chal);
+                  finv(fe_make(2ull << logd, 0)), finv(fe_make(1ull << logd, 0)), Ld, vscr, tr, ro.poly, ro.chal);
     GBZ_CUDA(cudaGetLastError());
     // pcs_sumcheck_phase2 (coPCS.cpp:571-587)
-    cophase2_launch(bcd, (uint64_t)N * n, Ld, logd, coef, s);
-    GBZ_CUDA(cudaMemcpyAsync(bcd, coef, 16ull * N * n / d, cudaMemcpyDeviceToDevice, s));
-    cophase2_launch(B, (uint64_t)N * n, Ld, logd, coef, s);
-    GBZ_CUDA(cudaMemcpyAsync(B, coef, 16ull * N * n / d, cudaMemcpyDeviceToDevice, s));
+    cophase2_launch(bcd, (uint64_t)N * n, Ld, logd, bcd2, s);
+    cophase2_launch(B, (uint64_t)N * n, Ld, logd, B2, s);
+    std::swap(bcd, bcd2);
+    std::swap(B, B2);
     n /= d;
     const bool last = i == nrounds - 1;
     fe *Cpn, *fold;
