@@ -241,6 +241,15 @@ void gbz_destroy(gbz_ctx *ctx) {
       cudaEventDestroy(ctx->side.join);
       cudaStreamDestroy(ctx->side.stream);
     }
+    for (cudaStream_t t : ctx->tail.s)
+      if (t) {
+        cudaStreamSynchronize(t);
+        cudaStreamDestroy(t);
+      }
+    for (cudaEvent_t e : ctx->tail.ready)
+      if (e) cudaEventDestroy(e);
+    for (cudaEvent_t e : ctx->tail.done)
+      if (e) cudaEventDestroy(e);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
   } catch (...) {
   }

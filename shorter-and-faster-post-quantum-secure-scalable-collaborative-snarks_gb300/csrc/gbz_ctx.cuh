@@ -13,6 +13,7 @@
 
 #include "../../include/gbz.h"
 #include "gbz_prover.cuh"
+#include "gbz_pcs_leader.cuh"
 #include "gbz_rounds.cuh"
 #include "gbz_sched.cuh"
 
@@ -100,6 +101,7 @@ struct gbz_ctx {
   bool graphs = true;  // gbz_prove replays captured graphs (gbz_set_graphs)
   bool group = true;   // gbz_prove_batch: proofs of one shape share launches (gbz_sched_set_grouping)
   SideStream side;     // second stream of the party sumcheck (created on first use)
+  TailStreams tail;    // streams of the PCS leader's tail (created on first use)
 
   const SideStream &side_stream() {
     if (!side.stream) {
@@ -108,6 +110,16 @@ struct gbz_ctx {
       GBZ_CUDA(cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming));
     }
     return side;
+  }
+
+  const TailStreams &tail_streams() {
+    for (auto &t : tail.s)
+      if (!t) GBZ_CUDA(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
+    for (auto &e : tail.ready)
+      if (!e) GBZ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    for (auto &e : tail.done)
+      if (!e) GBZ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    return tail;
   }
 
   void *buf(int slot, uint64_t bytes) {

@@ -1897,6 +1897,7 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
       GBZ_CUDA(cudaMemcpyAsync((void *)lr.y, y, 16ull * l, cudaMemcpyDeviceToDevice, s));
       GBZ_CUDA(cudaMemcpyAsync((void *)lr.qp, qp, 4ull * l, cudaMemcpyDeviceToDevice, s));
       GBZ_CUDA(cudaMemcpyAsync((void *)lr.qpos, qpos, 4ull * l, cudaMemcpyDeviceToDevice, s));
+      if (i) GBZ_CUDA(cudaEventRecord(ctx->tail_streams().ready[i], s));
     }
     if (!last) {
       launch_kernel(k_check_y, grid(l), 256, 0, s, Cpn, cpl_new, (uint32_t)sc.rate0[i + 2], (uint32_t)sc.rate0[i + 1],
@@ -1981,6 +1982,8 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
     GBZ_CUDA(cudaStreamWaitEvent(s, side->join, 0));
     LeaderResources LR;
     LR.s = s;
+    LR.side = &ctx->tail_streams();
+    LR.drawn = side->join;
     LR.alloc = [&ob](uint64_t bytes) -> void * { return ob.alloc<uint8_t>(bytes); };
     LR.tables = [ctx](int lg) -> NttTables & { return ctx->tables(lg); };
     Layout tl;

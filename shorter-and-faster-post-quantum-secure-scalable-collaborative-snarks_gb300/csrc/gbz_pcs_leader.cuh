@@ -79,8 +79,20 @@ enum : uint32_t {
   LF_FATAL = LF_DELEGATION | LF_DECODING | LF_WHIR | LF_FINAL | LF_BETAS | LF_LAG2
 };
 
+// Streams beside the call's own for the parts of the tail that do not wait for
+// one another: the first three take the rounds' delegations in turn, the last
+// the final evaluation and the delegation of the betas.  ready[i]: round i's
+// values are there (recorded by the caller; ready[0] is the tail's own).
+constexpr int kTailSides = 4, kTailRounds = 8;
+struct TailStreams {
+  cudaStream_t s[kTailSides] = {};
+  cudaEvent_t ready[kTailRounds] = {}, done[kTailSides] = {};
+};
+
 struct LeaderResources {
   cudaStream_t s = nullptr;
+  const TailStreams *side = nullptr;
+  cudaEvent_t drawn = nullptr;               // the script of draws has run
   std::function<void *(uint64_t)> alloc;     // device scratch held until the call ends
   std::function<NttTables &(int)> tables;    // twiddle tables by log2 length
 };
