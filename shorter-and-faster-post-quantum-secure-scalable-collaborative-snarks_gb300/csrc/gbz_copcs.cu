@@ -444,8 +444,7 @@ void aggregate_weights_launch(const fe *b, int N, fe *lambda, cudaStream_t s) {
 
 void aggregate_launch(const fe *msgs, int N, uint64_t len, const fe *lambda, fe *out, cudaStream_t s) {
   launch_kernel(aggregate_kernel, (unsigned)((len + kAggrCols - 1) / kAggrCols), dim3(kAggrCols, kAggrRows), 0, s,
-                msgs, N, len,
-                                                                                                 lambda, out);
+                msgs, N, len, lambda, out);
   GBZ_CUDA(cudaGetLastError());
 }
 

@@ -145,8 +145,7 @@ gbz_status gbz_dpcs_batch_commit(gbz_ctx *ctx, int N, uint64_t A, const uint64_t
   }
   // column hashes over the batch rows (distributed_PCS.cpp:76-88), every party's tree
   launch_kernel(k_dpcs_columns, dim3(nblk2(L), N), 256, 0, s, cw, batch, L, (uint64_t)batch * L,
-                ilog2((uint64_t)batch / 4), lv,
-                                                   32 * nh);
+                ilog2((uint64_t)batch / 4), lv, 32 * nh);
   GBZ_CUDA(cudaGetLastError());
   trees(ctx, lv, L, N, roots, leader_root);
   if (mem == GBZ_MEM_HOST) {
@@ -479,10 +478,9 @@ gbz_status gbz_dpcs_open(gbz_ctx *ctx, int N, int P, int rows, uint64_t S, int r
   fe *cdb = ob.alloc<fe>((uint64_t)P * N * S), *cwb = ob.alloc<fe>((uint64_t)P * N * L);
   for (int q = 0; q < P; q++) {
     launch_kernel(k_rowsum, dim3(nblk2(S), N), 256, 0, s, dcd + (uint64_t)q * N * rows * S, rows, S,
-                  db3 + (uint64_t)q * rows,
-                                              cdb + (uint64_t)q * N * S);
+                  db3 + (uint64_t)q * rows, cdb + (uint64_t)q * N * S);
     launch_kernel(k_rowsum_global, dim3(nblk2(L), N), 256, 0, s, dcw + (uint64_t)q * N * rows * L, rows, L, N,
-                                                     db3 + (uint64_t)q * rows, cwb + (uint64_t)q * N * L);
+                  db3 + (uint64_t)q * rows, cwb + (uint64_t)q * N * L);
   }
   GBZ_CUDA(cudaGetLastError());
   // the eval claims: every party's cross evaluations, summed with b1_j[p]

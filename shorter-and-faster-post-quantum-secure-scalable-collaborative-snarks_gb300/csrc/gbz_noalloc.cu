@@ -95,7 +95,7 @@ extern "C" gbz_status gbz_whir_update_betas_noalloc(uint64_t *b, uint64_t nb, co
   NoAllocScratch *scratch = nullptr;
   if (scratch_on_current_device(s, &scratch) != cudaSuccess) return GBZ_ECUDA;
   launch_kernel(noalloc_prep_kernel, 1, 256, 0, s, &scratch->st, queries, l, ilog2(N), fe_make(r[0], r[1]),
-                                        reinterpret_cast<fe *>(challenges));
+                reinterpret_cast<fe *>(challenges));
   if (cudaGetLastError() != cudaSuccess) return GBZ_ECUDA;
   if (nb == 0) return GBZ_OK;  // the weights are written; there is nothing to update
   try {

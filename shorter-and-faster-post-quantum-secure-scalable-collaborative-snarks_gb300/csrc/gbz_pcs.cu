@@ -1297,8 +1297,8 @@ CoscOut cosumcheck_run(gbz_ctx *ctx, int form, int N, uint64_t n, const fe *p1, 
     aggregate_launch(H, N, D, dl, poly, s);
     fe *LD = LDall + ro.off[i];
     launch_kernel(k_cosc_verify, 1, 256, 0, s, st, poly, logd[i], ext, i, finv(root_of_unity(logd[i] + ext)),
-                                    finv(fe_make((uint64_t)D, 0)), finv(fe_make(1ull << logd[i], 0)), LD, Ldh + at,
-                                    scr, tr, off_poly[i], off_chal[i]);
+                  finv(fe_make((uint64_t)D, 0)), finv(fe_make(1ull << logd[i], 0)), LD, Ldh + at, scr, tr,
+                  off_poly[i], off_chal[i]);
     launch_kernel(k_cosc_sparse, N, kCoscThreads, 0, s, dR, Rst, ro, i, LD, D, N, st);
     GBZ_CUDA(cudaGetLastError());
     // phase 2 (coSumcheck.cpp:66-148, 201-213): every vector folded by Ld
@@ -1512,8 +1512,7 @@ gbz_status gbz_pcs_claim(gbz_ctx *ctx, const gbz_pcs *pcs, const uint64_t *r, in
   fe *partial = ob.alloc<fe>((uint64_t)N * nblk);
   if (nb - 1 > 32) throw ArgError("pcs: F_ip over more than 32 rows");
   launch_kernel(k_fip_partial, dim3(nblk, N), kRedThreads, 0, s, pcs->cd, (uint64_t)nb * pcs->Bs, nb - 1, pcs->Bs,
-                brow, bcol,
-                                                       partial);
+                brow, bcol, partial);
   launch_kernel(k_fip_combine, 1, kPcsMaxParties, 0, s, partial, nblk, N, dl, dK);
   GBZ_CUDA(cudaGetLastError());
   if (mem == GBZ_MEM_DEVICE) GBZ_CUDA(cudaMemcpyAsync(K, dK, 16, cudaMemcpyDeviceToDevice, s));
@@ -1736,7 +1735,7 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
   ntt_launch_rows(tB, cdl, Bs, Bs, cdl, Bs, N, tmp, true, s);
   const NttTables &tw = ctx->tables(1 + sc.log_rate_offset + logBs);
   launch_kernel(k_open_prep, dim3(grid(Bs), N), 256, 0, s, bcd, cdl, B, b2, b3p, Bs, tw.lo_fwd, tw.hi_fwd, tw.lo_inv,
-                                                 tw.hi_inv);
+                tw.hi_inv);
   GBZ_CUDA(cudaGetLastError());
   // the batching round
   const int nblk = (int)std::min<uint64_t>(64, (Bs + kRedThreads - 1) / kRedThreads);
@@ -1747,8 +1746,7 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
   aggregate_launch(H, N, 3, dlam, poly, s);
   launch_kernel(k_first_verify, 1, 1, 0, s, st, poly, tr, off.poly0, off.chal0, off.K0);
   launch_kernel(k_first_fold, dim3(grid(L), N), 256, 0, s, bcd, cdl, B, Cp, pcs->cw + (uint64_t)(nb - 1) * L,
-                (uint64_t)nb * L,
-                                                Bs, L, st);
+                (uint64_t)nb * L, Bs, L, st);
   GBZ_CUDA(cudaGetLastError());
   // batch_commitments_new (coPCS.cpp:1242-1308): the root over C' in columns
   // of _degrees[1] entries depends on the first column's first leaf
@@ -1759,8 +1757,7 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
   {
     const uint64_t c = L / sc.degrees[1];
     launch_kernel(k_roots, 1, 64, 0, s, Cp, L, c, ilog2(sc.degrees[1] / 4) + ilog2(c), N, logN, nullptr, rts, tr,
-                  off.broots,
-                             off.bleader);
+                  off.broots, off.bleader);
     GBZ_CUDA(cudaGetLastError());
     // the batch tree is the commitment a tensor code would inherit when no
     // concatenated commitment follows it (levels over c column roots)
@@ -1862,8 +1859,7 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
       if (depth > prev_depth) throw ArgError("pcs: tensor code deeper than the previous commitment");
       const bool stale = prev_depth > depth;
       launch_kernel(k_roots, 1, 64, 0, s, Cpn, cpl_new, 1, depth, N, logN, stale ? prev_rts : nullptr, rts, tr,
-                    ro.roots,
-                               ro.leader);
+                    ro.roots, ro.leader);
       GBZ_CUDA(cudaGetLastError());
     }
     // delegate_checks (coPCS.cpp:740-891)
@@ -1889,8 +1885,7 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
       lr.seg = seg_copy;
     }
     launch_kernel(k_gather, grid((uint64_t)l * d), 256, 0, s, Cp, cpl, seg_n, d, fold, seg_n, qp, qpos, l, y, tr,
-                  ro.y, ro.seg,
-                                                   seg_copy);
+                  ro.y, ro.seg, seg_copy);
     GBZ_CUDA(cudaGetLastError());
     if (full) {
       GBZ_CUDA(cudaMemcpyAsync((void *)lr.L, Ld, 16ull * d, cudaMemcpyDeviceToDevice, s));
@@ -1901,8 +1896,7 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
     }
     if (!last) {
       launch_kernel(k_check_y, grid(l), 256, 0, s, Cpn, cpl_new, (uint32_t)sc.rate0[i + 2], (uint32_t)sc.rate0[i + 1],
-                    qp, qpos,
-                                        y, l, st);
+                    qp, qpos, y, l, st);
       GBZ_CUDA(cudaGetLastError());
     }
     launch_kernel(k_s_update, 1, 256, 0, s, st, y, l, last ? 0 : 1, tr, ro.s, ro.K);
@@ -1921,8 +1915,7 @@ static gbz_status pcs_open_impl(gbz_ctx *ctx, gbz_pcs *pcs, const uint64_t *r, i
       fe *tmp3 = logw > 13 ? ob.alloc<fe>((uint64_t)N * W) : nullptr;
       GBZ_CUDA(cudaMemsetAsync(V, 0, 16ull * N * W, s));
       launch_kernel(k_phase3_prep, grid(l), 256, 0, s, st, qp, qpos, l, (uint32_t)sc.rate0[i + 2],
-                    (uint32_t)sc.rate0[i + 1],
-                                             logw, dscale, N, q3, wts);
+                    (uint32_t)sc.rate0[i + 1], logw, dscale, N, q3, wts);
       launch_kernel(k_phase3_scatter, dim3(grid(l), N), 256, 0, s, q3, wts, l, W, V);
       GBZ_CUDA(cudaGetLastError());
       ntt_launch_rows(ctx->tables(logw), V, W, W, T, W, N, tmp3, false, s);

@@ -850,8 +850,7 @@ struct Tail {
       beta_launch(D, logS, b1, s);
       powers_launch(finv(root_of_unity(logd)), (uint64_t)d, twd, s);
       launch_kernel(k_pmf_vectors, (unsigned)S, 256, 32ull * d, s, rd.seg, rd.qpos, l, d, logd, twd, wn_inv, rd.L, b1,
-                    V[0],
-                                                         V[1], V[2], V[3]);
+                    V[0], V[1], V[2], V[3]);
       // K = d sum_t b1[t] y[t] (pad_vector(y): zeros beyond l)
       launch_kernel(k_dot, 1, kT, 0, s, b1, rd.y, (uint64_t)l, fe_make((uint64_t)d, 0), y);
       check();
@@ -1121,8 +1120,7 @@ struct Tail {
       draw_mod(la, (uint32_t)(Lw / 4), off_aq);
       if (!dry) {
         launch_kernel(k_whir_paths_chain, nblk((uint64_t)la * depth_a, 128), 128, 0, s, ro[0].W, Lw / 4, la, tr,
-                      off_aq, off_ap,
-                                                                             0, 0);
+                      off_aq, off_ap, 0, 0);
         launch_kernel(k_zero_tree_root, 1, 32, 0, s, ilog2(Lw / 8), tr, off_ar);
         check();
       }
@@ -1169,8 +1167,7 @@ struct Tail {
       if (!dry) {
         const NttTables &tf = R.tables(ilog2(wt.L_final));
         launch_kernel(k_reencode_check, nblk(wt.L_final), kT, 0, s, wt.final_arr, (int)wt.m_final, wt.last_codeword,
-                      wt.L_final,
-                                                        tf.lo_fwd, tf.hi_fwd, st);
+                      wt.L_final, tf.lo_fwd, tf.hi_fwd, st);
         launch_kernel(k_whir_flags, 1, 32, 0, s, st, flags);
         // the final claim (evaluate_vector(_initial_b, total_r), total_r)
         ChalOffs co{};

@@ -586,8 +586,7 @@ gbz_status gbz_piop_phase1(gbz_ctx *ctx, int N, uint64_t n, const uint64_t *vL, 
   fe *dl = ob.alloc<fe>(N), *dy = ob.alloc<fe>(3);
   GBZ_CUDA(cudaMemcpyAsync(dl, lambda.data(), 16ull * N, cudaMemcpyHostToDevice, s));
   launch_kernel(k_piop_y, 1, kPiopMaxParties, 0, s, dm, dR1, rlen, sg, N, bt[0], bt[1], bt[2], bt[3], dl, r1.back(),
-                dy, tr,
-                                         off_y);
+                dy, tr, off_y);
   GBZ_CUDA(cudaGetLastError());
   fe hy[3];
   GBZ_CUDA(cudaMemcpyAsync(hy, dy, sizeof hy, cudaMemcpyDeviceToHost, s));

@@ -943,7 +943,7 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
     for (; m > (uint64_t)kScTailMax; i += 2, m /= 4, pp ^= 1) {
       RUN(PC_PROTOCOL, 1,
           launch_kernel(k_sc_rounds_eq, B, 256, 0, s, p.partial, blocks, st, i, tr, i == 0 ? (int64_t)off_claim : -1,
-                                           off_poly0 + 80ull * (uint64_t)i, p.bs_part, trs));
+                        off_poly0 + 80ull * (uint64_t)i, p.bs_part, trs));
       blocks = sc_blocks(m / 4);
       BStr fs;  // (a, chal, a4, E, E4, partial)
       fs.s[0] = as;
@@ -965,8 +965,7 @@ void enqueue_proof(ProofPlan &p, const fe *witness, uint32_t prng_seed, cudaStre
   tb.s[2] = trs;
   RUN(PC_SUMCHECK, 1,
       (launch_kernel(k_sc_tail, B, kScTailThreads, kScTailShared, s, st, a, p.vb[pp], (int)m, i, logn, tr,
-                                                         i == 0 ? (int64_t)off_claim : -1,
-                                                         off_poly0 + 80ull * (uint64_t)i, off, tb)));
+                     i == 0 ? (int64_t)off_claim : -1, off_poly0 + 80ull * (uint64_t)i, off, tb)));
   };
 
   // The opening's randomness, drawn on the query stream while the

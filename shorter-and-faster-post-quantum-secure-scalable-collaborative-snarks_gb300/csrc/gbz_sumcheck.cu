@@ -522,8 +522,8 @@ void sc_fold2_launch(const fe *a, const fe *b, uint64_t m, const fe *chal0, cons
 void sc_fold2_eq_launch(const fe *a, const fe *E2, uint64_t m, const fe *c, const fe *chal0, const fe *chal1, fe *a4,
                         fe *b4, fe *partial0, fe *partial1, int blocks, cudaStream_t s, int batch, const BStr &bs) {
   if (m < 4) throw ArgError("two-round fold needs at least 4 entries");
-  launch_kernel(sc_fold2_eq_kernel, dim3(blocks, batch), kScThreads, 0, s, a, E2, m, c, chal0, chal1, a4, b4, partial0,
-                                                                partial1, bs);
+  launch_kernel(sc_fold2_eq_kernel, dim3(blocks, batch), kScThreads, 0, s, a, E2, m, c, chal0, chal1, a4, b4,
+                partial0, partial1, bs);
   GBZ_CUDA(cudaGetLastError());
 }
 

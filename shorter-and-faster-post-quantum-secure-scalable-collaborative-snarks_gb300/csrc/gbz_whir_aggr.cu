@@ -211,8 +211,7 @@ template <int TA, int TC>
 void pass_launch(const VecList &a, const fe *elo, const fe *ehi, int h, int lg, uint64_t n, const fe *bw,
                  const fe *aw, int first, fe *arr, fe *baggr, fe *partial, int blocks, cudaStream_t s) {
   launch_kernel(aggr_claims_pass_kernel<TA, TC>, blocks, kThreads, 0, s, a, elo, ehi, h, 1ull << h, 1ull << (lg - h),
-                n, bw,
-                                                              aw, first, arr, baggr, partial);
+                n, bw, aw, first, arr, baggr, partial);
   GBZ_CUDA(cudaGetLastError());
 }
 
