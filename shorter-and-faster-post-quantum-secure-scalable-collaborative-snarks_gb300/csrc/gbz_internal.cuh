@@ -146,8 +146,11 @@ inline bool is_pow2(uint64_t x) { return x && !(x & (x - 1)); }
 // Twiddle tables for one transform length, resident in device memory.
 struct NttTables {
   int logn = -1;
-  fe *sub_fwd = nullptr;   // omega_S^t for every sub-length S = 2^s, s <= 13, packed
-  fe *sub_inv = nullptr;
+  // the device's tables, shared by every length: the stage twiddles
+  // omega_{8 Ns}^{r k} (gbz_ntt.cu, stage_table_offset) and the half table of
+  // the small kernel
+  const fe *sub_fwd = nullptr, *sub_inv = nullptr;
+  const fe *half_fwd = nullptr, *half_inv = nullptr;
   fe *lo_fwd = nullptr, *hi_fwd = nullptr;  // omega_L^e = lo[e & 4095] * hi[e >> 12]
   fe *lo_inv = nullptr, *hi_inv = nullptr;
   fe inv_len;              // L^{-1}

@@ -56,7 +56,8 @@ struct PassArgs {
   // out_hstride + k out_kstride; l is the column of the outer twiddle.
   uint64_t in_gstride, in_hstride, in_jstride, out_gstride, out_hstride, out_kstride;
   int logG;
-  const fe *stages;  // stage twiddles of the direction
+  const fe *stages;   // stage twiddles of the direction
+  const fe *half_tw;  // omega_{2^kSmallLog}^k of the direction, k < 2^(kSmallLog - 1) (the small kernel)
   // The outer twiddle of output k is omega_L^{l k 2^tw_shift}.
   const fe *tw_lo;   // omega_L^t, t < 2^12 (nullptr: no outer twiddle)
   const fe *tw_hi;   // omega_L^{2^12 t}
@@ -527,8 +528,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs
 // which such a launch does not notice (2^6 to 2^10 by 4 cosets 10.4 -> 3.7 us,
 // 2^8 to 2^15 by 128 13.3 -> 5.0, 2^10 to 2^16 by 64 14.8 -> 8.9; one
 // transform of 2^11 gains nothing).
-// half_tw: omega_{2^kSmallLog}^k of the direction, k < 2^(kSmallLog - 1).
-__global__ void __launch_bounds__(1 << (kSmallLog - 1)) ntt_small_kernel(const PassArgs a, const fe *half_tw) {
+__global__ void __launch_bounds__(1 << (kSmallLog - 1)) ntt_small_kernel(const PassArgs a) {
   pdl_wait();
   if (a.run_if && *a.run_if == 0) return;
   extern __shared__ fe smem[];
@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(1 << (kSmallLog - 1)) ntt_small_kernel(const P
     if (r) x[1] = v;
     else x[0] = v;
   }
-  for (uint32_t t = tid; t < half; t += blockDim.x) tw[t] = half_tw[t << (kSmallLog - logS)];
+  for (uint32_t t = tid; t < half; t += blockDim.x) tw[t] = a.half_tw[t << (kSmallLog - logS)];
   fe y0 = fadd(x[0], x[1]), y1 = fsub(x[0], x[1]);
 #pragma unroll 1
   for (int s = 1; s < logS; s++) {  // x'[(j / Ns) 2 Ns + j mod Ns (+ Ns)], Ns = 2^(s-1), then the next level
@@ -714,44 +714,66 @@ PassKernel pass_kernel(int logS, bool inverse, int mode) {
   }
 }
 
-// Stage twiddle tables per direction, shared by every length.
-fe *g_stages[2] = {nullptr, nullptr};
-fe *g_half_tw[2] = {nullptr, nullptr};  // the small kernel's
-int g_stages_device = -1;
+// A device's tables that every length shares, per direction: the stage
+// twiddles and the small kernel's half table.
+struct DeviceTables {
+  fe *stages[2] = {nullptr, nullptr}, *half[2] = {nullptr, nullptr};
+};
 
-void ensure_stages() {
-  int dev;
-  GBZ_CUDA(cudaGetDevice(&dev));
-  if (g_stages[0] && g_stages_device == dev) return;
-  std::vector<fe> h(stage_table_offset(kSubLog - 2));
-  for (int dir = 0; dir < 2; dir++) {
-    for (int ns = 1; ns <= kSubLog - 3; ns++) {
-      fe w = root_of_unity(ns + 3);
-      if (dir) w = finv(w);
-      fe wr = w;
-      for (int r = 1; r < 8; r++, wr = fmul(wr, w)) {
-        fe x = fe_one();
-        for (uint32_t k = 0; k < (1u << ns); k++, x = fmul(x, wr)) h[stage_table_offset(ns) + ((r - 1) << ns) + k] = x;
+void upload_table(fe **d, const std::vector<fe> &h) {
+  GBZ_CUDA(device_malloc((void **)d, sizeof(fe) * h.size()));
+  GBZ_CUDA(cudaMemcpy(*d, h.data(), sizeof(fe) * h.size(), cudaMemcpyHostToDevice));
+}
+
+DeviceTables device_tables_build() {
+  DeviceTables t;
+  try {
+    std::vector<fe> h(stage_table_offset(kSubLog - 2)), half(1u << (kSmallLog - 1));
+    for (int dir = 0; dir < 2; dir++) {
+      for (int ns = 1; ns <= kSubLog - 3; ns++) {
+        fe w = root_of_unity(ns + 3);
+        if (dir) w = finv(w);
+        fe wr = w;
+        for (int r = 1; r < 8; r++, wr = fmul(wr, w)) {
+          fe x = fe_one();
+          for (uint32_t k = 0; k < (1u << ns); k++, x = fmul(x, wr)) h[stage_table_offset(ns) + ((r - 1) << ns) + k] = x;
+        }
       }
+      upload_table(&t.stages[dir], h);
+      fe w = root_of_unity(kSmallLog), x = fe_one();
+      if (dir) w = finv(w);
+      for (size_t k = 0; k < half.size(); k++, x = fmul(x, w)) half[k] = x;
+      upload_table(&t.half[dir], half);
     }
-    GBZ_CUDA(device_malloc((void **)&g_stages[dir], sizeof(fe) * h.size()));
-    GBZ_CUDA(cudaMemcpy(g_stages[dir], h.data(), sizeof(fe) * h.size(), cudaMemcpyHostToDevice));
+    // a copy from pageable memory may return before its last part has arrived
+    GBZ_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+    GBZ_CUDA(cudaFuncSetAttribute(ntt_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(sizeof(fe) * (5u << (kSmallLog - 1)))));
+    for (int logS = 0; logS <= kSubLog; logS++)
+      for (PassKernel k : {pass_kernel(logS, false, PASS_PLAIN), pass_kernel(logS, true, PASS_PLAIN),
+                           pass_kernel(logS, false, PASS_PACKED), pass_kernel(logS, false, PASS_SCATTER)})
+        GBZ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(fe) * kCtaElems)));
+  } catch (...) {
+    for (int dir = 0; dir < 2; dir++) {
+      cudaFree(t.stages[dir]);
+      cudaFree(t.half[dir]);
+    }
+    throw;
   }
-  for (int dir = 0; dir < 2; dir++) {
-    fe w = root_of_unity(kSmallLog);
-    if (dir) w = finv(w);
-    std::vector<fe> t(1u << (kSmallLog - 1), fe_one());
-    for (size_t k = 1; k < t.size(); k++) t[k] = fmul(t[k - 1], w);
-    GBZ_CUDA(device_malloc((void **)&g_half_tw[dir], sizeof(fe) * t.size()));
-    GBZ_CUDA(cudaMemcpy(g_half_tw[dir], t.data(), sizeof(fe) * t.size(), cudaMemcpyHostToDevice));
-  }
-  GBZ_CUDA(cudaFuncSetAttribute(ntt_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(fe) * (5u << (kSmallLog - 1)))));
-  g_stages_device = dev;
-  for (int logS = 0; logS <= kSubLog; logS++)
-    for (PassKernel k : {pass_kernel(logS, false, PASS_PLAIN), pass_kernel(logS, true, PASS_PLAIN),
-                         pass_kernel(logS, false, PASS_PACKED), pass_kernel(logS, false, PASS_SCATTER)})
-      GBZ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(fe) * kCtaElems)));
+  return t;
+}
+
+// The current device's, built on first use and kept for the process.  A
+// thread gets them when they are filled and the kernels' attributes are set;
+// launches take the pointers from the NttTables of their own device.
+DeviceTables device_tables() {
+  static std::mutex mu;
+  static std::map<int, DeviceTables> built;
+  int dev = 0;
+  GBZ_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  const auto it = built.find(dev);
+  return it != built.end() ? it->second : built.emplace(dev, device_tables_build()).first->second;
 }
 
 // Launches of up to 2^kSmallTotal elements in sub-transforms of up to
@@ -773,7 +795,7 @@ void launch_pass(PassArgs a, uint64_t groups, cudaStream_t s, int rows = 1) {
     a.logB = std::min(std::max(0, 6 - a.logS), ilog2(groups & (~groups + 1)));
     const uint32_t threads = 1u << (a.logS - 1 + a.logB);
     launch_kernel(ntt_small_kernel, dim3((unsigned)(groups >> a.logB), (unsigned)rows), threads,
-                  sizeof(fe) * 5 * threads, s, a, g_half_tw[a.inverse ? 1 : 0]);
+                  sizeof(fe) * 5 * threads, s, a);
     GBZ_CUDA(cudaGetLastError());
     return;
   }
@@ -933,10 +955,12 @@ Schedule schedule(int logn, int rows = 1) {
 }  // namespace
 
 void ntt_tables_build(NttTables &t, int logn) {
-  ensure_stages();
+  const DeviceTables dt = device_tables();
   t.logn = logn;
-  t.sub_fwd = g_stages[0];
-  t.sub_inv = g_stages[1];
+  t.sub_fwd = dt.stages[0];
+  t.sub_inv = dt.stages[1];
+  t.half_fwd = dt.half[0];
+  t.half_inv = dt.half[1];
   t.inv_len = finv(fe_make(1ull << logn, 0));
   const uint64_t L = 1ull << logn;
   const int nlo = 1 << kTwLoBits;
@@ -951,11 +975,10 @@ void ntt_tables_build(NttTables &t, int logn) {
     x = fe_one();
     for (uint64_t i = 0; i < nhi; i++) { hi[i] = x; x = fmul(x, w12); }
     fe **plo = dir ? &t.lo_inv : &t.lo_fwd, **phi = dir ? &t.hi_inv : &t.hi_fwd;
-    GBZ_CUDA(device_malloc((void **)plo, sizeof(fe) * nlo));
-    GBZ_CUDA(device_malloc((void **)phi, sizeof(fe) * nhi));
-    GBZ_CUDA(cudaMemcpy(*plo, lo.data(), sizeof(fe) * nlo, cudaMemcpyHostToDevice));
-    GBZ_CUDA(cudaMemcpy(*phi, hi.data(), sizeof(fe) * nhi, cudaMemcpyHostToDevice));
+    upload_table(plo, lo);
+    upload_table(phi, hi);
   }
+  GBZ_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // as for the device's tables
   if (logn > kSubLog) {
     if (g_shape[logn].k1 > 0) outer_table_build(logn, g_shape[logn].k1);
     const Schedule sc = schedule(logn);
@@ -1077,6 +1100,7 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
   a.row_in = row_in;
   a.row_out = row_out;
   a.stages = inverse ? t.sub_inv : t.sub_fwd;
+  a.half_tw = inverse ? t.half_inv : t.half_fwd;
   a.scale = t.inv_len;
   a.inverse = inverse ? 1 : 0;
   a.j_valid = 1u << kSubLog;
@@ -1279,6 +1303,7 @@ void ntt_batched(const NttTables &t, const fe *in, uint64_t in_stride, uint32_t 
   if (!count) return;
   PassArgs a{};
   a.stages = inverse ? t.sub_inv : t.sub_fwd;
+  a.half_tw = inverse ? t.half_inv : t.half_fwd;
   a.scale = t.inv_len;
   a.inverse = inverse ? 1 : 0;
   a.in = in;
@@ -1348,6 +1373,7 @@ void ntt_batched_strided(const NttTables &t, const fe *in, uint64_t col_stride, 
   if (!count) return;
   PassArgs a{};
   a.stages = inverse ? t.sub_inv : t.sub_fwd;
+  a.half_tw = inverse ? t.half_inv : t.half_fwd;
   a.scale = t.inv_len;
   a.inverse = inverse ? 1 : 0;
   a.in = in;
