@@ -19,7 +19,10 @@
  *   in and results out and returns when the results are in place.
  *   `mem` = GBZ_MEM_DEVICE: pointers are device memory of the context's
  *   device; the work is enqueued on the context's stream and the call may
- *   return before it finishes (gbz_synchronize waits).
+ *   return before it finishes (gbz_synchronize waits).  Device arrays of
+ *   field elements start on a 16-byte boundary; the vectors of
+ *   gbz_cosumcheck and gbz_pcs_commit may start at any word (they are copied
+ *   then).
  *
  * Errors
  *   Every call returns a gbz_status instead of the reference's printf+exit.

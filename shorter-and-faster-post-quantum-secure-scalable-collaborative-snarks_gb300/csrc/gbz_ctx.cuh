@@ -231,6 +231,8 @@ T *dev_view(gbz_ctx *ctx, int slot, T *p, uint64_t bytes, int mem, bool in) {
   if (in && bytes) GBZ_CUDA(cudaMemcpyAsync((void *)d, (const void *)p, bytes, cudaMemcpyHostToDevice, ctx->stream));
   return d;
 }
+// Whether kernels can load the elements where they are: 16 bytes at a time.
+inline bool fe_aligned(const void *p) { return ((uintptr_t)p & 15) == 0; }
 template <typename T>
 void copy_out(gbz_ctx *ctx, T *host, const T *dev, uint64_t bytes, int mem) {
   if (mem == GBZ_MEM_DEVICE || !bytes) return;

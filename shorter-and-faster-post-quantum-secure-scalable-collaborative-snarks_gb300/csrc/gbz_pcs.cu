@@ -1200,16 +1200,18 @@ CoscOut cosumcheck_run(gbz_ctx *ctx, int form, int N, uint64_t n, const fe *p1, 
   OpenBufs ob;
   {
     std::string key = "cosumcheck:" + std::to_string(form) + ":" + std::to_string(N) + ":" + std::to_string(n) + ":" +
-                      std::to_string((int)kin) + ":" + std::to_string(transcript != nullptr) + ":" + std::to_string(ip != nullptr);
+                      std::to_string((int)kin) + ":" + std::to_string(transcript != nullptr) + ":" + std::to_string(ip != nullptr) +
+                      ":" + std::to_string(fe_aligned(p1)) + std::to_string(fe_aligned(p2)) + std::to_string(fe_aligned(p3));
     for (int i = 0; i < ndeg; i++) key += ":" + std::to_string(degrees[i]);
     ob.pool = &ctx->pools[key];
   }
-  // party-major inputs, read where they are when they are device memory: a
-  // round folds into buffers of its own.  b1's table is one for all parties.
+  // party-major inputs, read where they are when they are device memory that
+  // starts on 16 bytes: a round folds into buffers of its own.  b1's table is
+  // one for all parties.
   const uint64_t Rst = ro.off[ndeg];
   const fe *cur[4] = {nullptr, nullptr, nullptr, nullptr};  // p1, p2, b1's table, p3
   auto input = [&](const fe *p) -> const fe * {
-    if (kin == cudaMemcpyDeviceToDevice) return p;
+    if (kin == cudaMemcpyDeviceToDevice && fe_aligned(p)) return p;
     fe *v = ob.alloc<fe>((uint64_t)N * n);
     GBZ_CUDA(cudaMemcpyAsync(v, p, 16ull * N * n, kin, s));
     return v;
@@ -1401,9 +1403,14 @@ gbz_status gbz_pcs_commit(gbz_ctx *ctx, int N, uint64_t M, int rounds, const int
   const uint64_t Bs = pc->Bs, L = pc->L, S = pc->S, R = pc->R;
   const int nb = pc->batches;
   cudaStream_t s = ctx->stream;
-  // inputs on the device
-  const fe *dsh = dev_view(ctx, 0, (const fe *)shares, 16 * S * N, mem, true);
-  const fe *drn = dev_view(ctx, 1, (const fe *)random, 16 * R * N, mem, true);
+  // inputs on the device, a caller's that starts off a 16-byte boundary copied
+  auto input = [&](int slot, const uint64_t *p, uint64_t bytes) -> const fe * {
+    if (mem == GBZ_MEM_HOST || fe_aligned(p)) return dev_view(ctx, slot, (const fe *)p, bytes, mem, true);
+    void *b = ctx->buf(slot, bytes);
+    GBZ_CUDA(cudaMemcpyAsync(b, p, bytes, cudaMemcpyDeviceToDevice, s));
+    return (const fe *)b;
+  };
+  const fe *dsh = input(0, shares, 16 * S * N), *drn = input(1, random, 16 * R * N);
   pc->alloc(ctx, (uint64_t)N * nb * Bs, (uint64_t)N * nb * L, 32ull * N * (2 * L - 1), 64ull * N);
   // prepare_data (coPCS.cpp:76-129): the rows of every party
   PrepareArgs pa{};

@@ -136,3 +136,67 @@ for kernel, _, seq, ptrs in launches:
         if p.known and p.filled():  # filled by a copy: a table
             assert p.filled() < seq, kernel
 """)
+
+
+@pytest.mark.parametrize("shift", [0, 8])
+def test_device_inputs_at_any_word(run, shift):
+    """Inputs that a call takes from device memory may start at any 64-bit word
+    (a tensor's slice): the kernels, which load 16 bytes at a time, get the
+    caller's pointer only where it is on such a boundary."""
+    run("SHIFT = %d" % shift + r"""
+ctx = gbz.Context(0)
+lib, N, u64 = gbz.lib, 8, ctypes.c_uint64
+for form, step in ((gbz.SC_QUADRATIC, 2), (gbz.SC_CUBIC, 4)):
+    n, deg = 4096, np.array([64, 8], dtype=np.int32)
+    p = [device_array(N * n, SHIFT) for _ in range(3)]
+    R = device_array(N * step * int(deg.sum()), SHIFT)
+    cubic = form == gbz.SC_CUBIC
+    r1, r2, K, Kr, fs, cl = [device_array(64, SHIFT) for _ in range(6)]
+    fl = ctypes.c_uint32()
+    check(lib.gbz_cosumcheck(ctx.h, form, N, n, p[0], p[1], p[2] if cubic else None, R, r1 if cubic else None,
+                             12 if cubic else 0, r2 if cubic else None, K, Kr, deg.ctypes.data, 2, fs, cl,
+                             ctypes.byref(fl), None, 0, gbz.MEM_DEVICE), ctx)
+rates = [(4,), (4,), (4, 4), (4, 4)]
+_, _, rnd = gbz.pcs_schedule(4, 1 << 14, rates)
+r0, r1 = gbz._rates(rates)
+h = ctypes.c_void_p()
+check(lib.gbz_pcs_commit(ctx.h, 4, 1 << 14, 4, r0.ctypes.data, r1.ctypes.data, device_array(4 << 14, SHIFT),
+                         device_array(4 * rnd, SHIFT), gbz.MEM_DEVICE, ctypes.byref(h), None, None), ctx)
+names = {k for k, *_ in launches}
+assert {"k_prepare", "coset_extend_kernel", "cophase2_kernel"} <= names, names
+for kernel, _, _, ptrs in launches:
+    for q in ptrs:
+        if q.known and ("fe" in q.kind or q.kind in SCAN):
+            assert q.value %% 16 == 0, (kernel, q.kind)
+""".replace("%%", "%"))
+
+
+def test_commitment_buffers_are_given_back(run):
+    run(r"""
+rates = [(4,), (4,), (4, 4), (4, 4)]
+_, _, rnd = gbz.pcs_schedule(4, 1 << 14, rates)
+shares, random = np.ones((4 << 14, 2), dtype=np.uint64), np.ones((4 * rnd, 2), dtype=np.uint64)
+
+def commit(c):
+    return gbz.pcs_commit(c, 4, 1 << 14, rates, shares, random)[0]
+
+c = gbz.Context(0)
+commit(c).free()
+c.sched_release()
+base = fake.fake_live()
+com = commit(c)
+assert fake.fake_live() == base + 4
+com.free()
+assert fake.fake_live() == base + 4  # one set is kept
+one, two = commit(c), commit(c)
+assert fake.fake_live() == base + 8
+one.free()
+two.free()
+assert fake.fake_live() == base + 4
+assert c.sched_release() > 0 and fake.fake_live() == base
+com = commit(c)
+c.close()
+live = fake.fake_live()
+com.free()  # a handle may outlive its context, and then nothing is kept
+assert fake.fake_live() == live - 4
+""")
