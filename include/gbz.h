@@ -870,26 +870,33 @@ gbz_status gbz_calibrate(gbz_ctx *ctx, double *fmul_per_s, double *blake3_per_s)
 
 /* ------------------------------------------------------------ autotuning */
 
-/* The shape of the two-pass (four-step) transforms of length 2^logn,
- * 14 <= logn <= 28: k1 = log2 of the contiguous second pass (the first pass
- * has length 2^(logn - k1)), 2^log_cols_a columns staged per CTA in the first
- * pass and 2^log_rows_b rows per CTA in the second.  Every valid shape
- * computes the same values; only speed differs.  Shapes are process-wide:
- * change them while no transform is in flight. */
+/* How transforms of length 2^logn, 14 <= logn <= 26, are split into passes.
+ * k1 = -1, the default: passes of the library's own choice, two up to 2^20 and
+ * three above.  k1 > 0: the two-pass (four-step) shape with a contiguous
+ * second pass of length 2^k1 (the first pass has length 2^(logn - k1)),
+ * 2^log_cols_a columns staged per CTA in the first pass and 2^log_rows_b rows
+ * per CTA in the second; both passes at most 2^13 long and 2^13 elements a
+ * CTA.  gbz_ntt_get_shape reports what is set ({-1, -1, -1}: nothing).  Every
+ * choice computes the same values; only speed differs.  Shapes are
+ * process-wide: change them while no transform is in flight. */
 gbz_status gbz_ntt_set_shape(int logn, int k1, int log_cols_a, int log_rows_b);
 gbz_status gbz_ntt_get_shape(int logn, int *shape);  /* shape: 3 ints */
 
-/* Times every candidate shape for 2^logn on the context's device (best of
- * reps forward transforms each) and installs the fastest; shape (3 ints),
+/* Times the library's own passes (*ms_default) and every candidate two-pass
+ * shape for 2^logn on the context's device (best of reps forward transforms
+ * each) and installs the fastest; shape (3 ints, k1 = -1 for the own passes),
  * ms_default and ms_best (optional) report the choice.  No counterpart in
  * the reference, whose fft has a single radix-2 schedule. */
 gbz_status gbz_ntt_autotune(gbz_ctx *ctx, int logn, int reps, int *shape, double *ms_default, double *ms_best);
 
-/* The first pass of a two-pass transform multiplies by omega_L^(n1 k2) read
- * from a table of L elements per (length, split, direction), built with the
- * length's twiddles (2 L * 16 bytes of device memory, kept for the process);
- * disabled, it forms each factor from two small tables with one more
- * multiply.  Same values either way; process-wide. */
+/* Every pass but the last multiplies by powers of omega read from a table:
+ * L elements per direction before the first pass and, in three passes, C
+ * before the second, C the length that the first pass leaves.  They are built
+ * with the length's twiddles, 2 (L + C) * 16 bytes of device memory, and kept
+ * for the process; a set shape has tables of its own beside them (2 L * 16
+ * bytes), and the autotuner frees those it built for shapes that it did not
+ * choose.  Disabled, a pass forms each factor from two small tables with one
+ * more multiply.  Same values either way; process-wide. */
 void gbz_ntt_full_twiddles(int enable);
 
 /* Merkle level fusion: each launch computes 2^log_nodes_per_cta nodes of a

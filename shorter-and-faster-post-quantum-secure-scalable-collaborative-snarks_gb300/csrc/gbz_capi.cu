@@ -1324,6 +1324,8 @@ gbz_status gbz_ntt_set_shape(int logn, int k1, int log_cols_a, int log_rows_b) {
     ntt_set_shape(logn, NttShape{k1, log_cols_a, log_rows_b});
   } catch (const ArgError &) {
     return GBZ_EINVAL;
+  } catch (const CudaError &) {
+    return GBZ_ECUDA;
   }
   return GBZ_OK;
 }
@@ -1334,7 +1336,7 @@ gbz_status gbz_ntt_get_shape(int logn, int *shape) {
   shape[0] = sh.k1;
   shape[1] = sh.logBA;
   shape[2] = sh.logBB;
-  return sh.k1 > 0 ? GBZ_OK : GBZ_EINVAL;
+  return ntt_shape_length(logn) ? GBZ_OK : GBZ_EINVAL;
 }
 
 void gbz_ntt_full_twiddles(int enable) { ntt_use_full_twiddles(enable != 0); }
@@ -1404,7 +1406,7 @@ gbz_status gbz_ntt_autotune(gbz_ctx *ctx, int logn, int reps, int *shape, double
   GBZ_CUDA(cudaMemsetAsync(buf, 0x11, 16 * L, ctx->stream));  // any canonical-looking data; timing only
   const NttTables &t = ctx->tables(logn);
   const NttShape before = ntt_get_shape(logn);
-  const NttShape dflt = ntt_default_shape(logn);
+  std::vector<int> splits = outer_table_splits(logn);
   cudaEvent_t a, b;
   GBZ_CUDA(cudaEventCreate(&a));
   GBZ_CUDA(cudaEventCreate(&b));
@@ -1423,10 +1425,10 @@ gbz_status gbz_ntt_autotune(gbz_ctx *ctx, int logn, int reps, int *shape, double
     }
     return best;
   };
-  NttShape best_sh = dflt;
+  NttShape best_sh;  // none: the library's own passes, timed first
   double best_ms = 0, def_ms = 0;
   try {
-    def_ms = best_ms = time_shape(dflt);
+    def_ms = best_ms = time_shape(best_sh);
     for (const NttShape &sh : ntt_shape_candidates(logn)) {
       const double ms = time_shape(sh);
       if (ms < best_ms * 0.98) {  // keep the default unless clearly faster
@@ -1436,6 +1438,7 @@ gbz_status gbz_ntt_autotune(gbz_ctx *ctx, int logn, int reps, int *shape, double
     }
   } catch (...) {
     ntt_set_shape(logn, before);
+    outer_table_keep_only(logn, splits);
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     throw;
@@ -1443,7 +1446,8 @@ gbz_status gbz_ntt_autotune(gbz_ctx *ctx, int logn, int reps, int *shape, double
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   ntt_set_shape(logn, best_sh);
-  outer_table_keep_only(logn, best_sh.k1);
+  splits.push_back(best_sh.k1);
+  outer_table_keep_only(logn, splits);
   if (shape) {
     shape[0] = best_sh.k1;
     shape[1] = best_sh.logBA;

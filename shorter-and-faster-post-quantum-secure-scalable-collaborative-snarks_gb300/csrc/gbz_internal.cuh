@@ -221,17 +221,20 @@ void ntt_batched_strided(const NttTables &t, const fe *in, uint64_t col_stride, 
 void ntt_tables_free(NttTables &t);
 // Four-step shape of the two-pass transforms (lengths above 2^13): pass B
 // length 2^k1 (contiguous rows), 2^logBA columns per CTA in pass A and
-// 2^logBB rows per CTA in pass B.  Every shape computes the same values.
+// 2^logBB rows per CTA in pass B.  k1 = -1: none set, the passes of
+// schedule() (gbz_ntt.cu).  Every shape computes the same values.
 struct NttShape {
   int k1 = -1, logBA = -1, logBB = -1;
 };
-NttShape ntt_default_shape(int logn);
 NttShape ntt_get_shape(int logn);
+bool ntt_shape_length(int logn);  // lengths that a shape can be set for
 bool ntt_shape_valid(int logn, const NttShape &sh);
 void ntt_set_shape(int logn, const NttShape &sh);  // process-wide
 std::vector<NttShape> ntt_shape_candidates(int logn);
-// Frees the first-pass twiddle tables of splits other than k1 (process-wide).
-void outer_table_keep_only(int logn, int k1);
+// The splits k1 of a length that have first-pass twiddle tables, and the
+// tables of the others freed (process-wide, the current device's).
+std::vector<int> outer_table_splits(int logn);
+void outer_table_keep_only(int logn, const std::vector<int> &splits);
 // Whether the first pass reads its twiddles from the full tables (default)
 // or forms them from the two-level tables; the values are the same.
 void ntt_use_full_twiddles(bool on);

@@ -44,7 +44,7 @@ constexpr int kPerThread = 8;            // elements per thread (CTA = max(32, E
 
 // Two-pass shape of a length set by ntt_set_shape (the autotuner): k1 = log2
 // of the contiguous second pass and the sub-transforms staged per CTA in each
-// pass.  Lengths without one take the passes of schedule().
+// pass.  Lengths without one (k1 = -1) take the passes of schedule().
 NttShape g_shape[kMaxLogN + 1];
 
 struct PassArgs {
@@ -839,8 +839,7 @@ __global__ void outer_table_kernel(fe w, int logL, int k1, fe *T) {
   }
 }
 
-// Tables of the default schedules (kScheduleTable added to the split) stay
-// for the process, whatever the autotuner does with its own.
+// The schedules' tables have kScheduleTable added to the split.
 constexpr int kScheduleTable = 64;
 
 const fe *outer_table_get(int logn, int key_k1, bool inverse) {
@@ -879,14 +878,25 @@ void outer_table_build(int logn, int key_k1) {
   }
 }
 
-// Frees the tables of other splits of this length (after autotuning).
-void outer_table_keep_only(int logn, int k1) {
+std::vector<int> outer_table_splits(int logn) {
+  int dev = 0;
+  GBZ_CUDA(cudaGetDevice(&dev));
+  std::vector<int> out;
+  std::lock_guard<std::mutex> lk(g_outer_mu);
+  for (const auto &e : g_outer)
+    if (std::get<0>(e.first) == dev && std::get<1>(e.first) == logn) out.push_back(std::get<2>(e.first));
+  return out;
+}
+
+// After autotuning: the tables that it built for shapes it did not choose.
+// Those that were there before stay, as captured proofs may read them.
+void outer_table_keep_only(int logn, const std::vector<int> &splits) {
   int dev = 0;
   GBZ_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(g_outer_mu);
   for (auto it = g_outer.begin(); it != g_outer.end();) {
-    if (std::get<0>(it->first) == dev && std::get<1>(it->first) == logn && std::get<2>(it->first) != k1 &&
-        std::get<2>(it->first) < kScheduleTable) {
+    if (std::get<0>(it->first) == dev && std::get<1>(it->first) == logn &&
+        std::find(splits.begin(), splits.end(), std::get<2>(it->first)) == splits.end()) {
       GBZ_CUDA(cudaDeviceSynchronize());
       cudaFree(it->second);
       it = g_outer.erase(it);
@@ -1010,7 +1020,9 @@ int ntt_launch_count(int logn, uint64_t n_valid, int rows) {
   return g_shape[logn].k1 > 0 ? 2 : schedule(logn).passes;
 }
 
-NttShape ntt_default_shape(int logn) {
+namespace {
+// The shape of a sparse transform (one second pass) whose length has none set.
+NttShape sparse_shape(int logn) {
   NttShape sh;
   sh.k1 = (logn + 1) / 2;
   const int k2 = logn - sh.k1;
@@ -1021,9 +1033,13 @@ NttShape ntt_default_shape(int logn) {
   sh.logBB = std::min(k2, std::max(0, std::min(kSubLog - 1, logn - 8) - sh.k1));
   return sh;
 }
+}  // namespace
+
+bool ntt_shape_length(int logn) { return logn > kSubLog && logn <= kMaxNttLogN; }
 
 bool ntt_shape_valid(int logn, const NttShape &sh) {
-  if (logn <= kSubLog || logn > kMaxNttLogN) return false;
+  if (!ntt_shape_length(logn)) return false;
+  if (sh.k1 == -1) return true;
   const int k2 = logn - sh.k1;
   if (sh.k1 < 1 || sh.k1 > kSubLog || k2 < 1 || k2 > kSubLog) return false;
   if (sh.logBA < 0 || sh.logBA > sh.k1 || k2 + sh.logBA > kSubLog) return false;
@@ -1031,20 +1047,12 @@ bool ntt_shape_valid(int logn, const NttShape &sh) {
   return true;
 }
 
-NttShape ntt_get_shape(int logn) {
-  if (logn <= kSubLog || logn > kMaxNttLogN) return NttShape{};
-  return g_shape[logn].k1 > 0 ? g_shape[logn] : ntt_default_shape(logn);
-}
+NttShape ntt_get_shape(int logn) { return ntt_shape_length(logn) ? g_shape[logn] : NttShape{}; }
 
 void ntt_set_shape(int logn, const NttShape &sh) {
   if (!ntt_shape_valid(logn, sh)) throw ArgError("ntt shape: invalid split or staging for this length");
-  const NttShape d = ntt_default_shape(logn);
-  if (sh.k1 == d.k1 && sh.logBA == d.logBA && sh.logBB == d.logBB) {  // back to the default schedule
-    g_shape[logn] = NttShape{};
-    return;
-  }
-  outer_table_build(logn, sh.k1);
-  g_shape[logn] = sh;
+  if (sh.k1 > 0) outer_table_build(logn, sh.k1);
+  g_shape[logn] = sh.k1 > 0 ? sh : NttShape{};
 }
 
 std::vector<NttShape> ntt_shape_candidates(int logn) {
@@ -1409,7 +1417,7 @@ void ntt_sparse_accumulate(const NttTables &t, const int32_t *q, const fe *c, in
   if (l < 1 || l > kMaxQueries) throw ArgError("sparse transform: 1..256 entries");
   const int logn = t.logn;
   const uint64_t L = 1ull << logn;
-  const NttShape sh = g_shape[logn].k1 > 0 ? g_shape[logn] : ntt_default_shape(logn);
+  const NttShape sh = g_shape[logn].k1 > 0 ? g_shape[logn] : sparse_shape(logn);
   const int k1 = sh.k1, k2 = logn - k1;
   const uint64_t N1 = 1ull << k1, N2 = 1ull << k2;
   // column chains in the (otherwise unused) scratch

@@ -663,8 +663,9 @@ class Context:
         return a.value, b.value
 
     def ntt_autotune(self, logn, reps=3):
-        """Installs the fastest two-pass shape for 2^logn; returns
-        (shape (k1, log_cols_a, log_rows_b), ms_default, ms_best)."""
+        """Installs the fastest of the library's own passes (k1 = -1) and the
+        two-pass shapes for 2^logn; returns (shape (k1, log_cols_a,
+        log_rows_b), ms_default, ms_best)."""
         sh = np.zeros(3, dtype=np.int32)
         a, b = ctypes.c_double(), ctypes.c_double()
         self.check(lib.gbz_ntt_autotune(self.h, logn, reps, _ptr(sh), ctypes.byref(a), ctypes.byref(b)))
@@ -708,7 +709,7 @@ class Context:
 def ntt_get_shape(logn):
     sh = np.zeros(3, dtype=np.int32)
     if lib.gbz_ntt_get_shape(logn, _ptr(sh)) != OK:
-        raise GbzError(EINVAL, "no two-pass shape for 2^%d" % logn)
+        raise GbzError(EINVAL, "no shapes for 2^%d" % logn)
     return tuple(int(x) for x in sh)
 
 

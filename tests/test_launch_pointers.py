@@ -200,3 +200,57 @@ live = fake.fake_live()
 com.free()  # a handle may outlive its context, and then nothing is kept
 assert fake.fake_live() == live - 4
 """)
+
+
+@pytest.mark.parametrize("logn", [14, 20, 21])
+def test_every_valid_shape_can_be_set(run, logn):
+    """A set shape is installed as given and reported; without one the library
+    takes passes of its own, which have a name of their own."""
+    run("LOGN = %d" % logn + r"""
+c, x = gbz.Context(0), np.ones((1 << LOGN, 2), dtype=np.uint64)
+
+def passes():
+    launches.clear()
+    c.fft(x, LOGN, False)
+    return sum(k == "ntt_pass_kernel" for k, *_ in launches)
+
+own = gbz.ntt_get_shape(LOGN)
+assert own[0] == -1, own
+assert passes() == (3 if LOGN > 20 else 2)
+k1 = (LOGN + 1) // 2
+valid = [(k1, a, b) for k1 in range(1, 14) for a in range(4) for b in range(4)
+         if 1 <= LOGN - k1 <= 13 and a <= k1 and b <= LOGN - k1 and LOGN - k1 + a <= 13 and k1 + b <= 13]
+for shape in [(k1, 1, 1)] + valid[::9]:
+    gbz.ntt_set_shape(LOGN, *shape)
+    assert gbz.ntt_get_shape(LOGN) == shape
+    assert passes() == 2, shape
+gbz.ntt_set_shape(LOGN, *own)
+assert gbz.ntt_get_shape(LOGN) == own and passes() == (3 if LOGN > 20 else 2)
+for bad in ((0, 0, 0), (-2, 0, 0), (14, 0, 0)):
+    assert gbz.lib.gbz_ntt_set_shape(LOGN, *bad) == gbz.EINVAL
+assert gbz.lib.gbz_ntt_set_shape(13, -1, -1, -1) == gbz.EINVAL
+assert gbz.lib.gbz_ntt_set_shape(27, -1, -1, -1) == gbz.EINVAL
+for n in (13, 27, -1):
+    assert gbz.lib.gbz_ntt_get_shape(n, (ctypes.c_int * 3)()) == gbz.EINVAL
+""")
+
+
+def test_autotuning_frees_the_tables_it_built(run):
+    run(r"""
+c = gbz.Context(0)
+x = np.ones((1 << 18, 2), dtype=np.uint64)
+c.fft(x, 18, False)
+shape, d, b = c.ntt_autotune(18, 1)  # every launch takes as long: the own passes stay
+assert shape[0] == -1 and gbz.ntt_get_shape(18) == shape and d == b
+base = fake.fake_live()
+gbz.ntt_set_shape(18, 8, 1, 1)
+assert fake.fake_live() == base + 2  # both directions
+c.fft(x, 18, False)
+c.ntt_autotune(18, 1)
+assert fake.fake_live() == base + 2  # what was there before may still be in use
+gbz.ntt_set_shape(18, 8, 1, 1)
+launches.clear()
+c.fft(x, 18, False)
+c.fft(x, 18, True)
+assert launches and not any(p.freed for _, _, _, ptrs in launches for p in ptrs)
+""")
