@@ -272,7 +272,7 @@ __global__ void sum_partials_kernel(const fe *partial, uint64_t nparts, uint32_t
 // lanes share an output and read consecutive entries of its block (whole
 // lines; one thread per output walked a block of its own, a line a lane and
 // step): 2^24 entries by 128 78 us, then 63; 1024 outputs of 1024 entries 38
-// us, then 3.
+// us, then 3.  A block of one entry is a product, with no sum to reduce.
 template <int LOGW>
 __global__ void __launch_bounds__(256) cophase2_kernel(const fe *v, uint64_t nout, const fe *L, int logd, fe *out) {
   pdl_wait();
@@ -281,6 +281,10 @@ __global__ void __launch_bounds__(256) cophase2_kernel(const fe *v, uint64_t nou
   for (uint32_t k = threadIdx.x; k < d; k += blockDim.x) sl[k] = L[k];
   __syncthreads();
   const uint64_t j = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> LOGW;
+  if (LOGW == 0 && d == 1) {
+    if (j < nout) out[j] = fmul(v[j], sl[0]);
+    return;
+  }
   facc acc = facc_zero();
   if (j < nout) {
 #pragma unroll 4
@@ -503,9 +507,14 @@ void cophase2_launch(const fe *v, uint64_t n, const fe *L, int logd, fe *out, cu
   if (logd > 10) throw ArgError("coSumcheck phase 2: block longer than 1024");
   const uint64_t nout = n >> logd;
   // eight lanes an output; a warp where that leaves SMs without work (1024
-  // outputs of 1024 entries: 38 us with one lane, 3 with 32); blocks below
-  // eight entries have no work for more lanes
+  // outputs of 1024 entries: 38 us with one lane, 3 with 32).  Short blocks
+  // leave more lanes too few products beside the reduction of each (2^24
+  // entries, the whole call, with 1, 2 and 8 lanes: blocks of 4 87, 115 and
+  // 165 us, of 8 103, 89 and 168, of 16 96, 80 and 127, of 32 94, 78 and 97,
+  // of 64 107, 82 and 92), which shows from 2^16 outputs on.
   if (logd < 3) launch_kernel(cophase2_kernel<0>, grid(nout), 256, 0, s, v, nout, L, logd, out);
+  else if (logd < 6 && nout >= (1u << 16)) launch_kernel(cophase2_kernel<1>, grid(nout << 1), 256, 0, s, v, nout, L,
+                                                         logd, out);
   else if (logd < 5 || nout >= (1u << 14)) launch_kernel(cophase2_kernel<3>, grid(nout << 3), 256, 0, s, v, nout, L,
                                                          logd, out);
   else launch_kernel(cophase2_kernel<5>, grid(nout << 5), 256, 0, s, v, nout, L, logd, out);
