@@ -460,6 +460,23 @@ __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs
   }
   const bool in_order = in_rows || a.sp_l > 0;
   if constexpr (LOGS <= 3) {  // the first stage is the last
+    if constexpr (LOGS == 3 && MODE == PASS_PLAIN) {
+      // A batch's outputs lie back to back: by way of shared memory neighbouring
+      // threads store neighbouring elements instead of a line each (block sums of
+      // 2^24 entries in pairs, extended fourfold: 2660 -> 2148 us).
+      if (in_order && a.out_kstride == 1 && a.out_gstride == S && !a.acc && !a.tw_lo && !tw_full) {
+        if (tid < (total >> 3)) {
+#pragma unroll
+          for (int r = 0; r < 8; r++) {
+            const fe x = v[0][r];
+            sm[(tid << 3) + (r ^ (tid & 7))] = a.has_scale ? fmul(x, a.scale) : canon_fe(x);
+          }
+        }
+        __syncthreads();
+        for (uint32_t e = tid; e < total; e += blockDim.x) out[l0 * S + e] = sm[(e & ~7u) + ((e ^ (e >> 3)) & 7)];
+        return;
+      }
+    }
 #pragma unroll
     for (int i = 0; i < PER; i++) {
       const uint32_t u = tid + i * blockDim.x;
@@ -801,7 +818,7 @@ void launch_pass(PassArgs a, uint64_t groups, cudaStream_t s, int rows = 1) {
   }
   const uint64_t tiles = groups >> a.logB;
   const uint32_t E = 1u << (a.logS + a.logB);
-  const size_t smem = a.logS > 3 || a.sp_l > 0 ? sizeof(fe) * E : 0;
+  const size_t smem = a.logS >= 3 || a.sp_l > 0 ? sizeof(fe) * E : 0;
   const unsigned threads = E / kPerThread > 32 ? E / kPerThread : 32;
   if (a.logG == 0) a.logG = 40;  // every g is a column of its own
   const uint64_t last = (groups - 1) * a.in_gstride + ((1ull << a.logS) - 1) * a.in_jstride;
