@@ -284,7 +284,8 @@ void sc_fold2_eq_launch(const fe *a, const fe *E2, uint64_t m, const fe *c, cons
 // kept as a shrinking table (E of m/4 entries for w of m entries): the four
 // sums T_k = sum_j a[4j + k] E[j] of both rounds (m a multiple of 4), and the
 // fold of a by chal[0], chal[1] into a4 (m/4, m a multiple of 128) with
-// E4 = sums of four of E (m/16) and, when reduce, the T sums of (a4, E4).
+// E4 = sums of four of E (m/16, always written); reduce adds the T sums of
+// (a4, E4).
 // Partials are (T0, T1, T2, T3) per block.
 void sc_eq_reduce_launch(const fe *a, const fe *E, uint64_t m, fe *partial, int blocks, cudaStream_t s,
                          int batch = 1, const BStr &bs = BStr());

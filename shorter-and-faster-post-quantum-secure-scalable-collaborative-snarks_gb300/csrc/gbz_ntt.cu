@@ -56,8 +56,7 @@ struct PassArgs {
   // out_hstride + k out_kstride; l is the column of the outer twiddle.
   uint64_t in_gstride, in_hstride, in_jstride, out_gstride, out_hstride, out_kstride;
   int logG;
-  const fe *stages;   // stage twiddles of the direction
-  const fe *half_tw;  // omega_{2^kSmallLog}^k of the direction, k < 2^(kSmallLog - 1) (the small kernel)
+  const fe *stages;  // twiddles of the direction: of the stages, or the small kernel's (set at launch)
   // The outer twiddle of output k is omega_L^{l k 2^tw_shift}.
   const fe *tw_lo;   // omega_L^t, t < 2^12 (nullptr: no outer twiddle)
   const fe *tw_hi;   // omega_L^{2^12 t}
@@ -224,8 +223,9 @@ __host__ __device__ constexpr int first_log(int logs) { return logs <= 3 ? logs 
 // read neighbouring k, whole lines out of L1 (57 KB for the last stage of
 // S = 2^12, beside 128 KB of staged data).  As a half table of omega_S in
 // shared memory, loaded by every CTA, the strided reads cost up to eight
-// wavefronts for one (60 % of a pass's shared-memory wavefronts were
-// conflicts) and r = 5..7 a conditional negation.
+// wavefronts for one (a pass's loads took three times their ideal wavefronts;
+// of the 12 million that a pass of 2^9 over 2^24 elements takes now, one is
+// a conflict) and r = 5..7 a conditional negation.
 __host__ __device__ constexpr uint32_t stage_table_offset(int logns) { return 7u * ((1u << logns) - 2); }
 
 // Entry j of sub-transform b in shared memory.  The exclusive or with j / 8
@@ -545,6 +545,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) ntt_pass_kernel(const PassArgs
 // which such a launch does not notice (2^6 to 2^10 by 4 cosets 10.4 -> 3.7 us,
 // 2^8 to 2^15 by 128 13.3 -> 5.0, 2^10 to 2^16 by 64 14.8 -> 8.9; one
 // transform of 2^11 gains nothing).
+// stages: omega_{2^kSmallLog}^k of the direction, k < 2^(kSmallLog - 1).
 __global__ void __launch_bounds__(1 << (kSmallLog - 1)) ntt_small_kernel(const PassArgs a) {
   pdl_wait();
   if (a.run_if && *a.run_if == 0) return;
@@ -581,7 +582,7 @@ __global__ void __launch_bounds__(1 << (kSmallLog - 1)) ntt_small_kernel(const P
     if (r) x[1] = v;
     else x[0] = v;
   }
-  for (uint32_t t = tid; t < half; t += blockDim.x) tw[t] = a.half_tw[t << (kSmallLog - logS)];
+  for (uint32_t t = tid; t < half; t += blockDim.x) tw[t] = a.stages[t << (kSmallLog - logS)];
   fe y0 = fadd(x[0], x[1]), y1 = fsub(x[0], x[1]);
 #pragma unroll 1
   for (int s = 1; s < logS; s++) {  // x'[(j / Ns) 2 Ns + j mod Ns (+ Ns)], Ns = 2^(s-1), then the next level
@@ -805,9 +806,11 @@ bool small_launch(const PassArgs &a, uint64_t groups, int rows) {
                      ((groups * (uint64_t)rows) << a.logS) <= (1ull << kSmallTotal));
 }
 
-void launch_pass(PassArgs a, uint64_t groups, cudaStream_t s, int rows = 1) {
+// Launches with the tables of the transform's own device (t).
+void launch_pass(const NttTables &t, PassArgs a, uint64_t groups, cudaStream_t s, int rows = 1) {
   if (rows < 1 || rows > 65535) throw ArgError("transform: 1..65535 rows per launch");
   if (small_launch(a, groups, rows)) {
+    a.stages = a.inverse ? t.half_inv : t.half_fwd;
     // a warp of butterflies a CTA at least
     a.logB = std::min(std::max(0, 6 - a.logS), ilog2(groups & (~groups + 1)));
     const uint32_t threads = 1u << (a.logS - 1 + a.logB);
@@ -816,6 +819,7 @@ void launch_pass(PassArgs a, uint64_t groups, cudaStream_t s, int rows = 1) {
     GBZ_CUDA(cudaGetLastError());
     return;
   }
+  a.stages = a.inverse ? t.sub_inv : t.sub_fwd;
   const uint64_t tiles = groups >> a.logB;
   const uint32_t E = 1u << (a.logS + a.logB);
   const size_t smem = a.logS >= 3 || a.sp_l > 0 ? sizeof(fe) * E : 0;
@@ -1124,8 +1128,6 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
   a.run_if = gate.run_if;
   a.row_in = row_in;
   a.row_out = row_out;
-  a.stages = inverse ? t.sub_inv : t.sub_fwd;
-  a.half_tw = inverse ? t.half_inv : t.half_fwd;
   a.scale = t.inv_len;
   a.inverse = inverse ? 1 : 0;
   a.j_valid = 1u << kSubLog;
@@ -1148,7 +1150,7 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
     a.out_kstride = out_elem_stride << (logn - logv);
     a.logS = logv;
     a.has_scale = inverse;
-    launch_pass(a, 1ull << (logn - logv), s, rows);
+    launch_pass(t, a, 1ull << (logn - logv), s, rows);
     return;
   }
   if (logn <= kSubLog) {
@@ -1168,7 +1170,7 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
     a.sc_lo = gate.sc_lo;
     a.sc_n = gate.sc_n;
     a.sc_stride = gate.sc_stride;
-    launch_pass(a, 1, s, rows);
+    launch_pass(t, a, 1, s, rows);
     return;
   }
   Schedule sc;
@@ -1204,7 +1206,7 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
     b.tw_hi = inverse ? t.hi_inv : t.hi_fwd;
     b.tw_shift = done;
     b.tw_full = g_use_outer ? outer_table_get(rest, lc + (set ? 0 : kScheduleTable), inverse) : nullptr;
-    launch_pass(b, L >> sc.log[i], s, rows);
+    launch_pass(t, b, L >> sc.log[i], s, rows);
     done += sc.log[i];
     rest = lc;
   }
@@ -1233,7 +1235,7 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
   b.sc_lo = gate.sc_lo;
   b.sc_n = gate.sc_n;
   b.sc_stride = gate.sc_stride;
-  launch_pass(b, L >> rest, s, rows);
+  launch_pass(t, b, L >> rest, s, rows);
 }
 
 }  // namespace
@@ -1327,8 +1329,6 @@ void ntt_batched(const NttTables &t, const fe *in, uint64_t in_stride, uint32_t 
   if (logS > kSubLog) throw ArgError("batched transform longer than 2^13");
   if (!count) return;
   PassArgs a{};
-  a.stages = inverse ? t.sub_inv : t.sub_fwd;
-  a.half_tw = inverse ? t.half_inv : t.half_fwd;
   a.scale = t.inv_len;
   a.inverse = inverse ? 1 : 0;
   a.in = in;
@@ -1347,13 +1347,13 @@ void ntt_batched(const NttTables &t, const fe *in, uint64_t in_stride, uint32_t 
   a.logB = logB;
   const uint64_t B = 1ull << logB;
   const uint64_t full = count / B * B;
-  if (full) launch_pass(a, full, s);
+  if (full) launch_pass(t, a, full, s);
   if (full < count) {  // remaining transforms one per CTA
     PassArgs r = a;
     r.in = in + full * in_stride;
     r.out = out + (full << logS);
     r.logB = 0;
-    launch_pass(r, count - full, s);
+    launch_pass(t, r, count - full, s);
   }
 }
 
@@ -1397,8 +1397,6 @@ void ntt_batched_strided(const NttTables &t, const fe *in, uint64_t col_stride, 
   if (logS > kSubLog) throw ArgError("batched transform longer than 2^13");
   if (!count) return;
   PassArgs a{};
-  a.stages = inverse ? t.sub_inv : t.sub_fwd;
-  a.half_tw = inverse ? t.half_inv : t.half_fwd;
   a.scale = t.inv_len;
   a.inverse = inverse ? 1 : 0;
   a.in = in;
@@ -1417,13 +1415,13 @@ void ntt_batched_strided(const NttTables &t, const fe *in, uint64_t col_stride, 
   a.logB = logB;
   const uint64_t B = 1ull << logB;
   const uint64_t full = count / B * B;
-  if (full) launch_pass(a, full, s);
+  if (full) launch_pass(t, a, full, s);
   if (full < count) {
     PassArgs r = a;
     r.in = in + full;
     r.out = out + (full << logS);
     r.logB = 0;
-    launch_pass(r, count - full, s);
+    launch_pass(t, r, count - full, s);
   }
 }
 
@@ -1443,7 +1441,6 @@ void ntt_sparse_accumulate(const NttTables &t, const int32_t *q, const fe *c, in
   launch_kernel(sparse_chain_kernel, 1, kMaxQueries, 0, s, q, l, q_shift, (uint32_t)(N1 - 1), next, lead);
   GBZ_CUDA(cudaGetLastError());
   PassArgs b{};
-  b.stages = t.sub_fwd;
   b.scale = t.inv_len;
   b.inverse = 0;
   b.j_valid = 1u << kSubLog;
@@ -1468,7 +1465,7 @@ void ntt_sparse_accumulate(const NttTables &t, const int32_t *q, const fe *c, in
   b.sp_lo = t.lo_fwd;
   b.sp_hi = t.hi_fwd;
   b.sp_mask = L - 1;
-  launch_pass(b, N2, s);
+  launch_pass(t, b, N2, s);
 }
 
 }  // namespace gbz
