@@ -58,13 +58,14 @@ sys.path.insert(0, PKG)
 sys.path.insert(0, ORACLE)
 
 LOGN, RATE = 24, 2
-# DRAM bytes of every transform launch of one proof (both passes of each
+# DRAM bytes of every transform launch of one proof (every pass of each
 # transform, the packed pass and the unpack), from one ncu capture of the
 # n = 2^22 proof (dram__bytes_read.sum, dram__bytes_write.sum, kernels
-# ntt_pass_kernel and real_unpack_kernel, four proofs within 0.3 %); scaled
-# by n for other sizes (the later, smaller transforms' writes stay in L2 at
-# 2^22, so the write figure is a lower bound).
-NTT_TRAFFIC_2E22 = {"read": 585.3e6, "write": 175.0e6}
+# ntt_pass_kernel, ntt_small_kernel and real_unpack_kernel, five proofs within
+# 0.01 % read and 1.3 % written); scaled by n for other sizes (the later,
+# smaller transforms' writes stay in L2 at 2^22, so the write figure is a
+# lower bound).
+NTT_TRAFFIC_2E22 = {"read": 744.2e6, "write": 181.3e6}
 E2E_LANES = 3  # slots of the batched end-to-end pass
 SERVE_REPEATS = 3  # interleaved repeats of the served and plain runs at 200 requests/s
 SEED = 0x5EED0000 + 2 * 65536  # witness seed of the 2^24 rate-1/2 workload
@@ -1245,13 +1246,12 @@ def main():
             a = work["ntt"] / t / 1e9
             r["int"] = {"achieved": a, "peak": fmul_peak / 1e9, "unit": "G F-mul/s (radix-2 butterflies)",
                         "frac": a / (fmul_peak / 1e9), "butterflies_per_proof": work["ntt"],
-                        "alu_pipe_ncu": "57 % (pass A) / 51 % (pass B), issue active 52 % / 46 % "
-                                        "(profiles/ntt_pass_2e23.md)"}
+                        "pipes_ncu": "multiply pipe 56 / 65 / 55 %, ALU 50 / 58 / 62 % in the passes of 2^24 "
+                                     "(profiles/ntt_pass_2e24.md)"}
         if cat == "update_betas":
             a = work["update_betas"] / t / 1e9
             r["int"] = {"achieved": a, "peak": fmul_peak / 1e9, "unit": "G F-mul/s",
-                        "frac": a / (fmul_peak / 1e9), "fmuls_per_proof": work["update_betas"],
-                        "alu_pipe_ncu": "54 % in the sparse-rows pass (profiles/update_betas_sparse_2e22.md)"}
+                        "frac": a / (fmul_peak / 1e9), "fmuls_per_proof": work["update_betas"]}
         if cat == "merkle":
             r["compressions_per_proof"] = work["merkle_chain"]
             r["note"] = "root and path chains only (latency bound); whole trees: rows.merkle_tree"
@@ -1265,8 +1265,8 @@ def main():
     roof = {"kernel": dom, "bound": "int" if "int" in d else "hbm", "ms_per_proof": per_proof_ms[dom],
             "traffic": traffic,
             "traffic_note": "DRAM bytes per proof of all transform launches: ncu capture of the n = 2^22 proof "
-                            "scaled by n; above the algorithmic bytes by the two-pass intermediate and the first "
-                            "pass's twiddle table" if traffic else None}
+                            "scaled by n; above the algorithmic bytes by the intermediates between passes and the "
+                            "outer twiddle tables" if traffic else None}
     if primary:
         roof.update({"achieved": primary["achieved"], "peak": primary["peak"], "unit": primary["unit"],
                      "frac": primary["frac"]})

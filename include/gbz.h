@@ -485,13 +485,22 @@ typedef struct gbz_pcs gbz_pcs;
 /* PCS_commit of every party: prepare_data (coPCS.cpp:76-129), Encode
  * (:131-147) and distributed_MT (:152-230).  shares: N x (4M/N) elements,
  * random: N x random_per_party elements, party-major.  *out receives the
- * commitment (device memory held until gbz_pcs_free); party_roots (N x 32 B)
- * and leader_root (32 B; the leader's tree over {root_0, 0, ..., 0}) may be
- * NULL.
+ * commitment (device memory held until gbz_pcs_free, see there); party_roots
+ * (N x 32 B) and leader_root (32 B; the leader's tree over {root_0, 0, ...,
+ * 0}) may be NULL.
  * replaces PCS_commit (coPCS.cpp:236-250) on N ranks. */
 gbz_status gbz_pcs_commit(gbz_ctx *ctx, int N, uint64_t M, int rounds, const int *rate0, const int *rate1,
                           const uint64_t *shares, const uint64_t *random, int mem, gbz_pcs **out,
                           uint8_t *party_roots, uint8_t *leader_root);
+/* Ends a commitment.  Its buffers (16 N batches (row_len + codeword_len) bytes
+ * and the trees) stay with the context that made it, for its next commitment
+ * of the same sizes on the same stream, when they are at most a sixteenth of
+ * the device's memory and no other context worked on them; otherwise they are
+ * freed.  A context keeps one such set at a time.  It is given back by
+ * gbz_sched_release, a commitment of other sizes or on another stream,
+ * gbz_destroy, and any allocation of the library that finds the device full;
+ * call gbz_sched_release before allocating that memory by other means.  May be
+ * called from any thread and after the context is gone. */
 void gbz_pcs_free(gbz_pcs *pcs);
 /* Shape of a commitment: Commit_data rows with entries (batches), their
  * length, the codeword length, and the transcript bytes of gbz_pcs_open. */

@@ -92,10 +92,10 @@ GBZ_HD uint64_t red125(unsigned __int128 v) {
 // counts.  The columns are chosen so that none of them needs a register
 // move: the cross products share one 64-bit accumulator (they stay below
 // 2^64 because the high words are short), the low ones chain their carry
-// into the high ones.  Measured (independent multiplies on every SM, one
-// operand kept): 42.6 instructions and 454 G multiplies/s folded, 48.6 and
-// 425 canonical, against 66.8 and 329 for the 128-bit form that the host
-// uses below.
+// into the high ones.  48.6 instructions canonical and 42.6 folded, against
+// 66.8 for the 128-bit form that the host uses below.  gbz_calibrate (four
+// chains a thread on every SM): 445 G canonical multiplies/s, 345 before;
+// folded ones are 7 % faster.
 struct dot_cols {
   uint32_t x0, x1, x2, x3;  // S, least significant word first
 };

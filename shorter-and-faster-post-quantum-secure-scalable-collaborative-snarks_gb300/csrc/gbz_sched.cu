@@ -58,8 +58,8 @@ SlotPlan::~SlotPlan() {
 }
 
 double proof_cost(int logn, int rate) {
-  // about one millisecond of dependent launches per proof plus a term
-  // proportional to the codeword length (2^21 elements per millisecond)
+  // relative weights: a chain of dependent launches counts as much as 2^21
+  // codeword elements
   const double L = std::ldexp(1.0, logn) * rate;
   return 1.0 + L / 2097152.0;
 }

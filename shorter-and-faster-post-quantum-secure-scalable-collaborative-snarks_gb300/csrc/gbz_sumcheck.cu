@@ -282,8 +282,9 @@ sc_eq_reduce_kernel(const fe *__restrict__ a, const fe *__restrict__ E, uint64_t
   block_sum_classes(acc, partial);
 }
 
-// Fold a (m entries, a multiple of 128) by chal[0] and chal[1] into a4, and
-// (reduce) E (m / 4 entries) into E4 and the T sums of a4 with E4.
+// Fold a (m entries, a multiple of 128) by chal[0] and chal[1] into a4 and E
+// (m / 4 entries) into E4, which the tail reads after the last pass too; with
+// reduce also the T sums of a4 with E4.
 __global__ void __launch_bounds__(kScThreads)
 sc_eq_fold_kernel(const fe *__restrict__ a, uint64_t m, const fe *chal, fe *__restrict__ a4,
                   const fe *__restrict__ E, fe *__restrict__ E4, int reduce, fe *partial, BStr bs) {
