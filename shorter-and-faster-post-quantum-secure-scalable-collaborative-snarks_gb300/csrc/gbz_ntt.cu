@@ -1170,6 +1170,30 @@ void ntt_passes(const NttTables &t, const fe *in, uint64_t n_valid, fe *out, fe 
     a.sc_lo = gate.sc_lo;
     a.sc_n = gate.sc_n;
     a.sc_stride = gate.sc_stride;
+    // Rows too short to fill a CTA of 2^11 elements share one, as neighbouring
+    // sub-transforms, where that leaves enough CTAs for every SM; what is left
+    // over of them goes row by row.  (The output factors and the scattered
+    // output are addressed by row.)  A CTA for every row of 2^9, 65535 of them
+    // from 2^5 entries, took 657 us, so 443.
+    if (rows <= 65535 && !gate.out_tab && !gate.sc_n && !small_launch(a, 1, rows)) {
+      int logB = std::max(0, 11 - logn);
+      while (logB > 0 && (rows >> logB) < 608) logB--;
+      const int full = rows >> logB << logB;
+      if (logB > 0) {
+        PassArgs b = a;
+        b.in_gstride = row_in;
+        b.out_gstride = row_out;
+        b.row_in = b.row_out = 0;
+        b.n_valid = ~0ull;
+        b.j_valid = (uint32_t)n_valid;
+        b.logB = logB;
+        launch_pass(t, b, (uint64_t)full, s);
+        if (full == rows) return;
+        a.in += full * row_in;
+        a.out += full * row_out;
+        rows -= full;
+      }
+    }
     launch_pass(t, a, 1, s, rows);
     return;
   }
